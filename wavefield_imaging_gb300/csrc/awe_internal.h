@@ -29,6 +29,17 @@ struct GeoPoint {
     float w[8];
 };
 
+// The cells a set of fixed sources injects into: entries [start[k], start[k+1])
+// of `ent` are (source * 8 + corner, weight bits) of cell[k], in the reference's
+// (source, corner) order, so one thread per cell adds what one thread walking
+// every source would, in the same order.
+struct InjCells {
+    int n;  // cells; 0: none
+    const long long *cell;
+    const int *start;
+    const int2 *ent;
+};
+
 // Padded grid, axis 1 fastest.
 struct Grid {
     int n1, n2, n3;  // n3 = 1 in 2D
@@ -117,6 +128,7 @@ struct Bnd3Params {
     float *rec_row;  // null: no gather this step
     const GeoPoint *src;
     int ns, src_stride;
+    InjCells inj;  // fixed sources by cell (n = 0: walk src)
     const float *wav;
     int it, ncs, one_wavelet;
     int n_int, nxr, nzr, rec_blocks;  // set by launch_bnd3
@@ -150,6 +162,10 @@ void launch_bnd3_adj(Bnd3AdjParams p, cudaStream_t s);
 void launch_injectB_off(int ndim, bool exact, float *u, const float *vel, const GeoPoint *pts, int ns,
                         const float *wav, int it, int ncs, bool one_wavelet, const long long *off, cudaStream_t s,
                         int stride = 1);
+
+// the same from a cell list (fixed sources)
+void launch_injectB_cells(bool exact, float *u, const float *vel, const InjCells &c, const float *wav, int it, int ncs,
+                          bool one_wavelet, cudaStream_t s);
 
 // receiver gather; when w1 != null the sponge factors are applied to each node
 // value first (the field carries a pending sponge)
@@ -200,6 +216,8 @@ void launch_rec_adjA(float *z, const GeoPoint *pts, int nr, const float *r, cons
 // wav [nt][ncs]: ncs = 1 (one wavelet for every source) or ns
 void launch_injectA(bool exact, int ndim, float *u, const GeoPoint *pts, const float *scale, int ns, const float *wav,
                     int it, bool scaled, const long long *off, cudaStream_t s, int stride = 1, int ncs = 1);
+void launch_injectA_cells(bool exact, float *u, const float *scale, const InjCells &c, const float *wav, int it,
+                          bool scaled, cudaStream_t s, int ncs);
 void launch_snapshot_transpose2(const float *u, float *dst, const Grid &g, int f1, int f2, int m1, int m2,
                                 cudaStream_t s);
 
@@ -225,8 +243,8 @@ void launch_abc_adjB(int nop, int fsrf, float *mu, float *kap, const AbcB &a, co
 void launch_kap_fold(float *mu, float *kap, const AdjParams &p, cudaStream_t s);
 void launch_rec_adj(float *mu, const GeoPoint *pts, int nr, const float *r, const AdjParams &p, const long long *off,
                     cudaStream_t s);
-void launch_src_grad(float2 *G, const float *nu, const GeoPoint *pts, int ns, const float *wav, int it, int ncs,
-                     bool one_wavelet, int nd, const long long *off, cudaStream_t s);
+void launch_src_grad_cells(float2 *G, const float *nu, const InjCells &c, const float *wav, int it, int ncs,
+                           bool one_wavelet, cudaStream_t s);
 void launch_residual(const float *d, const float *dobs, float *r, int nrows, int nr, double *row_sum, cudaStream_t s);
 void launch_ckpt_store16(bool fp16, const float *u, long long n, unsigned int *amax, void *q, float *scale, int grid,
                          cudaStream_t s);

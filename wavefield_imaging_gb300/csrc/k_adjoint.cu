@@ -341,25 +341,27 @@ void launch_rec_adj(float *mu, const GeoPoint *pts, int nr, const float *r, cons
     if (nr > 0) k_rec_adj<<<(nr + 127) / 128, 128, 0, s>>>(mu, pts, nr, r, p, off);
 }
 
-// source term of the gradient: dJ/dvel2[node] += nu[node] * wav * w (one
-// thread, sources and corners in order)
-__global__ void k_src_grad(float2 *G, const float *__restrict__ nu, const GeoPoint *__restrict__ pts, int ns,
-                           const float *__restrict__ wav, int it, int ncs, int one_wavelet, int nc,
-                           const long long *__restrict__ off) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    for (int s = 0; s < ns; s++) {
-        const float dd = one_wavelet ? wav[(long long)it * ncs] : wav[(long long)it * ncs + s];
-        const GeoPoint pt = pts[s];
-        for (int c = 0; c < nc; c++) {
-            const long long n = pt.base + off[c];
-            G[n] = gsum_add_prod(G[n], nu[n], dd * pt.w[c]);
-        }
+// source term of the gradient: dJ/dvel2[node] += nu[node] * wav * w, one thread
+// per cell, its (source, corner) entries in order
+__global__ void __launch_bounds__(128) k_src_grad_cells(float2 *G, const float *__restrict__ nu, const InjCells c,
+                                                        const float *__restrict__ wav, int it, int ncs,
+                                                        int one_wavelet) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= c.n) return;
+    const long long n = c.cell[k];
+    float2 g = G[n];
+    const float x = nu[n];
+    for (int e = c.start[k], e1 = c.start[k + 1]; e < e1; e++) {
+        const int2 en = c.ent[e];
+        const float dd = one_wavelet ? wav[(long long)it * ncs] : wav[(long long)it * ncs + (en.x >> 3)];
+        g = gsum_add_prod(g, x, dd * __int_as_float(en.y));
     }
+    G[n] = g;
 }
 
-void launch_src_grad(float2 *G, const float *nu, const GeoPoint *pts, int ns, const float *wav, int it, int ncs,
-                     bool one_wavelet, int nd, const long long *off, cudaStream_t s) {
-    if (ns > 0) k_src_grad<<<1, 1, 0, s>>>(G, nu, pts, ns, wav, it, ncs, one_wavelet, nd == 3 ? 8 : 4, off);
+void launch_src_grad_cells(float2 *G, const float *nu, const InjCells &c, const float *wav, int it, int ncs,
+                           bool one_wavelet, cudaStream_t s) {
+    if (c.n > 0) k_src_grad_cells<<<(c.n + 127) / 128, 128, 0, s>>>(G, nu, c, wav, it, ncs, one_wavelet ? 1 : 0);
 }
 
 // ---------------------------------------------------------------------------

@@ -290,6 +290,21 @@ __global__ void __launch_bounds__(b3::NT, 4) k_bnd3(const Bnd3Params p) {
         return;
     }
     blk -= p.rec_blocks;
+    if (p.inj.n > 0) {  // ---- injection, one thread per cell
+        const int k = blk * NT + tid;
+        if (k >= p.inj.n) return;
+        const long long n = p.inj.cell[k];
+        float v = p.uo[n];
+        const float vn = p.vel[n];
+        for (int e = p.inj.start[k], e1 = p.inj.start[k + 1]; e < e1; e++) {
+            const int2 en = p.inj.ent[e];
+            const float dd =
+                p.one_wavelet ? p.wav[(long long)p.it * p.ncs] : p.wav[(long long)p.it * p.ncs + (en.x >> 3)];
+            v = fadd<EXACT>(v, fmul<EXACT>(fmul<EXACT>(dd, __int_as_float(en.y)), vn));
+        }
+        p.uo[n] = v;
+        return;
+    }
     if (blk == 0 && p.ns > 0 && tid == 0) {  // ---- injection, sources and corners in order
         for (int s = 0; s < p.ns; s++) {
             const float dd = p.one_wavelet ? p.wav[(long long)p.it * p.ncs] : p.wav[(long long)p.it * p.ncs + s];
@@ -312,7 +327,7 @@ void launch_bnd3(bool exact, Bnd3Params p, cudaStream_t s) {
     p.nxr = p.g.n2 / XR > 0 ? p.g.n2 / XR : 1;
     p.nzr = p.g.n1 / ZR > 0 ? p.g.n1 / ZR : 1;
     p.rec_blocks = p.rec_row ? (p.nr + NT - 1) / NT : 0;
-    const int grid = p.n_int + 2 * p.nxr * p.nzr + p.rec_blocks + (p.ns > 0 ? 1 : 0);
+    const int grid = p.n_int + 2 * p.nxr * p.nzr + p.rec_blocks + (p.inj.n > 0 ? (p.inj.n + NT - 1) / NT : p.ns > 0 ? 1 : 0);
     if (exact) k_bnd3<true><<<grid, NT, 0, s>>>(p);
     else k_bnd3<false><<<grid, NT, 0, s>>>(p);
 }

@@ -468,6 +468,31 @@ void launch_injectA(bool exact, int ndim, float *u, const GeoPoint *pts, const f
     else k_injectA<false><<<1, 32, 0, s>>>(u, pts, scale, ns, wav, it, ncs, nc, scaled, off, stride);
 }
 
+// The same, one thread per cell (InjCells; the scale is per source and corner).
+template <bool EXACT>
+__global__ void __launch_bounds__(128) k_injectA_cells(float *u, const float *__restrict__ scale, const InjCells c,
+                                                       const float *__restrict__ wav, int it, int ncs, int scaled) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= c.n) return;
+    const long long n = c.cell[k];
+    float v = u[n];
+    for (int e = c.start[k], e1 = c.start[k + 1]; e < e1; e++) {
+        const int2 en = c.ent[e];
+        const float wa = wav[(long long)it * ncs + (ncs == 1 ? 0 : en.x >> 3)];
+        float a = fmul<EXACT>(wa, __int_as_float(en.y));
+        if (scaled) a = fmul<EXACT>(a, scale[en.x]);
+        v = fadd<EXACT>(v, a);
+    }
+    u[n] = v;
+}
+
+void launch_injectA_cells(bool exact, float *u, const float *scale, const InjCells &c, const float *wav, int it,
+                          bool scaled, cudaStream_t s, int ncs) {
+    if (c.n <= 0) return;
+    if (exact) k_injectA_cells<true><<<(c.n + 127) / 128, 128, 0, s>>>(u, scale, c, wav, it, ncs, scaled);
+    else k_injectA_cells<false><<<(c.n + 127) / 128, 128, 0, s>>>(u, scale, c, wav, it, ncs, scaled);
+}
+
 // polar snapshots are theta-fastest ([r][theta]) as sfAWEFDspher2Dgpu writes them
 __global__ void k_snapshot_transpose2(const float *__restrict__ u, float *__restrict__ dst, Grid g, int f1, int f2,
                                       int m1, int m2) {

@@ -385,13 +385,16 @@ awe_status awe_set_geometry(awe_plan *p, int ns, const float *sou, int nr, const
         k[7] = p->sponge_deferred;
         k[8] = p->src_in_shell;
         k[9] = p->pa.nshot;
+        k[10] = (long long)(uintptr_t)p->inj_buf;
+        k[11] = p->inj.n;
     };
-    long long before[10], after[10];
+    long long before[12], after[12];
     key(before);
     plan_gradient_graph_drop(p);  // its per-cell point lists follow the geometry
     CUDA_TRY(cudaSetDevice(p->device));
     set_move_mode(p, -1, 1, 1);
     awe_status st = set_geometry_common(p, ns, sou, nr, rec);
+    if (st == AWE_OK) st = set_inj_cells(p);
     if (st == AWE_OK) st = single_shot(p, ns, nr);
     key(after);
     if (st != AWE_OK || std::memcmp(before, after, sizeof before) != 0) plan_graph_drop(p);
@@ -436,6 +439,7 @@ awe_status awe_set_moving_geometry(awe_plan *p, int ns, int nst, const float *so
     CUDA_TRY(cudaSetDevice(p->device));
     awe_status st = set_geometry_common(p, ns * nst, sou, nr * nrt, rec);
     if (st != AWE_OK) return st;
+    p->inj = InjCells{};  // the lists hold fixed sources
     p->ns = ns;
     p->nr = nr;
     set_move_mode(p, mode, nst, nrt);
@@ -483,6 +487,8 @@ awe_status awe_set_shots(awe_plan *p, int nshots, const int *ns, const float *so
     }
     if (NS) CUDA_TRY(cudaMemcpy(p->src, p->h_src.data(), NS * sizeof(GeoPoint), cudaMemcpyHostToDevice));
     if (NR) CUDA_TRY(cudaMemcpy(p->rec, p->h_rec.data(), NR * sizeof(GeoPoint), cudaMemcpyHostToDevice));
+    st = set_inj_cells(p);
+    if (st != AWE_OK) return st;
     p->shot_ns.assign(ns, ns + nshots);
     p->shot_nr.assign(nr, nr + nshots);
     if (nshots != p->pa.nshot) {

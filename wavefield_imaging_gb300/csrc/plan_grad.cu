@@ -299,7 +299,8 @@ static awe_status gradient_spher_one(awe_plan *p, const float *d_wav, int ncs, c
         AWE_TRY(ckpt_load(p, 2 * seg + 1, slot + cells, s));
         for (int k = k0; k < k1; k++) {
             float *cur = slot + (size_t)(k - k0 + 1) * cells;
-            launch_injectA(false, 3, cur, p->src, nullptr, p->ns, d_wav, k, false, p->corner_off, s, 1, ncs);
+            if (p->inj.n > 0) launch_injectA_cells(false, cur, nullptr, p->inj, d_wav, k, false, s, ncs);
+            else launch_injectA(false, 3, cur, p->src, nullptr, p->ns, d_wav, k, false, p->corner_off, s, 1, ncs);
             if (k + 1 < k1) {
                 if (st->sph) {  // slot i = k - k0 + 1 from slots i and i - 1, into slot i + 1
                     const int i = k - k0 + 1;
@@ -388,7 +389,10 @@ static awe_status plan_gradient_spher(awe_plan *p, const float *d_wav, int ncs, 
     float *dobs_s = nullptr, *dsyn_s = nullptr;
     double *grad_s = nullptr;
     GeoPoint *src0 = p->src, *rec0 = p->rec;
+    const InjCells inj0 = p->inj;
+    p->inj = InjCells{};  // built for all shots' fields; the shots run one at a time here
     auto cleanup = [&]() {
+        p->inj = inj0;
         p->src = src0;
         p->rec = rec0;
         p->ns = NS;
@@ -662,7 +666,7 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
                 launches++;
             }
             if (p->ns > 0 && !xcorr && !fuse_pts) {
-                launch_src_grad(st->G, X, p->src, p->ns, d_wav, k, ncs, ncs == 1, d.ndim, p->corner_off, s);
+                launch_src_grad_cells(st->G, X, p->inj, d_wav, k, ncs, ncs == 1, s);
                 launches++;
             }
             std::swap(X, Y);

@@ -51,6 +51,10 @@ struct awe_plan {
     bool sponge_deferred = false;  // a source node lies in the sponge band outside the boundary shell
     bool src_in_shell = false;     // a source node lies within nop + 2 of a face (3D)
     int src_cap = 0, rec_cap = 0;  // points the src / rec device buffers hold
+    // fixed sources by cell (set_inj_cells): one buffer, kept while large enough
+    awe::InjCells inj{};
+    void *inj_buf = nullptr;
+    size_t inj_cap = 0;
     // moving geometry (awe_set_moving_geometry): src/rec hold ns*src_rows and
     // nr*rec_rows entries; move_mode < 0 = fixed points
     int move_mode = -1, src_rows = 1, rec_rows = 1;
@@ -129,6 +133,8 @@ awe_status deliver_snapshot(awe_plan *p, const float *d_frame, int isnap, int it
 // hand the last queued frame to the callback (end of a run)
 awe_status flush_snapshots(awe_plan *p);
 
+// (re)builds p->inj from h_src
+awe_status set_inj_cells(awe_plan *p);
 awe_status set_geometry_common(awe_plan *p, int ns, const float *sou, int nr, const float *rec);
 
 // The n points of a table active at step it: the first one and the stride

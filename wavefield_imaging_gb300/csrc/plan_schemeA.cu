@@ -375,8 +375,11 @@ awe_status planA_run(awe_plan *p, const float *d_wav, int ncs, float *d_dat, flo
         if (hook) AWE_TRY((*hook)(it, nxt, cur, s));
         if (p->ns > 0) {
             const PointsAt ps = points_at(p, p->src, p->ns, p->src_rows, it);
-            launch_injectA(exact, d.ndim, cur, ps.pts, p->inj_scale, p->ns, d_wav, it, scaled, p->corner_off, s,
-                           ps.stride, ncs);
+            if (p->move_mode < 0 && p->inj.n > 0)
+                launch_injectA_cells(exact, cur, p->inj_scale, p->inj, d_wav, it, scaled, s, ncs);
+            else
+                launch_injectA(exact, d.ndim, cur, ps.pts, p->inj_scale, p->ns, d_wav, it, scaled, p->corner_off, s,
+                               ps.stride, ncs);
             launches++;
         }
         prof_begin(p, s);

@@ -171,6 +171,48 @@ awe_status planB_model(awe_plan *p, const float *vel, const float *den) {
     return AWE_OK;
 }
 
+awe_status set_inj_cells(awe_plan *p) {
+    const int nc = p->d.ndim == 3 ? 8 : 4, ns = (int)p->h_src.size();
+    std::vector<std::pair<long long, int>> e;  // (cell, source * 8 + corner)
+    e.reserve((size_t)ns * nc);
+    for (int s = 0; s < ns; s++)
+        for (int c = 0; c < nc; c++) e.push_back({p->h_src[s].base + p->h_corner_off[c], 8 * s + c});
+    std::sort(e.begin(), e.end());
+    std::vector<long long> cell;
+    std::vector<int> start;
+    std::vector<int2> ent(e.size());
+    for (size_t k = 0; k < e.size(); k++) {
+        if (k == 0 || e[k].first != e[k - 1].first) {
+            cell.push_back(e[k].first);
+            start.push_back((int)k);
+        }
+        int w;
+        std::memcpy(&w, &p->h_src[e[k].second >> 3].w[e[k].second & 7], sizeof w);
+        ent[k] = make_int2(e[k].second, w);
+    }
+    start.push_back((int)e.size());
+    p->inj = InjCells{};
+    if (cell.empty()) return AWE_OK;
+    // sizes for every source at cells of its own, so that points that only
+    // move keep the buffer (a captured time loop reads it)
+    const size_t nmax = (size_t)ns * nc;
+    const size_t o_ent = nmax * sizeof(long long), o_start = o_ent + nmax * sizeof(int2);
+    const size_t bytes = o_start + (nmax + 1) * sizeof(int);
+    if (p->inj_cap < bytes) {
+        dev_free(p, p->inj_buf);
+        p->inj_buf = nullptr;
+        p->inj_cap = 0;
+        AWE_TRY(dev_alloc(p, &p->inj_buf, bytes));
+        p->inj_cap = bytes;
+    }
+    char *b = (char *)p->inj_buf;
+    CUDA_TRY(cudaMemcpy(b, cell.data(), cell.size() * sizeof(long long), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(b + o_ent, ent.data(), ent.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(b + o_start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice));
+    p->inj = InjCells{(int)cell.size(), (const long long *)b, (const int *)(b + o_start), (const int2 *)(b + o_ent)};
+    return AWE_OK;
+}
+
 awe_status set_geometry_common(awe_plan *p, int ns, const float *sou, int nr, const float *rec) {
     const awe_desc &d = p->d;
     const Grid &g = p->g;
@@ -353,8 +395,11 @@ awe_status stepB_full(awe_plan *p, const StepBParams &sp0, const float *prv, con
     const bool inj_in_bnd = bnd && !p->src_in_shell;
     if (p->ns > 0 && !fuse_src && !inj_in_bnd) {
         const PointsAt ps = points_at(p, p->src, p->ns, p->src_rows, it);
-        launch_injectB_off(d.ndim, exact, nxt, p->vel, ps.pts, p->ns, d_wav, it, ncs, ncs == 1, p->corner_off, s,
-                           ps.stride);
+        if (p->move_mode < 0 && p->inj.n > 0)
+            launch_injectB_cells(exact, nxt, p->vel, p->inj, d_wav, it, ncs, ncs == 1, s);
+        else
+            launch_injectB_off(d.ndim, exact, nxt, p->vel, ps.pts, p->ns, d_wav, it, ncs, ncs == 1, p->corner_off, s,
+                               ps.stride);
         launches++;
     }
     if (bnd) {
@@ -387,6 +432,7 @@ awe_status stepB_full(awe_plan *p, const StepBParams &sp0, const float *prv, con
             bp.src = ps.pts;
             bp.ns = p->ns;
             bp.src_stride = ps.stride;
+            if (p->move_mode < 0) bp.inj = p->inj;
             bp.wav = d_wav;
             bp.it = it;
             bp.ncs = ncs;
