@@ -367,6 +367,7 @@ struct Step3Launch {
 };
 bool stepB3_tma_eligible(int ndim, int nop, bool rho, const Grid &g);
 bool stepB3_tma_maps(CUtensorMap *maps, float *const u[2], const float *vel, const Grid &g);
+int march_planes(int n3, long long columns, int slots, int halo);
 Step3Launch stepB3_tma_shape(const Grid &g, int num_sms, int L);
 cudaError_t launch_stepB3_tma(bool exact, const CUtensorMap *maps, int icur, float *nxt, const StepBParams &sp,
                               const Step3Launch &sh, unsigned long long *counter, unsigned long long base, int *err,

@@ -292,9 +292,9 @@ bool sphA_tma_maps(CUtensorMap *maps, float *const u[2], const float *vel, const
 Step3Launch sphA_tma_shape(const Grid &g, int nshot, int num_sms, int L) {
     using namespace sp3;
     Step3Launch s{};
-    s.L = L > 0 ? L : 64;
     s.ntz = (g.n1 + TR - 1) / TR;
     s.ntx = (g.n2 + TT - 1) / TT;
+    s.L = L > 0 ? L : march_planes(g.n3, (long long)s.ntz * s.ntx * (nshot > 0 ? nshot : 1), 2 * num_sms, 2);
     s.nchunks = (g.n3 + s.L - 1) / s.L;
     s.items = s.ntz * s.ntx * s.nchunks * (nshot > 0 ? nshot : 1);
     s.grid = std::min(s.items, 2 * num_sms);
