@@ -206,6 +206,27 @@ void launch_stepA_oop(int geom, bool exact, const float *cur, const float *prv, 
                       const StepAParams &p, cudaStream_t s);
 void launch_stepA(int geom, bool exact, const float *cur, float *nxt, const float *vel, const StepAParams &p,
                   cudaStream_t s);
+// 2D step in one launch (k_stepA2d.cu): out of place (cur, prv and nxt differ)
+constexpr int kFusedCorners = 32;  // one bit per corner in the block's mask
+struct StepA2Fused {
+    // source corners whose injection is added when a level is read (inj_n = 0:
+    // the levels hold it already), in (source, corner) order; none on the last
+    // line that the one-way boundary reads
+    int inj_n;
+    int inj_i1[kFusedCorners], inj_i2[kFusedCorners];  // cell
+    int inj_src[kFusedCorners];                        // source * 8 + corner
+    float inj_w[kFusedCorners];
+    const float *scale;
+    int scaled;
+    const float *wav;
+    int it, ncs;
+    // receivers gathered from cur (nr = 0: none)
+    const GeoPoint *rec;
+    int nr;
+    float *rec_row;
+};
+void launch_stepA2(int geom, bool exact, const float *cur, const float *prv, float *nxt, const float *vel,
+                   const StepAParams &p, const StepA2Fused &f, cudaStream_t s);
 void launch_bcA(bool exact, const float *um, float *uo, float *aux, const StepAParams &p, cudaStream_t s);
 // adjoint of the spherical step (AWE_FAST): Y <- W M (L^T(I c X) + 2 X - W Y),
 // G += X L(A) on the interior (xcorr: G += X A; A null: none); receivers z += W M (w r)

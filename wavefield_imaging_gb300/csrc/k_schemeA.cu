@@ -58,11 +58,9 @@ __device__ __forceinline__ int sponge_index(const int *c, const int *n, const St
 // free-surface masks (value forced to zero), see StepAParams::mask
 __device__ __forceinline__ bool masked(const int *c, const int *n, const StepAParams &p) {
     switch (p.mask) {
-        case 1:  // cart 2D: x > nxpad - nb, plus the next-row spill of the rounded-up grid
-            return c[1] > n[1] - p.nb || (c[1] < p.spill && c[0] >= 1);
         case 2:  // cart 3D (before the boundary): z < nb
             return c[0] < p.nb;
-        case 3:  // polar / spherical: r > nrapad - nb, plus the next-line spill
+        case 3:  // spherical: r > nrapad - nb, plus the next-line spill
             return c[0] > n[0] - p.nb || (c[0] < p.spill && (c[1] >= 1 || c[2] >= 1));
     }
     return false;
@@ -87,23 +85,11 @@ __device__ __forceinline__ float laplacian(const float *__restrict__ A, long lon
     };
     // AWE_EXACT divides as the reference; AWE_FAST multiplies by the reciprocal
     auto div = [&](float a, float b, float rb) { return EXACT ? __fdiv_rn(a, b) : a * rb; };
-    if constexpr (GEOM == 0) {  // cart 2D (x = axis 2, z = axis 1): pxx + pzz
-        const float pxx = div(d2(A[i - s2], A[i + s2]), p.dd2, p.rd[1]);
-        const float pzz = div(d2(A[i - 1], A[i + 1]), p.dd1, p.rd[0]);
-        return fadd<EXACT>(pxx, pzz);
-    } else if constexpr (GEOM == 1) {  // cart 3D: (pxx + pyy) + pzz
+    if constexpr (GEOM == 1) {  // cart 3D: (pxx + pyy) + pzz
         const float pxx = div(d2(A[i - s2], A[i + s2]), p.dd2, p.rd[1]);
         const float pyy = div(d2(A[i - s3], A[i + s3]), p.dd3, p.rd[2]);
         const float pzz = div(d2(A[i - 1], A[i + 1]), p.dd1, p.rd[0]);
         return fadd<EXACT>(fadd<EXACT>(pxx, pyy), pzz);
-    } else if constexpr (GEOM == 2) {  // polar (r = axis 1, theta = axis 2)
-        const int ir = c[0];
-        const float am = __ldg(p.tr0 + ir), ap = __ldg(p.tr1 + ir), b = __ldg(p.tr2 + ir), b0 = __ldg(p.tr3 + ir);
-        const float compra =
-            fadd<EXACT>(fadd<EXACT>(fmul<EXACT>(am, A[i - 1]), fmul<EXACT>(p.a0, u)), fmul<EXACT>(ap, A[i + 1]));
-        const float compth =
-            fadd<EXACT>(fadd<EXACT>(fmul<EXACT>(b, A[i - s2]), fmul<EXACT>(b0, u)), fmul<EXACT>(b, A[i + s2]));
-        return fadd<EXACT>(compra, compth);
     } else {  // spherical (r = axis 1, theta = axis 2, phi = axis 3)
         const int ir = c[0];
         const float pra = div(fsub<EXACT>(A[i + 1], A[i - 1]), p.dd1, p.rd[0]);    // / (2 dra)
@@ -318,9 +304,7 @@ static void step_geom(int geom, const float *cur, const float *prv, float *nxt, 
         return;
     }
     switch (geom) {
-        case 0: k_stepA<0, EXACT><<<grid, block, 0, s>>>(cur, nxt, vel, p); break;
         case 1: k_stepA<1, EXACT><<<grid, block, 0, s>>>(cur, nxt, vel, p); break;
-        case 2: k_stepA<2, EXACT><<<grid, block, 0, s>>>(cur, nxt, vel, p); break;
         default: k_stepA<3, EXACT><<<grid, block, 0, s>>>(cur, nxt, vel, p); break;
     }
 }
@@ -345,29 +329,6 @@ void launch_stepA_oop(int geom, bool exact, const float *cur, const float *prv, 
 template <bool EXACT>
 __device__ __forceinline__ float oneway(float um_n, float um_c, float uo_n, float b) {
     return fadd<EXACT>(um_n, fmul<EXACT>(fsub<EXACT>(um_c, uo_n), b));
-}
-
-// 2D programs: rows 1..4 and n-5..n-2 of the swept axis, read from the last
-// sample of the other axis (the reference kernel's loop leaves that one).
-// geom 0: swept axis z (axis 1), other axis x (axis 2), rows limited to < nxpad
-// geom 2: swept axis theta (axis 2), other axis r (axis 1)
-template <bool EXACT>
-__global__ void k_bcA2_phase1(const float *__restrict__ um, const float *__restrict__ uo, float *__restrict__ aux,
-                              const StepAParams p) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const Grid g = p.g;
-    const bool cart = p.geom == 0;
-    const int nsw = cart ? g.n1 : g.n2, noth = cart ? g.n2 : g.n1;
-    if (t >= 8 * noth) return;
-    const int k = t / noth, o = t % noth;  // k: 0..3 top rows 1..4, 4..7 bottom rows n-5..n-2
-    const int row = k < 4 ? 1 + k : nsw - 5 + (k - 4);
-    if (cart && row >= g.n2) return;  // the kernel's `iz < nxpad` test
-    auto at = [&](int r, int oo) -> long long {
-        return cart ? (long long)oo * g.n1 + r : (long long)r * g.n1 + oo;
-    };
-    const int nbr = k < 4 ? row + 1 : row - 1;
-    const float b = k < 4 ? p.b2lo : p.b2hi;
-    aux[at(row, o)] = oneway<EXACT>(um[at(nbr, noth - 1)], um[at(row, o)], uo[at(nbr, noth - 1)], b);
 }
 
 // cart 3D (onewayBC_3D): cells within 4 (low) / 5 (high) of a face; the last
@@ -406,34 +367,22 @@ __global__ void k_bcA_phase2(float *__restrict__ uo, const float *__restrict__ a
     const int c[3] = {i1, i2, i3}, n[3] = {g.n1, g.n2, g.n3};
     if (!in_shell(c, n, p)) return;
     const long long i = ((long long)i3 * g.n2 + i2) * g.n1 + i1;
-    bool bc;
-    if (p.geom == 0) bc = ((i1 >= 1 && i1 <= 4) || (i1 >= g.n1 - 5 && i1 <= g.n1 - 2)) && i1 < g.n2;
-    else if (p.geom == 2) bc = (i2 >= 1 && i2 <= 4) || (i2 >= g.n2 - 5 && i2 <= g.n2 - 2);
-    else bc = i1 <= 4 || i1 >= g.n1 - 5 || i2 <= 4 || i2 >= g.n2 - 5 || i3 <= 4 || i3 >= g.n3 - 5;
+    const bool bc = i1 <= 4 || i1 >= g.n1 - 5 || i2 <= 4 || i2 >= g.n2 - 5 || i3 <= 4 || i3 >= g.n3 - 5;
     float v = uo[i];
-    if (p.geom == 1 && masked(c, n, p)) v = 0.f;  // cart 3D: free surface before the boundary
+    if (masked(c, n, p)) v = 0.f;  // the free surface before the boundary
     if (bc) v = aux[i];
     v = damp_a<EXACT>(v, sponge_index(c, n, p), p.dtab, p.ftab);
-    if (p.geom != 1 && p.mask && masked(c, n, p)) v = 0.f;  // 2D programs: free surface after the sponge
     uo[i] = v;
 }
 
 void launch_bcA(bool exact, const float *um, float *uo, float *aux, const StepAParams &p, cudaStream_t s) {
     const Grid &g = p.g;
     const int T = 128;
-    if (p.geom == 0 || p.geom == 2) {
-        const int noth = p.geom == 0 ? g.n2 : g.n1;
-        const int n = 8 * noth;
-        if (exact) k_bcA2_phase1<true><<<(n + T - 1) / T, T, 0, s>>>(um, uo, aux, p);
-        else k_bcA2_phase1<false><<<(n + T - 1) / T, T, 0, s>>>(um, uo, aux, p);
-    } else {
-        dim3 grid((g.n1 + T - 1) / T, g.n2, g.n3);
-        if (exact) k_bcA3_phase1<true><<<grid, T, 0, s>>>(um, uo, aux, p);
-        else k_bcA3_phase1<false><<<grid, T, 0, s>>>(um, uo, aux, p);
-    }
-    dim3 grid2((g.n1 + T - 1) / T, g.n2, g.n3);
-    if (exact) k_bcA_phase2<true><<<grid2, T, 0, s>>>(uo, aux, p);
-    else k_bcA_phase2<false><<<grid2, T, 0, s>>>(uo, aux, p);
+    dim3 grid((g.n1 + T - 1) / T, g.n2, g.n3);
+    if (exact) k_bcA3_phase1<true><<<grid, T, 0, s>>>(um, uo, aux, p);
+    else k_bcA3_phase1<false><<<grid, T, 0, s>>>(um, uo, aux, p);
+    if (exact) k_bcA_phase2<true><<<grid, T, 0, s>>>(uo, aux, p);
+    else k_bcA_phase2<false><<<grid, T, 0, s>>>(uo, aux, p);
 }
 
 // ---------------------------------------------------------------------------

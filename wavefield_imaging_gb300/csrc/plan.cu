@@ -55,7 +55,9 @@ void plan_graph_drop(awe_plan *p) {
     p->gexec = nullptr;
     p->g_wav = nullptr;
     p->g_dat = nullptr;
+    p->g_wfl = nullptr;
     p->g_ncs = 0;
+    p->g_seen = false;
 }
 
 // Optional cap on the device memory one plan may hold (AWE_DEVICE_BYTES_LIMIT,
@@ -393,11 +395,14 @@ awe_status awe_set_geometry(awe_plan *p, int ns, const float *sou, int nr, const
     plan_gradient_graph_drop(p);  // its per-cell point lists follow the geometry
     CUDA_TRY(cudaSetDevice(p->device));
     set_move_mode(p, -1, 1, 1);
+    p->inj_scale_ok = false;
     awe_status st = set_geometry_common(p, ns, sou, nr, rec);
     if (st == AWE_OK) st = set_inj_cells(p);
     if (st == AWE_OK) st = single_shot(p, ns, nr);
     key(after);
-    if (st != AWE_OK || std::memcmp(before, after, sizeof before) != 0) plan_graph_drop(p);
+    // (the 2D GPU-program loop bakes in where its sources lie)
+    if (st != AWE_OK || p->d.scheme == AWE_SCHEME_GPU || std::memcmp(before, after, sizeof before) != 0)
+        plan_graph_drop(p);
     if (st == AWE_OK) p->geom_set = true;
     return st;
 }
@@ -437,6 +442,7 @@ awe_status awe_set_moving_geometry(awe_plan *p, int ns, int nst, const float *so
     }
     plan_graph_drop(p);  // the captured time loop baked in the old state
     CUDA_TRY(cudaSetDevice(p->device));
+    p->inj_scale_ok = false;
     awe_status st = set_geometry_common(p, ns * nst, sou, nr * nrt, rec);
     if (st != AWE_OK) return st;
     p->inj = InjCells{};  // the lists hold fixed sources
@@ -476,6 +482,7 @@ awe_status awe_set_shots(awe_plan *p, int nshots, const int *ns, const float *so
     }
     CUDA_TRY(cudaSetDevice(p->device));
     set_move_mode(p, -1, 1, 1);
+    p->inj_scale_ok = false;
     awe_status st = set_geometry_common(p, NS, sou, NR, rec);
     if (st != AWE_OK) return st;
     // points of shot s address field s
@@ -577,20 +584,25 @@ awe_status awe_forward_device(awe_plan *p, const float *d_wav, int ncs, float *d
     }
     CUDA_TRY(cudaSetDevice(p->device));
     cudaStream_t s = stream ? (cudaStream_t)stream : p->stream;
-    // the CPU-program scheme's loop is pure stream work without snapshots and
-    // profiling: capture it once as a CUDA graph and replay it (one launch per
-    // run instead of several per time step - what matters for small 2D grids)
-    const bool graph = p->d.scheme == AWE_SCHEME_CPU && !(p->nsnap > 0 && (d_wfl || p->snap_cb)) && !p->profile;
+    // the CPU-program scheme's loop and the 2D GPU-program one are pure stream
+    // work without a frame callback and profiling.  The first run with its
+    // pointers launches it directly (300 captured and instantiated steps cost
+    // 0.9 ms before the first one runs); a second one captures it as a CUDA
+    // graph, replayed from then on (what matters for small 2D grids).
+    const bool cpu = p->d.scheme == AWE_SCHEME_CPU;
+    const bool graph = (cpu || p->d.ndim == 2) && !(p->nsnap > 0 && p->snap_cb) && !p->profile;
     awe_status st = AWE_OK;
-    if (graph) {
-        if (!p->gexec || p->g_wav != d_wav || p->g_dat != d_dat || p->g_ncs != ncs) {
-            plan_graph_drop(p);
+    if (!cpu) st = planA_prepare(p);  // uploads: not inside a capture
+    if (st != AWE_OK) return st;
+    const bool same = p->g_wav == d_wav && p->g_dat == d_dat && p->g_wfl == d_wfl && p->g_ncs == ncs;
+    if (graph && same && (p->gexec || p->g_seen)) {
+        if (!p->gexec) {
             cudaStream_t cs;
             CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
             cudaGraph_t gr = nullptr;
             cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
             if (e == cudaSuccess) {
-                st = planB_run(p, d_wav, ncs, d_dat, nullptr, cs);
+                st = cpu ? planB_run(p, d_wav, ncs, d_dat, d_wfl, cs) : planA_run(p, d_wav, ncs, d_dat, d_wfl, cs);
                 e = cudaStreamEndCapture(cs, &gr);
             }
             if (st == AWE_OK && e == cudaSuccess) e = cudaGraphInstantiate(&p->gexec, gr, 0);
@@ -602,14 +614,20 @@ awe_status awe_forward_device(awe_plan *p, const float *d_wav, int ncs, float *d
                 set_error("CUDA graph capture of the time loop failed: %s", cudaGetErrorString(e));
                 return AWE_ERR_CUDA;
             }
-            p->g_wav = d_wav;
-            p->g_dat = d_dat;
-            p->g_ncs = ncs;
             p->g_launches = p->launches;
         }
         CUDA_TRY(cudaGraphLaunch(p->gexec, s));
         p->launches = p->g_launches;
     } else {
+        if (graph) {
+            if (p->gexec) cudaGraphExecDestroy(p->gexec);
+            p->gexec = nullptr;
+            p->g_wav = d_wav;
+            p->g_dat = d_dat;
+            p->g_wfl = d_wfl;
+            p->g_ncs = ncs;
+            p->g_seen = true;
+        }
         st = (p->d.scheme == AWE_SCHEME_CPU) ? planB_run(p, d_wav, ncs, d_dat, d_wfl, s)
                                              : planA_run(p, d_wav, ncs, d_dat, d_wfl, s);
     }

@@ -537,7 +537,7 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
     // receivers and sources in the adjoint step itself (one launch per step)
     // where the grid is small enough for per-cell lists and no ABC transpose
     // follows the step
-    const bool fuse_pts = !st->tma && !st->kap && cells <= (1LL << 24);
+    const bool fuse_pts = !st->tma && !st->kap && cells <= kFusedCells;
     // 3D TMA path: one boundary launch per adjoint step (k_bnd3_adj) instead of
     // the kappa fold, three ABC-transpose launches and the g pass; AWE_BND3=0
     // keeps the separate launches (the tests compare both)

@@ -64,6 +64,9 @@ struct awe_plan {
     awe::StepAParams pa{};             // step / boundary parameters
     std::vector<float> h_rfl_pad;      // padded reflectivity image (cart 2D refl=y)
     float *inj_scale = nullptr;        // per source corner injection scale
+    bool inj_scale_ok = false;         // inj_scale follows the current model and points
+    float *u3 = nullptr;               // third level buffer (2D: the step is out of place)
+    bool inj_fused = false;            // 2D: the step adds the injection itself (StepA2Fused)
     int snap_transpose = 0;            // polar snapshots are theta-fastest
 
     bool model_set = false, geom_set = false;
@@ -106,7 +109,9 @@ struct awe_plan {
     cudaGraphExec_t gexec = nullptr;
     const float *g_wav = nullptr;
     float *g_dat = nullptr;
+    float *g_wfl = nullptr;
     int g_ncs = 0;
+    bool g_seen = false;  // the last run had these pointers and ran directly
     long long g_launches = 0;
     float *stage_wav = nullptr, *stage_dat = nullptr;  // awe_forward's device staging buffers
     size_t stage_wav_bytes = 0, stage_dat_bytes = 0;
@@ -171,6 +176,8 @@ awe_status stepB_full(awe_plan *p, const StepBParams &sp, const float *prv, cons
                       int ext_n = 0, int ext_stride = 1, float *ext_row = nullptr);
 // 2D steps add the sources in the step kernel (one launch per step) up to this many sources
 constexpr int kFusedSources = 8;
+// the gradient's adjoint step adds the point terms itself up to this many cells
+constexpr long long kFusedCells = 1LL << 24;
 // 3D CPU-program scheme with sponge + one-way ABC: the boundary work of a step
 // (ABC, shell sponge, receiver gather, injection) is one launch (k_bnd3)
 bool stepB3_bnd(const awe_plan *p);
@@ -182,6 +189,8 @@ void plan_gradient_free(awe_plan *p);
 void plan_gradient_graph_drop(awe_plan *p);
 
 awe_status planA_init(awe_plan *p);
+// the per-corner injection scales, when the model or the points changed since
+awe_status planA_prepare(awe_plan *p);
 awe_status planA_model(awe_plan *p, const float *vel, const float *rfl);
 awe_status planA_run(awe_plan *p, const float *d_wav, int ncs, float *d_dat, float *d_wfl, cudaStream_t s,
                      const StepHook *hook = nullptr);

@@ -168,7 +168,8 @@ awe_status planA_init(awe_plan *p) {
     AWE_TRY(dev_alloc(p, (void **)&p->u[1], cells * sizeof(float)));
     AWE_TRY(dev_alloc(p, (void **)&p->vel, cells * sizeof(float)));
     AWE_TRY(dev_alloc(p, (void **)&p->corner_off, 8 * sizeof(long long)));
-    if (pa.shell > 0) AWE_TRY(dev_alloc(p, (void **)&p->aux, cells * sizeof(float)));
+    if (d.ndim == 2) AWE_TRY(dev_alloc(p, (void **)&p->u3, cells * sizeof(float)));
+    else if (pa.shell > 0) AWE_TRY(dev_alloc(p, (void **)&p->aux, cells * sizeof(float)));
 
     pa.nshot = 1;
     pa.shot_cells = g.cells();
@@ -226,6 +227,7 @@ awe_status planA_model(awe_plan *p, const float *vel, const float *rfl) {
     StepAParams &pa = p->pa;
     const size_t cells = (size_t)g.cells();
     const int nb = p->nbd;
+    p->inj_scale_ok = false;
     p->h_vel_raw.assign(cells, 0.f);
     expand_model(d.ndim, vel, p->h_vel_raw.data(), nb, d.n);
     AWE_TRY(upload_t(p, &p->vel, p->h_vel_raw.data(), cells));
@@ -305,12 +307,20 @@ static float refl_scale(const std::vector<float> &v, long long s, long long rs, 
     return 0.f;
 }
 
-static awe_status prepare_injection(awe_plan *p, bool &scaled) {
+awe_status planA_prepare(awe_plan *p) {
     const awe_desc &d = p->d;
     const Grid &g = p->g;
     const int geom = p->pa.geom, ns = p->ns;
-    scaled = d.expl != 0;
-    if (!scaled || ns == 0) return AWE_OK;
+    // 2D: few source corners, none on the line the one-way boundary reads, are
+    // added by the step itself
+    static_assert(4 * kFusedSources <= kFusedCorners, "fused corners");
+    p->inj_fused = (geom == 0 || geom == 2) && p->move_mode < 0 && (int)p->h_src.size() <= kFusedSources;
+    for (const GeoPoint &pt : p->h_src)
+        for (int c = 0; p->inj_fused && c < 4; c++) {
+            const long long n = pt.base + p->h_corner_off[c];
+            if (geom == 0 ? n / g.n1 >= g.n2 - 1 : n % g.n1 >= g.n1 - 1) p->inj_fused = false;
+        }
+    if (d.expl == 0 || ns == 0 || p->inj_scale_ok) return AWE_OK;
     std::vector<float> sc((size_t)ns * 8, 1.f);
     for (int s = 0; s < ns; s++) {
         const Lint &l = p->h_src_lint[s];
@@ -335,7 +345,85 @@ static awe_status prepare_injection(awe_plan *p, bool &scaled) {
     if (p->inj_scale) dev_free(p, p->inj_scale);
     p->inj_scale = nullptr;
     AWE_TRY(upload_t(p, &p->inj_scale, sc.data(), sc.size()));
+    p->inj_scale_ok = true;
     return AWE_OK;
+}
+
+// 2D: one launch a step (k_stepA2d.cu).  Sources the step adds itself leave the
+// levels without their injection, so the traces of step it - 1 come from the
+// level step it reads; otherwise the injection and the gather keep their own
+// launches around the step.
+static awe_status run2d(awe_plan *p, const float *d_wav, int ncs, float *d_dat, float *d_wfl, cudaStream_t s) {
+    const awe_desc &d = p->d;
+    const Grid &g = p->g;
+    const StepAParams &pa = p->pa;
+    const bool exact = d.precision == AWE_EXACT, scaled = d.expl != 0;
+    long long launches = 0;
+    float *prv = p->u[0], *cur = p->u[1], *nxt = p->u3;
+    StepA2Fused f{};
+    if (p->inj_fused)
+        for (size_t k = 0; k < p->h_src.size(); k++)
+            for (int c = 0; c < 4; c++) {
+                const long long n = p->h_src[k].base + p->h_corner_off[c];
+                f.inj_i1[f.inj_n] = (int)(n % g.n1);
+                f.inj_i2[f.inj_n] = (int)(n / g.n1);
+                f.inj_src[f.inj_n] = 8 * (int)k + c;
+                f.inj_w[f.inj_n++] = p->h_src[k].w[c];
+            }
+    f.scale = p->inj_scale;
+    f.scaled = scaled;
+    f.wav = d_wav;
+    f.ncs = ncs;
+    auto gather = [&](int it, const float *lev) {
+        const PointsAt pr = points_at(p, p->rec, p->nr, p->rec_rows, it);
+        launch_extract_off(2, exact, lev, pr.pts, p->nr, d_dat + (size_t)it * p->nr, nullptr, nullptr, nullptr, g,
+                           p->corner_off, s, pr.stride);
+        launches++;
+    };
+    int isnap = 0;
+    for (int it = 0; it < d.nt; it++) {
+        f.it = it;
+        f.nr = 0;
+        if (!p->inj_fused && p->ns > 0) {
+            const PointsAt ps = points_at(p, p->src, p->ns, p->src_rows, it);
+            if (p->inj.n > 0)
+                launch_injectA_cells(exact, cur, p->inj_scale, p->inj, d_wav, it, scaled, s, ncs);
+            else
+                launch_injectA(exact, 2, cur, ps.pts, p->inj_scale, p->ns, d_wav, it, scaled, p->corner_off, s,
+                               ps.stride, ncs);
+            launches++;
+        } else if (p->move_mode < 0 && p->nr > 0 && it > 0 && it - 1 < p->nsmp) {
+            f.rec = p->rec;
+            f.nr = p->nr;
+            f.rec_row = d_dat + (size_t)(it - 1) * p->nr;
+        }
+        prof_begin(p, s);
+        launch_stepA2(pa.geom, exact, cur, prv, nxt, p->vel, pa, f, s);
+        prof_end(p, s);
+        launches++;
+        float *t = prv;
+        prv = cur;
+        cur = nxt;
+        nxt = t;
+        const bool own = (!p->inj_fused && p->ns > 0) || p->move_mode >= 0;
+        if (p->nr > 0 && it < p->nsmp && (own || it == d.nt - 1)) gather(it, cur);
+        if (p->nsnap > 0 && it % d.jsnap == 0) {
+            float *frame = d_wfl ? d_wfl + (size_t)isnap * p->snap_elems : p->d_snap_tmp;
+            if (frame) {
+                if (p->snap_transpose)
+                    launch_snapshot_transpose2(cur, frame, g, p->snap_f[0], p->snap_f[1], p->snap_m[0], p->snap_m[1],
+                                               s);
+                else
+                    launch_snapshot(2, cur, frame, g, p->snap_f[0], p->snap_f[1], 0, p->snap_m[0], p->snap_m[1], 1,
+                                    nullptr, nullptr, nullptr, s);
+                launches++;
+                AWE_TRY(deliver_snapshot(p, frame, isnap, it, s));
+            }
+            isnap++;
+        }
+    }
+    p->launches = launches;
+    return flush_snapshots(p);
 }
 
 // hook (may be null): called at the start of every iteration, before the
@@ -348,14 +436,15 @@ awe_status planA_run(awe_plan *p, const float *d_wav, int ncs, float *d_dat, flo
     const StepAParams &pa = p->pa;
     const bool exact = d.precision == AWE_EXACT;
     const size_t bytes = (size_t)g.cells() * sizeof(float) * (pa.nshot > 0 ? pa.nshot : 1);
-    bool scaled = false;
-    AWE_TRY(prepare_injection(p, scaled));
+    const bool scaled = d.expl != 0;
+    AWE_TRY(planA_prepare(p));
     CUDA_TRY(cudaMemsetAsync(p->u[0], 0, bytes, s));
     CUDA_TRY(cudaMemsetAsync(p->u[1], 0, bytes, s));
     CUDA_TRY(cudaMemsetAsync(d_dat, 0, (size_t)p->nsmp * p->nr * sizeof(float), s));
     if (p->nsnap > 0 && !d_wfl && p->snap_cb && !p->d_snap_tmp)
         AWE_TRY(dev_alloc(p, (void **)&p->d_snap_tmp, p->snap_elems * sizeof(float)));
     p->snap_pending = -1;  // a frame left queued by a failed run is not delivered
+    if (d.ndim == 2) return run2d(p, d_wav, ncs, d_dat, d_wfl, s);
 
     if (p->sph_tma) {  // maps of this run's level fields; the work counter restarts with every run
         if (!sphA_tma_maps(p->sph_maps, p->u, p->vel, g, pa.nshot)) {
@@ -409,9 +498,7 @@ awe_status planA_run(awe_plan *p, const float *d_wav, int ncs, float *d_dat, flo
                 itr += 1;
                 if (itr < p->nsmp) row = itr;
             }
-        } else if (pa.geom == 3) {
-            row = it;
-        } else if (it < p->nsmp) {
+        } else {
             row = it;
         }
         if (row >= 0 && p->nr > 0) {
@@ -423,12 +510,8 @@ awe_status planA_run(awe_plan *p, const float *d_wav, int ncs, float *d_dat, flo
         if (p->nsnap > 0 && it % d.jsnap == 0) {
             float *frame = d_wfl ? d_wfl + (size_t)isnap * p->snap_elems : p->d_snap_tmp;
             if (frame) {
-                if (p->snap_transpose)
-                    launch_snapshot_transpose2(cur, frame, g, p->snap_f[0], p->snap_f[1], p->snap_m[0], p->snap_m[1],
-                                               s);
-                else
-                    launch_snapshot(d.ndim, cur, frame, g, p->snap_f[0], p->snap_f[1], p->snap_f[2], p->snap_m[0],
-                                    p->snap_m[1], p->snap_m[2], nullptr, nullptr, nullptr, s);
+                launch_snapshot(d.ndim, cur, frame, g, p->snap_f[0], p->snap_f[1], p->snap_f[2], p->snap_m[0],
+                                p->snap_m[1], p->snap_m[2], nullptr, nullptr, nullptr, s);
                 launches++;
                 AWE_TRY(deliver_snapshot(p, frame, isnap, it, s));
             }

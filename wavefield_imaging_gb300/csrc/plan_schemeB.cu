@@ -173,6 +173,10 @@ awe_status planB_model(awe_plan *p, const float *vel, const float *den) {
 
 awe_status set_inj_cells(awe_plan *p) {
     const int nc = p->d.ndim == 3 ? 8 : 4, ns = (int)p->h_src.size();
+    p->inj = InjCells{};
+    // 2D steps add a few sources themselves; the gradient's fused adjoint step
+    // (up to 2^24 cells) has lists of its own
+    if (p->d.ndim == 2 && ns <= kFusedSources && p->g.cells() <= kFusedCells) return AWE_OK;
     std::vector<std::pair<long long, int>> e;  // (cell, source * 8 + corner)
     e.reserve((size_t)ns * nc);
     for (int s = 0; s < ns; s++)
@@ -191,7 +195,6 @@ awe_status set_inj_cells(awe_plan *p) {
         ent[k] = make_int2(e[k].second, w);
     }
     start.push_back((int)e.size());
-    p->inj = InjCells{};
     if (cell.empty()) return AWE_OK;
     // sizes for every source at cells of its own, so that points that only
     // move keep the buffer (a captured time loop reads it)
