@@ -1,4 +1,4 @@
-"""The 2D GPU-program step in one launch at its edges: grids one block wide or
+"""The cartesian and polar GPU-program steps in one launch at their edges: grids one block wide or
 ending inside a block, sources at block edges and on the last line (where the
 injection keeps its own launch), more sources than the step adds itself, a
 graph replay and kept points.  AWE_EXACT equals the oracle bit for bit."""
@@ -50,3 +50,33 @@ def test_one_launch_step_is_bit_exact(kind, n, ns, edge):
             np.testing.assert_array_equal(p.forward(wav), ref)
         p.set_geometry(sou, rec)
         np.testing.assert_array_equal(p.forward(wav), ref)
+
+
+@pytest.mark.parametrize("n,n3,ns", [(12, 12, 2), (13, 15, 3), (33, 17, 8), (34, 44, 9), (45, 30, 2)])
+def test_one_launch_step_3d_is_bit_exact(n, n3, ns):
+    """Planes per block, face planes and shifted boundary lines; sources next
+    to the boundary lines and on the padded faces."""
+    from oracle import oracle
+    import wavefield_imaging_gb300 as awe
+
+    rng = np.random.default_rng(n + n3)
+    nb, nt = 4, 40
+    vel = (150 + 30 * rng.random((n3, n, n))).astype(np.float32)
+    c = np.stack([rng.integers(0, q - 1, ns) + rng.choice([0.0, 0.5], ns) for q in (n, n3, n)], 1)
+    c[0] = (-nb + 2.0, -nb + 5.5, -nb + 3.25)  # in the boundary shell
+    sou = (c * D).astype(np.float32)
+    rec = np.stack([rng.uniform(-nb, q + nb - 1.01, 12) * D for q in (n, n3, n)], 1).astype(np.float32)
+    par = dict(kind="cart3d", n=[n, n, n3], d=[D] * 3, o=[0.0] * 3, nb=nb, nt=nt, dt=0.005, jsnap=15, bnds=1, jdata=2)
+    wav = ricker(nt, 0.005)
+    ref, rsn = oracle.gpu_scheme("cart3d", par, vel, wav, sou, rec)
+    desc = awe.make_desc(3, (n, n, n3), (D,) * 3, (0.0,) * 3, nt, 0.005, scheme=awe.SCHEME_GPU, nb=nb, jsnap=15,
+                         bnds=1, jdata=2, precision=awe.EXACT)
+    with awe.Plan(desc) as p:
+        p.set_model(vel)
+        p.set_geometry(sou, rec)
+        dat, snaps = p.forward(wav, snapshots=True)
+        again = p.forward(wav)
+    assert np.abs(ref).max() > 0
+    np.testing.assert_array_equal(dat, ref)
+    np.testing.assert_array_equal(snaps, rsn)
+    np.testing.assert_array_equal(again, ref)

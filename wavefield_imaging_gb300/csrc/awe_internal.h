@@ -186,7 +186,6 @@ struct StepAParams {
     int pri[3];      // sponge priority over memory axes (the kernel's x, y, z)
     int mask;        // 0 none, 1 cart 2D x band, 2 cart 3D z < nb, 3 r band (polar/spherical)
     int spill;       // samples of the next line zeroed by the free-surface grid rounding
-    int shell, shell_axes;  // boundary shell width and the axes it spans (bit a = axis a+1)
     float dt2;
     float dd1, dd2, dd3, dd4, dd5;  // divisors of the Laplacian terms
     float rd[5];                    // their reciprocals (AWE_FAST)
@@ -201,11 +200,9 @@ struct StepAParams {
     long long shot_cells;                // cells of one shot's field
 };
 // out of place (the spherical AWE_FAST march kernels): prv the previous level, out the new one
-bool stepA_out_of_place(int geom, bool exact);
-void launch_stepA_oop(int geom, bool exact, const float *cur, const float *prv, float *out, const float *vel,
+void launch_stepA_oop(const float *cur, const float *prv, float *out, const float *vel,
                       const StepAParams &p, cudaStream_t s);
-void launch_stepA(int geom, bool exact, const float *cur, float *nxt, const float *vel, const StepAParams &p,
-                  cudaStream_t s);
+void launch_stepA(bool exact, const float *cur, float *nxt, const float *vel, const StepAParams &p, cudaStream_t s);
 // 2D step in one launch (k_stepA2d.cu): out of place (cur, prv and nxt differ)
 constexpr int kFusedCorners = 32;  // one bit per corner in the block's mask
 struct StepA2Fused {
@@ -227,7 +224,23 @@ struct StepA2Fused {
 };
 void launch_stepA2(int geom, bool exact, const float *cur, const float *prv, float *nxt, const float *vel,
                    const StepAParams &p, const StepA2Fused &f, cudaStream_t s);
-void launch_bcA(bool exact, const float *um, float *uo, float *aux, const StepAParams &p, cudaStream_t s);
+// cartesian 3D step in one launch (k_stepA3d.cu), the same for 3D
+constexpr int kFusedCorners3 = 64;  // one bit per corner in the block's mask
+struct StepA3Fused {
+    int inj_n;
+    int inj_i1[kFusedCorners3], inj_i2[kFusedCorners3], inj_i3[kFusedCorners3];
+    int inj_src[kFusedCorners3];
+    float inj_w[kFusedCorners3];
+    const float *scale;
+    int scaled;
+    const float *wav;
+    int it, ncs;
+    const GeoPoint *rec;
+    int nr;
+    float *rec_row;
+};
+void launch_stepA3(bool exact, const float *cur, const float *prv, float *nxt, const float *vel, const StepAParams &p,
+                   const StepA3Fused &f, cudaStream_t s);
 // adjoint of the spherical step (AWE_FAST): Y <- W M (L^T(I c X) + 2 X - W Y),
 // G += X L(A) on the interior (xcorr: G += X A; A null: none); receivers z += W M (w r)
 void launch_adjA_sph(const float *X, float *Y, const float *A, const float *vel, float2 *G, const StepAParams &p,

@@ -1,19 +1,15 @@
-// Kernels for the scheme of the reference's GPU programs
-// (CODE/MAWEFD{cart,spher}{2D,3D}gpu.cu over cart_kernels.cu / spher_kernels.cu):
-// 2nd-order Laplacian (cartesian, polar, or spherical with metric terms),
-// injection into the current level before the update, one-way boundary,
-// quadratic-alpha sponge on both time levels, free-surface masks.
+// Kernels for the spherical scheme of the reference's GPU programs
+// (CODE/MAWEFDspher3Dgpu.cu over spher_kernels.cu: 2nd-order Laplacian with
+// metric terms, injection into the current level before the update,
+// quadratic-alpha sponge on both time levels, free-surface mask), its adjoint,
+// and the injection and frame kernels all geometries share.  The cartesian and
+// polar steps are in k_stepA2d.cu and k_stepA3d.cu.
 //
 // Two buffers hold the time levels.  The reference shifts three (ppo <- po,
 // po <- fpo) and then sponges both po and ppo; here the new level overwrites
 // the previous one in place and the sponge of the level that becomes
 // "previous" is applied when it is next read, the same float operation on the
-// same value.  Cells that the one-way boundary rewrites or reads (the
-// `shell`) are stored unsponged by the step kernel and finished by a two-phase
-// boundary pass: phase 1 computes the boundary values from the unmodified
-// fields (every read sees the field before the pass - the race-free reading
-// of the reference's boundary kernels), phase 2 writes them with the sponge
-// and masks.
+// same value.
 #include <cuda_runtime.h>
 
 #include "awe_internal.h"
@@ -31,170 +27,8 @@ __device__ __forceinline__ float damp_a(float v, int i, const double *__restrict
     else return v * ftab[i];
 }
 
-// sponge index: priority over memory axes pri[0..nd-1] (the kernel's x, y, z)
-__device__ __forceinline__ int sponge_index(const int *c, const int *n, const StepAParams &p) {
-    const int nb = p.nb;
-    bool low = false, high = false;
-    for (int k = 0; k < p.nd; k++) {
-        const int a = p.pri[k];
-        low = low || c[a] < nb;
-        high = high || c[a] > n[a] - nb;
-    }
-    if (low) {
-        for (int k = 0; k < p.nd; k++) {
-            const int a = p.pri[k];
-            if (c[a] < nb) return nb - c[a];
-        }
-    }
-    if (high) {
-        for (int k = 0; k < p.nd; k++) {
-            const int a = p.pri[k];
-            if (c[a] > n[a] - nb) return c[a] - (n[a] - nb);
-        }
-    }
-    return 0;
-}
-
-// free-surface masks (value forced to zero), see StepAParams::mask
-__device__ __forceinline__ bool masked(const int *c, const int *n, const StepAParams &p) {
-    switch (p.mask) {
-        case 2:  // cart 3D (before the boundary): z < nb
-            return c[0] < p.nb;
-        case 3:  // spherical: r > nrapad - nb, plus the next-line spill
-            return c[0] > n[0] - p.nb || (c[0] < p.spill && (c[1] >= 1 || c[2] >= 1));
-    }
-    return false;
-}
-
-__device__ __forceinline__ bool in_shell(const int *c, const int *n, const StepAParams &p) {
-    if (p.shell_axes == 0) return false;
-    for (int a = 0; a < 3; a++)
-        if ((p.shell_axes >> a) & 1)
-            if (c[a] < p.shell || c[a] >= n[a] - p.shell) return true;
-    return false;
-}
-
-template <int GEOM, bool EXACT>
-__device__ __forceinline__ float laplacian(const float *__restrict__ A, long long i, const int *c,
-                                           const StepAParams &p) {
-    const long long s2 = p.g.n1, s3 = (long long)p.g.n1 * p.g.n2;
-    const float u = A[i];
-    const float u2 = fadd<EXACT>(u, u);  // 2*p, exact
-    auto d2 = [&](float m, float pl) {   // (p[+1] - 2 p) + p[-1]
-        return fadd<EXACT>(fsub<EXACT>(pl, u2), m);
-    };
-    // AWE_EXACT divides as the reference; AWE_FAST multiplies by the reciprocal
-    auto div = [&](float a, float b, float rb) { return EXACT ? __fdiv_rn(a, b) : a * rb; };
-    if constexpr (GEOM == 1) {  // cart 3D: (pxx + pyy) + pzz
-        const float pxx = div(d2(A[i - s2], A[i + s2]), p.dd2, p.rd[1]);
-        const float pyy = div(d2(A[i - s3], A[i + s3]), p.dd3, p.rd[2]);
-        const float pzz = div(d2(A[i - 1], A[i + 1]), p.dd1, p.rd[0]);
-        return fadd<EXACT>(fadd<EXACT>(pxx, pyy), pzz);
-    } else {  // spherical (r = axis 1, theta = axis 2, phi = axis 3)
-        const int ir = c[0];
-        const float pra = div(fsub<EXACT>(A[i + 1], A[i - 1]), p.dd1, p.rd[0]);    // / (2 dra)
-        const float ppra = div(d2(A[i - 1], A[i + 1]), p.dd2, p.rd[1]);              // / dra^2
-        const float pth = div(fsub<EXACT>(A[i + s2], A[i - s2]), p.dd3, p.rd[2]);  // / (2 dth)
-        const float ppth = div(d2(A[i - s2], A[i + s2]), p.dd4, p.rd[3]);            // / dth^2
-        const float ppph = div(d2(A[i - s3], A[i + s3]), p.dd5, p.rd[4]);            // / dph^2
-        const long long t = (long long)c[1] * p.g.n1 + ir;
-        const float A2 = __ldg(p.tr0 + ir), Cr = __ldg(p.tr1 + ir), B = __ldg(p.tt0 + t), D = __ldg(p.tt1 + t);
-        float lap = fadd<EXACT>(fmul<EXACT>(A2, pra), ppra);
-        lap = fadd<EXACT>(lap, fmul<EXACT>(B, pth));
-        lap = fadd<EXACT>(lap, fmul<EXACT>(Cr, ppth));
-        return fadd<EXACT>(lap, fmul<EXACT>(D, ppph));
-    }
-}
-
-// One step: nxt (previous level, sponge pending) <- new level.
-template <int GEOM, bool EXACT>
-__global__ void __launch_bounds__(256) k_stepA(const float *__restrict__ cur, float *__restrict__ nxt,
-                                               const float *__restrict__ vel, const StepAParams p) {
-    const int i1 = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i2 = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i3 = blockIdx.z;
-    const Grid g = p.g;
-    if (i1 >= g.n1 || i2 >= g.n2) return;
-    const int c[3] = {i1, i2, i3}, n[3] = {g.n1, g.n2, g.n3};
-    const long long i = ((long long)i3 * g.n2 + i2) * g.n1 + i1;
-    const int si = sponge_index(c, n, p);
-    const float q = damp_a<EXACT>(nxt[i], si, p.dtab, p.ftab);  // previous level, its sponge applied now
-    bool interior = true;
-    for (int a = 0; a < p.nd; a++) interior = interior && c[a] >= 4 && c[a] < n[a] - 4;
-    const float lap = interior ? laplacian<GEOM, EXACT>(cur, i, c, p) : 0.f;
-    const float v = __ldg(vel + i), u = cur[i];
-    // cart: (dt*dt)*(v*v*lap) + 2p - pp ; polar/spherical: (dt*dt)*(v*v)*lap + 2p - pp
-    float a;
-    if constexpr (GEOM <= 1)
-        a = fmul<EXACT>(p.dt2, fmul<EXACT>(fmul<EXACT>(v, v), lap));
-    else
-        a = fmul<EXACT>(fmul<EXACT>(p.dt2, fmul<EXACT>(v, v)), lap);
-    float f = fsub<EXACT>(fadd<EXACT>(a, fadd<EXACT>(u, u)), q);
-    if (!in_shell(c, n, p)) {
-        if (p.mask && masked(c, n, p)) f = 0.f;
-        f = damp_a<EXACT>(f, si, p.dtab, p.ftab);
-    }
-    nxt[i] = f;
-}
-
-// Spherical step, AWE_FAST: each thread owns one (r, theta) column and marches
-// along phi through a chunk of planes.  The phi neighbours stay in registers,
-// the per-radius and per-(theta, r) metric tables are read once per column,
-// and the r / theta neighbours come through L1 from the lanes and warps that
-// load the same plane.  Same formula and operation order as k_stepA<3>,
-// with fused multiply-adds and reciprocal multiplies.
-constexpr int kSphChunk = 16;
-
-// prv: the previous level (the same buffer as nxt for the in-place step)
-__global__ void __launch_bounds__(256) k_stepA_sph_march(const float *__restrict__ cur, const float *prv, float *nxt,
-                                                         const float *__restrict__ vel, const StepAParams p) {
-    const int i1 = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i2 = blockIdx.y * blockDim.y + threadIdx.y;
-    const Grid g = p.g;
-    if (i1 >= g.n1 || i2 >= g.n2) return;
-    const int n[3] = {g.n1, g.n2, g.n3};
-    const long long s2 = g.n1, s3 = (long long)g.n1 * g.n2;
-    const int p0 = blockIdx.z * kSphChunk, p1 = min(p0 + kSphChunk, g.n3);
-    const bool in12 = i1 >= 4 && i1 < g.n1 - 4 && i2 >= 4 && i2 < g.n2 - 4;
-    const long long t = (long long)i2 * g.n1 + i1;
-    const float A2 = __ldg(p.tr0 + i1), Cr = __ldg(p.tr1 + i1), B = __ldg(p.tt0 + t), D = __ldg(p.tt1 + t);
-    const long long base = (long long)i2 * s2 + i1;
-    float um = p0 > 0 ? cur[base + (p0 - 1) * s3] : 0.f;
-    float uc = cur[base + p0 * s3];
-    for (int i3 = p0; i3 < p1; i3++) {
-        const long long i = base + i3 * s3;
-        const float up = i3 + 1 < g.n3 ? cur[i + s3] : 0.f;
-        const int c[3] = {i1, i2, i3};
-        const int si = sponge_index(c, n, p);
-        const float q = damp_a<false>(prv[i], si, p.dtab, p.ftab);
-        float lap = 0.f;
-        if (in12 && i3 >= 4 && i3 < g.n3 - 4) {
-            const float u2 = uc + uc;
-            const float rm = cur[i - 1], rp = cur[i + 1], tm = cur[i - s2], tp = cur[i + s2];
-            const float pra = (rp - rm) * p.rd[0];
-            const float ppra = ((rp - u2) + rm) * p.rd[1];
-            const float pth = (tp - tm) * p.rd[2];
-            const float ppth = ((tp - u2) + tm) * p.rd[3];
-            const float ppph = ((up - u2) + um) * p.rd[4];
-            lap = fmaf(A2, pra, ppra);
-            lap = fmaf(B, pth, lap);
-            lap = fmaf(Cr, ppth, lap);
-            lap = fmaf(D, ppph, lap);
-        }
-        const float v = __ldg(vel + i);
-        float f = fmaf(p.dt2 * (v * v), lap, uc + uc) - q;
-        if (!in_shell(c, n, p)) {
-            if (p.mask && masked(c, n, p)) f = 0.f;
-            f = damp_a<false>(f, si, p.dtab, p.ftab);
-        }
-        nxt[i] = f;
-        um = uc;
-        uc = up;
-    }
-}
-
-// sponge_index for a 3D grid with the coordinates in registers (no indexed
-// arrays): the all-interior case first, then the priority walk
+// sponge_index of the spherical grid with the coordinates in registers (no
+// indexed arrays): the all-interior case first, then the priority walk
 __device__ __forceinline__ int sel3(int a, int v0, int v1, int v2) { return a == 0 ? v0 : (a == 1 ? v1 : v2); }
 
 __device__ __forceinline__ int sponge_index3(int c0, int c1, int c2, int n0, int n1, int n2, const StepAParams &p) {
@@ -216,6 +50,100 @@ __device__ __forceinline__ int sponge_index3(int c0, int c1, int c2, int n0, int
         if (!low && c > n - nb) return c - (n - nb);
     }
     return 0;
+}
+
+// free-surface mask (value forced to zero): r > nrapad - nb, plus the
+// next-line spill of the rounded-up grid
+__device__ __forceinline__ bool masked(int c0, int c1, int c2, const Grid &g, const StepAParams &p) {
+    return c0 > g.n1 - p.nb || (c0 < p.spill && (c1 >= 1 || c2 >= 1));
+}
+
+
+// One step of the spherical scheme, AWE_EXACT: nxt (previous level, sponge
+// pending) <- new level.
+__global__ void __launch_bounds__(256) k_stepA_exact(const float *__restrict__ cur, float *__restrict__ nxt,
+                                                     const float *__restrict__ vel, const StepAParams p) {
+    const int i1 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i2 = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i3 = blockIdx.z;
+    const Grid g = p.g;
+    if (i1 >= g.n1 || i2 >= g.n2) return;
+    const long long s2 = g.n1, s3 = (long long)g.n1 * g.n2;
+    const long long i = i3 * s3 + i2 * s2 + i1;
+    const int si = sponge_index3(i1, i2, i3, g.n1, g.n2, g.n3, p);
+    const float q = damp_a<true>(nxt[i], si, p.dtab, p.ftab);  // previous level, its sponge applied now
+    const float u = cur[i], u2 = __fadd_rn(u, u);
+    float lap = 0.f;
+    if (i1 >= 4 && i1 < g.n1 - 4 && i2 >= 4 && i2 < g.n2 - 4 && i3 >= 4 && i3 < g.n3 - 4) {
+        auto d2 = [&](float m, float pl) { return __fadd_rn(__fsub_rn(pl, u2), m); };  // (p[+1] - 2 p) + p[-1]
+        const float pra = __fdiv_rn(__fsub_rn(cur[i + 1], cur[i - 1]), p.dd1);      // / (2 dra)
+        const float ppra = __fdiv_rn(d2(cur[i - 1], cur[i + 1]), p.dd2);            // / dra^2
+        const float pth = __fdiv_rn(__fsub_rn(cur[i + s2], cur[i - s2]), p.dd3);    // / (2 dth)
+        const float ppth = __fdiv_rn(d2(cur[i - s2], cur[i + s2]), p.dd4);          // / dth^2
+        const float ppph = __fdiv_rn(d2(cur[i - s3], cur[i + s3]), p.dd5);          // / dph^2
+        const long long t = (long long)i2 * g.n1 + i1;
+        const float A2 = __ldg(p.tr0 + i1), Cr = __ldg(p.tr1 + i1), B = __ldg(p.tt0 + t), D = __ldg(p.tt1 + t);
+        lap = __fadd_rn(__fmul_rn(A2, pra), ppra);
+        lap = __fadd_rn(lap, __fmul_rn(B, pth));
+        lap = __fadd_rn(lap, __fmul_rn(Cr, ppth));
+        lap = __fadd_rn(lap, __fmul_rn(D, ppph));
+    }
+    const float v = __ldg(vel + i);
+    const float a = __fmul_rn(__fmul_rn(p.dt2, __fmul_rn(v, v)), lap);
+    float f = __fsub_rn(__fadd_rn(a, u2), q);
+    if (p.mask && masked(i1, i2, i3, g, p)) f = 0.f;
+    nxt[i] = damp_a<true>(f, si, p.dtab, p.ftab);
+}
+
+// The spherical step, AWE_FAST: each thread owns one (r, theta) column and marches
+// along phi through a chunk of planes.  The phi neighbours stay in registers,
+// the per-radius and per-(theta, r) metric tables are read once per column,
+// and the r / theta neighbours come through L1 from the lanes and warps that
+// load the same plane.  Same formula and operation order as k_stepA_exact,
+// with fused multiply-adds and reciprocal multiplies.
+constexpr int kSphChunk = 16;
+
+// prv: the previous level (the same buffer as nxt for the in-place step)
+__global__ void __launch_bounds__(256) k_stepA_sph_march(const float *__restrict__ cur, const float *prv, float *nxt,
+                                                         const float *__restrict__ vel, const StepAParams p) {
+    const int i1 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i2 = blockIdx.y * blockDim.y + threadIdx.y;
+    const Grid g = p.g;
+    if (i1 >= g.n1 || i2 >= g.n2) return;
+    const long long s2 = g.n1, s3 = (long long)g.n1 * g.n2;
+    const int p0 = blockIdx.z * kSphChunk, p1 = min(p0 + kSphChunk, g.n3);
+    const bool in12 = i1 >= 4 && i1 < g.n1 - 4 && i2 >= 4 && i2 < g.n2 - 4;
+    const long long t = (long long)i2 * g.n1 + i1;
+    const float A2 = __ldg(p.tr0 + i1), Cr = __ldg(p.tr1 + i1), B = __ldg(p.tt0 + t), D = __ldg(p.tt1 + t);
+    const long long base = (long long)i2 * s2 + i1;
+    float um = p0 > 0 ? cur[base + (p0 - 1) * s3] : 0.f;
+    float uc = cur[base + p0 * s3];
+    for (int i3 = p0; i3 < p1; i3++) {
+        const long long i = base + i3 * s3;
+        const float up = i3 + 1 < g.n3 ? cur[i + s3] : 0.f;
+        const int si = sponge_index3(i1, i2, i3, g.n1, g.n2, g.n3, p);
+        const float q = damp_a<false>(prv[i], si, p.dtab, p.ftab);
+        float lap = 0.f;
+        if (in12 && i3 >= 4 && i3 < g.n3 - 4) {
+            const float u2 = uc + uc;
+            const float rm = cur[i - 1], rp = cur[i + 1], tm = cur[i - s2], tp = cur[i + s2];
+            const float pra = (rp - rm) * p.rd[0];
+            const float ppra = ((rp - u2) + rm) * p.rd[1];
+            const float pth = (tp - tm) * p.rd[2];
+            const float ppth = ((tp - u2) + tm) * p.rd[3];
+            const float ppph = ((up - u2) + um) * p.rd[4];
+            lap = fmaf(A2, pra, ppra);
+            lap = fmaf(B, pth, lap);
+            lap = fmaf(Cr, ppth, lap);
+            lap = fmaf(D, ppph, lap);
+        }
+        const float v = __ldg(vel + i);
+        float f = fmaf(p.dt2 * (v * v), lap, uc + uc) - q;
+        if (p.mask && masked(i1, i2, i3, g, p)) f = 0.f;
+        nxt[i] = damp_a<false>(f, si, p.dtab, p.ftab);
+        um = uc;
+        uc = up;
+    }
 }
 
 // The same march with two consecutive radii per thread (n1 even): 8-byte
@@ -288,101 +216,27 @@ __global__ void __launch_bounds__(256) k_stepA_sph_march2(const float *__restric
     }
 }
 
-template <bool EXACT>
-static void step_geom(int geom, const float *cur, const float *prv, float *nxt, const float *vel, const StepAParams &p,
+static void step_fast(const float *cur, const float *prv, float *nxt, const float *vel, const StepAParams &p,
                       cudaStream_t s) {
+    const int nchunk = (p.g.n3 + kSphChunk - 1) / kSphChunk;
+    if (p.g.n1 % 2 == 0) {
+        dim3 block(32, 8, 1), grid((p.g.n1 / 2 + 31) / 32, (p.g.n2 + 7) / 8, nchunk * (p.nshot > 0 ? p.nshot : 1));
+        k_stepA_sph_march2<<<grid, block, 0, s>>>(cur, prv, nxt, vel, p);
+    } else {
+        dim3 block(64, 4, 1), grid((p.g.n1 + 63) / 64, (p.g.n2 + 3) / 4, nchunk);
+        k_stepA_sph_march<<<grid, block, 0, s>>>(cur, prv, nxt, vel, p);
+    }
+}
+
+void launch_stepA(bool exact, const float *cur, float *nxt, const float *vel, const StepAParams &p, cudaStream_t s) {
+    if (!exact) return step_fast(cur, nxt, nxt, vel, p, s);
     dim3 block(64, 4, 1), grid((p.g.n1 + 63) / 64, (p.g.n2 + 3) / 4, p.g.n3);
-    if (!EXACT && geom == 3) {
-        if (p.g.n1 % 2 == 0) {
-            const int nchunk = (p.g.n3 + kSphChunk - 1) / kSphChunk;
-            dim3 b2(32, 8, 1), g2((p.g.n1 / 2 + 31) / 32, (p.g.n2 + 7) / 8, nchunk * (p.nshot > 0 ? p.nshot : 1));
-            k_stepA_sph_march2<<<g2, b2, 0, s>>>(cur, prv, nxt, vel, p);
-        } else {
-            dim3 mg((p.g.n1 + 63) / 64, (p.g.n2 + 3) / 4, (p.g.n3 + kSphChunk - 1) / kSphChunk);
-            k_stepA_sph_march<<<mg, block, 0, s>>>(cur, prv, nxt, vel, p);
-        }
-        return;
-    }
-    switch (geom) {
-        case 1: k_stepA<1, EXACT><<<grid, block, 0, s>>>(cur, nxt, vel, p); break;
-        default: k_stepA<3, EXACT><<<grid, block, 0, s>>>(cur, nxt, vel, p); break;
-    }
+    k_stepA_exact<<<grid, block, 0, s>>>(cur, nxt, vel, p);
 }
 
-void launch_stepA(int geom, bool exact, const float *cur, float *nxt, const float *vel, const StepAParams &p,
-                  cudaStream_t s) {
-    if (exact) step_geom<true>(geom, cur, nxt, nxt, vel, p, s);
-    else step_geom<false>(geom, cur, nxt, nxt, vel, p, s);
-}
-
-bool stepA_out_of_place(int geom, bool exact) { return geom == 3 && !exact; }
-
-void launch_stepA_oop(int geom, bool exact, const float *cur, const float *prv, float *out, const float *vel,
-                      const StepAParams &p, cudaStream_t s) {
-    if (stepA_out_of_place(geom, exact)) step_geom<false>(geom, cur, prv, out, vel, p, s);
-}
-
-// ---------------------------------------------------------------------------
-// One-way boundary, phase 1: boundary values from the unmodified fields.
-// um = the level that just became "previous" (before its sponge), uo = the
-// new level as stored by the step kernel (unsponged inside the shell).
-template <bool EXACT>
-__device__ __forceinline__ float oneway(float um_n, float um_c, float uo_n, float b) {
-    return fadd<EXACT>(um_n, fmul<EXACT>(fsub<EXACT>(um_c, uo_n), b));
-}
-
-// cart 3D (onewayBC_3D): cells within 4 (low) / 5 (high) of a face; the last
-// applicable face formula wins; neighbours read masked (z < nb zeroed).
-template <bool EXACT>
-__global__ void k_bcA3_phase1(const float *__restrict__ um, const float *__restrict__ uo, float *__restrict__ aux,
-                              const StepAParams p) {
-    const int i1 = blockIdx.x * blockDim.x + threadIdx.x;  // z
-    const int i2 = blockIdx.y, i3 = blockIdx.z;           // x, y
-    const Grid g = p.g;
-    if (i1 >= g.n1) return;
-    const int iz = i1, ix = i2, iy = i3;
-    const bool zl = iz <= 4, zh = iz >= g.n1 - 5, xl = ix <= 4, xh = ix >= g.n2 - 5, yl = iy <= 4, yh = iy >= g.n3 - 5;
-    if (!(zl || zh || xl || xh || yl || yh)) return;
-    const long long s2 = g.n1, s3 = (long long)g.n1 * g.n2, c = iy * s3 + ix * s2 + iz;
-    auto ps = [&](long long n, int nz) { return nz < p.nb ? 0.f : uo[n]; };  // freeSurf_3D before the boundary
-    const int nx = g.n2, nz = g.n1;
-    float val = 0.f;
-    if (zl) val = oneway<EXACT>(um[c + 1], um[c], ps(c + 1, iz + 1), p.tb[0][iy * nx + ix]);
-    if (zh) val = oneway<EXACT>(um[c - 1], um[c], ps(c - 1, iz - 1), p.tb[1][iy * nx + ix]);
-    if (xl) val = oneway<EXACT>(um[c + s2], um[c], ps(c + s2, iz), p.tb[2][iy * nz + iz]);
-    if (xh) val = oneway<EXACT>(um[c - s2], um[c], ps(c - s2, iz), p.tb[1][iy * nz + iz]);  // the z-high table, as the reference
-    if (yl) val = oneway<EXACT>(um[c + s3], um[c], ps(c + s3, iz), p.tb[4][iz * nx + ix]);
-    if (yh) val = oneway<EXACT>(um[c - s3], um[c], ps(c - s3, iz), p.tb[5][iz * nx + ix]);
-    aux[c] = val;
-}
-
-// phase 2: every shell cell gets its final value: the boundary value where
-// the boundary applies, else the (masked) new level; then sponge and masks.
-template <bool EXACT>
-__global__ void k_bcA_phase2(float *__restrict__ uo, const float *__restrict__ aux, const StepAParams p) {
-    const int i1 = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i2 = blockIdx.y, i3 = blockIdx.z;
-    const Grid g = p.g;
-    if (i1 >= g.n1) return;
-    const int c[3] = {i1, i2, i3}, n[3] = {g.n1, g.n2, g.n3};
-    if (!in_shell(c, n, p)) return;
-    const long long i = ((long long)i3 * g.n2 + i2) * g.n1 + i1;
-    const bool bc = i1 <= 4 || i1 >= g.n1 - 5 || i2 <= 4 || i2 >= g.n2 - 5 || i3 <= 4 || i3 >= g.n3 - 5;
-    float v = uo[i];
-    if (masked(c, n, p)) v = 0.f;  // the free surface before the boundary
-    if (bc) v = aux[i];
-    v = damp_a<EXACT>(v, sponge_index(c, n, p), p.dtab, p.ftab);
-    uo[i] = v;
-}
-
-void launch_bcA(bool exact, const float *um, float *uo, float *aux, const StepAParams &p, cudaStream_t s) {
-    const Grid &g = p.g;
-    const int T = 128;
-    dim3 grid((g.n1 + T - 1) / T, g.n2, g.n3);
-    if (exact) k_bcA3_phase1<true><<<grid, T, 0, s>>>(um, uo, aux, p);
-    else k_bcA3_phase1<false><<<grid, T, 0, s>>>(um, uo, aux, p);
-    if (exact) k_bcA_phase2<true><<<grid, T, 0, s>>>(uo, aux, p);
-    else k_bcA_phase2<false><<<grid, T, 0, s>>>(uo, aux, p);
+void launch_stepA_oop(const float *cur, const float *prv, float *out, const float *vel, const StepAParams &p,
+                      cudaStream_t s) {
+    step_fast(cur, prv, out, vel, p, s);
 }
 
 // ---------------------------------------------------------------------------

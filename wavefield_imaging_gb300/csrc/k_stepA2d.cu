@@ -69,12 +69,13 @@ __device__ __forceinline__ float inj2(float v, int e, int it, const StepA2Fused 
 // one wave of blocks.  What no earlier launch writes (velocity, tables) is
 // loaded before the wait for the previous step, the levels after it, all of
 // them unconditionally (clamped), so their latencies overlap.
-template <int GEOM, bool EXACT>
+// Idx: int up to 2^31 - 1 cells (64-bit indices cost 6 % of a step)
+template <int GEOM, bool EXACT, typename Idx>
 __global__ void __launch_bounds__(256) k_stepA2(const float *__restrict__ cur, const float *__restrict__ prv,
                                                 float *__restrict__ nxt, const float *__restrict__ vel,
                                                 const StepAParams p, const StepA2Fused f) {
     const Grid g = p.g;
-    const int s2 = g.n1, last = g.n1 * g.n2 - 1;
+    const Idx s2 = g.n1, last = s2 * g.n2 - 1;
     const int rows = (g.n2 + 7) / 8;  // blocks of cells
     if ((int)blockIdx.y >= rows) {    // receiver gather of cur, extract_2D's order
         const int r = (((int)blockIdx.y - rows) * (int)gridDim.x + (int)blockIdx.x) * 256 +
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(256) k_stepA2(const float *__restrict__ cur, c
     if constexpr (GEOM == 2) {
         am = __ldg(p.tr0 + j1), ap = __ldg(p.tr1 + j1), b = __ldg(p.tr2 + j1), b0 = __ldg(p.tr3 + j1);
     }
-    int i[2];
+    Idx i[2];
     Damp2<EXACT> damp[2];
     float v[2];
 #pragma unroll
@@ -122,16 +123,17 @@ __global__ void __launch_bounds__(256) k_stepA2(const float *__restrict__ cur, c
     for (int r = 0; r < 2; r++) {
         u[r] = cur[i[r]];
         q[r] = prv[i[r]];
-        zm[r] = cur[max(i[r] - 1, 0)];
+        zm[r] = cur[max(i[r] - 1, (Idx)0)];
         zp[r] = cur[min(i[r] + 1, last)];
-        xm[r] = cur[max(i[r] - s2, 0)];
+        xm[r] = cur[max(i[r] - s2, (Idx)0)];
         xp[r] = cur[min(i[r] + s2, last)];
     }
     for (; near; near &= near - 1) {  // in (source, corner) order
-        const int e = __ffs(near) - 1, c = f.inj_i2[e] * s2 + f.inj_i1[e];
+        const int e = __ffs(near) - 1;
+        const Idx c = f.inj_i2[e] * s2 + f.inj_i1[e];
 #pragma unroll
         for (int r = 0; r < 2; r++) {
-            const int d = c - i[r];
+            const Idx d = c - i[r];
             if (d == 0) {
                 u[r] = inj2<EXACT>(u[r], e, f.it, f);
                 if (f.it > 0) q[r] = inj2<EXACT>(q[r], e, f.it - 1, f);
@@ -184,7 +186,8 @@ __global__ void __launch_bounds__(256) k_stepA2(const float *__restrict__ cur, c
         const bool lo = row >= 1 && row <= 4, hi = row >= nsw - 5 && row <= nsw - 2;
         if ((lo || hi) && (GEOM != 0 || row < g.n2)) {
             const int nbr = lo ? row + 1 : row - 1;
-            const int l1 = GEOM == 0 ? nbr : g.n1 - 1, l2 = GEOM == 0 ? g.n2 - 1 : nbr, l = l2 * s2 + l1;
+            const int l1 = GEOM == 0 ? nbr : g.n1 - 1, l2 = GEOM == 0 ? g.n2 - 1 : nbr;
+            const Idx l = l2 * s2 + l1;
             const float um = cur[l];
             const float ql = Damp2<EXACT>(sponge2<GEOM>(l1, l2, g, p.nb), p)(prv[l]);
             const float d = __fsub_rn(u[r], __fsub_rn(__fadd_rn(um, um), ql)), c = lo ? p.b2lo : p.b2hi;
@@ -199,8 +202,9 @@ __global__ void __launch_bounds__(256) k_stepA2(const float *__restrict__ cur, c
 
 }  // namespace
 
-void launch_stepA2(int geom, bool exact, const float *cur, const float *prv, float *nxt, const float *vel,
-                   const StepAParams &p, const StepA2Fused &f, cudaStream_t s) {
+template <typename Idx>
+static void launch_a2(int geom, bool exact, const float *cur, const float *prv, float *nxt, const float *vel,
+                      const StepAParams &p, const StepA2Fused &f, cudaStream_t s) {
     dim3 grid((p.g.n1 + 63) / 64, (p.g.n2 + 7) / 8);
     if (f.nr > 0) grid.y += (unsigned)((f.nr + grid.x * 256 - 1) / (grid.x * 256));
     cudaLaunchConfig_t cfg = {};
@@ -213,12 +217,18 @@ void launch_stepA2(int geom, bool exact, const float *cur, const float *prv, flo
     cfg.attrs = at;
     cfg.numAttrs = 1;
     if (geom == 0) {
-        if (exact) cudaLaunchKernelEx(&cfg, k_stepA2<0, true>, cur, prv, nxt, vel, p, f);
-        else cudaLaunchKernelEx(&cfg, k_stepA2<0, false>, cur, prv, nxt, vel, p, f);
+        if (exact) cudaLaunchKernelEx(&cfg, k_stepA2<0, true, Idx>, cur, prv, nxt, vel, p, f);
+        else cudaLaunchKernelEx(&cfg, k_stepA2<0, false, Idx>, cur, prv, nxt, vel, p, f);
     } else {
-        if (exact) cudaLaunchKernelEx(&cfg, k_stepA2<2, true>, cur, prv, nxt, vel, p, f);
-        else cudaLaunchKernelEx(&cfg, k_stepA2<2, false>, cur, prv, nxt, vel, p, f);
+        if (exact) cudaLaunchKernelEx(&cfg, k_stepA2<2, true, Idx>, cur, prv, nxt, vel, p, f);
+        else cudaLaunchKernelEx(&cfg, k_stepA2<2, false, Idx>, cur, prv, nxt, vel, p, f);
     }
+}
+
+void launch_stepA2(int geom, bool exact, const float *cur, const float *prv, float *nxt, const float *vel,
+                   const StepAParams &p, const StepA2Fused &f, cudaStream_t s) {
+    if (p.g.cells() + p.g.n1 < (1ll << 31)) launch_a2<int>(geom, exact, cur, prv, nxt, vel, p, f, s);
+    else launch_a2<long long>(geom, exact, cur, prv, nxt, vel, p, f, s);
 }
 
 }  // namespace awe

@@ -400,7 +400,7 @@ awe_status awe_set_geometry(awe_plan *p, int ns, const float *sou, int nr, const
     if (st == AWE_OK) st = set_inj_cells(p);
     if (st == AWE_OK) st = single_shot(p, ns, nr);
     key(after);
-    // (the 2D GPU-program loop bakes in where its sources lie)
+    // (the GPU-program loop bakes in where its sources lie)
     if (st != AWE_OK || p->d.scheme == AWE_SCHEME_GPU || std::memcmp(before, after, sizeof before) != 0)
         plan_graph_drop(p);
     if (st == AWE_OK) p->geom_set = true;
@@ -584,13 +584,14 @@ awe_status awe_forward_device(awe_plan *p, const float *d_wav, int ncs, float *d
     }
     CUDA_TRY(cudaSetDevice(p->device));
     cudaStream_t s = stream ? (cudaStream_t)stream : p->stream;
-    // the CPU-program scheme's loop and the 2D GPU-program one are pure stream
+    // the loops of the CPU-program scheme and of the cartesian and polar
+    // GPU-program ones are pure stream
     // work without a frame callback and profiling.  The first run with its
     // pointers launches it directly (300 captured and instantiated steps cost
     // 0.9 ms before the first one runs); a second one captures it as a CUDA
     // graph, replayed from then on (what matters for small 2D grids).
     const bool cpu = p->d.scheme == AWE_SCHEME_CPU;
-    const bool graph = (cpu || p->d.ndim == 2) && !(p->nsnap > 0 && p->snap_cb) && !p->profile;
+    const bool graph = (cpu || p->pa.geom != 3) && !(p->nsnap > 0 && p->snap_cb) && !p->profile;
     awe_status st = AWE_OK;
     if (!cpu) st = planA_prepare(p);  // uploads: not inside a capture
     if (st != AWE_OK) return st;

@@ -307,7 +307,7 @@ static awe_status gradient_spher_one(awe_plan *p, const float *d_wav, int ncs, c
                     AWE_TRY(sph_tma_step(p, st->sl_halo, st->sl_tile, cur + cells, i * g.n3, (i - 1) * g.n3, s));
                 } else {
                     prof_begin(p, s);
-                    launch_stepA_oop(pa.geom, false, cur, cur - cells, cur + cells, p->vel, pa, s);
+                    launch_stepA_oop(cur, cur - cells, cur + cells, p->vel, pa, s);
                     prof_end(p, s);
                 }
             }

@@ -60,13 +60,12 @@ struct awe_plan {
     int move_mode = -1, src_rows = 1, rec_rows = 1;
 
     // scheme-GPU specific
-    float *aux = nullptr;              // boundary values (phase 1 -> phase 2)
     awe::StepAParams pa{};             // step / boundary parameters
     std::vector<float> h_rfl_pad;      // padded reflectivity image (cart 2D refl=y)
     float *inj_scale = nullptr;        // per source corner injection scale
     bool inj_scale_ok = false;         // inj_scale follows the current model and points
-    float *u3 = nullptr;               // third level buffer (2D: the step is out of place)
-    bool inj_fused = false;            // 2D: the step adds the injection itself (StepA2Fused)
+    float *u3 = nullptr;               // third level buffer (cartesian, polar: the step is out of place)
+    bool inj_fused = false;            // the step adds the injection itself (StepA2Fused, StepA3Fused)
     int snap_transpose = 0;            // polar snapshots are theta-fastest
 
     bool model_set = false, geom_set = false;

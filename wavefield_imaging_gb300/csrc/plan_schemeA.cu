@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "awe_internal.h"
@@ -76,14 +77,12 @@ awe_status planA_init(awe_plan *p) {
             pa.pri[0] = 1, pa.pri[1] = 0;
             pa.mask = 1;  // freeSurf_2D unconditional (MAWEFDcart2Dgpu.cu:424)
             pa.spill = round2 - g.n2;
-            pa.shell = 6, pa.shell_axes = 1;
             pa.dd1 = d.d[0] * d.d[0];
             pa.dd2 = d.d[1] * d.d[1];
             break;
         case 1:  // cart 3D: kernel axes (x, y, z) = memory (2, 3, 1)
             pa.pri[0] = 1, pa.pri[1] = 2, pa.pri[2] = 0;
             pa.mask = 2;  // freeSurf_3D unconditional before the boundary (MAWEFDcart3Dgpu.cu:417)
-            pa.shell = 6, pa.shell_axes = 7;
             pa.dd1 = d.d[0] * d.d[0];
             pa.dd2 = d.d[1] * d.d[1];
             pa.dd3 = d.d[2] * d.d[2];
@@ -92,13 +91,11 @@ awe_status planA_init(awe_plan *p) {
             pa.pri[0] = 0, pa.pri[1] = 1;
             pa.mask = d.fsrf ? 3 : 0;
             pa.spill = round1 - g.n1;
-            pa.shell = 6, pa.shell_axes = 2;
             break;
         default:  // spherical: kernel axes (r, phi, theta) = memory (1, 3, 2)
             pa.pri[0] = 0, pa.pri[1] = 2, pa.pri[2] = 1;
             pa.mask = d.fsrf ? 3 : 0;
             pa.spill = round1 - g.n1;
-            pa.shell = 0, pa.shell_axes = 0;
             break;
     }
     (void)round1;
@@ -168,8 +165,7 @@ awe_status planA_init(awe_plan *p) {
     AWE_TRY(dev_alloc(p, (void **)&p->u[1], cells * sizeof(float)));
     AWE_TRY(dev_alloc(p, (void **)&p->vel, cells * sizeof(float)));
     AWE_TRY(dev_alloc(p, (void **)&p->corner_off, 8 * sizeof(long long)));
-    if (d.ndim == 2) AWE_TRY(dev_alloc(p, (void **)&p->u3, cells * sizeof(float)));
-    else if (pa.shell > 0) AWE_TRY(dev_alloc(p, (void **)&p->aux, cells * sizeof(float)));
+    if (geom != 3) AWE_TRY(dev_alloc(p, (void **)&p->u3, cells * sizeof(float)));
 
     pa.nshot = 1;
     pa.shot_cells = g.cells();
@@ -311,12 +307,12 @@ awe_status planA_prepare(awe_plan *p) {
     const awe_desc &d = p->d;
     const Grid &g = p->g;
     const int geom = p->pa.geom, ns = p->ns;
-    // 2D: few source corners, none on the line the one-way boundary reads, are
-    // added by the step itself
-    static_assert(4 * kFusedSources <= kFusedCorners, "fused corners");
-    p->inj_fused = (geom == 0 || geom == 2) && p->move_mode < 0 && (int)p->h_src.size() <= kFusedSources;
+    // few source corners are added by the step itself (2D: none on the line the
+    // one-way boundary reads)
+    static_assert(4 * kFusedSources <= kFusedCorners && 8 * kFusedSources <= kFusedCorners3, "fused corners");
+    p->inj_fused = geom != 3 && p->move_mode < 0 && (int)p->h_src.size() <= kFusedSources;
     for (const GeoPoint &pt : p->h_src)
-        for (int c = 0; p->inj_fused && c < 4; c++) {
+        for (int c = 0; d.ndim == 2 && p->inj_fused && c < 4; c++) {
             const long long n = pt.base + p->h_corner_off[c];
             if (geom == 0 ? n / g.n1 >= g.n2 - 1 : n % g.n1 >= g.n1 - 1) p->inj_fused = false;
         }
@@ -349,24 +345,28 @@ awe_status planA_prepare(awe_plan *p) {
     return AWE_OK;
 }
 
-// 2D: one launch a step (k_stepA2d.cu).  Sources the step adds itself leave the
-// levels without their injection, so the traces of step it - 1 come from the
-// level step it reads; otherwise the injection and the gather keep their own
-// launches around the step.
-static awe_status run2d(awe_plan *p, const float *d_wav, int ncs, float *d_dat, float *d_wfl, cudaStream_t s) {
+// Cartesian and polar: one launch a step (k_stepA2d.cu, k_stepA3d.cu).  Sources
+// the step adds itself leave the levels without their injection, so the traces
+// of step it - 1 come from the level step it reads; otherwise the injection and
+// the gather keep their own launches around the step.
+template <class Fused>
+static awe_status run_fused(awe_plan *p, const float *d_wav, int ncs, float *d_dat, float *d_wfl, cudaStream_t s) {
     const awe_desc &d = p->d;
     const Grid &g = p->g;
     const StepAParams &pa = p->pa;
     const bool exact = d.precision == AWE_EXACT, scaled = d.expl != 0;
+    const int nc = d.ndim == 3 ? 8 : 4;
     long long launches = 0;
     float *prv = p->u[0], *cur = p->u[1], *nxt = p->u3;
-    StepA2Fused f{};
+    Fused f{};
     if (p->inj_fused)
         for (size_t k = 0; k < p->h_src.size(); k++)
-            for (int c = 0; c < 4; c++) {
+            for (int c = 0; c < nc; c++) {
                 const long long n = p->h_src[k].base + p->h_corner_off[c];
                 f.inj_i1[f.inj_n] = (int)(n % g.n1);
-                f.inj_i2[f.inj_n] = (int)(n / g.n1);
+                f.inj_i2[f.inj_n] = (int)(n / g.n1 % g.n2);
+                if constexpr (std::is_same<Fused, StepA3Fused>::value)
+                    f.inj_i3[f.inj_n] = (int)(n / g.n1 / g.n2);
                 f.inj_src[f.inj_n] = 8 * (int)k + c;
                 f.inj_w[f.inj_n++] = p->h_src[k].w[c];
             }
@@ -374,39 +374,48 @@ static awe_status run2d(awe_plan *p, const float *d_wav, int ncs, float *d_dat, 
     f.scaled = scaled;
     f.wav = d_wav;
     f.ncs = ncs;
-    auto gather = [&](int it, const float *lev) {
-        const PointsAt pr = points_at(p, p->rec, p->nr, p->rec_rows, it);
-        launch_extract_off(2, exact, lev, pr.pts, p->nr, d_dat + (size_t)it * p->nr, nullptr, nullptr, nullptr, g,
-                           p->corner_off, s, pr.stride);
-        launches++;
+    // the trace row of step it, or -1 (cartesian 3D: MAWEFDcart3Dgpu.cu:432-442, pre-incremented)
+    auto row_of = [&](int it) {
+        const int r = d.ndim == 2 ? it : it % d.jdata == 0 ? it / d.jdata + 1 : -1;
+        return p->nr > 0 && r < p->nsmp ? r : -1;
     };
     int isnap = 0;
     for (int it = 0; it < d.nt; it++) {
         f.it = it;
         f.nr = 0;
-        if (!p->inj_fused && p->ns > 0) {
+        const bool inj = !p->inj_fused && p->ns > 0;
+        const bool own = inj || p->move_mode >= 0;  // the traces keep their own launch
+        if (inj) {
             const PointsAt ps = points_at(p, p->src, p->ns, p->src_rows, it);
             if (p->inj.n > 0)
                 launch_injectA_cells(exact, cur, p->inj_scale, p->inj, d_wav, it, scaled, s, ncs);
             else
-                launch_injectA(exact, 2, cur, ps.pts, p->inj_scale, p->ns, d_wav, it, scaled, p->corner_off, s,
+                launch_injectA(exact, d.ndim, cur, ps.pts, p->inj_scale, p->ns, d_wav, it, scaled, p->corner_off, s,
                                ps.stride, ncs);
             launches++;
-        } else if (p->move_mode < 0 && p->nr > 0 && it > 0 && it - 1 < p->nsmp) {
+        }
+        if (!own && it > 0 && row_of(it - 1) >= 0) {
             f.rec = p->rec;
             f.nr = p->nr;
-            f.rec_row = d_dat + (size_t)(it - 1) * p->nr;
+            f.rec_row = d_dat + (size_t)row_of(it - 1) * p->nr;
         }
         prof_begin(p, s);
-        launch_stepA2(pa.geom, exact, cur, prv, nxt, p->vel, pa, f, s);
+        if constexpr (std::is_same<Fused, StepA3Fused>::value)
+            launch_stepA3(exact, cur, prv, nxt, p->vel, pa, f, s);
+        else
+            launch_stepA2(pa.geom, exact, cur, prv, nxt, p->vel, pa, f, s);
         prof_end(p, s);
         launches++;
         float *t = prv;
         prv = cur;
         cur = nxt;
         nxt = t;
-        const bool own = (!p->inj_fused && p->ns > 0) || p->move_mode >= 0;
-        if (p->nr > 0 && it < p->nsmp && (own || it == d.nt - 1)) gather(it, cur);
+        if (row_of(it) >= 0 && (own || it == d.nt - 1)) {
+            const PointsAt pr = points_at(p, p->rec, p->nr, p->rec_rows, it);
+            launch_extract_off(d.ndim, exact, cur, pr.pts, p->nr, d_dat + (size_t)row_of(it) * p->nr, nullptr, nullptr,
+                               nullptr, g, p->corner_off, s, pr.stride);
+            launches++;
+        }
         if (p->nsnap > 0 && it % d.jsnap == 0) {
             float *frame = d_wfl ? d_wfl + (size_t)isnap * p->snap_elems : p->d_snap_tmp;
             if (frame) {
@@ -414,8 +423,8 @@ static awe_status run2d(awe_plan *p, const float *d_wav, int ncs, float *d_dat, 
                     launch_snapshot_transpose2(cur, frame, g, p->snap_f[0], p->snap_f[1], p->snap_m[0], p->snap_m[1],
                                                s);
                 else
-                    launch_snapshot(2, cur, frame, g, p->snap_f[0], p->snap_f[1], 0, p->snap_m[0], p->snap_m[1], 1,
-                                    nullptr, nullptr, nullptr, s);
+                    launch_snapshot(d.ndim, cur, frame, g, p->snap_f[0], p->snap_f[1], p->snap_f[2], p->snap_m[0],
+                                    p->snap_m[1], p->snap_m[2], nullptr, nullptr, nullptr, s);
                 launches++;
                 AWE_TRY(deliver_snapshot(p, frame, isnap, it, s));
             }
@@ -444,7 +453,8 @@ awe_status planA_run(awe_plan *p, const float *d_wav, int ncs, float *d_dat, flo
     if (p->nsnap > 0 && !d_wfl && p->snap_cb && !p->d_snap_tmp)
         AWE_TRY(dev_alloc(p, (void **)&p->d_snap_tmp, p->snap_elems * sizeof(float)));
     p->snap_pending = -1;  // a frame left queued by a failed run is not delivered
-    if (d.ndim == 2) return run2d(p, d_wav, ncs, d_dat, d_wfl, s);
+    if (d.ndim == 2) return run_fused<StepA2Fused>(p, d_wav, ncs, d_dat, d_wfl, s);
+    if (pa.geom == 1) return run_fused<StepA3Fused>(p, d_wav, ncs, d_dat, d_wfl, s);
 
     if (p->sph_tma) {  // maps of this run's level fields; the work counter restarts with every run
         if (!sphA_tma_maps(p->sph_maps, p->u, p->vel, g, pa.nshot)) {
@@ -456,10 +466,9 @@ awe_status planA_run(awe_plan *p, const float *d_wav, int ncs, float *d_dat, flo
         CUDA_TRY(cudaMemsetAsync(p->sched_counter, 0, sizeof(unsigned long long), s));
         p->sched_base = 0;
     }
-    const int jdata = d.jdata > 0 ? d.jdata : 1;
     long long launches = 0;
     float *cur = p->u[1], *nxt = p->u[0];
-    int itr = 0, isnap = 0;
+    int isnap = 0;
     for (int it = 0; it < d.nt; it++) {
         if (hook) AWE_TRY((*hook)(it, nxt, cur, s));
         if (p->ns > 0) {
@@ -483,28 +492,15 @@ awe_status planA_run(awe_plan *p, const float *d_wav, int ncs, float *d_dat, flo
                 return AWE_ERR_CUDA;
             }
         } else {
-            launch_stepA(pa.geom, exact, cur, nxt, p->vel, pa, s);
+            launch_stepA(exact, cur, nxt, p->vel, pa, s);
         }
         prof_end(p, s);
         launches++;
-        if (pa.shell > 0) {
-            launch_bcA(exact, cur, nxt, p->aux, pa, s);
-            launches += 2;
-        }
         std::swap(cur, nxt);  // cur: the new level (final); nxt: previous (sponge pending)
-        int row = -1;
-        if (pa.geom == 1) {  // MAWEFDcart3Dgpu.cu:432-442: pre-incremented row
-            if (it % jdata == 0) {
-                itr += 1;
-                if (itr < p->nsmp) row = itr;
-            }
-        } else {
-            row = it;
-        }
-        if (row >= 0 && p->nr > 0) {
+        if (p->nr > 0) {
             const PointsAt pr = points_at(p, p->rec, p->nr, p->rec_rows, it);
-            launch_extract_off(d.ndim, exact, cur, pr.pts, p->nr, d_dat + (size_t)row * p->nr, nullptr, nullptr,
-                               nullptr, g, p->corner_off, s, pr.stride);
+            launch_extract_off(d.ndim, exact, cur, pr.pts, p->nr, d_dat + (size_t)it * p->nr, nullptr, nullptr, nullptr,
+                               g, p->corner_off, s, pr.stride);
             launches++;
         }
         if (p->nsnap > 0 && it % d.jsnap == 0) {
