@@ -81,6 +81,38 @@ void undamped_range(const std::vector<float> &w, int &lo, int &hi);
 void launch_stepB(int ndim, int nop, bool exact, bool rho, const float *cur, float *nxt, const float *vel,
                   const float *den, const StepBParams &p, cudaStream_t s);
 
+// ---- several 2D steps in one launch (k_tb2d.cu) ----
+constexpr int kTb2Threads = 512;
+constexpr size_t kTb2SmemMax = 200 * 1024;
+// tile of tz x tx cells, k steps a launch, region of the tile and its halos
+// (rz x rx; hz >= nop k a multiple of 4, hx = nop k), cx columns a thread
+struct Tb2Shape {
+    int k, tz, tx, hz, hx, rz, rx, ntz, ntx, cx;
+};
+struct Tb2Params {
+    int n1, n2, k, it;
+    int tz, tx, hz, hx, rz, rx;
+    float c0, cz[5], cx[5];
+    const float *cur, *prv, *vel;  // levels it, it - 1; v^2 dt^2
+    float *ocur, *oprv;            // levels it + k, it + k - 1 (other buffers; null: not stored)
+    float *slots;                  // every new level j at slots + j * slot_stride (null: none)
+    long long slot_stride;
+    const float *w1, *w2;            // sponge factors (null: no sponge)
+    int ilo1, ihi1, ilo2, ihi2;      // every factor in the range is 1
+    // per tile: source cells of its region (z, x, first and last entry) with
+    // their entries (source * 8 + corner, weight bits), and the receivers of its
+    // cells (z, x, receiver) with their weights; the longest lists of a tile
+    const int *inj_start, *ent_start, *rec_start;
+    const int4 *inj_cell, *rec_pt;
+    const int2 *inj_ent;
+    const float *rec_wt;
+    int max_rec, max_cell, max_ent;
+    const float *wav;
+    int ncs, jdata, nr;
+    float *dat;
+};
+void launch_tb2(int nop, bool exact, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s);
+
 struct AbcB {
     const float *zl, *zh;  // [n3][n2]
     const float *xl, *xh;  // [n3][n1]

@@ -1,0 +1,329 @@
+// Several 2D time steps of the CPU-program scheme in one launch (temporal
+// blocking over overlapping tiles).
+//
+// A single shot's levels (592 x 592 cells: 1.4 MB each) live in L2, and a step
+// of its own is launch and latency: 4.35 us for 0.5 us of work.  Here a block
+// loads its tile of both levels and of v^2 dt^2 with a halo of k * nop cells
+// once, steps k times in shared memory, and stores the tile of the last two
+// levels; halo cells are computed by every tile that needs them.  A thread owns
+// 4 (axis 1) x 1, 2 or 4 (axis 2) cells: their two levels and v^2 dt^2 stay in
+// registers, the current level also in one of two shared-memory buffers that
+// the neighbours read.  Sources, the receivers of every step's level and the
+// sponge are inside.  The operations of a cell are k_stepB's in the same order
+// (with the products that its compiled form fuses), so the result is the same
+// bits.  Measured, us a step, one-step kernel and this one (replayed graphs):
+// 592 x 592 8th order 4.35, 1.91; 141 x 183 4th order 2.45, 0.79; 1480 x 1480
+// 8th order 16.4, 8.6.  What bounds it now is the latency of a step in one
+// block per SM (0.4 of the issue slots), then shared-memory reads.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "awe_internal.h"
+#include "fp_exact.cuh"
+
+namespace awe {
+
+namespace {
+
+template <int NOP, bool EXACT, int CX>
+__global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
+    extern __shared__ float smem[];
+    const int zt = p.rz / 4, rz = p.rz, tid = threadIdx.x;
+    const int xg = tid / zt, zs = tid - xg * zt;
+    // four columns of padding on either side: outer halo strips read past the region
+    const int plane = (p.rx + 8) * rz;
+    float *S0 = smem + 4 * rz, *S1 = S0 + plane;
+    const int tz0 = blockIdx.x * p.tz, tx0 = blockIdx.y * p.tx;
+    const int z0 = tz0 - p.hz + 4 * zs, x0 = tx0 - p.hx + CX * xg;  // the thread's first cell
+    const int n1 = p.n1, n2 = p.n2;
+    const int own = CX * xg * rz + 4 * zs;
+    const bool vec = (n1 & 3) == 0;
+
+    // cells outside the grid take the nearest one's values: nothing a step keeps depends on them
+    const int zc[4] = {min(max(z0, 0), vec ? n1 - 4 : n1 - 1), min(max(z0 + 1, 0), n1 - 1), min(max(z0 + 2, 0), n1 - 1),
+                       min(max(z0 + 3, 0), n1 - 1)};
+    auto load = [&](const float *src, int c) {
+        const float *q = src + (long long)min(max(x0 + c, 0), n2 - 1) * n1;
+        return vec ? *reinterpret_cast<const float4 *>(q + zc[0]) : make_float4(q[zc[0]], q[zc[1]], q[zc[2]], q[zc[3]]);
+    };
+    float4 cur[CX], prv[CX], vel[CX];
+    float wz[4], wx[CX];
+    // what no step writes, before the wait for the previous launch
+#pragma unroll
+    for (int c = 0; c < CX; c++) {
+        vel[c] = load(p.vel, c);
+        wx[c] = p.w2 ? __ldg(p.w2 + min(max(x0 + c, 0), n2 - 1)) : 1.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) wz[i] = p.w1 ? __ldg(p.w1 + min(max(z0 + i, 0), n1 - 1)) : 1.f;
+    // The tile's receivers and sources, with the wavelet samples of the launch's
+    // steps, go to shared memory here: read from global memory in every step,
+    // the chain of their loads made the tiles that hold them twice as slow.
+    const int tile = blockIdx.y * gridDim.x + blockIdx.x;
+    const int nrec = p.rec_start ? p.rec_start[tile + 1] - p.rec_start[tile] : 0;
+    const int ncell = p.inj_start ? p.inj_start[tile + 1] - p.inj_start[tile] : 0;
+    float4 *rec_w = reinterpret_cast<float4 *>(smem + 2 * plane), *rec_d = rec_w + p.max_rec;
+    int4 *cells = reinterpret_cast<int4 *>(rec_d + p.max_rec);  // cell, first and last entry, v^2 dt^2
+    int2 *rec_l = reinterpret_cast<int2 *>(cells + p.max_cell);  // cell, receiver
+    float *ent_w = reinterpret_cast<float *>(rec_l + p.max_rec), *ent_d = ent_w + p.max_ent;
+    for (int r = tid; r < nrec; r += blockDim.x) {
+        const int4 q = p.rec_pt[p.rec_start[tile] + r];  // z, x, receiver
+        rec_l[r] = make_int2((q.y - tx0 + p.hx) * rz + q.x - tz0 + p.hz, q.z);
+        rec_w[r] = *reinterpret_cast<const float4 *>(p.rec_wt + 4 * (p.rec_start[tile] + r));
+        if (p.w1) rec_d[r] = make_float4(p.w1[q.x], p.w1[q.x + 1], p.w2[q.y], p.w2[q.y + 1]);
+    }
+    if (ncell > 0) {
+        const int e0 = p.ent_start[tile], nent = p.ent_start[tile + 1] - e0;
+        for (int s = tid; s < ncell; s += blockDim.x) {
+            const int4 q = p.inj_cell[p.inj_start[tile] + s];  // z, x, first and last entry
+            cells[s] = make_int4((q.y - tx0 + p.hx) * rz + q.x - tz0 + p.hz, q.z - e0, q.w - e0,
+                                 __float_as_int(p.vel[(long long)q.y * n1 + q.x]));
+        }
+        for (int e = tid; e < nent; e += blockDim.x) {
+            const int2 en = p.inj_ent[e0 + e];
+            ent_w[e] = __int_as_float(en.y);
+            for (int j = 0; j < p.k; j++)
+                ent_d[j * p.max_ent + e] = p.wav[(long long)(p.it + j) * p.ncs + (p.ncs == 1 ? 0 : en.x >> 3)];
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+#pragma unroll
+    for (int c = 0; c < CX; c++) {
+        cur[c] = load(p.cur, c);
+        prv[c] = load(p.prv, c);
+        *reinterpret_cast<float4 *>(S0 + own + c * rz) = cur[c];
+    }
+    __syncthreads();
+
+    const int tz1 = min(tz0 + p.tz, n1), tx1 = min(tx0 + p.tx, n2);
+    // uniform: every cell the steps compute is interior / keeps its value under the sponge
+    const int e0 = NOP * (p.k - 1);
+    const bool inner = tz0 - e0 - 3 >= NOP && tz1 + e0 + 3 <= n1 - NOP && tx0 - e0 - 3 >= NOP && tx1 + e0 + 3 <= n2 - NOP;
+    const bool damp = p.w1 && !(tz0 - e0 >= p.ilo1 && tz1 + e0 <= p.ihi1 && tx0 - e0 >= p.ilo2 && tx1 + e0 <= p.ihi2);
+
+    // the thread's cells are within `need` of the tile: computed while the later
+    // steps of the launch still need them
+    int need = max(max(max(tz0 - (z0 + 3), z0 - (tz1 - 1)), max(tx0 - (x0 + CX - 1), x0 - (tx1 - 1))), 0);
+    if (z0 + 3 < 0 || z0 >= n1 || x0 + CX - 1 < 0 || x0 >= n2) need = 1 << 30;
+    // GEN: cells that are not interior, or change under the sponge (a factor of 1 changes nothing)
+    auto steps = [&](auto gen_) {
+        constexpr bool GEN = decltype(gen_)::value;
+        for (int j = 0; j < p.k; j++) {
+            const int it = p.it + j;
+            if (need <= NOP * (p.k - 1 - j)) {
+                float4 W[CX + 2 * NOP];  // columns x0 - NOP .. x0 + CX - 1 + NOP of the strip
+#pragma unroll
+                for (int k = 0; k < CX + 2 * NOP; k++)
+                    W[k] = k >= NOP && k < NOP + CX ? cur[k - NOP < CX ? k - NOP : 0]
+                                                    : *reinterpret_cast<const float4 *>(S0 + own + (k - NOP) * rz);
+#pragma unroll
+                for (int c = 0; c < CX; c++) {
+                    const float4 a = *reinterpret_cast<const float4 *>(S0 + own + c * rz - 4);
+                    const float4 b = *reinterpret_cast<const float4 *>(S0 + own + c * rz + 4);
+                    const float4 m = W[NOP + c];
+                    const float zw[12] = {a.x, a.y, a.z, a.w, m.x, m.y, m.z, m.w, b.x, b.y, b.z, b.w};
+                    float4 pr = prv[c], o;
+                    if (GEN) {
+                        pr.x = __fmul_rn(__fmul_rn(pr.x, wz[0]), wx[c]);
+                        pr.y = __fmul_rn(__fmul_rn(pr.y, wz[1]), wx[c]);
+                        pr.z = __fmul_rn(__fmul_rn(pr.z, wz[2]), wx[c]);
+                        pr.w = __fmul_rn(__fmul_rn(pr.w, wz[3]), wx[c]);
+                    }
+                    // ts_kernel.c:140-144: lap = u*c0 + sum_k [(z pair)*cz + (x pair)*cx]
+                    if constexpr (EXACT) {
+                        float *ov = &o.x;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            const float u = zw[4 + i];
+                            float lap = __fmul_rn(u, p.c0);
+#pragma unroll
+                            for (int k = 1; k <= NOP; k++) {
+                                const float zp = __fadd_rn(zw[4 + i - k], zw[4 + i + k]);
+                                const float xp = __fadd_rn((&W[NOP + c - k].x)[i], (&W[NOP + c + k].x)[i]);
+                                lap = __fadd_rn(lap, __fadd_rn(__fmul_rn(zp, p.cz[k]), __fmul_rn(xp, p.cx[k])));
+                            }
+                            ov[i] = sum3_rn(__fmul_rn((&vel[c].x)[i], lap), __fadd_rn(u, u), -(&pr.x)[i]);
+                        }
+                    } else {
+                        // two cells per instruction, with the products that k_stepB's compiled form fuses
+                        const float2 u0 = make_float2(m.x, m.y), u1 = make_float2(m.z, m.w);
+                        float2 l0, l1;
+#pragma unroll
+                        for (int k = 1; k <= NOP; k++) {
+                            const float4 xm = W[NOP + c - k], xp = W[NOP + c + k];
+                            const float2 cz = make_float2(p.cz[k], p.cz[k]), cx = make_float2(p.cx[k], p.cx[k]);
+                            float2 z0p, z1p;
+                            if (k % 2 == 0) {  // pairs aligned with the 16-byte loads
+                                z0p = __fadd2_rn(make_float2(zw[4 - k], zw[5 - k]), make_float2(zw[4 + k], zw[5 + k]));
+                                z1p = __fadd2_rn(make_float2(zw[6 - k], zw[7 - k]), make_float2(zw[6 + k], zw[7 + k]));
+                            } else {
+                                z0p = make_float2(__fadd_rn(zw[4 - k], zw[4 + k]), __fadd_rn(zw[5 - k], zw[5 + k]));
+                                z1p = make_float2(__fadd_rn(zw[6 - k], zw[6 + k]), __fadd_rn(zw[7 - k], zw[7 + k]));
+                            }
+                            const float2 x0p = __fadd2_rn(make_float2(xm.x, xm.y), make_float2(xp.x, xp.y));
+                            const float2 x1p = __fadd2_rn(make_float2(xm.z, xm.w), make_float2(xp.z, xp.w));
+                            const float2 t0 = __ffma2_rn(z0p, cz, __fmul2_rn(x0p, cx));
+                            const float2 t1 = __ffma2_rn(z1p, cz, __fmul2_rn(x1p, cx));
+                            const float2 c0 = make_float2(p.c0, p.c0);
+                            l0 = k == 1 ? __ffma2_rn(u0, c0, t0) : __fadd2_rn(l0, t0);
+                            l1 = k == 1 ? __ffma2_rn(u1, c0, t1) : __fadd2_rn(l1, t1);
+                        }
+                        const float2 m1 = make_float2(-1.f, -1.f);
+                        const float2 d0 = __ffma2_rn(make_float2(pr.x, pr.y), m1, __fadd2_rn(u0, u0));  // 2 u - pr
+                        const float2 d1 = __ffma2_rn(make_float2(pr.z, pr.w), m1, __fadd2_rn(u1, u1));
+                        const float2 o0 = __ffma2_rn(make_float2(vel[c].x, vel[c].y), l0, d0);
+                        const float2 o1 = __ffma2_rn(make_float2(vel[c].z, vel[c].w), l1, d1);
+                        o = make_float4(o0.x, o0.y, o1.x, o1.y);
+                    }
+                    if (GEN) {
+                        const bool xin = x0 + c >= NOP && x0 + c < n2 - NOP;
+                        if (!(xin && z0 >= NOP && z0 < n1 - NOP)) o.x = pr.x;
+                        if (!(xin && z0 + 1 >= NOP && z0 + 1 < n1 - NOP)) o.y = pr.y;
+                        if (!(xin && z0 + 2 >= NOP && z0 + 2 < n1 - NOP)) o.z = pr.z;
+                        if (!(xin && z0 + 3 >= NOP && z0 + 3 < n1 - NOP)) o.w = pr.w;
+                        o.x = __fmul_rn(__fmul_rn(o.x, wz[0]), wx[c]);
+                        o.y = __fmul_rn(__fmul_rn(o.y, wz[1]), wx[c]);
+                        o.z = __fmul_rn(__fmul_rn(o.z, wz[2]), wx[c]);
+                        o.w = __fmul_rn(__fmul_rn(o.w, wz[3]), wx[c]);
+                    }
+                    prv[c] = m;
+                    cur[c] = o;
+                    *reinterpret_cast<float4 *>(S1 + own + c * rz) = o;
+                }
+            }
+            // receivers of the level this step reads, pending sponge applied (lint2d_extract)
+            if (nrec > 0 && (p.jdata == 1 || it % p.jdata == 0)) {
+                float *row = p.dat + (long long)(it / p.jdata) * p.nr;
+                for (int r = tid; r < nrec; r += blockDim.x) {
+                    const int2 li = rec_l[r];
+                    const float4 w = rec_w[r], d = rec_d[r];
+                    float v0 = S0[li.x], v1 = S0[li.x + 1], v2 = S0[li.x + rz], v3 = S0[li.x + rz + 1];
+                    if (p.w1) {
+                        v0 = __fmul_rn(__fmul_rn(v0, d.x), d.z), v1 = __fmul_rn(__fmul_rn(v1, d.y), d.z);
+                        v2 = __fmul_rn(__fmul_rn(v2, d.x), d.w), v3 = __fmul_rn(__fmul_rn(v3, d.y), d.w);
+                    }
+                    float acc = __fmul_rn(v0, w.x);
+                    if constexpr (EXACT) {
+                        acc = __fadd_rn(acc, __fmul_rn(v1, w.y));
+                        acc = __fadd_rn(acc, __fmul_rn(v2, w.z));
+                        acc = __fadd_rn(acc, __fmul_rn(v3, w.w));
+                    } else {
+                        acc = fmaf(v3, w.w, fmaf(v2, w.z, fmaf(v1, w.y, acc)));
+                    }
+                    row[li.y] = acc;
+                }
+            }
+            __syncthreads();
+            if (ncell > 0) {  // sources on the new level, one thread per cell, in (source, corner) order
+                const float *dd = ent_d + j * p.max_ent;
+                for (int s = tid; s < ncell; s += blockDim.x) {
+                    const int4 q = cells[s];
+                    const float vn = __int_as_float(q.w);
+                    float v = S1[q.x];
+#pragma unroll 1
+                    for (int e = q.y; e < q.z; e++) {
+                        const float a = __fmul_rn(dd[e], ent_w[e]);
+                        v = EXACT ? __fadd_rn(v, __fmul_rn(a, vn)) : fmaf(a, vn, v);
+                    }
+                    S1[q.x] = v;
+                }
+                __syncthreads();
+#pragma unroll
+                for (int c = 0; c < CX; c++) cur[c] = *reinterpret_cast<const float4 *>(S1 + own + c * rz);
+            }
+            float *t = S0;
+            S0 = S1;
+            S1 = t;
+            if (p.slots) {  // every new level (the gradient's recompute)
+                float *dst = p.slots + (long long)j * p.slot_stride;
+                if (z0 >= tz0 && z0 < tz1 && x0 + CX - 1 >= tx0 && x0 < tx1)
+#pragma unroll
+                    for (int c = 0; c < CX; c++) {
+                        const int x = x0 + c;
+                        if (x < tx0 || x >= tx1) continue;
+                        const float4 v = *reinterpret_cast<const float4 *>(S0 + own + c * rz);
+                        float *d = dst + (long long)x * n1 + z0;
+                        if (vec) {
+                            *reinterpret_cast<float4 *>(d) = v;
+                        } else {
+                            const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                            for (int i = 0; i < 4; i++)
+                                if (z0 + i < tz1) d[i] = e[i];
+                        }
+                    }
+            }
+        }
+    };
+    if (inner && !damp) steps(std::false_type());
+    else steps(std::true_type());
+    if (!p.ocur) return;
+    // the tile's cells of the last two levels (tz and hz are multiples of 4, so strips do not straddle its low edge)
+    if (z0 >= tz0 && z0 < tz1)
+#pragma unroll
+        for (int c = 0; c < CX; c++) {
+            const int x = x0 + c;
+            if (x < tx0 || x >= tx1) continue;
+            const float4 a = *reinterpret_cast<const float4 *>(S0 + own + c * rz);
+            const float4 b = *reinterpret_cast<const float4 *>(S1 + own + c * rz);
+            const long long i = (long long)x * n1 + z0;
+            if (vec) {
+                *reinterpret_cast<float4 *>(p.ocur + i) = a;
+                *reinterpret_cast<float4 *>(p.oprv + i) = b;
+            } else {
+                const float va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (z0 + q < tz1) {
+                        p.ocur[i + q] = va[q];
+                        p.oprv[i + q] = vb[q];
+                    }
+            }
+        }
+}
+
+template <int NOP, bool EXACT, int CX>
+static void launch_cx(const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sh.ntz, sh.ntx);
+    cfg.blockDim = dim3((sh.rz / 4) * (sh.rx / CX));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaFuncSetAttribute(k_tb2<NOP, EXACT, CX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTb2SmemMax);
+    cudaLaunchKernelEx(&cfg, k_tb2<NOP, EXACT, CX>, p);
+}
+
+template <int NOP>
+static void launch_nop(bool exact, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
+    if (sh.cx == 1) {
+        if (exact) launch_cx<NOP, true, 1>(p, sh, smem, s);
+        else launch_cx<NOP, false, 1>(p, sh, smem, s);
+    } else if (sh.cx == 4) {
+        if (exact) launch_cx<NOP, true, 4>(p, sh, smem, s);
+        else launch_cx<NOP, false, 4>(p, sh, smem, s);
+    } else {
+        if (exact) launch_cx<NOP, true, 2>(p, sh, smem, s);
+        else launch_cx<NOP, false, 2>(p, sh, smem, s);
+    }
+}
+
+}  // namespace
+
+void launch_tb2(int nop, bool exact, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
+    switch (nop) {
+        case 1: launch_nop<1>(exact, p, sh, smem, s); break;
+        case 2: launch_nop<2>(exact, p, sh, smem, s); break;
+        case 3: launch_nop<3>(exact, p, sh, smem, s); break;
+        default: launch_nop<4>(exact, p, sh, smem, s); break;
+    }
+}
+
+}  // namespace awe

@@ -568,7 +568,7 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
         AWE_TRY(ckpt_store(p, 2 * seg + 1, cur, ss));
         return AWE_OK;
     };
-    AWE_TRY(planB_run_hooked(p, d_wav, ncs, dat, nullptr, s, &hook));
+    AWE_TRY(planB_run_hooked(p, d_wav, ncs, dat, nullptr, s, &hook, T));
     launches += p->launches;
 
     // 2. residual and misfit (FP64 per row, summed in row order on the host);

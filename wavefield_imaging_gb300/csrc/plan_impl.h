@@ -68,6 +68,16 @@ struct awe_plan {
     bool inj_fused = false;            // the step adds the injection itself (StepA2Fused, StepA3Fused)
     int snap_transpose = 0;            // polar snapshots are theta-fastest
 
+    // 2D CPU-program scheme: several steps a launch (k_tb2d.cu)
+    bool tb2 = false;        // the plan's kind allows it
+    bool tb2_geom = false;   // and so do its points
+    awe::Tb2Shape tb2_shape{};
+    float *tb2_u = nullptr;  // two more levels (the launch is out of place)
+    int *tb2_lists = nullptr;  // per tile lists (set_tb2_lists)
+    size_t tb2_cap = 0;
+    size_t tb2_off[7] = {0, 0, 0, 0, 0, 0, 0};  // of Tb2Params' lists, in their order
+    int tb2_max[3] = {0, 0, 0};                   // max_rec, max_cell, max_ent
+
     bool model_set = false, geom_set = false;
     awe_snap_fn snap_cb = nullptr;
     void *snap_user = nullptr;
@@ -163,8 +173,14 @@ awe_status planB_run(awe_plan *p, const float *d_wav, int ncs, float *d_dat, flo
 // called at the start of step it with the two levels (prev = V_{it-1} with its
 // second sponge pending, cur = V_it)
 typedef std::function<awe_status(int it, const float *prev, const float *cur, cudaStream_t s)> StepHook;
+// hook_every: the hook does nothing but at multiples of it
 awe_status planB_run_hooked(awe_plan *p, const float *d_wav, int ncs, float *d_dat, float *d_wfl, cudaStream_t s,
-                            const StepHook *hook);
+                            const StepHook *hook, int hook_every = 1);
+// tile lists of the points for k_tb2d.cu; sets p->tb2_geom
+awe_status set_tb2_lists(awe_plan *p);
+// steps it .. it + k - 1 from levels prv, cur
+void tb2_launch(awe_plan *p, const float *prv, const float *cur, float *oprv, float *ocur, float *slots,
+                long long slot_stride, int it, int k, const float *d_wav, int ncs, float *d_dat, cudaStream_t s);
 StepBParams stepB_params(const awe_plan *p);
 // lap_out: the TMA path also stores L(cur) of interior cells there (gradient recompute)
 // ext_*: 2D, the receivers of `cur` (pending sponge applied) gathered into

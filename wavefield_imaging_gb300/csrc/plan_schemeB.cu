@@ -36,6 +36,183 @@ static awe_status upload(awe_plan *p, float **dst, const float *src, size_t n) {
     return AWE_OK;
 }
 
+// Tile, steps per launch and columns per thread of k_tb2d.cu.  A launch costs
+// about 1.5 us besides its steps, a step 0.35 us (barrier, load and arithmetic
+// latency of a few warps) and 0.15 ns per cell of the region; a tile occupies
+// an SM (512 threads of 4 x cx cells).  Fitted to 141 x 183 (4th order) to 1480
+// x 1480 (8th order) cells, where the best of 17 shapes took 0.79 to 8.6 us a
+// step and the one-step kernel 2.45 to 16.4.
+static Tb2Shape tb2_shape(const Grid &g, int nop, int sms) {
+    Tb2Shape best{};
+    double cost = 1e30;
+    for (int tz0 = 8; tz0 <= 104; tz0 += 4)
+        for (int tx0 = 8; tx0 <= 104; tx0 += 4)
+            for (int k = 1; k <= 12; k++) {
+                Tb2Shape s{};
+                s.k = k;
+                s.ntz = (g.n1 + tz0 - 1) / tz0;
+                s.ntx = (g.n2 + tx0 - 1) / tx0;
+                s.tz = ((g.n1 + s.ntz - 1) / s.ntz + 3) / 4 * 4;  // even tiles
+                s.tx = (g.n2 + s.ntx - 1) / s.ntx;
+                s.hx = nop * k;
+                s.hz = (s.hx + 3) / 4 * 4;
+                s.rz = s.tz + 2 * s.hz;
+                s.rx = (s.tx + 2 * s.hx + 3) / 4 * 4;
+                for (s.cx = 1; s.cx <= 4 && (s.rz / 4) * (s.rx / s.cx) > kTb2Threads;) s.cx *= 2;
+                if (s.cx > 4) break;
+                const long long rounds = ((long long)s.ntz * s.ntx + sms - 1) / sms;
+                const double c = rounds * (1.5 / k + 0.35 + 1.5e-4 * s.rz * s.rx);
+                if (c < cost) {
+                    cost = c;
+                    best = s;
+                }
+            }
+    best.ntz = (g.n1 + best.tz - 1) / best.tz;
+    best.ntx = (g.n2 + best.tx - 1) / best.tx;
+    return best;
+}
+
+// two level buffers with their padding columns, and the longest lists of a tile
+static size_t tb2_smem(const awe_plan *p) {
+    const Tb2Shape &sh = p->tb2_shape;
+    const int *m = p->tb2_max;
+    return (size_t)2 * (sh.rx + 8) * sh.rz * 4 + (size_t)m[0] * 40 + (size_t)m[1] * 16 + (size_t)m[2] * 4 * (1 + sh.k);
+}
+
+awe_status set_tb2_lists(awe_plan *p) {
+    p->tb2_geom = false;
+    if (!p->tb2 || p->move_mode >= 0 || p->sponge_deferred) return AWE_OK;
+    const Grid &g = p->g;
+    const Tb2Shape &sh = p->tb2_shape;
+    const int ntile = sh.ntz * sh.ntx;
+    struct Cell {
+        int tile;
+        int4 q;
+    };
+    // receivers by the tile of their base cell (all four corners are in its region)
+    std::vector<Cell> rec;
+    for (int r = 0; r < (int)p->h_rec.size(); r++) {
+        const int z = (int)(p->h_rec[r].base % g.n1), x = (int)(p->h_rec[r].base / g.n1);
+        if (z >= g.n1 - 1 || x >= g.n2 - 1) return AWE_OK;
+        rec.push_back({(x / sh.tx) * sh.ntz + z / sh.tz, make_int4(z, x, r, 0)});
+    }
+    // source cells, each with its entries in (source, corner) order, in every
+    // tile whose region holds the cell
+    std::vector<std::pair<long long, int>> e;
+    for (int s = 0; s < (int)p->h_src.size(); s++)
+        for (int c = 0; c < 4; c++) {
+            const long long n = p->h_src[s].base + p->h_corner_off[c];
+            if (n >= g.cells()) return AWE_OK;
+            e.push_back({n, 8 * s + c});
+        }
+    std::sort(e.begin(), e.end());
+    std::vector<Cell> cell;
+    for (size_t k = 0, k1; k < e.size(); k = k1) {
+        for (k1 = k; k1 < e.size() && e[k1].first == e[k].first;) k1++;
+        const int z = (int)(e[k].first % g.n1), x = (int)(e[k].first / g.n1);
+        for (int bx = std::max(0, (x - sh.hx) / sh.tx - 1); bx < sh.ntx && bx * sh.tx - sh.hx <= x; bx++)
+            for (int bz = std::max(0, (z - sh.hz) / sh.tz - 1); bz < sh.ntz && bz * sh.tz - sh.hz <= z; bz++)
+                if (x < bx * sh.tx - sh.hx + sh.rx && z < bz * sh.tz - sh.hz + sh.rz)
+                    cell.push_back({bx * sh.ntz + bz, make_int4(z, x, (int)k, (int)k1)});
+    }
+    auto by_tile = [](const Cell &a, const Cell &b) { return a.tile < b.tile; };
+    std::stable_sort(rec.begin(), rec.end(), by_tile);
+    std::stable_sort(cell.begin(), cell.end(), by_tile);
+    std::vector<int> start[3];  // cells, entries, receivers
+    for (auto &v : start) v.assign(ntile + 1, 0);
+    std::vector<int2> ent;
+    for (Cell &c : cell) {
+        const int k0 = c.q.z, k1 = c.q.w;
+        c.q.z = (int)ent.size();
+        for (int k = k0; k < k1; k++) {
+            int w;
+            std::memcpy(&w, &p->h_src[e[k].second >> 3].w[e[k].second & 7], sizeof w);
+            ent.push_back(make_int2(e[k].second, w));
+        }
+        c.q.w = (int)ent.size();
+        start[0][c.tile + 1]++;
+        start[1][c.tile + 1] += k1 - k0;
+    }
+    for (const Cell &c : rec) start[2][c.tile + 1]++;
+    int most[3] = {0, 0, 0};
+    for (int k = 0; k < 3; k++)
+        for (int t = 0; t < ntile; t++) {
+            most[k] = std::max(most[k], start[k][t + 1]);
+            start[k][t + 1] += start[k][t];
+        }
+    p->tb2_max[0] = most[2];
+    p->tb2_max[1] = most[0];
+    p->tb2_max[2] = most[1];
+    if (tb2_smem(p) > kTb2SmemMax) return AWE_OK;  // the points of one tile do not fit beside its levels
+    // one buffer and one copy; sized for source corners in four tiles each, so
+    // that points that only move keep it (a captured time loop reads it)
+    const size_t nst = (size_t)(ntile + 4) / 4 * 4 + 4, ns = p->h_src.size(), nr = p->h_rec.size();
+    const size_t ncell = std::max(cell.size(), 16 * ns), nent = std::max(ent.size() + 1, 16 * ns + 1) / 2 * 2;
+    size_t *off = p->tb2_off;
+    off[0] = 0;
+    off[1] = off[0] + nst;
+    off[2] = off[1] + nst;
+    off[3] = off[2] + nst;          // inj_cell
+    off[4] = off[3] + 4 * ncell;    // rec_pt
+    off[5] = off[4] + 4 * nr;       // inj_ent
+    off[6] = off[5] + 2 * nent;     // rec_wt
+    const size_t total = off[6] + 4 * nr;
+    std::vector<int> buf(total, 0);
+    for (int k = 0; k < 3; k++) std::copy(start[k].begin(), start[k].end(), buf.begin() + off[k]);
+    for (size_t k = 0; k < cell.size(); k++) std::memcpy(&buf[off[3] + 4 * k], &cell[k].q, sizeof(int4));
+    if (!ent.empty()) std::memcpy(&buf[off[5]], ent.data(), ent.size() * sizeof(int2));
+    for (size_t k = 0; k < rec.size(); k++) {
+        std::memcpy(&buf[off[4] + 4 * k], &rec[k].q, sizeof(int4));
+        std::memcpy(&buf[off[6] + 4 * k], p->h_rec[rec[k].q.z].w, 4 * sizeof(float));
+    }
+    if (p->tb2_cap < total) {
+        dev_free(p, p->tb2_lists);
+        p->tb2_lists = nullptr;
+        p->tb2_cap = 0;
+        AWE_TRY(dev_alloc(p, (void **)&p->tb2_lists, total * sizeof(int)));
+        p->tb2_cap = total;
+    }
+    CUDA_TRY(cudaMemcpy(p->tb2_lists, buf.data(), total * sizeof(int), cudaMemcpyHostToDevice));
+    p->tb2_geom = true;
+    return AWE_OK;
+}
+
+void tb2_launch(awe_plan *p, const float *prv, const float *cur, float *oprv, float *ocur, float *slots,
+                long long slot_stride, int it, int k, const float *d_wav, int ncs, float *d_dat, cudaStream_t s) {
+    const awe_desc &d = p->d;
+    const Tb2Shape &sh = p->tb2_shape;
+    const bool sponge = d.dabc && !d.hybrid;
+    Tb2Params q{};
+    q.n1 = p->g.n1;
+    q.n2 = p->g.n2;
+    q.k = k;
+    q.it = it;
+    q.tz = sh.tz, q.tx = sh.tx, q.hz = sh.hz, q.hx = sh.hx, q.rz = sh.rz, q.rx = sh.rx;
+    q.c0 = p->k.c0;
+    for (int i = 0; i <= p->nop; i++) q.cz[i] = p->k.c[0][i], q.cx[i] = p->k.c[1][i];
+    q.cur = cur, q.prv = prv, q.vel = p->vel, q.ocur = ocur, q.oprv = oprv;
+    q.slots = slots;
+    q.slot_stride = slot_stride;
+    if (sponge) q.w1 = p->w[0], q.w2 = p->w[1];
+    q.ilo1 = p->wlo[0], q.ihi1 = p->whi[0], q.ilo2 = p->wlo[1], q.ihi2 = p->whi[1];
+    const int *b = p->tb2_lists;
+    const size_t *off = p->tb2_off;
+    if (p->tb2_max[1] > 0) q.inj_start = b + off[0];
+    q.ent_start = b + off[1];
+    if (p->tb2_max[0] > 0 && d_dat) q.rec_start = b + off[2];
+    q.inj_cell = (const int4 *)(b + off[3]);
+    q.rec_pt = (const int4 *)(b + off[4]);
+    q.inj_ent = (const int2 *)(b + off[5]);
+    q.rec_wt = (const float *)(b + off[6]);
+    q.max_rec = p->tb2_max[0], q.max_cell = p->tb2_max[1], q.max_ent = p->tb2_max[2];
+    q.wav = d_wav;
+    q.ncs = ncs;
+    q.jdata = d.jdata;
+    q.nr = p->nr;
+    q.dat = d_dat;
+    launch_tb2(p->nop, d.precision == AWE_EXACT, q, sh, tb2_smem(p), s);
+}
+
 awe_status planB_init(awe_plan *p) {
     awe_desc &d = p->d;
     if (d.fdorder == 0) d.fdorder = 4;  // MAWEFDcart2Dcpu.c:126
@@ -95,6 +272,13 @@ awe_status planB_init(awe_plan *p) {
         if (stepB3_tma_maps(p->tmaps, p->u, p->vel, p->g)) p->use_tma = true;
         const char *spin = std::getenv("AWE_PIPELINE_SPIN_LIMIT");
         if (spin && *spin) p->spin_limit = std::atoll(spin);
+    }
+    if (d.ndim == 2 && !force_simple && p->nop <= 4 && !d.hybrid) {
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+        p->tb2_shape = tb2_shape(p->g, p->nop, sms > 0 ? sms : 1);
+        p->tb2 = true;
+        AWE_TRY(dev_alloc(p, (void **)&p->tb2_u, 2 * cells * sizeof(float)));
     }
     // line-end copies of the 3D boundary launch (made before any capture of
     // the time loop; AWE_BND_ENDS=0: the launch reads the level itself)
@@ -476,7 +660,7 @@ awe_status planB_run(awe_plan *p, const float *d_wav, int ncs, float *d_dat, flo
 }
 
 awe_status planB_run_hooked(awe_plan *p, const float *d_wav, int ncs, float *d_dat, float *d_wfl, cudaStream_t s,
-                            const StepHook *hook) {
+                            const StepHook *hook, int hook_every) {
     const awe_desc &d = p->d;
     const Grid &g = p->g;
     const bool exact = d.precision == AWE_EXACT;
@@ -515,6 +699,33 @@ awe_status planB_run_hooked(awe_plan *p, const float *d_wav, int ncs, float *d_d
     // 2D: the traces of step it (the level the step reads, pending sponge
     // applied, as the reference extracts after its swap) are gathered by the
     // step's own launch; 3D: by the step's boundary launch
+    if (p->tb2_geom && !p->den && !p->profile) {
+        // several steps a launch, stopping at steps whose levels the hook or a frame reads
+        float *alt_prv = p->tb2_u, *alt_cur = p->tb2_u + g.cells();
+        float *prv = nxt;
+        const bool frames = p->nsnap > 0 && (d_wfl || p->d_snap_tmp);
+        for (int it = 0; it < d.nt;) {
+            if (hook && it % hook_every == 0) AWE_TRY((*hook)(it, prv, cur, s));
+            if (frames && it % d.jsnap == 0) {
+                float *frame = d_wfl ? d_wfl + (size_t)isnap * p->snap_elems : p->d_snap_tmp;
+                launch_snapshot(2, cur, frame, g, p->snap_f[0], p->snap_f[1], p->snap_f[2], p->snap_m[0], p->snap_m[1],
+                                p->snap_m[2], pw1, p->w[1], p->w[2], s);
+                launches++;
+                AWE_TRY(deliver_snapshot(p, frame, isnap, it, s));
+                isnap++;
+            }
+            int k = std::min(p->tb2_shape.k, d.nt - it);
+            if (hook) k = std::min(k, hook_every - it % hook_every);
+            if (frames) k = std::min(k, d.jsnap - it % d.jsnap);
+            tb2_launch(p, prv, cur, alt_prv, alt_cur, nullptr, 0, it, k, d_wav, ncs, d_dat, s);
+            launches++;
+            std::swap(prv, alt_prv);
+            std::swap(cur, alt_cur);
+            it += k;
+        }
+        p->launches = launches;
+        return flush_snapshots(p);
+    }
     const bool fuse_rec = (d.ndim == 2 || stepB3_bnd(p)) && p->nr > 0;
     for (int it = 0; it < d.nt; it++) {
         if (hook) AWE_TRY((*hook)(it, nxt, cur, s));
