@@ -48,3 +48,38 @@ def test_fast_equals_the_one_step_kernel(n, nb, order, nt, ns, nr, kw, monkeypat
     np.testing.assert_array_equal(dat, ref)
     if par.get("jsnap"):
         np.testing.assert_array_equal(snaps, rsn)
+
+
+@pytest.mark.parametrize("n,nb,order,nt,ns,nr,kw", [
+    ((30, 41), 7, 8, 61, 3, 40, dict(fsrf=1)), ((50, 37), 10, 4, 62, 9, 700, dict(jdata=2)),
+    ((101, 64), 9, 2, 63, 2, 30, {}), ((150, 170), 10, 8, 45, 1, 60, {}), ((64, 250), 11, 6, 50, 2, 0, {})])
+def test_gradient_and_image_equal_the_one_step_kernels(n, nb, order, nt, ns, nr, kw, monkeypatch):
+    """The gradient's recompute and adjoint sweep several steps a launch, the
+    imaging condition once per segment: the same bits as one step a launch,
+    for one segment, segments of one step, and segments that end inside a launch."""
+    import wavefield_imaging_gb300 as awe
+    from helpers import desc_from_par
+
+    par, vel, wav, sou, rec = _case(n, nb, order, nt, ns, nr, n[1], **kw)
+    rng = np.random.default_rng(1)
+    dobs = rng.standard_normal(((nt - 1) // par.get("jdata", 1) + 1, nr)).astype(np.float32)
+
+    def run():
+        out = []
+        with awe.Plan(desc_from_par(par)) as p:
+            p.set_model(vel)
+            p.set_geometry(sou, rec)
+            for every in (0, 1, 1000):
+                g, J = p.gradient(wav, dobs, ckpt_every=every)
+                out += [g, np.float64(J)]
+            out.append(p.rtm(wav, dobs, awe.IMAGE_XCORR))
+            out.append(p.rtm(wav, dobs, awe.IMAGE_BORN))
+            p.profile(True)  # profiled runs go one step a launch: the lists of both forms
+            out.append(p.gradient(wav, dobs)[0])
+        return out
+
+    ours = run()
+    monkeypatch.setenv("AWE_STEP_KERNEL", "simple")
+    for a, b in zip(ours, run()):
+        np.testing.assert_array_equal(a, b)
+    assert nr == 0 or np.abs(ours[0]).max() > 0

@@ -95,8 +95,11 @@ struct Tb2Params {
     float c0, cz[5], cx[5];
     const float *cur, *prv, *vel;  // levels it, it - 1; v^2 dt^2
     float *ocur, *oprv;            // levels it + k, it + k - 1 (other buffers; null: not stored)
-    float *slots;                  // every new level j at slots + j * slot_stride (null: none)
+    // stored by step j at slots + j * slot_stride (null: nothing): L of the level
+    // it reads, or (slot_level) that level; the adjoint step nu_k
+    float *slots;
     long long slot_stride;
+    int slot_level;
     const float *w1, *w2;            // sponge factors (null: no sponge)
     int ilo1, ihi1, ilo2, ihi2;      // every factor in the range is 1
     // per tile: source cells of its region (z, x, first and last entry) with
@@ -111,7 +114,8 @@ struct Tb2Params {
     int ncs, jdata, nr;
     float *dat;
 };
-void launch_tb2(int nop, bool exact, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s);
+// mode 0: AWE_FAST, 1: AWE_EXACT, 2: the adjoint step, 3: AWE_FAST with slots
+void launch_tb2(int nop, int mode, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s);
 
 struct AbcB {
     const float *zl, *zh;  // [n3][n2]
@@ -305,6 +309,8 @@ struct AdjParams {
 };
 void launch_adjB(const float *X, float *Y, const float *V, const float *vel, float2 *G, const AdjParams &p,
                  cudaStream_t s);
+void launch_tb2_image(float2 *G, const float *lap, const float *nu, long long stride, const AdjParams &p, int k0,
+                      int k1, cudaStream_t s);
 void launch_abc_adjB(int nop, int fsrf, float *mu, float *kap, const AbcB &a, const Grid &g, cudaStream_t s);
 void launch_kap_fold(float *mu, float *kap, const AdjParams &p, cudaStream_t s);
 void launch_rec_adj(float *mu, const GeoPoint *pts, int nr, const float *r, const AdjParams &p, const long long *off,

@@ -22,13 +22,18 @@
 
 #include "awe_internal.h"
 #include "fp_exact.cuh"
+#include "gsum.cuh"
 
 namespace awe {
 
 namespace {
 
-template <int NOP, bool EXACT, int CX>
+// MODE 0: AWE_FAST, 1: AWE_EXACT, 3: AWE_FAST storing slots (the gradient's recompute),
+// 2 (ADJ): the adjoint step (k_adjB): cur = nu_k, prv = nu_{k+1}, shared memory holds
+// I vel2 nu; step j is time step it - j; the cells' entries are receiver residuals
+template <int NOP, int MODE, int CX>
 __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
+    constexpr bool EXACT = MODE == 1, ADJ = MODE == 2, SLOTS = MODE >= 2;
     extern __shared__ float smem[];
     const int zt = p.rz / 4, rz = p.rz, tid = threadIdx.x;
     const int xg = tid / zt, zs = tid - xg * zt;
@@ -37,7 +42,7 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
     float *S0 = smem + 4 * rz, *S1 = S0 + plane;
     const int tz0 = blockIdx.x * p.tz, tx0 = blockIdx.y * p.tx;
     const int z0 = tz0 - p.hz + 4 * zs, x0 = tx0 - p.hx + CX * xg;  // the thread's first cell
-    const int n1 = p.n1, n2 = p.n2;
+    const int n1 = p.n1, n2 = p.n2, tz1 = min(tz0 + p.tz, n1), tx1 = min(tx0 + p.tx, n2);
     const int own = CX * xg * rz + 4 * zs;
     const bool vec = (n1 & 3) == 0;
 
@@ -65,40 +70,79 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
     const int nrec = p.rec_start ? p.rec_start[tile + 1] - p.rec_start[tile] : 0;
     const int ncell = p.inj_start ? p.inj_start[tile + 1] - p.inj_start[tile] : 0;
     float4 *rec_w = reinterpret_cast<float4 *>(smem + 2 * plane), *rec_d = rec_w + p.max_rec;
-    int4 *cells = reinterpret_cast<int4 *>(rec_d + p.max_rec);  // cell, first and last entry, v^2 dt^2
+    int4 *cells = reinterpret_cast<int4 *>(rec_d + p.max_rec);  // cell, first and last entry, v^2 dt^2 (ADJ: sponge)
     int2 *rec_l = reinterpret_cast<int2 *>(cells + p.max_cell);  // cell, receiver
-    float *ent_w = reinterpret_cast<float *>(rec_l + p.max_rec), *ent_d = ent_w + p.max_ent;
+    int *mine = reinterpret_cast<int *>(rec_l + p.max_rec);      // per thread: first cell * 65536 + cells
+    float *ent_w = reinterpret_cast<float *>(mine + kTb2Threads), *ent_d = ent_w + p.max_ent;
     for (int r = tid; r < nrec; r += blockDim.x) {
         const int4 q = p.rec_pt[p.rec_start[tile] + r];  // z, x, receiver
         rec_l[r] = make_int2((q.y - tx0 + p.hx) * rz + q.x - tz0 + p.hz, q.z);
         rec_w[r] = *reinterpret_cast<const float4 *>(p.rec_wt + 4 * (p.rec_start[tile] + r));
         if (p.w1) rec_d[r] = make_float4(p.w1[q.x], p.w1[q.x + 1], p.w2[q.y], p.w2[q.y + 1]);
     }
+    if (ADJ) mine[tid] = 0;
     if (ncell > 0) {
-        const int e0 = p.ent_start[tile], nent = p.ent_start[tile + 1] - e0;
+        const int i0 = p.inj_start[tile], e0 = p.ent_start[tile], nent = p.ent_start[tile + 1] - e0;
+        if (ADJ) __syncthreads();
+        auto owner = [&](const int4 &q) { return (q.y - tx0 + p.hx) / CX * zt + (q.x - tz0 + p.hz) / 4; };
         for (int s = tid; s < ncell; s += blockDim.x) {
-            const int4 q = p.inj_cell[p.inj_start[tile] + s];  // z, x, first and last entry
-            cells[s] = make_int4((q.y - tx0 + p.hx) * rz + q.x - tz0 + p.hz, q.z - e0, q.w - e0,
-                                 __float_as_int(p.vel[(long long)q.y * n1 + q.x]));
+            const int4 q = p.inj_cell[i0 + s];  // z, x, first and last entry, a thread's cells one after the other
+            float f = ADJ ? 1.f : p.vel[(long long)q.y * n1 + q.x];
+            if (ADJ && p.w1) f = __fmul_rn(p.w1[q.x], p.w2[q.y]);
+            cells[s] = make_int4((q.y - tx0 + p.hx) * rz + q.x - tz0 + p.hz, q.z - e0, q.w - e0, __float_as_int(f));
+            const int o = owner(q);
+            if (ADJ && (s == 0 || owner(p.inj_cell[i0 + s - 1]) != o)) {
+                int n = 1;
+                while (s + n < ncell && owner(p.inj_cell[i0 + s + n]) == o) n++;
+                mine[o] = s * 65536 + n;
+            }
         }
         for (int e = tid; e < nent; e += blockDim.x) {
             const int2 en = p.inj_ent[e0 + e];
             ent_w[e] = __int_as_float(en.y);
-            for (int j = 0; j < p.k; j++)
-                ent_d[j * p.max_ent + e] = p.wav[(long long)(p.it + j) * p.ncs + (p.ncs == 1 ? 0 : en.x >> 3)];
+            for (int j = 0; j < p.k; j++) {
+                const int it = ADJ ? p.it - j : p.it + j;
+                float d = 0.f;
+                if (!ADJ) d = p.wav[(long long)it * p.ncs + (p.ncs == 1 ? 0 : en.x >> 3)];
+                else if (it % p.jdata == 0) d = p.wav[(long long)(it / p.jdata) * p.ncs + (en.x >> 3)];
+                ent_d[j * p.max_ent + e] = d;
+            }
         }
     }
+    // I vel2 nu of a strip
+    auto weighted = [&](const float4 &v, int c) {
+        const bool xin = x0 + c >= NOP && x0 + c < n2 - NOP;
+        return make_float4(xin && z0 >= NOP && z0 < n1 - NOP ? __fmul_rn(vel[c].x, v.x) : 0.f,
+                           xin && z0 + 1 >= NOP && z0 + 1 < n1 - NOP ? __fmul_rn(vel[c].y, v.y) : 0.f,
+                           xin && z0 + 2 >= NOP && z0 + 2 < n1 - NOP ? __fmul_rn(vel[c].z, v.z) : 0.f,
+                           xin && z0 + 3 >= NOP && z0 + 3 < n1 - NOP ? __fmul_rn(vel[c].w, v.w) : 0.f);
+    };
+    // a strip of the tile to global memory
+    auto store = [&](float *dst, int c, const float4 &v) {
+        const int x = x0 + c;
+        if (z0 < tz0 || z0 >= tz1 || x < tx0 || x >= tx1) return;
+        float *d = dst + (long long)x * n1 + z0;
+        if (vec) {
+            *reinterpret_cast<float4 *>(d) = v;
+        } else {
+            d[0] = v.x;
+            if (z0 + 1 < tz1) d[1] = v.y;
+            if (z0 + 2 < tz1) d[2] = v.z;
+            if (z0 + 3 < tz1) d[3] = v.w;
+        }
+    };
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
 #pragma unroll
     for (int c = 0; c < CX; c++) {
         cur[c] = load(p.cur, c);
         prv[c] = load(p.prv, c);
-        *reinterpret_cast<float4 *>(S0 + own + c * rz) = cur[c];
+        *reinterpret_cast<float4 *>(S0 + own + c * rz) = ADJ ? weighted(cur[c], c) : cur[c];
     }
     __syncthreads();
+    // (ADJ) the thread's cells with entries
+    const int my0 = ADJ ? mine[tid] >> 16 : 0, my1 = ADJ ? my0 + (mine[tid] & 65535) : 0;
 
-    const int tz1 = min(tz0 + p.tz, n1), tx1 = min(tx0 + p.tx, n2);
     // uniform: every cell the steps compute is interior / keeps its value under the sponge
     const int e0 = NOP * (p.k - 1);
     const bool inner = tz0 - e0 - 3 >= NOP && tz1 + e0 + 3 <= n1 - NOP && tx0 - e0 - 3 >= NOP && tx1 + e0 + 3 <= n2 - NOP;
@@ -108,16 +152,31 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
     // steps of the launch still need them
     int need = max(max(max(tz0 - (z0 + 3), z0 - (tz1 - 1)), max(tx0 - (x0 + CX - 1), x0 - (tx1 - 1))), 0);
     if (z0 + 3 < 0 || z0 >= n1 || x0 + CX - 1 < 0 || x0 >= n2) need = 1 << 30;
+    // v with its cell's entries of step j added, in (point, corner) order
+    auto with_entries = [&](float v, const int4 &q, int j) {
+        const float f = __int_as_float(q.w), *dd = ent_d + j * p.max_ent;
+#pragma unroll 1
+        for (int e = q.y; e < q.z; e++) {
+            if constexpr (ADJ) {
+                v = __fadd_rn(v, __fmul_rn(f, __fmul_rn(f, __fmul_rn(ent_w[e], dd[e]))));
+            } else {
+                const float a = __fmul_rn(dd[e], ent_w[e]);
+                v = EXACT ? __fadd_rn(v, __fmul_rn(a, f)) : fmaf(a, f, v);
+            }
+        }
+        return v;
+    };
     // GEN: cells that are not interior, or change under the sponge (a factor of 1 changes nothing)
     auto steps = [&](auto gen_) {
         constexpr bool GEN = decltype(gen_)::value;
         for (int j = 0; j < p.k; j++) {
             const int it = p.it + j;
+            float *slot = SLOTS ? p.slots + j * p.slot_stride : nullptr;
             if (need <= NOP * (p.k - 1 - j)) {
                 float4 W[CX + 2 * NOP];  // columns x0 - NOP .. x0 + CX - 1 + NOP of the strip
 #pragma unroll
                 for (int k = 0; k < CX + 2 * NOP; k++)
-                    W[k] = k >= NOP && k < NOP + CX ? cur[k - NOP < CX ? k - NOP : 0]
+                    W[k] = !ADJ && k >= NOP && k < NOP + CX ? cur[k - NOP < CX ? k - NOP : 0]
                                                     : *reinterpret_cast<const float4 *>(S0 + own + (k - NOP) * rz);
 #pragma unroll
                 for (int c = 0; c < CX; c++) {
@@ -126,12 +185,13 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
                     const float4 m = W[NOP + c];
                     const float zw[12] = {a.x, a.y, a.z, a.w, m.x, m.y, m.z, m.w, b.x, b.y, b.z, b.w};
                     float4 pr = prv[c], o;
-                    if (GEN) {
+                    if (!ADJ && GEN) {
                         pr.x = __fmul_rn(__fmul_rn(pr.x, wz[0]), wx[c]);
                         pr.y = __fmul_rn(__fmul_rn(pr.y, wz[1]), wx[c]);
                         pr.z = __fmul_rn(__fmul_rn(pr.z, wz[2]), wx[c]);
                         pr.w = __fmul_rn(__fmul_rn(pr.w, wz[3]), wx[c]);
                     }
+                    float4 lp = make_float4(0.f, 0.f, 0.f, 0.f);  // L(V) of the strip
                     // ts_kernel.c:140-144: lap = u*c0 + sum_k [(z pair)*cz + (x pair)*cx]
                     if constexpr (EXACT) {
                         float *ov = &o.x;
@@ -147,6 +207,41 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
                             }
                             ov[i] = sum3_rn(__fmul_rn((&vel[c].x)[i], lap), __fadd_rn(u, u), -(&pr.x)[i]);
                         }
+                    } else if constexpr (ADJ) {
+                        // lambda = 2 I nu + L(I vel2 nu) + W (1 - 2 I) nu_{k+1}, mu = W lambda
+                        const float2 c0 = make_float2(p.c0, p.c0);
+                        float2 l0 = __fmul2_rn(c0, make_float2(m.x, m.y)), l1 = __fmul2_rn(c0, make_float2(m.z, m.w));
+#pragma unroll
+                        for (int k = 1; k <= NOP; k++) {
+                            const float4 xm = W[NOP + c - k], xp = W[NOP + c + k];
+                            const float2 cz = make_float2(p.cz[k], p.cz[k]), cx = make_float2(p.cx[k], p.cx[k]);
+                            float2 z0p, z1p;
+                            if (k % 2 == 0) {
+                                z0p = __fadd2_rn(make_float2(zw[4 - k], zw[5 - k]), make_float2(zw[4 + k], zw[5 + k]));
+                                z1p = __fadd2_rn(make_float2(zw[6 - k], zw[7 - k]), make_float2(zw[6 + k], zw[7 + k]));
+                            } else {
+                                z0p = make_float2(__fadd_rn(zw[4 - k], zw[4 + k]), __fadd_rn(zw[5 - k], zw[5 + k]));
+                                z1p = make_float2(__fadd_rn(zw[6 - k], zw[6 + k]), __fadd_rn(zw[7 - k], zw[7 + k]));
+                            }
+                            l0 = __ffma2_rn(z0p, cz, l0);
+                            l1 = __ffma2_rn(z1p, cz, l1);
+                            l0 = __ffma2_rn(__fadd2_rn(make_float2(xm.x, xm.y), make_float2(xp.x, xp.y)), cx, l0);
+                            l1 = __ffma2_rn(__fadd2_rn(make_float2(xm.z, xm.w), make_float2(xp.z, xp.w)), cx, l1);
+                        }
+                        const float4 u = cur[c];
+                        const float lt[4] = {l0.x, l0.y, l1.x, l1.y}, uv[4] = {u.x, u.y, u.z, u.w};
+                        const float yv[4] = {pr.x, pr.y, pr.z, pr.w};
+                        float ov[4];
+                        const bool xin = x0 + c >= NOP && x0 + c < n2 - NOP;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            const bool in = !GEN || (xin && z0 + i >= NOP && z0 + i < n1 - NOP);
+                            const float w = GEN ? __fmul_rn(wz[i], wx[c]) : 1.f;
+                            const float t = __fadd_rn(in ? __fadd_rn(uv[i], uv[i]) : 0.f, lt[i]);
+                            const float lam = fmaf(in ? -w : w, yv[i], t);
+                            ov[i] = GEN ? __fmul_rn(w, lam) : lam;
+                        }
+                        o = make_float4(ov[0], ov[1], ov[2], ov[3]);
                     } else {
                         // two cells per instruction, with the products that k_stepB's compiled form fuses
                         const float2 u0 = make_float2(m.x, m.y), u1 = make_float2(m.z, m.w);
@@ -177,8 +272,9 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
                         const float2 o0 = __ffma2_rn(make_float2(vel[c].x, vel[c].y), l0, d0);
                         const float2 o1 = __ffma2_rn(make_float2(vel[c].z, vel[c].w), l1, d1);
                         o = make_float4(o0.x, o0.y, o1.x, o1.y);
+                        lp = make_float4(l0.x, l0.y, l1.x, l1.y);
                     }
-                    if (GEN) {
+                    if (!ADJ && GEN) {
                         const bool xin = x0 + c >= NOP && x0 + c < n2 - NOP;
                         if (!(xin && z0 >= NOP && z0 < n1 - NOP)) o.x = pr.x;
                         if (!(xin && z0 + 1 >= NOP && z0 + 1 < n1 - NOP)) o.y = pr.y;
@@ -189,13 +285,25 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
                         o.z = __fmul_rn(__fmul_rn(o.z, wz[2]), wx[c]);
                         o.w = __fmul_rn(__fmul_rn(o.w, wz[3]), wx[c]);
                     }
-                    prv[c] = m;
+                    if (SLOTS) store(slot, c, ADJ || p.slot_level ? cur[c] : lp);
+                    prv[c] = cur[c];
                     cur[c] = o;
-                    *reinterpret_cast<float4 *>(S1 + own + c * rz) = o;
                 }
+                // residuals of the thread's own cells: on mu, before it is weighted
+                if (ADJ && my1 > my0) {
+#pragma unroll
+                    for (int c = 0; c < CX; c++) *reinterpret_cast<float4 *>(S1 + own + c * rz) = cur[c];
+#pragma unroll 1
+                    for (int s = my0; s < my1; s++) S1[cells[s].x] = with_entries(S1[cells[s].x], cells[s], j);
+#pragma unroll
+                    for (int c = 0; c < CX; c++) cur[c] = *reinterpret_cast<const float4 *>(S1 + own + c * rz);
+                }
+#pragma unroll
+                for (int c = 0; c < CX; c++)
+                    *reinterpret_cast<float4 *>(S1 + own + c * rz) = ADJ ? weighted(cur[c], c) : cur[c];
             }
             // receivers of the level this step reads, pending sponge applied (lint2d_extract)
-            if (nrec > 0 && (p.jdata == 1 || it % p.jdata == 0)) {
+            if (!ADJ && nrec > 0 && (p.jdata == 1 || it % p.jdata == 0)) {
                 float *row = p.dat + (long long)(it / p.jdata) * p.nr;
                 for (int r = tid; r < nrec; r += blockDim.x) {
                     const int2 li = rec_l[r];
@@ -217,19 +325,9 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
                 }
             }
             __syncthreads();
-            if (ncell > 0) {  // sources on the new level, one thread per cell, in (source, corner) order
-                const float *dd = ent_d + j * p.max_ent;
-                for (int s = tid; s < ncell; s += blockDim.x) {
-                    const int4 q = cells[s];
-                    const float vn = __int_as_float(q.w);
-                    float v = S1[q.x];
-#pragma unroll 1
-                    for (int e = q.y; e < q.z; e++) {
-                        const float a = __fmul_rn(dd[e], ent_w[e]);
-                        v = EXACT ? __fadd_rn(v, __fmul_rn(a, vn)) : fmaf(a, vn, v);
-                    }
-                    S1[q.x] = v;
-                }
+            if (!ADJ && ncell > 0) {  // sources on the new level, one thread per cell
+                for (int s = tid; s < ncell; s += blockDim.x)
+                    S1[cells[s].x] = with_entries(S1[cells[s].x], cells[s], j);
                 __syncthreads();
 #pragma unroll
                 for (int c = 0; c < CX; c++) cur[c] = *reinterpret_cast<const float4 *>(S1 + own + c * rz);
@@ -237,55 +335,19 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
             float *t = S0;
             S0 = S1;
             S1 = t;
-            if (p.slots) {  // every new level (the gradient's recompute)
-                float *dst = p.slots + (long long)j * p.slot_stride;
-                if (z0 >= tz0 && z0 < tz1 && x0 + CX - 1 >= tx0 && x0 < tx1)
-#pragma unroll
-                    for (int c = 0; c < CX; c++) {
-                        const int x = x0 + c;
-                        if (x < tx0 || x >= tx1) continue;
-                        const float4 v = *reinterpret_cast<const float4 *>(S0 + own + c * rz);
-                        float *d = dst + (long long)x * n1 + z0;
-                        if (vec) {
-                            *reinterpret_cast<float4 *>(d) = v;
-                        } else {
-                            const float e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                            for (int i = 0; i < 4; i++)
-                                if (z0 + i < tz1) d[i] = e[i];
-                        }
-                    }
-            }
         }
     };
     if (inner && !damp) steps(std::false_type());
     else steps(std::true_type());
     if (!p.ocur) return;
-    // the tile's cells of the last two levels (tz and hz are multiples of 4, so strips do not straddle its low edge)
-    if (z0 >= tz0 && z0 < tz1)
 #pragma unroll
-        for (int c = 0; c < CX; c++) {
-            const int x = x0 + c;
-            if (x < tx0 || x >= tx1) continue;
-            const float4 a = *reinterpret_cast<const float4 *>(S0 + own + c * rz);
-            const float4 b = *reinterpret_cast<const float4 *>(S1 + own + c * rz);
-            const long long i = (long long)x * n1 + z0;
-            if (vec) {
-                *reinterpret_cast<float4 *>(p.ocur + i) = a;
-                *reinterpret_cast<float4 *>(p.oprv + i) = b;
-            } else {
-                const float va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (z0 + q < tz1) {
-                        p.ocur[i + q] = va[q];
-                        p.oprv[i + q] = vb[q];
-                    }
-            }
-        }
+    for (int c = 0; c < CX; c++) {  // the last two levels
+        store(p.ocur, c, cur[c]);
+        store(p.oprv, c, prv[c]);
+    }
 }
 
-template <int NOP, bool EXACT, int CX>
+template <int NOP, int MODE, int CX>
 static void launch_cx(const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sh.ntz, sh.ntx);
@@ -297,33 +359,74 @@ static void launch_cx(const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaS
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaFuncSetAttribute(k_tb2<NOP, EXACT, CX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTb2SmemMax);
-    cudaLaunchKernelEx(&cfg, k_tb2<NOP, EXACT, CX>, p);
+    cudaFuncSetAttribute(k_tb2<NOP, MODE, CX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTb2SmemMax);
+    cudaLaunchKernelEx(&cfg, k_tb2<NOP, MODE, CX>, p);
+}
+
+template <int NOP, int CX>
+static void launch_mode(int mode, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
+    switch (mode) {
+        case 0: launch_cx<NOP, 0, CX>(p, sh, smem, s); break;
+        case 1: launch_cx<NOP, 1, CX>(p, sh, smem, s); break;
+        case 2: launch_cx<NOP, 2, CX>(p, sh, smem, s); break;
+        default: launch_cx<NOP, 3, CX>(p, sh, smem, s); break;
+    }
 }
 
 template <int NOP>
-static void launch_nop(bool exact, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
-    if (sh.cx == 1) {
-        if (exact) launch_cx<NOP, true, 1>(p, sh, smem, s);
-        else launch_cx<NOP, false, 1>(p, sh, smem, s);
-    } else if (sh.cx == 4) {
-        if (exact) launch_cx<NOP, true, 4>(p, sh, smem, s);
-        else launch_cx<NOP, false, 4>(p, sh, smem, s);
-    } else {
-        if (exact) launch_cx<NOP, true, 2>(p, sh, smem, s);
-        else launch_cx<NOP, false, 2>(p, sh, smem, s);
-    }
+static void launch_nop(int mode, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
+    if (sh.cx == 1) launch_mode<NOP, 1>(mode, p, sh, smem, s);
+    else if (sh.cx == 2) launch_mode<NOP, 2>(mode, p, sh, smem, s);
+    else launch_mode<NOP, 4>(mode, p, sh, smem, s);
 }
 
 }  // namespace
 
-void launch_tb2(int nop, bool exact, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
+void launch_tb2(int nop, int mode, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
     switch (nop) {
-        case 1: launch_nop<1>(exact, p, sh, smem, s); break;
-        case 2: launch_nop<2>(exact, p, sh, smem, s); break;
-        case 3: launch_nop<3>(exact, p, sh, smem, s); break;
-        default: launch_nop<4>(exact, p, sh, smem, s); break;
+        case 1: launch_nop<1>(mode, p, sh, smem, s); break;
+        case 2: launch_nop<2>(mode, p, sh, smem, s); break;
+        case 3: launch_nop<3>(mode, p, sh, smem, s); break;
+        default: launch_nop<4>(mode, p, sh, smem, s); break;
     }
+}
+
+// The imaging condition of a segment: G += I nu_k L(V_k) (or I nu_k V_k, the
+// cross-correlation) and, at source cells, nu_k wav w, k from k1 - 1 down to
+// k0.  One thread per cell keeps its compensated sum in registers over the
+// segment; the levels come from the slots that the recompute (lap) and the
+// adjoint sweep (nu) wrote, both read once.
+__global__ void __launch_bounds__(256) k_tb2_image(float2 *__restrict__ G, const float *__restrict__ lap,
+                                                   const float *__restrict__ nu, long long stride, const AdjParams p,
+                                                   int k0, int k1) {
+    const Grid g = p.g;
+    const int i1 = blockIdx.x * 64 + threadIdx.x, i2 = blockIdx.y * 4 + threadIdx.y;
+    if (i1 >= g.n1 || i2 >= g.n2) return;
+    const long long i = (long long)i2 * g.n1 + i1;
+    const bool in = i1 >= p.nop && i1 < g.n1 - p.nop && i2 >= p.nop && i2 < g.n2 - p.nop;
+    const int e0 = p.wav && !p.xcorr ? p.sc_start[i] : 0, e1 = p.wav && !p.xcorr ? p.sc_start[i + 1] : 0;
+    if (!in && e1 == e0) return;
+    float2 a = G[i];
+    const float *l = lap + i + (k1 - k0) * stride;  // slot k - k0: L(V_k)
+    const float *n = nu + i;                        // slot k1 - 1 - k: nu_k
+#pragma unroll 4
+    for (int k = k1 - 1; k >= k0; k--) {
+        l -= stride;
+        const float x = *n;
+        n += stride;
+        if (in) a = gsum_add(a, __fmul_rn(x, *l));
+        for (int e = e0; e < e1; e++) {
+            const int2 en = p.sc_ent[e];
+            const float dd = p.one_wavelet ? p.wav[(long long)k * p.ncs] : p.wav[(long long)k * p.ncs + en.x];
+            a = gsum_add_prod(a, x, dd * __int_as_float(en.y));
+        }
+    }
+    G[i] = a;
+}
+
+void launch_tb2_image(float2 *G, const float *lap, const float *nu, long long stride, const AdjParams &p, int k0,
+                      int k1, cudaStream_t s) {
+    k_tb2_image<<<dim3((p.g.n1 + 63) / 64, (p.g.n2 + 3) / 4), dim3(64, 4), 0, s>>>(G, lap, nu, stride, p, k0, k1);
 }
 
 }  // namespace awe

@@ -389,10 +389,10 @@ awe_status awe_set_geometry(awe_plan *p, int ns, const float *sou, int nr, const
         k[9] = p->pa.nshot;
         k[10] = (long long)(uintptr_t)p->inj_buf;
         k[11] = p->inj.n;
-        k[12] = (long long)(uintptr_t)p->tb2_lists;
-        k[13] = p->tb2_geom;
-        for (int q = 0; q < 7; q++) k[14 + q] = (long long)p->tb2_off[q];
-        for (int q = 0; q < 3; q++) k[21 + q] = p->tb2_max[q];
+        k[12] = (long long)(uintptr_t)p->tb2_fwd.buf;
+        k[13] = p->tb2_fwd.ok;
+        for (int q = 0; q < 7; q++) k[14 + q] = (long long)p->tb2_fwd.off[q];
+        for (int q = 0; q < 3; q++) k[21 + q] = p->tb2_fwd.most[q];
     };
     long long before[24], after[24];
     key(before);
@@ -402,7 +402,7 @@ awe_status awe_set_geometry(awe_plan *p, int ns, const float *sou, int nr, const
     p->inj_scale_ok = false;
     awe_status st = set_geometry_common(p, ns, sou, nr, rec);
     if (st == AWE_OK) st = set_inj_cells(p);
-    if (st == AWE_OK) st = set_tb2_lists(p);
+    if (st == AWE_OK) st = set_tb2_lists(p, p->tb2_fwd, p->h_src, &p->h_rec);
     if (st == AWE_OK) st = single_shot(p, ns, nr);
     key(after);
     // (the GPU-program loop bakes in where its sources lie)
@@ -451,7 +451,7 @@ awe_status awe_set_moving_geometry(awe_plan *p, int ns, int nst, const float *so
     awe_status st = set_geometry_common(p, ns * nst, sou, nr * nrt, rec);
     if (st != AWE_OK) return st;
     p->inj = InjCells{};  // the lists hold fixed sources
-    p->tb2_geom = false;
+    p->tb2_fwd.ok = false;
     p->ns = ns;
     p->nr = nr;
     set_move_mode(p, mode, nst, nrt);

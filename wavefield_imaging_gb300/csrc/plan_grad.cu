@@ -55,8 +55,12 @@ struct GradState {
     int *rc_start = nullptr, *sc_start = nullptr;
     int2 *rc_ent = nullptr, *sc_ent = nullptr;
     size_t rc_cap = 0, sc_cap = 0;
-    bool lists_ok = false;  // cleared when the geometry changes
+    bool lists_ok = false, rc_ok = false;  // cleared when the geometry changes
     size_t nd_cap = 0;      // trace samples dat and r hold
+    // 2D, several steps a launch (k_tb2d.cu): slots hold T levels of L(V_k) and
+    // T of nu_k, xy2 two more levels for the adjoint sweep
+    bool tb2 = false;
+    float *xy2 = nullptr;
     // misfit rows (pinned, written by the stream) and the captured gradient
     double *h_rows = nullptr;
     size_t h_rows_n = 0;
@@ -75,7 +79,7 @@ void plan_gradient_graph_drop(awe_plan *p) {
     if (st->gexec) cudaGraphExecDestroy(st->gexec);
     st->gexec = nullptr;
     st->g_seen = false;
-    st->lists_ok = false;
+    st->lists_ok = st->rc_ok = false;
 }
 
 void plan_gradient_free(awe_plan *p) {
@@ -86,7 +90,7 @@ void plan_gradient_free(awe_plan *p) {
     for (void *ptr : {(void *)st->slots, st->ckpt, (void *)st->scales, (void *)st->amax, (void *)st->X, (void *)st->Y,
                       (void *)st->kap, (void *)st->G, (void *)st->dat, (void *)st->r, (void *)st->row_sum,
                       (void *)st->vr, (void *)st->gbuf, (void *)st->rc_start, (void *)st->sc_start,
-                      (void *)st->rc_ent, (void *)st->sc_ent})
+                      (void *)st->rc_ent, (void *)st->sc_ent, (void *)st->xy2})
         if (ptr) dev_free(p, ptr);
     delete st;
     p->grad = nullptr;
@@ -105,7 +109,18 @@ static awe_status grad_alloc(awe_plan *p, int T, int fmt) {
     st->nseg = (d.nt + T - 1) / T;
     const size_t es = fmt == AWE_CKPT_FP32 ? 4 : 2;
     st->tma = p->use_tma && d.precision == AWE_FAST;
-    AWE_TRY(dev_alloc(p, (void **)&st->slots, (size_t)(st->tma ? T : T + 1) * cells * sizeof(float)));
+    // 2D: two slots a step and two more levels, where memory allows them
+    st->tb2 = p->tb2 && (long long)cells <= kFusedCells;
+    if (st->tb2) {
+        st->tb2 = dev_alloc(p, (void **)&st->slots, (size_t)std::max(2 * T, T + 1) * cells * sizeof(float)) == AWE_OK;
+        if (st->tb2 && dev_alloc(p, (void **)&st->xy2, 2 * cells * sizeof(float)) != AWE_OK) {
+            dev_free(p, st->slots);
+            st->slots = nullptr;
+            st->tb2 = false;
+        }
+        cudaGetLastError();
+    }
+    if (!st->tb2) AWE_TRY(dev_alloc(p, (void **)&st->slots, (size_t)(st->tma ? T : T + 1) * cells * sizeof(float)));
     AWE_TRY(dev_alloc(p, &st->ckpt, (size_t)2 * st->nseg * cells * es));
     st->nblk = fmt == AWE_CKPT_BFP16 ? ((long long)cells + kBfpBlock - 1) / kBfpBlock : 1;
     AWE_TRY(dev_alloc(p, (void **)&st->scales, (size_t)2 * st->nseg * st->nblk * sizeof(float)));
@@ -542,12 +557,21 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
     // the kappa fold, three ABC-transpose launches and the g pass; AWE_BND3=0
     // keeps the separate launches (the tests compare both)
     const bool bnd_adj = st->tma && st->kap && stepB3_bnd(p);
+    // 2D: several steps of the recompute and of the adjoint sweep per launch, and
+    // the imaging condition once per segment
+    bool tb2 = false;
     if (fuse_pts) {
+        const int nc = d.ndim == 3 ? 8 : 4;
         if (!st->lists_ok) {
-            const int nc = d.ndim == 3 ? 8 : 4;
-            AWE_TRY(build_cell_lists(p, p->h_rec, nc, &st->rc_start, &st->rc_ent, &st->rc_cap, s));
+            p->tb2_adj.ok = false;
+            if (st->tb2 && p->tb2_fwd.ok) AWE_TRY(set_tb2_lists(p, p->tb2_adj, p->h_rec, nullptr));
             AWE_TRY(build_cell_lists(p, p->h_src, nc, &st->sc_start, &st->sc_ent, &st->sc_cap, s));
             st->lists_ok = true;
+        }
+        tb2 = st->tb2 && p->tb2_fwd.ok && p->tb2_adj.ok && !p->profile;
+        if (!tb2 && !st->rc_ok) {
+            AWE_TRY(build_cell_lists(p, p->h_rec, nc, &st->rc_start, &st->rc_ent, &st->rc_cap, s));
+            st->rc_ok = true;
         }
         ap.rc_start = st->rc_start;
         ap.rc_ent = st->rc_ent;
@@ -587,10 +611,37 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
     CUDA_TRY(cudaMemsetAsync(st->G, 0, (size_t)cells * sizeof(float2), s));
     if (st->kap) CUDA_TRY(cudaMemsetAsync(st->kap, 0, bytes, s));
     float *X = st->X, *Y = st->Y;
+    float *X2 = st->xy2, *Y2 = X2 + cells;  // (tb2)
     const CUtensorMap *xmap = &st->x_tile, *ymap = &st->y_tile;
     for (int seg = st->nseg - 1; seg >= 0; seg--) {
         const int k0 = seg * T, k1 = std::min(k0 + T, d.nt);
         float *slot0 = st->slots;
+        if (tb2) {
+            float *nu0 = slot0 + (size_t)T * cells;
+            float *A = p->u[0], *B = p->u[1], *A2 = p->tb2_u, *B2 = p->tb2_u + cells;
+            AWE_TRY(ckpt_load(p, 2 * seg, A, s));
+            AWE_TRY(ckpt_load(p, 2 * seg + 1, B, s));
+            for (int k = k0; k < k1; k += p->tb2_shape.k) {
+                const int n = std::min(p->tb2_shape.k, k1 - k);
+                tb2_launch(p, false, A, B, A2, B2, slot0 + (size_t)(k - k0) * cells, xcorr, k, n, d_wav, ncs, nullptr, s);
+                launches++;
+                std::swap(A, A2);
+                std::swap(B, B2);
+            }
+            for (int k = k1 - 1; k >= k0;) {
+                const int n = std::min(p->tb2_shape.k, k - k0 + 1);
+                tb2_launch(p, true, Y, X, Y2, X2, nu0 + (size_t)(k1 - 1 - k) * cells, true, k, n,
+                           p->nr > 0 ? st->r : nullptr, p->nr, nullptr, s);
+                launches++;
+                std::swap(X, X2);
+                std::swap(Y, Y2);
+                k -= n;
+            }
+            ap.wav = (p->ns > 0 && !xcorr) ? d_wav : nullptr;
+            launch_tb2_image(st->G, slot0, nu0, cells, ap, k0, k1, s);
+            launches++;
+            continue;
+        }
         if (st->tma) {
             // recompute with three rolling levels; the step kernel stores L(V_k) in slot k - k0
             AWE_TRY(ckpt_load(p, 2 * seg, st->vr, s));

@@ -11,6 +11,14 @@
 
 namespace awe {
 struct GradState;
+// per-tile point lists of k_tb2d.cu in one device buffer, kept while large enough
+struct Tb2Lists {
+    int *buf = nullptr;
+    size_t cap = 0;
+    size_t off[7] = {0, 0, 0, 0, 0, 0, 0};  // of Tb2Params' lists, in their order
+    int most[3] = {0, 0, 0};                // max_rec, max_cell, max_ent
+    bool ok = false;                        // false: the points do not allow the kernel
+};
 }
 
 struct awe_plan {
@@ -70,13 +78,9 @@ struct awe_plan {
 
     // 2D CPU-program scheme: several steps a launch (k_tb2d.cu)
     bool tb2 = false;        // the plan's kind allows it
-    bool tb2_geom = false;   // and so do its points
     awe::Tb2Shape tb2_shape{};
     float *tb2_u = nullptr;  // two more levels (the launch is out of place)
-    int *tb2_lists = nullptr;  // per tile lists (set_tb2_lists)
-    size_t tb2_cap = 0;
-    size_t tb2_off[7] = {0, 0, 0, 0, 0, 0, 0};  // of Tb2Params' lists, in their order
-    int tb2_max[3] = {0, 0, 0};                   // max_rec, max_cell, max_ent
+    awe::Tb2Lists tb2_fwd, tb2_adj;  // per tile: sources and receivers; receivers as the adjoint's sources
 
     bool model_set = false, geom_set = false;
     awe_snap_fn snap_cb = nullptr;
@@ -176,11 +180,13 @@ typedef std::function<awe_status(int it, const float *prev, const float *cur, cu
 // hook_every: the hook does nothing but at multiples of it
 awe_status planB_run_hooked(awe_plan *p, const float *d_wav, int ncs, float *d_dat, float *d_wfl, cudaStream_t s,
                             const StepHook *hook, int hook_every = 1);
-// tile lists of the points for k_tb2d.cu; sets p->tb2_geom
-awe_status set_tb2_lists(awe_plan *p);
-// steps it .. it + k - 1 from levels prv, cur
-void tb2_launch(awe_plan *p, const float *prv, const float *cur, float *oprv, float *ocur, float *slots,
-                long long slot_stride, int it, int k, const float *d_wav, int ncs, float *d_dat, cudaStream_t s);
+// tile lists for k_tb2d.cu of points that inject (entries per cell) and of
+// receivers (may be null)
+awe_status set_tb2_lists(awe_plan *p, Tb2Lists &t, const std::vector<GeoPoint> &inj, const std::vector<GeoPoint> *rec);
+// k steps from levels prv, cur: it .. it + k - 1 forward, it .. it - k + 1 of
+// the adjoint (d_wav the residual rows then)
+void tb2_launch(awe_plan *p, bool adj, const float *prv, const float *cur, float *oprv, float *ocur, float *slots,
+                bool slot_level, int it, int k, const float *d_wav, int ncs, float *d_dat, cudaStream_t s);
 StepBParams stepB_params(const awe_plan *p);
 // lap_out: the TMA path also stores L(cur) of interior cells there (gradient recompute)
 // ext_*: 2D, the receivers of `cur` (pending sponge applied) gathered into

@@ -72,36 +72,35 @@ static Tb2Shape tb2_shape(const Grid &g, int nop, int sms) {
     return best;
 }
 
-// two level buffers with their padding columns, and the longest lists of a tile
-static size_t tb2_smem(const awe_plan *p) {
-    const Tb2Shape &sh = p->tb2_shape;
-    const int *m = p->tb2_max;
-    return (size_t)2 * (sh.rx + 8) * sh.rz * 4 + (size_t)m[0] * 40 + (size_t)m[1] * 16 + (size_t)m[2] * 4 * (1 + sh.k);
+// two level buffers with their padding columns, the longest lists of a tile, a word per thread
+static size_t tb2_smem(const Tb2Shape &sh, const int *most) {
+    return (size_t)2 * (sh.rx + 8) * sh.rz * 4 + (size_t)most[0] * 40 + (size_t)most[1] * 16 + kTb2Threads * 4 +
+           (size_t)most[2] * 4 * (1 + sh.k);
 }
 
-awe_status set_tb2_lists(awe_plan *p) {
-    p->tb2_geom = false;
+awe_status set_tb2_lists(awe_plan *p, Tb2Lists &t, const std::vector<GeoPoint> &inj, const std::vector<GeoPoint> *rec) {
+    t.ok = false;
     if (!p->tb2 || p->move_mode >= 0 || p->sponge_deferred) return AWE_OK;
     const Grid &g = p->g;
     const Tb2Shape &sh = p->tb2_shape;
     const int ntile = sh.ntz * sh.ntx;
     struct Cell {
-        int tile;
+        int tile, owner;  // owner: the thread that holds the cell
         int4 q;
     };
     // receivers by the tile of their base cell (all four corners are in its region)
-    std::vector<Cell> rec;
-    for (int r = 0; r < (int)p->h_rec.size(); r++) {
-        const int z = (int)(p->h_rec[r].base % g.n1), x = (int)(p->h_rec[r].base / g.n1);
+    std::vector<Cell> rc;
+    for (int r = 0; rec && r < (int)rec->size(); r++) {
+        const int z = (int)((*rec)[r].base % g.n1), x = (int)((*rec)[r].base / g.n1);
         if (z >= g.n1 - 1 || x >= g.n2 - 1) return AWE_OK;
-        rec.push_back({(x / sh.tx) * sh.ntz + z / sh.tz, make_int4(z, x, r, 0)});
+        rc.push_back({(x / sh.tx) * sh.ntz + z / sh.tz, 0, make_int4(z, x, r, 0)});
     }
-    // source cells, each with its entries in (source, corner) order, in every
-    // tile whose region holds the cell
+    // cells that points inject into, each with its entries in (point, corner)
+    // order, in every tile whose region holds the cell
     std::vector<std::pair<long long, int>> e;
-    for (int s = 0; s < (int)p->h_src.size(); s++)
+    for (int s = 0; s < (int)inj.size(); s++)
         for (int c = 0; c < 4; c++) {
-            const long long n = p->h_src[s].base + p->h_corner_off[c];
+            const long long n = inj[s].base + p->h_corner_off[c];
             if (n >= g.cells()) return AWE_OK;
             e.push_back({n, 8 * s + c});
         }
@@ -111,13 +110,15 @@ awe_status set_tb2_lists(awe_plan *p) {
         for (k1 = k; k1 < e.size() && e[k1].first == e[k].first;) k1++;
         const int z = (int)(e[k].first % g.n1), x = (int)(e[k].first / g.n1);
         for (int bx = std::max(0, (x - sh.hx) / sh.tx - 1); bx < sh.ntx && bx * sh.tx - sh.hx <= x; bx++)
-            for (int bz = std::max(0, (z - sh.hz) / sh.tz - 1); bz < sh.ntz && bz * sh.tz - sh.hz <= z; bz++)
-                if (x < bx * sh.tx - sh.hx + sh.rx && z < bz * sh.tz - sh.hz + sh.rz)
-                    cell.push_back({bx * sh.ntz + bz, make_int4(z, x, (int)k, (int)k1)});
+            for (int bz = std::max(0, (z - sh.hz) / sh.tz - 1); bz < sh.ntz && bz * sh.tz - sh.hz <= z; bz++) {
+                const int lx = x - bx * sh.tx + sh.hx, lz = z - bz * sh.tz + sh.hz;
+                if (lx < sh.rx && lz < sh.rz)
+                    cell.push_back({bx * sh.ntz + bz, lx / sh.cx * (sh.rz / 4) + lz / 4, make_int4(z, x, (int)k, (int)k1)});
+            }
     }
-    auto by_tile = [](const Cell &a, const Cell &b) { return a.tile < b.tile; };
-    std::stable_sort(rec.begin(), rec.end(), by_tile);
-    std::stable_sort(cell.begin(), cell.end(), by_tile);
+    auto order = [](const Cell &a, const Cell &b) { return a.tile != b.tile ? a.tile < b.tile : a.owner < b.owner; };
+    std::stable_sort(rc.begin(), rc.end(), order);
+    std::stable_sort(cell.begin(), cell.end(), order);
     std::vector<int> start[3];  // cells, entries, receivers
     for (auto &v : start) v.assign(ntile + 1, 0);
     std::vector<int2> ent;
@@ -126,29 +127,29 @@ awe_status set_tb2_lists(awe_plan *p) {
         c.q.z = (int)ent.size();
         for (int k = k0; k < k1; k++) {
             int w;
-            std::memcpy(&w, &p->h_src[e[k].second >> 3].w[e[k].second & 7], sizeof w);
+            std::memcpy(&w, &inj[e[k].second >> 3].w[e[k].second & 7], sizeof w);
             ent.push_back(make_int2(e[k].second, w));
         }
         c.q.w = (int)ent.size();
         start[0][c.tile + 1]++;
         start[1][c.tile + 1] += k1 - k0;
     }
-    for (const Cell &c : rec) start[2][c.tile + 1]++;
+    for (const Cell &c : rc) start[2][c.tile + 1]++;
     int most[3] = {0, 0, 0};
     for (int k = 0; k < 3; k++)
-        for (int t = 0; t < ntile; t++) {
-            most[k] = std::max(most[k], start[k][t + 1]);
-            start[k][t + 1] += start[k][t];
+        for (int q = 0; q < ntile; q++) {
+            most[k] = std::max(most[k], start[k][q + 1]);
+            start[k][q + 1] += start[k][q];
         }
-    p->tb2_max[0] = most[2];
-    p->tb2_max[1] = most[0];
-    p->tb2_max[2] = most[1];
-    if (tb2_smem(p) > kTb2SmemMax) return AWE_OK;  // the points of one tile do not fit beside its levels
-    // one buffer and one copy; sized for source corners in four tiles each, so
+    t.most[0] = most[2];
+    t.most[1] = most[0];
+    t.most[2] = most[1];
+    if (most[0] >= 32768 || tb2_smem(sh, t.most) > kTb2SmemMax) return AWE_OK;  // one tile's points do not fit
+    // one buffer and one copy; sized for injected corners in four tiles each, so
     // that points that only move keep it (a captured time loop reads it)
-    const size_t nst = (size_t)(ntile + 4) / 4 * 4 + 4, ns = p->h_src.size(), nr = p->h_rec.size();
+    const size_t nst = (size_t)(ntile + 4) / 4 * 4 + 4, ns = inj.size(), nr = rc.size();
     const size_t ncell = std::max(cell.size(), 16 * ns), nent = std::max(ent.size() + 1, 16 * ns + 1) / 2 * 2;
-    size_t *off = p->tb2_off;
+    size_t *off = t.off;
     off[0] = 0;
     off[1] = off[0] + nst;
     off[2] = off[1] + nst;
@@ -161,27 +162,27 @@ awe_status set_tb2_lists(awe_plan *p) {
     for (int k = 0; k < 3; k++) std::copy(start[k].begin(), start[k].end(), buf.begin() + off[k]);
     for (size_t k = 0; k < cell.size(); k++) std::memcpy(&buf[off[3] + 4 * k], &cell[k].q, sizeof(int4));
     if (!ent.empty()) std::memcpy(&buf[off[5]], ent.data(), ent.size() * sizeof(int2));
-    for (size_t k = 0; k < rec.size(); k++) {
-        std::memcpy(&buf[off[4] + 4 * k], &rec[k].q, sizeof(int4));
-        std::memcpy(&buf[off[6] + 4 * k], p->h_rec[rec[k].q.z].w, 4 * sizeof(float));
+    for (size_t k = 0; k < rc.size(); k++) {
+        std::memcpy(&buf[off[4] + 4 * k], &rc[k].q, sizeof(int4));
+        std::memcpy(&buf[off[6] + 4 * k], (*rec)[rc[k].q.z].w, 4 * sizeof(float));
     }
-    if (p->tb2_cap < total) {
-        dev_free(p, p->tb2_lists);
-        p->tb2_lists = nullptr;
-        p->tb2_cap = 0;
-        AWE_TRY(dev_alloc(p, (void **)&p->tb2_lists, total * sizeof(int)));
-        p->tb2_cap = total;
+    if (t.cap < total) {
+        dev_free(p, t.buf);
+        t.buf = nullptr;
+        t.cap = 0;
+        AWE_TRY(dev_alloc(p, (void **)&t.buf, total * sizeof(int)));
+        t.cap = total;
     }
-    CUDA_TRY(cudaMemcpy(p->tb2_lists, buf.data(), total * sizeof(int), cudaMemcpyHostToDevice));
-    p->tb2_geom = true;
+    CUDA_TRY(cudaMemcpy(t.buf, buf.data(), total * sizeof(int), cudaMemcpyHostToDevice));
+    t.ok = true;
     return AWE_OK;
 }
 
-void tb2_launch(awe_plan *p, const float *prv, const float *cur, float *oprv, float *ocur, float *slots,
-                long long slot_stride, int it, int k, const float *d_wav, int ncs, float *d_dat, cudaStream_t s) {
+void tb2_launch(awe_plan *p, bool adj, const float *prv, const float *cur, float *oprv, float *ocur, float *slots,
+                bool slot_level, int it, int k, const float *d_wav, int ncs, float *d_dat, cudaStream_t s) {
     const awe_desc &d = p->d;
     const Tb2Shape &sh = p->tb2_shape;
-    const bool sponge = d.dabc && !d.hybrid;
+    const Tb2Lists &t = adj ? p->tb2_adj : p->tb2_fwd;
     Tb2Params q{};
     q.n1 = p->g.n1;
     q.n2 = p->g.n2;
@@ -192,25 +193,24 @@ void tb2_launch(awe_plan *p, const float *prv, const float *cur, float *oprv, fl
     for (int i = 0; i <= p->nop; i++) q.cz[i] = p->k.c[0][i], q.cx[i] = p->k.c[1][i];
     q.cur = cur, q.prv = prv, q.vel = p->vel, q.ocur = ocur, q.oprv = oprv;
     q.slots = slots;
-    q.slot_stride = slot_stride;
-    if (sponge) q.w1 = p->w[0], q.w2 = p->w[1];
+    q.slot_stride = p->g.cells();
+    q.slot_level = slot_level;
+    if (d.dabc && !d.hybrid) q.w1 = p->w[0], q.w2 = p->w[1];
     q.ilo1 = p->wlo[0], q.ihi1 = p->whi[0], q.ilo2 = p->wlo[1], q.ihi2 = p->whi[1];
-    const int *b = p->tb2_lists;
-    const size_t *off = p->tb2_off;
-    if (p->tb2_max[1] > 0) q.inj_start = b + off[0];
-    q.ent_start = b + off[1];
-    if (p->tb2_max[0] > 0 && d_dat) q.rec_start = b + off[2];
-    q.inj_cell = (const int4 *)(b + off[3]);
-    q.rec_pt = (const int4 *)(b + off[4]);
-    q.inj_ent = (const int2 *)(b + off[5]);
-    q.rec_wt = (const float *)(b + off[6]);
-    q.max_rec = p->tb2_max[0], q.max_cell = p->tb2_max[1], q.max_ent = p->tb2_max[2];
+    if (t.most[1] > 0 && d_wav) q.inj_start = t.buf + t.off[0];
+    q.ent_start = t.buf + t.off[1];
+    if (t.most[0] > 0 && d_dat) q.rec_start = t.buf + t.off[2];
+    q.inj_cell = (const int4 *)(t.buf + t.off[3]);
+    q.rec_pt = (const int4 *)(t.buf + t.off[4]);
+    q.inj_ent = (const int2 *)(t.buf + t.off[5]);
+    q.rec_wt = (const float *)(t.buf + t.off[6]);
+    q.max_rec = t.most[0], q.max_cell = t.most[1], q.max_ent = t.most[2];
     q.wav = d_wav;
     q.ncs = ncs;
     q.jdata = d.jdata;
     q.nr = p->nr;
     q.dat = d_dat;
-    launch_tb2(p->nop, d.precision == AWE_EXACT, q, sh, tb2_smem(p), s);
+    launch_tb2(p->nop, adj ? 2 : slots ? 3 : d.precision == AWE_EXACT ? 1 : 0, q, sh, tb2_smem(sh, t.most), s);
 }
 
 awe_status planB_init(awe_plan *p) {
@@ -277,8 +277,9 @@ awe_status planB_init(awe_plan *p) {
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
         p->tb2_shape = tb2_shape(p->g, p->nop, sms > 0 ? sms : 1);
-        p->tb2 = true;
-        AWE_TRY(dev_alloc(p, (void **)&p->tb2_u, 2 * cells * sizeof(float)));
+        // (without room for two more levels: one step a launch)
+        p->tb2 = dev_alloc(p, (void **)&p->tb2_u, 2 * cells * sizeof(float)) == AWE_OK;
+        cudaGetLastError();
     }
     // line-end copies of the 3D boundary launch (made before any capture of
     // the time loop; AWE_BND_ENDS=0: the launch reads the level itself)
@@ -699,7 +700,7 @@ awe_status planB_run_hooked(awe_plan *p, const float *d_wav, int ncs, float *d_d
     // 2D: the traces of step it (the level the step reads, pending sponge
     // applied, as the reference extracts after its swap) are gathered by the
     // step's own launch; 3D: by the step's boundary launch
-    if (p->tb2_geom && !p->den && !p->profile) {
+    if (p->tb2_fwd.ok && !p->den && !p->profile) {
         // several steps a launch, stopping at steps whose levels the hook or a frame reads
         float *alt_prv = p->tb2_u, *alt_cur = p->tb2_u + g.cells();
         float *prv = nxt;
@@ -717,7 +718,7 @@ awe_status planB_run_hooked(awe_plan *p, const float *d_wav, int ncs, float *d_d
             int k = std::min(p->tb2_shape.k, d.nt - it);
             if (hook) k = std::min(k, hook_every - it % hook_every);
             if (frames) k = std::min(k, d.jsnap - it % d.jsnap);
-            tb2_launch(p, prv, cur, alt_prv, alt_cur, nullptr, 0, it, k, d_wav, ncs, d_dat, s);
+            tb2_launch(p, false, prv, cur, alt_prv, alt_cur, nullptr, false, it, k, d_wav, ncs, d_dat, s);
             launches++;
             std::swap(prv, alt_prv);
             std::swap(cur, alt_cur);
