@@ -179,7 +179,7 @@ def measured_peak():
         return 6800.0, "fallback"
 
 
-# DRAM bytes per cell of one step-kernel launch (k_stepB3_o8, AWE_FAST),
+# DRAM bytes per cell of one step-kernel launch (k_stepB3 at 8th order, AWE_FAST),
 # from the ncu capture of a 384^3-padded launch: 895.2 MB read + written
 # over 56.62 M padded cells (profiles/k_stepB3_o8_tma_n320.md).  A full
 # 576^3 launch is too large for a capture; DRAM traffic scales with the cells
@@ -468,7 +468,7 @@ def run_ours(args):
                         "traffic_source": ("ncu DRAM bytes per cell of a 384^3-padded launch of the same kernel "
                                            "(profiles/k_stepB3_o8_tma_n320.md) x this launch's cells"
                                            if traffic else None),
-                        "kernel": ("k_stepB3_o8 (TMA-staged, 3D 8th order)" if plan.step_kernel == "tma3d"
+                        "kernel": ("k_stepB3 (TMA-staged, 3D 8th order)" if plan.step_kernel == "tma3d"
                                    else "k_stepB (one thread per cell, 3D 8th order)"),
                         "peak_source": peak_kind, "avg_launch_us": avg_kernel_s * 1e6,
                         "kernel_share": (kern_ms / ms) if ms > 0 else None},
@@ -736,8 +736,8 @@ def extra_gradients_3d(args, local, peak, peak_kind):
         dobs = plan.forward(wav)
         plan.set_model(v0)
         r = _timed_gradient(plan, wav, dobs, nt, padded_cells(w), peak, peak_kind, None, 36,
-                            {"step": "k_stepB3_o8 (forward 16 B, recompute 20 B per cell)",
-                             "adjoint": "k_stepB3_o8 adjoint step"})
+                            {"step": "k_stepB3 (forward 16 B, recompute 20 B per cell)",
+                             "adjoint": "k_stepB3 adjoint step"})
     r["workload"] = w["name"].replace("nt=%d" % nt, "nt=%d of 3000" % nt) + ", gradient, BFP16 checkpoints"
     res["cartesian"] = r
     # the spherical shell, one source

@@ -40,18 +40,24 @@ struct InjCells {
     const int2 *ent;
 };
 
-// Padded grid, axis 1 fastest.
+// Padded grid, axis 1 fastest.  Lines are p1 >= n1 cells apart: a multiple of 4
+// where a kernel's tensor maps or 16-byte accesses want it (the cells past n1
+// hold nothing that is read), else n1.
 struct Grid {
-    int n1, n2, n3;  // n3 = 1 in 2D
-    long long s2() const { return n1; }
-    long long s3() const { return (long long)n1 * n2; }
-    long long cells() const { return (long long)n1 * n2 * n3; }
+    int n1 = 0, n2 = 0, n3 = 0;  // n3 = 1 in 2D
+    int p1 = 0;
+    Grid() = default;
+    Grid(int a, int b, int c, int p = 0) : n1(a), n2(b), n3(c), p1(p ? p : a) {}
+    long long s2() const { return p1; }
+    long long s3() const { return (long long)p1 * n2; }
+    long long cells() const { return (long long)p1 * n2 * n3; }  // of storage
 };
 
 // ---- scheme of the reference CPU programs (MAWEFDcart{2D,3D}cpu.c) ----
 struct StepBParams {
     Grid g;
     Coef k;
+    int nop;
     const float *w1, *w2, *w3;  // per-axis sponge factor (1 where undamped); null = no sponge
     int damp_prev;              // prev level carries the sponge of the previous step
     int sponge_new;             // apply the sponge to the new level in the step kernel
@@ -150,7 +156,7 @@ void launch_model_abc(const float *raw, const ModelPrep &m, float *const abc[6],
 // of the six faces, sponge of the shell the step kernel left unsponged
 // (cells within nop + 2 of a face), the receiver gather of the level the step
 // read, and the injection (ns > 0; only when no source corner lies in that
-// shell, whose cells the ABC reads).  nop = 4.
+// shell, whose cells the ABC reads).
 struct Bnd3Params {
     Grid g;
     float *uo;        // the new level
@@ -168,6 +174,7 @@ struct Bnd3Params {
     const float *wav;
     int it, ncs, one_wavelet;
     int n_int, nxr, nzr, rec_blocks;  // set by launch_bnd3
+    int nop;                          // 1 .. 4
     // compact copies of the line ends ([n3][n2][16]: axis-1 cells 0..7, then
     // n1-8..n1-1) of um (em: written by the previous step's launch; null:
     // read um itself) and of the new level once final (eo; null: none)
@@ -318,15 +325,18 @@ void launch_rec_adj(float *mu, const GeoPoint *pts, int nr, const float *r, cons
 void launch_src_grad_cells(float2 *G, const float *nu, const InjCells &c, const float *wav, int it, int ncs,
                            bool one_wavelet, cudaStream_t s);
 void launch_residual(const float *d, const float *dobs, float *r, int nrows, int nr, double *row_sum, cudaStream_t s);
+// n1, p1: checkpoints hold the n cells of the levels' lines without their padding
 void launch_ckpt_store16(bool fp16, const float *u, long long n, unsigned int *amax, void *q, float *scale, int grid,
-                         cudaStream_t s);
+                         cudaStream_t s, int n1 = 1, int p1 = 1);
 void launch_ckpt_load16(bool fp16, const void *q, long long n, const float *scale, float *u, int grid,
-                        cudaStream_t s);
+                        cudaStream_t s, int n1 = 1, int p1 = 1);
 // block floating point checkpoints: kBfpBlock consecutive cells share one FP32 scale
 constexpr int kBfpBlock = 64;
 constexpr float kBfpTiny = 1e-30f;  // blocks with max |v| <= this are stored as zero
-void launch_ckpt_store_bfp(const float *u, long long n, short *q, float *scale, int grid, cudaStream_t s);
-void launch_ckpt_load_bfp(const short *q, const float *scale, long long n, float *u, int grid, cudaStream_t s);
+void launch_ckpt_store_bfp(const float *u, long long n, short *q, float *scale, int grid, cudaStream_t s, int n1 = 1,
+                           int p1 = 1);
+void launch_ckpt_load_bfp(const short *q, const float *scale, long long n, float *u, int grid, cudaStream_t s,
+                          int n1 = 1, int p1 = 1);
 // image on the model grid: the padded grid's model window of G
 void launch_add_f64(double *dst, const double *src, long long n, cudaStream_t s);
 void launch_image_cut(const float2 *G, const Grid &g, int nb, const int *n, int nd, double *out, cudaStream_t s);
@@ -438,9 +448,10 @@ struct Step3Launch {
     size_t smem;
 };
 bool stepB3_tma_eligible(int ndim, int nop, bool rho, const Grid &g);
-bool stepB3_tma_maps(CUtensorMap *maps, float *const u[2], const float *vel, const Grid &g);
+// (orders 2 to 8; g.p1 a multiple of 4)
+bool stepB3_tma_maps(CUtensorMap *maps, float *const u[2], const float *vel, const Grid &g, int nop);
 int march_planes(int n3, long long columns, int slots, int halo);
-Step3Launch stepB3_tma_shape(const Grid &g, int num_sms, int L);
+Step3Launch stepB3_tma_shape(const Grid &g, int num_sms, int L, int nop = 4);
 cudaError_t launch_stepB3_tma(bool exact, const CUtensorMap *maps, int icur, float *nxt, const StepBParams &sp,
                               const Step3Launch &sh, unsigned long long *counter, unsigned long long base, int *err,
                               cudaStream_t s);
@@ -455,7 +466,8 @@ cudaError_t launch_stepB3_adj(const CUtensorMap &g_halo, const CUtensorMap &y_ti
                               cudaStream_t s);
 // g = I vel2 nu (cells at least nop from every face), elementwise
 void launch_adj_g(const float *nu, const float *vel2, float *g, const Grid &gr, int nop, cudaStream_t s);
-bool make_tmap_3d(CUtensorMap *m, const float *base, int n1, int n2, int n3, int b1, int b2);
+// p1: cells from line to line (0: n1)
+bool make_tmap_3d(CUtensorMap *m, const float *base, int n1, int n2, int n3, int b1, int b2, int p1 = 0);
 // tensor-map boxes of the TMA step: the current level's halo box and the tile box
 void stepB3_tma_boxes(int *halo1, int *halo2, int *tile1, int *tile2);
 

@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(256) k_adjB(const float *__restrict__ X, float
     const int i3 = (NDIM == 3) ? (int)blockIdx.z : 0;
     const Grid g = p.g;
     if (i1 >= g.n1 || i2 >= g.n2) return;
-    const long long s2 = g.n1, s3 = (long long)g.n1 * g.n2;
+    const long long s2 = g.p1, s3 = (long long)g.p1 * g.n2;
     const long long i = i3 * s3 + i2 * s2 + i1;
     const bool in = interior<NOP, NDIM>(g, i1, i2, i3);
     const float x = X[i];
@@ -173,18 +173,18 @@ __global__ void k_abc_adj(float *mu, float *kap, const float *__restrict__ bl, c
     int n;
     if (AXIS == 1) {  // line (i3, i2), coefficients [n3][n2]
         if (t >= (long long)g.n2 * g.n3) return;
-        base = t * g.n1;
+        base = t * g.p1;
         st = 1;
         n = g.n1;
     } else if (AXIS == 2) {  // line (i3, i1), coefficients [n3][n1]
         if (t >= (long long)g.n1 * g.n3) return;
-        base = (t / g.n1) * g.n1 * (long long)g.n2 + t % g.n1;
-        st = g.n1;
+        base = (t / g.n1) * g.p1 * (long long)g.n2 + t % g.n1;
+        st = g.p1;
         n = g.n2;
     } else {  // line (i2, i1), coefficients [n2][n1]
         if (t >= (long long)g.n1 * g.n2) return;
-        base = t;
-        st = (long long)g.n1 * g.n2;
+        base = t / g.n1 * g.p1 + t % g.n1;
+        st = (long long)g.p1 * g.n2;
         n = g.n3;
     }
     const float cl = bl[t], ch = bh[t];
@@ -225,8 +225,8 @@ __global__ void k_abc_adj1_v4(float *__restrict__ mu, float *__restrict__ kap, c
     const long long line = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (line >= (long long)g.n2 * g.n3) return;
     const int q = g.n1 / 4;
-    float4 *M = reinterpret_cast<float4 *>(mu + line * g.n1);
-    float4 *K = reinterpret_cast<float4 *>(kap + line * g.n1);
+    float4 *M = reinterpret_cast<float4 *>(mu + line * g.p1);
+    float4 *K = reinterpret_cast<float4 *>(kap + line * g.p1);
     {  // i = n1-2, n1-3, n1-4, n1-5 (the forward's last update first), b = i - 1
         const float h = bh[line];
         float4 ma = M[q - 2], mb = M[q - 1], ka = K[q - 2], kb = K[q - 1];
@@ -302,7 +302,7 @@ __global__ void k_kap_fold(float *mu, float *kap, AdjParams p, int width) {
     } else {
         return;
     }
-    const long long i = ((long long)i3 * g.n2 + i2) * g.n1 + i1;
+    const long long i = ((long long)i3 * g.n2 + i2) * g.p1 + i1;
     const float kv = kap[i];
     if (kv != 0.f) {
         mu[i] += wcell(p, i1, i2, i3) * kv;
@@ -330,7 +330,7 @@ __global__ void k_rec_adj(float *mu, const GeoPoint *__restrict__ pts, int nr, c
     const int nc = p.nd == 3 ? 8 : 4;
     for (int c = 0; c < nc; c++) {
         const long long n = pt.base + off[c];
-        const int i1 = (int)(n % g.n1), i2 = (int)((n / g.n1) % g.n2), i3 = (int)(n / ((long long)g.n1 * g.n2));
+        const int i1 = (int)(n % g.p1), i2 = (int)((n / g.p1) % g.n2), i3 = (int)(n / ((long long)g.p1 * g.n2));
         const float w = wcell(p, i1, i2, i3);
         atomicAdd(mu + n, w * (w * (pt.w[c] * rv)));
     }
@@ -394,10 +394,15 @@ void launch_residual(const float *d, const float *dobs, float *r, int nrows, int
 // ---------------------------------------------------------------------------
 // Checkpoints: BF16 or FP16 with one FP32 scale per level (the level's
 // max |v|), or plain FP32 copies.
-__global__ void k_absmax(const float *__restrict__ u, long long n, unsigned int *out) {
+// cell i of the lines without their padding, in the level (p1 == n1: i itself)
+__device__ __forceinline__ long long line_cell(long long i, int n1, int p1) {
+    return p1 == n1 ? i : i / n1 * p1 + i % n1;
+}
+
+__global__ void k_absmax(const float *__restrict__ u, long long n, unsigned int *out, int n1, int p1) {
     float m = 0.f;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        m = fmaxf(m, fabsf(u[i]));
+        m = fmaxf(m, fabsf(u[line_cell(i, n1, p1)]));
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));  // non-negative floats order as unsigned
 }
@@ -411,35 +416,35 @@ __device__ __forceinline__ float from16(__half q) { return __half2float(q); }
 // values land in [-1, 1], inside FP16's normal range down to 6e-5 of the max
 template <typename Q>
 __global__ void k_quant16(const float *__restrict__ u, long long n, const unsigned int *__restrict__ amax,
-                          Q *__restrict__ q, float *__restrict__ scale_out) {
+                          Q *__restrict__ q, float *__restrict__ scale_out, int n1, int p1) {
     const float a = __uint_as_float(*amax);
     const float scale = a > 0.f ? a : 1.f;
     const float inv = 1.f / scale;
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        to16(u[i] * inv, q[i]);
+        to16(u[line_cell(i, n1, p1)] * inv, q[i]);
 }
 
 template <typename Q>
 __global__ void k_dequant16(const Q *__restrict__ q, long long n, const float *__restrict__ scale,
-                            float *__restrict__ u) {
+                            float *__restrict__ u, int n1, int p1) {
     const float sc = *scale;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        u[i] = from16(q[i]) * sc;
+        u[line_cell(i, n1, p1)] = from16(q[i]) * sc;
 }
 
 void launch_ckpt_store16(bool fp16, const float *u, long long n, unsigned int *amax, void *q, float *scale, int grid,
-                         cudaStream_t s) {
+                         cudaStream_t s, int n1, int p1) {
     cudaMemsetAsync(amax, 0, sizeof(unsigned int), s);
-    k_absmax<<<grid, 256, 0, s>>>(u, n, amax);
-    if (fp16) k_quant16<__half><<<grid, 256, 0, s>>>(u, n, amax, (__half *)q, scale);
-    else k_quant16<__nv_bfloat16><<<grid, 256, 0, s>>>(u, n, amax, (__nv_bfloat16 *)q, scale);
+    k_absmax<<<grid, 256, 0, s>>>(u, n, amax, n1, p1);
+    if (fp16) k_quant16<__half><<<grid, 256, 0, s>>>(u, n, amax, (__half *)q, scale, n1, p1);
+    else k_quant16<__nv_bfloat16><<<grid, 256, 0, s>>>(u, n, amax, (__nv_bfloat16 *)q, scale, n1, p1);
 }
 
 void launch_ckpt_load16(bool fp16, const void *q, long long n, const float *scale, float *u, int grid,
-                        cudaStream_t s) {
-    if (fp16) k_dequant16<__half><<<grid, 256, 0, s>>>((const __half *)q, n, scale, u);
-    else k_dequant16<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16 *)q, n, scale, u);
+                        cudaStream_t s, int n1, int p1) {
+    if (fp16) k_dequant16<__half><<<grid, 256, 0, s>>>((const __half *)q, n, scale, u, n1, p1);
+    else k_dequant16<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16 *)q, n, scale, u, n1, p1);
 }
 
 // Block floating point: each block of 64 consecutive cells keeps 16-bit
@@ -451,13 +456,13 @@ void launch_ckpt_load16(bool fp16, const void *q, long long n, const float *scal
 // restatement gets the same integers.  Unlike the per-level formats no
 // separate max pass over the level is needed.
 __global__ void k_bfp_store(const float *__restrict__ u, long long n, short *__restrict__ q,
-                            float *__restrict__ scale) {
+                            float *__restrict__ scale, int n1, int p1) {
     const int lane = threadIdx.x & 31;
     const long long nblk = (n + kBfpBlock - 1) / kBfpBlock;
     const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
     for (long long b = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < nblk; b += warps) {
         const long long i0 = b * kBfpBlock + lane, i1 = i0 + 32;
-        const float v0 = i0 < n ? u[i0] : 0.f, v1 = i1 < n ? u[i1] : 0.f;
+        const float v0 = i0 < n ? u[line_cell(i0, n1, p1)] : 0.f, v1 = i1 < n ? u[line_cell(i1, n1, p1)] : 0.f;
         float m = fmaxf(fabsf(v0), fabsf(v1));
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
         // blocks at or below kBfpTiny store zeros (keeps s and 1/s normal floats)
@@ -472,17 +477,19 @@ __global__ void k_bfp_store(const float *__restrict__ u, long long n, short *__r
 }
 
 __global__ void k_bfp_load(const short *__restrict__ q, const float *__restrict__ scale, long long n,
-                           float *__restrict__ u) {
+                           float *__restrict__ u, int n1, int p1) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        u[i] = __fmul_rn(__int2float_rn(q[i]), scale[i / kBfpBlock]);
+        u[line_cell(i, n1, p1)] = __fmul_rn(__int2float_rn(q[i]), scale[i / kBfpBlock]);
 }
 
-void launch_ckpt_store_bfp(const float *u, long long n, short *q, float *scale, int grid, cudaStream_t s) {
-    k_bfp_store<<<grid, 256, 0, s>>>(u, n, q, scale);
+void launch_ckpt_store_bfp(const float *u, long long n, short *q, float *scale, int grid, cudaStream_t s, int n1,
+                           int p1) {
+    k_bfp_store<<<grid, 256, 0, s>>>(u, n, q, scale, n1, p1);
 }
 
-void launch_ckpt_load_bfp(const short *q, const float *scale, long long n, float *u, int grid, cudaStream_t s) {
-    k_bfp_load<<<grid, 256, 0, s>>>(q, scale, n, u);
+void launch_ckpt_load_bfp(const short *q, const float *scale, long long n, float *u, int grid, cudaStream_t s, int n1,
+                          int p1) {
+    k_bfp_load<<<grid, 256, 0, s>>>(q, scale, n, u, n1, p1);
 }
 
 // ---------------------------------------------------------------------------
@@ -524,7 +531,7 @@ __global__ void k_grad_fold(const float2 *__restrict__ G, const float *__restric
     for (int i3 = a3; i3 <= b3; i3++)
         for (int i2 = a2; i2 <= b2; i2++)
             for (int i1 = a1; i1 <= b1; i1++) {
-                const long long i = ((long long)i3 * g.n2 + i2) * g.n1 + i1;
+                const long long i = ((long long)i3 * g.n2 + i2) * g.p1 + i1;
                 const double v2 = fold_c(vel2, i, cscale);
                 acc += gsum_value(G[i]) * (-v2 * v2 * inv_dt2);
             }
@@ -536,7 +543,7 @@ __global__ void k_image_cut(const float2 *__restrict__ G, Grid g, int nb, int m1
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)m1 * m2 * m3) return;
     const int j1 = (int)(t % m1), j2 = (int)((t / m1) % m2), j3 = (int)(t / ((long long)m1 * m2));
-    out[t] = gsum_value(G[((long long)(nd == 3 ? j3 + nb : 0) * g.n2 + j2 + nb) * g.n1 + j1 + nb]);
+    out[t] = gsum_value(G[((long long)(nd == 3 ? j3 + nb : 0) * g.n2 + j2 + nb) * g.p1 + j1 + nb]);
 }
 
 // dst += src (gradients of several shots)
@@ -589,7 +596,7 @@ __global__ void __launch_bounds__(256) k_grad_fold_big(const float2 *__restrict_
     double acc = 0;
     for (long long k = threadIdx.x; k < vol; k += blockDim.x) {
         const long long i1 = a1 + k % w1, i2 = a2 + (k / w1) % w2, i3 = a3 + k / (w1 * w2);
-        const long long i = (i3 * g.n2 + i2) * g.n1 + i1;
+        const long long i = (i3 * g.n2 + i2) * g.p1 + i1;
         const double v2 = fold_c(vel2, i, cscale);
         acc += gsum_value(G[i]) * (-v2 * v2 * inv_dt2);
     }

@@ -7,12 +7,12 @@
 //
 // The reference applies the ABC as three passes over the whole grid (axis-1
 // lines, then axis-2 lines, then axis-3 lines, each an outward recurrence over
-// the nop = 4 outer cells from the fifth), then the sponge.  The passes only
-// meet in the shell (cells within 6 of a face), so the work splits into
+// the nop outer cells from cell nop + 1), then the sponge.  The passes only
+// meet in the shell (cells within nop + 2 of a face), so the work splits into
 // blocks that each own a whole chain of dependencies:
-//  * a plane y in [6, n3-6) (no axis-3 face cell): its axis-1 line ends, then
+//  * a plane y in [nop+2, n3-nop-2) (no axis-3 face cell): its axis-1 line ends, then
 //    (after a barrier) its axis-2 line ends, each sponged once it is final;
-//  * a face block (planes 0..5 or n3-6..n3-1) x a 16-column x-range x a
+//  * a face block (the nop + 2 planes of a y face) x a 16-column x-range x a
 //    64-cell z-range: the axis-1 pass of its lines, the axis-2 pass of its
 //    z-range (x-ranges holding a face), the axis-3 pass of its columns, then
 //    the sponge of all its cells;
@@ -22,7 +22,7 @@
 // the order in which blocks run.
 //
 // The axis-1 ends (8 cells at each end of every line, 32 bytes of every
-// n1*4-byte line) are the scattered part of the work.  Within a forward run
+// p1*4-byte line) are the scattered part of the work.  Within a forward run
 // each launch also writes the final ends of the new level to a compact
 // [n3][n2][16] copy, and the next step's launch reads the ends of the level
 // its step read (the same values) from that copy with coalesced loads
@@ -35,7 +35,7 @@
 namespace awe {
 
 namespace b3 {
-constexpr int SHELL = 6;  // nop + 2: cells the ABC writes (1..4) or reads (5), and the face cell 0
+constexpr int SHELL = 6;  // the adjoint's nop + 2 (nop = 4): cells the ABC writes (1..4) or reads (5), and the face cell 0
 constexpr int XR = 16, ZR = 64;
 constexpr int NT = 256;
 }  // namespace b3
@@ -51,142 +51,160 @@ __device__ __forceinline__ float b3_damp(float v, float wz, float wx, float wy) 
     return fmul<EXACT>(fmul<EXACT>(fmul<EXACT>(v, wz), wx), wy);
 }
 
-// axis-1 low face of one line: cells 4, 3, 2, 1 from cell 5 (a = cells 0..3, b = 4..7)
-template <bool EXACT>
-__device__ __forceinline__ void b3_zlow(float4 &a, float4 &b, const float4 ma, const float4 mb, float c) {
-    const float u4 = b3_abc<EXACT>(mb.y, mb.x, b.y, c);
-    const float u3 = b3_abc<EXACT>(mb.x, ma.w, u4, c);
-    const float u2 = b3_abc<EXACT>(ma.w, ma.z, u3, c);
-    a.y = b3_abc<EXACT>(ma.z, ma.y, u2, c);
-    a.z = u2;
-    a.w = u3;
-    b.x = u4;
+// Axis-1 line ends: cells 0..7 and n1-8..n1-1 in registers.  Lines start on
+// 16-byte boundaries (the pitch p1), so the low end is two 16-byte accesses;
+// the high end is too where n1 % 4 == 0 (AL), else 8 scalar ones in the same
+// two sectors.
+template <bool AL>
+__device__ __forceinline__ void b3_ld8(float (&v)[8], const float *a) {
+    if constexpr (AL) {
+        const float4 x = *reinterpret_cast<const float4 *>(a), y = *reinterpret_cast<const float4 *>(a + 4);
+        v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = a[k];
+    }
 }
 
-// axis-1 high face: cells n1-5 .. n1-2 from n1-6 (a = cells n1-8..n1-5, b = n1-4..n1-1)
-template <bool EXACT>
-__device__ __forceinline__ void b3_zhigh(float4 &a, float4 &b, const float4 ma, const float4 mb, float c) {
-    const float v5 = b3_abc<EXACT>(ma.z, ma.w, a.z, c);
-    const float v4 = b3_abc<EXACT>(ma.w, mb.x, v5, c);
-    const float v3 = b3_abc<EXACT>(mb.x, mb.y, v4, c);
-    b.z = b3_abc<EXACT>(mb.y, mb.z, v3, c);
-    a.w = v5;
-    b.x = v4;
-    b.y = v3;
+template <bool AL>
+__device__ __forceinline__ void b3_st8(float *a, const float (&v)[8]) {
+    if constexpr (AL) {
+        *reinterpret_cast<float4 *>(a) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4 *>(a + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; k++) a[k] = v[k];
+    }
 }
 
-template <bool EXACT>
-__device__ __forceinline__ void b3_damp4(float4 &v, const float *w1, int z, float wx, float wy, unsigned mask) {
-    const float4 wz = __ldg(reinterpret_cast<const float4 *>(w1 + z));
-    if (mask & 1u) v.x = b3_damp<EXACT>(v.x, wz.x, wx, wy);
-    if (mask & 2u) v.y = b3_damp<EXACT>(v.y, wz.y, wx, wy);
-    if (mask & 4u) v.z = b3_damp<EXACT>(v.z, wz.z, wx, wy);
-    if (mask & 8u) v.w = b3_damp<EXACT>(v.w, wz.w, wx, wy);
+// low face: cells NOP .. 1 from cell NOP+1
+template <bool EXACT, int NOP>
+__device__ __forceinline__ void b3_zlow(float (&v)[8], const float (&m)[8], float c) {
+#pragma unroll
+    for (int k = NOP; k >= 1; k--) v[k] = b3_abc<EXACT>(m[k + 1], m[k], v[k + 1], c);
 }
 
-// one axis-2 face line (y, z): cells x = xa+dx .. xa+4dx from xa (outward),
-// optionally sponged (cells xs .. xs+5 of the line, the axis-2 shell)
-template <bool EXACT>
+// high face: cells n1-1-NOP .. n1-2 from n1-2-NOP (v[7] is cell n1-1)
+template <bool EXACT, int NOP>
+__device__ __forceinline__ void b3_zhigh(float (&v)[8], const float (&m)[8], float c) {
+#pragma unroll
+    for (int k = NOP; k >= 1; k--) v[7 - k] = b3_abc<EXACT>(m[6 - k], m[7 - k], v[6 - k], c);
+}
+
+// sponge of the elements of an end that lie in the shell (mask bit per element; w = w1 at element 0)
+template <bool EXACT, bool AL>
+__device__ __forceinline__ void b3_damp8(float (&v)[8], const float *w, float wx, float wy, unsigned mask) {
+    float wz[8];
+    b3_ld8<AL>(wz, w);
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        if ((mask >> k) & 1u) v[k] = b3_damp<EXACT>(v[k], wz[k], wx, wy);
+}
+
+// one axis-2 face line (y, z): the NOP cells outward from xa, optionally
+// sponged (the NOP + 2 shell cells of the line)
+template <bool EXACT, int NOP>
 __device__ __forceinline__ void b3_xline(const Bnd3Params &p, long long c0, int y, int z, bool low, bool damp) {
-    const long long s2 = p.g.n1;
-    const int xa = low ? 5 : p.g.n2 - b3::SHELL, dx = low ? -1 : 1;
+    constexpr int SHELL = NOP + 2;
+    const long long s2 = p.g.p1;
+    const int xa = low ? NOP + 1 : p.g.n2 - SHELL, dx = low ? -1 : 1;
     const float b = __ldg((low ? p.xl : p.xh) + (long long)y * p.g.n1 + z);
-    float v[6];  // cells xa .. xa + 5dx (the last one is the face cell 0 / n2-1)
+    float v[SHELL];  // cells xa .. the face cell 0 / n2-1
 #pragma unroll
-    for (int k = 0; k < 6; k++) v[k] = p.uo[c0 + (long long)(xa + k * dx) * s2];
-    float m[5];
+    for (int k = 0; k < SHELL; k++) v[k] = p.uo[c0 + (long long)(xa + k * dx) * s2];
+    float m[NOP + 1];
 #pragma unroll
-    for (int k = 0; k < 5; k++) m[k] = __ldg(p.um + c0 + (long long)(xa + k * dx) * s2);
+    for (int k = 0; k <= NOP; k++) m[k] = __ldg(p.um + c0 + (long long)(xa + k * dx) * s2);
 #pragma unroll
-    for (int k = 1; k <= 4; k++) v[k] = b3_abc<EXACT>(m[k - 1], m[k], v[k - 1], b);
+    for (int k = 1; k <= NOP; k++) v[k] = b3_abc<EXACT>(m[k - 1], m[k], v[k - 1], b);
     if (damp) {
         const float wz = __ldg(p.w1 + z), wy = __ldg(p.w3 + y);
 #pragma unroll
-        for (int k = 0; k < 6; k++) v[k] = b3_damp<EXACT>(v[k], wz, __ldg(p.w2 + xa + k * dx), wy);
+        for (int k = 0; k < SHELL; k++) v[k] = b3_damp<EXACT>(v[k], wz, __ldg(p.w2 + xa + k * dx), wy);
         p.uo[c0 + (long long)xa * s2] = v[0];
-        p.uo[c0 + (long long)(xa + 5 * dx) * s2] = v[5];
+        p.uo[c0 + (long long)(xa + (NOP + 1) * dx) * s2] = v[NOP + 1];
     }
 #pragma unroll
-    for (int k = 1; k <= 4; k++) p.uo[c0 + (long long)(xa + k * dx) * s2] = v[k];
+    for (int k = 1; k <= NOP; k++) p.uo[c0 + (long long)(xa + k * dx) * s2] = v[k];
 }
 
-// float4 `part` of line `line`'s ends (parts 0, 1: cells 0..7; 2, 3: cells
-// n1-8..n1-1) of the level the step read: from the compact copy of its line
-// ends the previous step's launch wrote (em), else from the level itself
-__device__ __forceinline__ float4 b3_mend(const Bnd3Params &p, long long line, int part) {
-    if (p.em) return __ldg(reinterpret_cast<const float4 *>(p.em) + line * 4 + part);
-    const float4 *m = reinterpret_cast<const float4 *>(p.um + line * p.g.n1);
-    return __ldg(m + (part < 2 ? part : p.g.n1 / 4 - 4 + part));
+// an end (0: cells 0..7, 1: cells n1-8..n1-1) of line `line` of the level the
+// step read: from the compact copy of its line ends the previous step's
+// launch wrote (em), else from the level itself
+template <bool AL>
+__device__ __forceinline__ void b3_mend(const Bnd3Params &p, float (&m)[8], long long line, int end) {
+    if (p.em) return b3_ld8<true>(m, p.em + line * 16 + 8 * end);
+    const float *r = p.um + line * p.g.p1;
+    if (end == 0) b3_ld8<true>(m, r);
+    else b3_ld8<AL>(m, r + p.g.n1 - 8);
 }
 
 // the compact copy of the new level's line ends (eo), read back from uo once
-// the line's cells are final
+// the line's cells are final; part 0..3: 4 cells each
+template <bool AL>
 __device__ __forceinline__ void b3_eput_from_uo(const Bnd3Params &p, long long line, int part) {
-    const float4 *o = reinterpret_cast<const float4 *>(p.uo + line * p.g.n1);
-    reinterpret_cast<float4 *>(p.eo)[line * 4 + part] = o[part < 2 ? part : p.g.n1 / 4 - 4 + part];
+    const float *o = p.uo + line * p.g.p1 + (part < 2 ? 4 * part : p.g.n1 - 16 + 4 * part);
+    float4 v;
+    if (AL || part < 2) v = *reinterpret_cast<const float4 *>(o);
+    else v = make_float4(o[0], o[1], o[2], o[3]);
+    reinterpret_cast<float4 *>(p.eo)[line * 4 + part] = v;
 }
 
-template <bool EXACT>
+template <bool EXACT, int NOP, bool AL>
 __global__ void __launch_bounds__(b3::NT, 4) k_bnd3(const Bnd3Params p) {
-    using namespace b3;
+    using b3::NT, b3::XR, b3::ZR;
+    constexpr int SHELL = NOP + 2;
+    // elements of an end (of 8) that lie in the shell
+    constexpr unsigned LOW = (1u << SHELL) - 1u, HIGH = LOW << (8 - SHELL);
     const int tid = threadIdx.x;
     const int n1 = p.g.n1, n2 = p.g.n2, n3 = p.g.n3;
-    const long long s2 = n1, s3 = (long long)n1 * n2;
+    const long long s2 = p.g.p1, s3 = s2 * n2;
     int blk = blockIdx.x;
 
     if (blk < p.n_int) {  // ---- one plane without axis-3 face cells
         const int y = SHELL + blk;
         const float wy = p.w3 ? __ldg(p.w3 + y) : 1.f;
-        const int q = n1 / 4;
         for (int x = tid; x < n2; x += NT) {
             const long long line = (long long)y * n2 + x;
-            float4 *o = reinterpret_cast<float4 *>(p.uo + line * n1);
+            float *o = p.uo + line * s2;
             // lines in the axis-2 shell are sponged by the axis-2 pass below
             const bool xshell = x < SHELL || x >= n2 - SHELL;
             const bool damp = p.w1 && !xshell;
             const float wx = damp ? __ldg(p.w2 + x) : 1.f;
-            float4 lo0 = make_float4(0.f, 0.f, 0.f, 0.f), lo1 = lo0;  // cells 0..7 as left
+            float lo[8] = {}, hi[8], m[8];  // both ends as left
             if (p.top || damp) {
-                lo0 = o[0];
-                lo1 = o[1];
-                if (p.top) b3_zlow<EXACT>(lo0, lo1, b3_mend(p, line, 0), b3_mend(p, line, 1), __ldg(p.zl + line));
-                if (damp) {
-                    b3_damp4<EXACT>(lo0, p.w1, 0, wx, wy, 15u);
-                    b3_damp4<EXACT>(lo1, p.w1, 4, wx, wy, 3u);
+                b3_ld8<true>(lo, o);
+                if (p.top) {
+                    b3_mend<AL>(p, m, line, 0);
+                    b3_zlow<EXACT, NOP>(lo, m, __ldg(p.zl + line));
                 }
-                o[0] = lo0;
-                o[1] = lo1;
+                if (damp) b3_damp8<EXACT, true>(lo, p.w1, wx, wy, LOW);
+                b3_st8<true>(o, lo);
             }
-            float4 a = o[q - 2], b = o[q - 1];
-            b3_zhigh<EXACT>(a, b, b3_mend(p, line, 2), b3_mend(p, line, 3), __ldg(p.zh + line));
-            if (damp) {
-                b3_damp4<EXACT>(a, p.w1, n1 - 8, wx, wy, 12u);
-                b3_damp4<EXACT>(b, p.w1, n1 - 4, wx, wy, 15u);
-            }
-            o[q - 2] = a;
-            o[q - 1] = b;
+            b3_ld8<AL>(hi, o + n1 - 8);
+            b3_mend<AL>(p, m, line, 1);
+            b3_zhigh<EXACT, NOP>(hi, m, __ldg(p.zh + line));
+            if (damp) b3_damp8<EXACT, AL>(hi, p.w1 + n1 - 8, wx, wy, HIGH);
+            b3_st8<AL>(o + n1 - 8, hi);
             // final unless the axis-2 pass changes the line (the axis-2 shell);
             // without a sponge and with a free surface the low end is not
             // read (nor needed: the next step's low-end ABC is off)
             if (p.eo && !xshell) {
-                float4 *e = reinterpret_cast<float4 *>(p.eo) + line * 4;
-                e[0] = lo0;
-                e[1] = lo1;
-                e[2] = a;
-                e[3] = b;
+                b3_st8<true>(p.eo + line * 16, lo);
+                b3_st8<true>(p.eo + line * 16 + 8, hi);
             }
         }
-        __syncthreads();  // the axis-2 pass reads the axis-1 results of lines x = 1..5
+        __syncthreads();  // the axis-2 pass reads the axis-1 results of lines x = 1..NOP+1
         for (int z = tid; z < n1; z += NT) {
             const long long c0 = (long long)y * s3 + z;
-            b3_xline<EXACT>(p, c0, y, z, true, p.w1 != nullptr);
-            b3_xline<EXACT>(p, c0, y, z, false, p.w1 != nullptr);
+            b3_xline<EXACT, NOP>(p, c0, y, z, true, p.w1 != nullptr);
+            b3_xline<EXACT, NOP>(p, c0, y, z, false, p.w1 != nullptr);
         }
         if (p.eo) {  // the axis-2 shell lines' ends, final now
             __syncthreads();
             for (int l = tid; l < 2 * SHELL * 4; l += NT) {
                 const int k = l >> 2, x = k < SHELL ? k : n2 - 2 * SHELL + k;
-                b3_eput_from_uo(p, (long long)y * n2 + x, l & 3);
+                b3_eput_from_uo<AL>(p, (long long)y * n2 + x, l & 3);
             }
         }
         return;
@@ -196,26 +214,27 @@ __global__ void __launch_bounds__(b3::NT, 4) k_bnd3(const Bnd3Params p) {
         const int f = blk / (p.nxr * p.nzr), r = blk % (p.nxr * p.nzr), xr = r / p.nzr, zr = r % p.nzr;
         const int xa = xr * XR, xb = xr == p.nxr - 1 ? n2 : xa + XR;
         const int za = zr * ZR, zb = zr == p.nzr - 1 ? n1 : za + ZR;
-        const int ya = f == 0 ? 0 : n3 - SHELL;  // planes [ya, ya + 6)
-        const int ncol = xb - xa, nz = zb - za, q = n1 / 4;
+        const int ya = f == 0 ? 0 : n3 - SHELL;  // planes [ya, ya + SHELL)
+        const int ncol = xb - xa, nz = zb - za;
         // axis 1: the line ends inside this z-range
         const bool zlo = zr == 0 && p.top, zhi = zr == p.nzr - 1;
         if (zlo || zhi)
             for (int l = tid; l < SHELL * ncol; l += NT) {
                 const int y = ya + l / ncol, x = xa + l % ncol;
                 const long long line = (long long)y * n2 + x;
-                float4 *o = reinterpret_cast<float4 *>(p.uo + line * n1);
+                float *o = p.uo + line * s2;
+                float v[8], m[8];
                 if (zlo) {
-                    float4 a = o[0], b = o[1];
-                    b3_zlow<EXACT>(a, b, b3_mend(p, line, 0), b3_mend(p, line, 1), __ldg(p.zl + line));
-                    o[0] = a;
-                    o[1] = b;
+                    b3_ld8<true>(v, o);
+                    b3_mend<AL>(p, m, line, 0);
+                    b3_zlow<EXACT, NOP>(v, m, __ldg(p.zl + line));
+                    b3_st8<true>(o, v);
                 }
                 if (zhi) {
-                    float4 a = o[q - 2], b = o[q - 1];
-                    b3_zhigh<EXACT>(a, b, b3_mend(p, line, 2), b3_mend(p, line, 3), __ldg(p.zh + line));
-                    o[q - 2] = a;
-                    o[q - 1] = b;
+                    b3_ld8<AL>(v, o + n1 - 8);
+                    b3_mend<AL>(p, m, line, 1);
+                    b3_zhigh<EXACT, NOP>(v, m, __ldg(p.zh + line));
+                    b3_st8<AL>(o + n1 - 8, v);
                 }
             }
         __syncthreads();
@@ -225,19 +244,19 @@ __global__ void __launch_bounds__(b3::NT, 4) k_bnd3(const Bnd3Params p) {
             for (int l = tid; l < SHELL * nz; l += NT) {
                 const int y = ya + l / nz, z = za + l % nz;
                 const long long c0 = (long long)y * s3 + z;
-                if (xlo) b3_xline<EXACT>(p, c0, y, z, true, false);
-                if (xhi) b3_xline<EXACT>(p, c0, y, z, false, false);
+                if (xlo) b3_xline<EXACT, NOP>(p, c0, y, z, true, false);
+                if (xhi) b3_xline<EXACT, NOP>(p, c0, y, z, false, false);
             }
         __syncthreads();
-        // axis 3: columns (x, z), planes 4..1 from 5 or n3-5..n3-2 from n3-6
+        // axis 3: columns (x, z), planes NOP..1 from NOP+1 or n3-1-NOP..n3-2 from n3-2-NOP
         for (int l = tid; l < ncol * nz; l += NT) {
             const int x = xa + l / nz, z = za + l % nz;
             const long long c0 = (long long)x * s2 + z;
-            const int y0 = f == 0 ? 5 : n3 - SHELL, dy = f == 0 ? -1 : 1;
+            const int y0 = f == 0 ? NOP + 1 : n3 - SHELL, dy = f == 0 ? -1 : 1;
             const float b = __ldg((f == 0 ? p.yl : p.yh) + (long long)x * n1 + z);
             float v = p.uo[c0 + (long long)y0 * s3], mprev = __ldg(p.um + c0 + (long long)y0 * s3);
 #pragma unroll
-            for (int k = 1; k <= 4; k++) {
+            for (int k = 1; k <= NOP; k++) {
                 const long long c = c0 + (long long)(y0 + k * dy) * s3;
                 const float mc = __ldg(p.um + c);
                 v = b3_abc<EXACT>(mprev, mc, v, b);
@@ -247,13 +266,17 @@ __global__ void __launch_bounds__(b3::NT, 4) k_bnd3(const Bnd3Params p) {
         }
         if (p.w1) {
             __syncthreads();
-            // sponge of every cell of the block (all lie in the axis-3 shell)
-            const int nq = nz / 4;
+            // sponge of every cell of the block (all lie in the axis-3 shell);
+            // the pad cells of a line hold 0, their factors 1
+            const int nq = (nz + 3) / 4;
             for (int l = tid; l < SHELL * ncol * nq; l += NT) {
                 const int y = ya + l / (ncol * nq), k = l % (ncol * nq), x = xa + k / nq, z = za + 4 * (k % nq);
                 float4 *c = reinterpret_cast<float4 *>(p.uo + (long long)y * s3 + (long long)x * s2 + z);
                 float4 v = *c;
-                b3_damp4<EXACT>(v, p.w1, z, __ldg(p.w2 + x), __ldg(p.w3 + y), 15u);
+                const float4 wz = __ldg(reinterpret_cast<const float4 *>(p.w1 + z));
+                const float wx = __ldg(p.w2 + x), wy = __ldg(p.w3 + y);
+                v = make_float4(b3_damp<EXACT>(v.x, wz.x, wx, wy), b3_damp<EXACT>(v.y, wz.y, wx, wy),
+                                b3_damp<EXACT>(v.z, wz.z, wx, wy), b3_damp<EXACT>(v.w, wz.w, wx, wy));
                 *c = v;
             }
         }
@@ -262,7 +285,7 @@ __global__ void __launch_bounds__(b3::NT, 4) k_bnd3(const Bnd3Params p) {
             for (int l = tid; l < SHELL * ncol * 4; l += NT) {
                 const int k = l >> 2, part = l & 3;
                 if (part < 2 ? zr != 0 : zr != p.nzr - 1) continue;
-                b3_eput_from_uo(p, (long long)(ya + k / ncol) * n2 + xa + k % ncol, part);
+                b3_eput_from_uo<AL>(p, (long long)(ya + k / ncol) * n2 + xa + k % ncol, part);
             }
         }
         return;
@@ -279,8 +302,8 @@ __global__ void __launch_bounds__(b3::NT, 4) k_bnd3(const Bnd3Params p) {
             float v = __ldg(p.um + n);
             if (p.w1) {
                 const int i3 = (int)(n / s3), rem = (int)(n % s3);
-                v = fmul<EXACT>(v, __ldg(p.w1 + rem % n1));
-                v = fmul<EXACT>(v, __ldg(p.w2 + rem / n1));
+                v = fmul<EXACT>(v, __ldg(p.w1 + rem % (int)s2));
+                v = fmul<EXACT>(v, __ldg(p.w2 + rem / (int)s2));
                 v = fmul<EXACT>(v, __ldg(p.w3 + i3));
             }
             const float t = fmul<EXACT>(v, pt.w[c]);
@@ -318,18 +341,29 @@ __global__ void __launch_bounds__(b3::NT, 4) k_bnd3(const Bnd3Params p) {
 }
 
 bool bnd3_eligible(int nop, const Grid &g) {
-    return nop == 4 && g.n1 % 4 == 0 && g.n1 >= 16 && g.n2 >= 2 * b3::SHELL && g.n3 >= 2 * b3::SHELL;
+    // both ends of a line in their 8 cells, every face's shell apart from the opposite one
+    return nop <= 4 && g.p1 % 4 == 0 && g.n1 >= 16 && g.n2 >= 2 * (nop + 2) && g.n3 >= 2 * (nop + 2);
+}
+
+template <bool EXACT, int NOP>
+static void launch_bnd3_nop(const Bnd3Params &p, int grid, cudaStream_t s) {
+    if (p.g.n1 % 4 == 0) k_bnd3<EXACT, NOP, true><<<grid, b3::NT, 0, s>>>(p);
+    else k_bnd3<EXACT, NOP, false><<<grid, b3::NT, 0, s>>>(p);
 }
 
 void launch_bnd3(bool exact, Bnd3Params p, cudaStream_t s) {
     using namespace b3;
-    p.n_int = p.g.n3 - 2 * SHELL;
+    p.n_int = p.g.n3 - 2 * (p.nop + 2);
     p.nxr = p.g.n2 / XR > 0 ? p.g.n2 / XR : 1;
     p.nzr = p.g.n1 / ZR > 0 ? p.g.n1 / ZR : 1;
     p.rec_blocks = p.rec_row ? (p.nr + NT - 1) / NT : 0;
     const int grid = p.n_int + 2 * p.nxr * p.nzr + p.rec_blocks + (p.inj.n > 0 ? (p.inj.n + NT - 1) / NT : p.ns > 0 ? 1 : 0);
-    if (exact) k_bnd3<true><<<grid, NT, 0, s>>>(p);
-    else k_bnd3<false><<<grid, NT, 0, s>>>(p);
+    switch (p.nop) {
+        case 1: return exact ? launch_bnd3_nop<true, 1>(p, grid, s) : launch_bnd3_nop<false, 1>(p, grid, s);
+        case 2: return exact ? launch_bnd3_nop<true, 2>(p, grid, s) : launch_bnd3_nop<false, 2>(p, grid, s);
+        case 3: return exact ? launch_bnd3_nop<true, 3>(p, grid, s) : launch_bnd3_nop<false, 3>(p, grid, s);
+        default: return exact ? launch_bnd3_nop<true, 4>(p, grid, s) : launch_bnd3_nop<false, 4>(p, grid, s);
+    }
 }
 
 // ---------------------------------------------------------------------------

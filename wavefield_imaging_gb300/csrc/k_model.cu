@@ -39,7 +39,7 @@ __global__ void k_model_pad(const float *__restrict__ raw, float *__restrict__ o
         v = __fmul_rn(v, __fmul_rn(v, m.dt2));
         if (i1 < m.zero1) v = 0.f;
     }
-    out[i] = v;
+    out[r * m.g.p1 + i1] = v;
 }
 
 __device__ __forceinline__ float abc_coef(float v, float dt, float dd) {
@@ -75,7 +75,7 @@ __global__ void k_model_abc(const float *__restrict__ raw, const ModelPrep m, fl
 }  // namespace
 
 void launch_model_pad(const float *raw, float *out, const ModelPrep &m, bool vel2, cudaStream_t s) {
-    const long long cells = m.g.cells();
+    const long long cells = (long long)m.g.n1 * m.g.n2 * m.g.n3;
     k_model_pad<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(raw, out, m, vel2 ? 1 : 0);
 }
 

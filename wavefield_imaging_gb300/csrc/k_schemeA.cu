@@ -550,7 +550,7 @@ __global__ void k_rec_adjA(float *z, const GeoPoint *__restrict__ pts, int nr, c
     const Grid g = p.g;
     for (int k = 0; k < 8; k++) {
         const long long j = pt.base + off[k];
-        const int c0 = (int)(j % g.n1), c1 = (int)((j / g.n1) % g.n2), c2 = (int)(j / ((long long)g.n1 * g.n2));
+        const int c0 = (int)(j % g.p1), c1 = (int)((j / g.p1) % g.n2), c2 = (int)(j / ((long long)g.p1 * g.n2));
         if (p.mask == 3 && (c0 > g.n1 - p.nb || (c0 < p.spill && (c1 >= 1 || c2 >= 1)))) continue;
         const int si = sponge_index3(c0, c1, c2, g.n1, g.n2, g.n3, p);
         atomicAdd(z + j, damp_a<false>(pt.w[k] * rv, si, p.dtab, p.ftab));

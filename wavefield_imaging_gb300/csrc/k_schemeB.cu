@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(256) k_stepB(const float *__restrict__ cur, fl
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
     const Grid g = p.g;
-    const long long s2 = g.n1, s3 = (long long)g.n1 * g.n2;
+    const long long s2 = g.p1, s3 = (long long)g.p1 * g.n2;
     if (NDIM == 2 && p.ext_n > 0) {
         const int rows = (g.n2 + (int)blockDim.y - 1) / (int)blockDim.y;  // blocks of cells
         if ((int)blockIdx.y >= rows) {  // receiver gather of `cur`, lint2d_extract's order
@@ -212,7 +212,7 @@ __global__ void k_abc_axis1(float *__restrict__ uo, const float *__restrict__ um
                             const float *__restrict__ bh, Grid g, int nop, int top) {
     const int line = blockIdx.x * blockDim.x + threadIdx.x;  // (i3, i2)
     if (line >= g.n2 * g.n3) return;
-    const long long c = (long long)line * g.n1;
+    const long long c = (long long)line * g.p1;
     const float l = bl[line], h = bh[line];
     // the sweep keeps the value it just wrote in a register (the next cell
     // reads it), so each face costs one pass over its nop+2 samples; the two
@@ -256,8 +256,8 @@ __global__ void k_abc_axis1_v4(float *__restrict__ uo, const float *__restrict__
     if (line >= g.n2 * g.n3) return;
     const int q = g.n1 / 4, i2 = line % g.n2, i3 = line / g.n2;
     const bool sp = w1 && i2 >= band && i2 < g.n2 - band && i3 >= band && i3 < g.n3 - band;
-    const float4 *m = reinterpret_cast<const float4 *>(um + (long long)line * g.n1);
-    float4 *o = reinterpret_cast<float4 *>(uo + (long long)line * g.n1);
+    const float4 *m = reinterpret_cast<const float4 *>(um + (long long)line * g.p1);
+    float4 *o = reinterpret_cast<float4 *>(uo + (long long)line * g.p1);
     if (top || sp) {  // iz = 4, 3, 2, 1 from uo[5]
         float4 oa = o[0], ob = o[1];
         if (top) {
@@ -302,7 +302,7 @@ __global__ void k_abc_axis2(float *uo, const float *__restrict__ um, const float
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)g.n1 * g.n3) return;
     const long long i3 = t / g.n1, i1 = t % g.n1;
-    const long long s2 = g.n1, base = i3 * g.n1 * (long long)g.n2 + i1;
+    const long long s2 = g.p1, base = i3 * g.p1 * (long long)g.n2 + i1;
     const float l = bl[t], h = bh[t];
     for (int iop = 0; iop < nop; iop++) {
         long long c = base + (long long)(nop - iop) * s2;
@@ -318,12 +318,12 @@ __global__ void k_abc_axis3(float *uo, const float *__restrict__ um, const float
                             const float *__restrict__ bh, Grid g, int nop) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)g.n1 * g.n2) return;
-    const long long s3 = (long long)g.n1 * g.n2;
+    const long long s3 = (long long)g.p1 * g.n2, o = t / g.n1 * g.p1 + t % g.n1;
     const float l = bl[t], h = bh[t];
     for (int iop = 0; iop < nop; iop++) {
-        long long c = (long long)(nop - iop) * s3 + t;
+        long long c = (long long)(nop - iop) * s3 + o;
         uo[c] = abc_update<EXACT>(um[c + s3], um[c], uo[c + s3], l);
-        c = (long long)(g.n3 - nop + iop - 1) * s3 + t;
+        c = (long long)(g.n3 - nop + iop - 1) * s3 + o;
         uo[c] = abc_update<EXACT>(um[c - s3], um[c], uo[c - s3], h);
     }
 }
@@ -378,20 +378,20 @@ __global__ void k_hybrid_axis(float *u2, const float *__restrict__ u1, const flo
     if (axis == 1) {
         nlines = (long long)g.n2 * g.n3;
         if (t >= nlines) return;
-        base = t * g.n1;
+        base = t * g.p1;
         stride = 1;
         n = g.n1;
     } else if (axis == 2) {
         nlines = (long long)g.n1 * g.n3;
         if (t >= nlines) return;
-        base = (t / g.n1) * g.n1 * (long long)g.n2 + t % g.n1;
-        stride = g.n1;
+        base = (t / g.n1) * g.p1 * (long long)g.n2 + t % g.n1;
+        stride = g.p1;
         n = g.n2;
     } else {
         nlines = (long long)g.n1 * g.n2;
         if (t >= nlines) return;
-        base = t;
-        stride = (long long)g.n1 * g.n2;
+        base = t / g.n1 * g.p1 + t % g.n1;
+        stride = (long long)g.p1 * g.n2;
         n = g.n3;
     }
     const float l = bl[t], h = bh[t];
@@ -446,7 +446,7 @@ __global__ void k_sponge_slab1(float *u, const float *__restrict__ w1, const flo
     if (t >= g.n2 * g.n3 * per) return;
     const int line = t / per, k = t - line * per;
     const int i1 = k < W ? k : g.n1 - per + k, i2 = line % g.n2, i3 = line / g.n2;
-    const long long i = (long long)line * g.n1 + i1;
+    const long long i = (long long)line * g.p1 + i1;
     u[i] = damp_cell<EXACT, NDIM>(u[i], i1, i2, i3, w1, w2, w3);
 }
 
@@ -456,7 +456,7 @@ __global__ void k_sponge_slab2(float *u, const float *__restrict__ w1, const flo
     const int i1 = W + blockIdx.x * blockDim.x + threadIdx.x;
     if (i1 >= g.n1 - W) return;
     const int k = blockIdx.y, i2 = k < W ? k : g.n2 - 2 * W + k, i3 = blockIdx.z;
-    const long long i = ((long long)i3 * g.n2 + i2) * g.n1 + i1;
+    const long long i = ((long long)i3 * g.n2 + i2) * g.p1 + i1;
     u[i] = damp_cell<EXACT, NDIM>(u[i], i1, i2, i3, w1, w2, w3);
 }
 
@@ -466,7 +466,7 @@ __global__ void k_sponge_slab3(float *u, const float *__restrict__ w1, const flo
     const int i1 = W + blockIdx.x * blockDim.x + threadIdx.x;
     if (i1 >= g.n1 - W) return;
     const int i2 = W + blockIdx.y, k = blockIdx.z, i3 = k < W ? k : g.n3 - 2 * W + k;
-    const long long i = ((long long)i3 * g.n2 + i2) * g.n1 + i1;
+    const long long i = ((long long)i3 * g.n2 + i2) * g.p1 + i1;
     u[i] = damp_cell<EXACT, 3>(u[i], i1, i2, i3, w1, w2, w3);
 }
 
@@ -494,7 +494,7 @@ __global__ void k_sponge_slab1_v4(float *u, const float *__restrict__ w1, const 
     const int i2 = line % g.n2, i3 = line / g.n2, i1 = 4 * chunk;
     // lines away from the axis-2/3 bands were finished by the fused axis-1 ABC pass
     if (zfused && i2 >= W && i2 < g.n2 - W && i3 >= W && i3 < g.n3 - W) return;
-    float4 *p = reinterpret_cast<float4 *>(u + (long long)line * g.n1) + chunk;
+    float4 *p = reinterpret_cast<float4 *>(u + (long long)line * g.p1) + chunk;
     float4 v = *p;
     if (k < c) damp4<EXACT, NDIM>(v, i1, 0, W, i2, i3, w1, w2, w3);
     else damp4<EXACT, NDIM>(v, i1, g.n1 - W, g.n1, i2, i3, w1, w2, w3);
@@ -519,7 +519,7 @@ __global__ void k_sponge_slab23_v4(float *u, const float *__restrict__ w1, const
         const int k = blockIdx.z;
         i3 = k < W ? k : g.n3 - 2 * W + k;
     }
-    float4 *p = reinterpret_cast<float4 *>(u + ((long long)i3 * g.n2 + i2) * g.n1) + chunk;
+    float4 *p = reinterpret_cast<float4 *>(u + ((long long)i3 * g.n2 + i2) * g.p1) + chunk;
     float4 v = *p;
     damp4<EXACT, NDIM>(v, 4 * chunk, W, g.n1 - W, i2, i3, w1, w2, w3);
     *p = v;
@@ -637,9 +637,9 @@ __global__ void k_extract(const float *__restrict__ u, const GeoPoint *__restric
         const long long n = pt.base + off[c];
         float v = __ldg(u + n);
         if (w1) {
-            const long long s3 = (long long)g.n1 * g.n2;
+            const long long s3 = (long long)g.p1 * g.n2;
             const int i3 = (int)(n / s3), rem = (int)(n % s3);
-            v = damp_cell<EXACT, NDIM>(v, rem % g.n1, rem / g.n1, i3, w1, w2, w3);
+            v = damp_cell<EXACT, NDIM>(v, rem % g.p1, rem / g.p1, i3, w1, w2, w3);
         }
         const float t = fmul<EXACT>(v, pt.w[c]);
         acc = (c == 0) ? t : fadd<EXACT>(acc, t);
@@ -681,7 +681,7 @@ __global__ void k_snapshot(const float *__restrict__ u, float *__restrict__ dst,
     if (t >= (long long)m1 * m2 * m3) return;
     const int j1 = (int)(t % m1), j2 = (int)((t / m1) % m2), j3 = (int)(t / ((long long)m1 * m2));
     const int i1 = f1 + j1, i2 = f2 + j2, i3 = f3 + j3;
-    float v = u[((long long)i3 * g.n2 + i2) * g.n1 + i1];
+    float v = u[((long long)i3 * g.n2 + i2) * g.p1 + i1];
     if (w1) v = damp_cell<true, NDIM>(v, i1, i2, i3, w1, w2, w3);
     dst[t] = v;
 }

@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(sp3::NTHREADS, 2)
     const int n1 = p.a.g.n1, n2 = p.a.g.n2, n3 = p.a.g.n3, nb = p.a.nb;
     const int per_chunk = p.ntr * p.ntt;
     const int nitems = per_chunk * p.nchunks * p.nshot;
-    const long long plane = (long long)n1 * n2;
+    const int p1 = p.a.g.p1;
+    const long long plane = (long long)p1 * n2;
     const float2 r0v = make_float2(p.a.rd[0], p.a.rd[0]), r1v = make_float2(p.a.rd[1], p.a.rd[1]);
     const float2 r2v = make_float2(p.a.rd[2], p.a.rd[2]), r3v = make_float2(p.a.rd[3], p.a.rd[3]);
     const float2 r4v = make_float2(p.a.rd[4], p.a.rd[4]), dt2v = make_float2(p.a.dt2, p.a.dt2);
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(sp3::NTHREADS, 2)
 
         // per-thread constants: 4 radii r .. r+3 of theta row t
         const int r = r0 + 4 * rq, t = t0 + ti;
-        const bool col_ok = r < n1 && t < n2;  // n1 % 4 == 0: the 4 cells exist together
+        const bool col_ok = r < n1 && t < n2;  // p1 % 4 == 0: the 4 cells are stored together
         const bool th_in = t >= 4 && t < n2 - 4;
         bool rin[4];
         bool any_r = false;
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(sp3::NTHREADS, 2)
         }
         float4 A2 = make_float4(0.f, 0.f, 0.f, 0.f), Cr = A2, B = A2, D = A2;
         if (col_ok) {
-            const long long tt = (long long)t * n1 + r;
+            const long long tt = (long long)t * p1 + r;
             A2 = __ldg(reinterpret_cast<const float4 *>(p.a.tr0 + r));
             Cr = __ldg(reinterpret_cast<const float4 *>(p.a.tr1 + r));
             B = __ldg(reinterpret_cast<const float4 *>(p.a.tt0 + tt));
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(sp3::NTHREADS, 2)
         }
         // every (r, theta) cell of the tile is outside the r and theta sponge bands
         const bool tile_undamped = r0 >= nb && r0 + TR - 1 <= n1 - nb && t0 >= nb && t0 + TT - 1 <= n2 - nb;
-        float *dst = p.nxt + ((long long)(fo + y0) * n2 + t) * n1 + r;
+        float *dst = p.nxt + ((long long)(fo + y0) * n2 + t) * p1 + r;
 
         int slot = slot0;  // ring slot and parity of stage s
         uint32_t ph = ph0;
@@ -274,7 +275,8 @@ __global__ void __launch_bounds__(sp3::NTHREADS, 2)
 }
 
 bool sphA_tma_eligible(const Grid &g, int nb) {
-    return g.n1 % 4 == 0 && g.n1 >= 16 && g.n2 >= 16 && g.n3 >= 3 && nb < sp3::FTAB_MAX;
+    // (cells between n1 and p1 look up to 3 entries past the sponge table)
+    return g.p1 % 4 == 0 && g.n1 >= 16 && g.n2 >= 16 && g.n3 >= 3 && nb + (g.p1 - g.n1) < sp3::FTAB_MAX;
 }
 
 // tensor maps: [0] u[0] halo box, [1] u[1] halo box, [2] u[0] tile, [3] u[1]
@@ -282,11 +284,11 @@ bool sphA_tma_eligible(const Grid &g, int nb) {
 bool sphA_tma_maps(CUtensorMap *maps, float *const u[2], const float *vel, const Grid &g, int nshot) {
     using namespace sp3;
     const int n3s = g.n3 * (nshot > 0 ? nshot : 1);
-    return make_tmap_3d(&maps[0], u[0], g.n1, g.n2, n3s, WR, WT) &&
-           make_tmap_3d(&maps[1], u[1], g.n1, g.n2, n3s, WR, WT) &&
-           make_tmap_3d(&maps[2], u[0], g.n1, g.n2, n3s, TR, TT) &&
-           make_tmap_3d(&maps[3], u[1], g.n1, g.n2, n3s, TR, TT) &&
-           make_tmap_3d(&maps[4], vel, g.n1, g.n2, g.n3, TR, TT);
+    return make_tmap_3d(&maps[0], u[0], g.n1, g.n2, n3s, WR, WT, g.p1) &&
+           make_tmap_3d(&maps[1], u[1], g.n1, g.n2, n3s, WR, WT, g.p1) &&
+           make_tmap_3d(&maps[2], u[0], g.n1, g.n2, n3s, TR, TT, g.p1) &&
+           make_tmap_3d(&maps[3], u[1], g.n1, g.n2, n3s, TR, TT, g.p1) &&
+           make_tmap_3d(&maps[4], vel, g.n1, g.n2, g.n3, TR, TT, g.p1);
 }
 
 Step3Launch sphA_tma_shape(const Grid &g, int nshot, int num_sms, int L) {
@@ -404,7 +406,8 @@ __global__ void __launch_bounds__(sa3::NTHREADS, 2)
     const int n1 = p.a.g.n1, n2 = p.a.g.n2, n3 = p.a.g.n3, nb = p.a.nb;
     const int per_chunk = p.ntr * p.ntt;
     const int nitems = per_chunk * p.nchunks;
-    const long long plane = (long long)n1 * n2;
+    const int p1 = p.a.g.p1;
+    const long long plane = (long long)p1 * n2;
     const float rd0 = p.a.rd[0], rd1 = p.a.rd[1], rd2 = p.a.rd[2], rd3 = p.a.rd[3], rd4 = p.a.rd[4];
     const float2 r0v = make_float2(rd0, rd0), r1v = make_float2(rd1, rd1), r2v = make_float2(rd2, rd2);
     const float2 r3v = make_float2(rd3, rd3), r4v = make_float2(rd4, rd4);
@@ -476,7 +479,7 @@ __global__ void __launch_bounds__(sa3::NTHREADS, 2)
               D[4] = {0.f, 0.f, 0.f, 0.f}, Bm[4] = {0.f, 0.f, 0.f, 0.f}, Bp[4] = {0.f, 0.f, 0.f, 0.f};
         float trm = 0.f, trp = 0.f;
         if (col_ok) {
-            const long long tt = (long long)t * n1 + r;
+            const long long tt = (long long)t * p1 + r;
             const float4 a4 = __ldg(reinterpret_cast<const float4 *>(p.a.tr0 + r));
             const float4 c4 = __ldg(reinterpret_cast<const float4 *>(p.a.tr1 + r));
             const float4 b4 = __ldg(reinterpret_cast<const float4 *>(p.a.tt0 + tt));
@@ -486,11 +489,11 @@ __global__ void __launch_bounds__(sa3::NTHREADS, 2)
             B[0] = b4.x, B[1] = b4.y, B[2] = b4.z, B[3] = b4.w;
             D[0] = d4.x, D[1] = d4.y, D[2] = d4.z, D[3] = d4.w;
             if (tm_ok) {
-                const float4 m4 = __ldg(reinterpret_cast<const float4 *>(p.a.tt0 + tt - n1));
+                const float4 m4 = __ldg(reinterpret_cast<const float4 *>(p.a.tt0 + tt - p1));
                 Bm[0] = m4.x, Bm[1] = m4.y, Bm[2] = m4.z, Bm[3] = m4.w;
             }
             if (tp_ok) {
-                const float4 q4 = __ldg(reinterpret_cast<const float4 *>(p.a.tt0 + tt + n1));
+                const float4 q4 = __ldg(reinterpret_cast<const float4 *>(p.a.tt0 + tt + p1));
                 Bp[0] = q4.x, Bp[1] = q4.y, Bp[2] = q4.z, Bp[3] = q4.w;
             }
             if (r >= 1) trm = __ldg(p.a.tr0 + r - 1);
@@ -510,7 +513,7 @@ __global__ void __launch_bounds__(sa3::NTHREADS, 2)
             wph[j] = D[j] * rd4;
         }
         const bool tile_undamped = r0 >= nb && r0 + TR - 1 <= n1 - nb && t0 >= nb && t0 + TT - 1 <= n2 - nb;
-        const long long col = (long long)t * n1 + r;
+        const long long col = (long long)t * p1 + r;
 
         int slot = slot0;
         uint32_t ph = ph0;
@@ -662,13 +665,13 @@ __global__ void __launch_bounds__(sa3::NTHREADS, 2)
 
 bool sphA_tma_level_maps(CUtensorMap *halo, CUtensorMap *tile, const float *base, const Grid &g, int nlevels) {
     const int n3s = g.n3 * (nlevels > 0 ? nlevels : 1);
-    return (!halo || make_tmap_3d(halo, base, g.n1, g.n2, n3s, sp3::WR, sp3::WT)) &&
-           (!tile || make_tmap_3d(tile, base, g.n1, g.n2, n3s, sp3::TR, sp3::TT));
+    return (!halo || make_tmap_3d(halo, base, g.n1, g.n2, n3s, sp3::WR, sp3::WT, g.p1)) &&
+           (!tile || make_tmap_3d(tile, base, g.n1, g.n2, n3s, sp3::TR, sp3::TT, g.p1));
 }
 
 // the accumulator pairs as a float field of 2 n1 floats per line, 128 x 16 boxes
 bool sphA_tma_pair_map(CUtensorMap *m, const float2 *base, const Grid &g) {
-    return make_tmap_3d(m, reinterpret_cast<const float *>(base), 2 * g.n1, g.n2, g.n3, 2 * sp3::TR, sp3::TT);
+    return make_tmap_3d(m, reinterpret_cast<const float *>(base), 2 * g.n1, g.n2, g.n3, 2 * sp3::TR, sp3::TT, 2 * g.p1);
 }
 
 cudaError_t launch_adjA_sph_tma(const CUtensorMap &x_halo, const CUtensorMap &v_halo, const CUtensorMap &a_halo,

@@ -1,12 +1,12 @@
-// 3D 8th-order step of the CPU-program scheme, TMA-staged 2.5D blocking.
+// 3D step of the CPU-program scheme (orders 2 to 8), TMA-staged 2.5D blocking.
 //
 // A CTA owns a 64 (z) x 16 (x) tile and marches along y over a chunk of
 // planes.  For every plane it TMA-loads (cp.async.bulk.tensor, mbarrier
-// completion) the current level's 72 x 24 halo tile into a 9-deep ring (the
-// halo of plane y is read when plane y+4 arrives, so five slots are in use)
+// completion) the current level's halo tile (72 x 24 at 8th order) into a
+// (nop + 5)-deep ring (the halo of plane y is read when plane y + nop arrives)
 // and, for the plane being updated, the previous level and v^2 dt^2 64 x 16
-// tiles into a 5-deep ring, five planes ahead of the compute.  y-neighbours come from a 9-plane register queue
-// (each thread owns a 4-cell z strip of one x column), z- and x-neighbours
+// tiles into a 5-deep ring, five planes ahead of the compute.  y-neighbours
+// come from a register queue of 2 nop + 1 planes (each thread owns a 4-cell z strip of one x column), z- and x-neighbours
 // from the halo tile in shared memory; the leapfrog update, the sponge of
 // the previous level (applied on read) and of the new level (outside the ABC
 // shell) are fused, and the 4-cell result is written with one 16-byte store.
@@ -16,6 +16,12 @@
 // Operation order per cell is that of ts_kernel.c:286-307
 // (lap = u*c0 + sum_k [(z pair)*cz + (x pair)*cx + (y pair)*cy]), so the
 // EXACT instantiation is bit-identical to k_stepB.
+//
+// Lines of a level are p1 cells apart, n1 rounded up to 16 bytes, so that the
+// copies and the 16-byte stores take any n1.  HBM bounds the large grids.  A
+// step of 251 x 223 x 199 cells at 4th order (n1 % 4 != 0) with its boundary took
+// 120 us as one-thread-per-cell kernels and separate passes, 56 us so: 16
+// bytes a cell at 3.2 TB/s, the boundary launch included.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -29,27 +35,34 @@
 namespace awe {
 
 namespace s3 {
-constexpr int TZ = 64, TX = 16, HALO = 4, RING = 9, TRING = 5, NOPQ = 4;
-constexpr int HZ = TZ + 2 * HALO, HX = TX + 2 * HALO;
+constexpr int TZ = 64, TX = 16, HALO = 4, AHEAD = 5, TRING = 5;
+constexpr int HZ = TZ + 2 * HALO;  // axis-1 halo: 4 cells at any order (16-byte boundaries)
 constexpr int NTHREADS = 256;
-constexpr uint32_t BYTES_HALO = HZ * HX * 4, BYTES_TILE = TZ * TX * 4;
+constexpr uint32_t BYTES_TILE = TZ * TX * 4;
 constexpr long long SPIN_LIMIT = 1ll << 22;
 
-struct __align__(128) Stage {  // halo ring entry
-    float cur[HX][HZ];
+template <int NOP>
+struct Ring {
+    static constexpr int HX = TX + 2 * NOP;     // axis-2 halo: the stencil's
+    static constexpr int N = NOP + AHEAD;       // the halo of plane y is read when plane y + NOP arrives
+    static constexpr int Q = 2 * NOP + 1;       // planes of the register queue
+    static constexpr uint32_t BYTES = HZ * HX * 4;
+    struct __align__(128) Stage {
+        float cur[HX][HZ];
+    };
 };
 struct __align__(128) Tile {  // tile ring entry
     float prv[TX][TZ];
     float vel[TX][TZ];
 };
-static_assert(sizeof(Stage) % 128 == 0 && sizeof(Tile) % 128 == 0, "stage size");
-// the tile of output plane o is refilled (for o + TRING) only after plane o
-// is computed: the refill is issued after stage o + 2 NOPQ + TRING - RING + NOPQ
-static_assert(TRING >= RING - NOPQ, "tile ring depth");
+static_assert(sizeof(Tile) % 128 == 0, "tile size");
+// the tile of output plane o is refilled (for o + TRING) only after plane o is
+// computed: the refill is issued after stage o + 2 NOP + TRING - N + NOP
+static_assert(TRING >= AHEAD, "tile ring depth");
 }  // namespace s3
 
 struct Step3Params {
-    int n1, n2, n3;
+    int n1, n2, n3, p1;
     float c0, cz[5], cx[5], cy[5];
     const float *w1, *w2, *w3;
     int damp_prev, sponge_new, shell;
@@ -75,11 +88,13 @@ __device__ __forceinline__ float damp3(float v, float a, float b, float c) {
 
 // MODE 0: forward step; 1: forward step that also stores L(cur); 2: adjoint
 // step of the misfit gradient (the tile loads are the same, the epilogue differs)
-template <bool EXACT, int MODE>
+template <int NOPQ, bool EXACT, int MODE>
 __global__ void __launch_bounds__(s3::NTHREADS, 2)
-    k_stepB3_o8(const __grid_constant__ CUtensorMap tm_cur, const __grid_constant__ CUtensorMap tm_prv,
+    k_stepB3(const __grid_constant__ CUtensorMap tm_cur, const __grid_constant__ CUtensorMap tm_prv,
                 const __grid_constant__ CUtensorMap tm_vel, const Step3Params p) {
     using namespace s3;
+    using Stage = typename Ring<NOPQ>::Stage;
+    constexpr int RING = Ring<NOPQ>::N, Q = Ring<NOPQ>::Q;
     extern __shared__ unsigned char smem_raw[];
     Stage *st = reinterpret_cast<Stage *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
     Tile *tl = reinterpret_cast<Tile *>(st + RING);
@@ -101,7 +116,7 @@ __global__ void __launch_bounds__(s3::NTHREADS, 2)
     if (__syncthreads_or(tid == 0 && *(volatile int *)p.err != 0)) return;
 
     const int nitems = p.ntz * p.ntx * p.nchunks;
-    const long long plane = (long long)p.n1 * p.n2;
+    const long long plane = (long long)p.p1 * p.n2;
     // ring position of the current item's first plane: slot and mbarrier
     // parity; tile ring slot of its first output plane
     int slot0 = 0, tile0 = 0;
@@ -119,8 +134,8 @@ __global__ void __launch_bounds__(s3::NTHREADS, 2)
         auto issue = [&](int s) {
             const int slot = (slot0 + s) % RING;
             const bool out = s >= 2 * NOPQ;
-            mbar_expect_tx(&full[slot], BYTES_HALO + (out ? 2 * BYTES_TILE : 0));
-            tma_load_3d(&st[slot].cur[0][0], &tm_cur, &full[slot], z0 - HALO, x0 - HALO, y0 - NOPQ + s);
+            mbar_expect_tx(&full[slot], Ring<NOPQ>::BYTES + (out ? 2 * BYTES_TILE : 0));
+            tma_load_3d(&st[slot].cur[0][0], &tm_cur, &full[slot], z0 - HALO, x0 - NOPQ, y0 - NOPQ + s);
             if (out) {
                 const int pl = y0 + s - 2 * NOPQ;
                 Tile &t = tl[(tile0 + s - 2 * NOPQ) % TRING];
@@ -150,15 +165,15 @@ __global__ void __launch_bounds__(s3::NTHREADS, 2)
         const bool tile_undamped = z0 >= p.ilo[0] && z0 + TZ <= p.ihi[0] && x0 >= p.ilo[1] && x0 + TX <= p.ihi[1];
         // every column of the tile is at least NOPQ from the z and x faces
         const bool tile_inner = z0 >= NOPQ && z0 + TZ <= p.n1 - NOPQ && x0 >= NOPQ && x0 + TX <= p.n2 - NOPQ;
-        float *dst = p.nxt + ((long long)y0 * p.n2 + x) * p.n1 + zg;
+        float *dst = p.nxt + ((long long)y0 * p.n2 + x) * p.p1 + zg;
 
         int slot = slot0;  // ring slot and parity of plane s
         uint32_t ph = ph0;
-        float q[9][4];  // y queue: plane y0-4+s lives in q[s % 9]
+        float q[Q][4];  // y queue: plane y0 - NOPQ + s lives in q[s % Q]
 #pragma unroll 1
-        for (int blk = 0; blk < S; blk += 9) {
+        for (int blk = 0; blk < S; blk += Q) {
 #pragma unroll
-            for (int u = 0; u < 9; u++) {
+            for (int u = 0; u < Q; u++) {
                 const int s = blk + u;
                 if (s < S) {
                     // adjoint: the plane's L(V) and gradient loads go out before the
@@ -171,7 +186,7 @@ __global__ void __launch_bounds__(s3::NTHREADS, 2)
                         if (s >= 2 * NOPQ) {
                             const int yp = y0 + s - 2 * NOPQ;
                             gok = col_ok && xin && yp >= NOPQ && yp < p.n3 - NOPQ;
-                            gip = ((long long)yp * p.n2 + x) * p.n1 + zg;
+                            gip = ((long long)yp * p.n2 + x) * p.p1 + zg;
                             if (gok) {
                                 lvp = __ldcs(reinterpret_cast<const float4 *>(p.lap_v + gip));
                                 gp0 = __ldcs(reinterpret_cast<const float4 *>(p.grad + gip));
@@ -181,7 +196,7 @@ __global__ void __launch_bounds__(s3::NTHREADS, 2)
                     }
                     const bool bad = !mbar_wait(&full[slot], ph, p.spin);
                     if (bad) atomicExch(p.err, 1);
-                    const float4 cq = *reinterpret_cast<const float4 *>(&st[slot].cur[xi + HALO][4 * zq + HALO]);
+                    const float4 cq = *reinterpret_cast<const float4 *>(&st[slot].cur[xi + NOPQ][4 * zq + HALO]);
                     q[u][0] = cq.x;
                     q[u][1] = cq.y;
                     q[u][2] = cq.z;
@@ -193,27 +208,27 @@ __global__ void __launch_bounds__(s3::NTHREADS, 2)
                         float zw[12];
 #pragma unroll
                         for (int v = 0; v < 3; v++) {
-                            const float4 t = *reinterpret_cast<const float4 *>(&H[xi + HALO][4 * zq + 4 * v]);
+                            const float4 t = *reinterpret_cast<const float4 *>(&H[xi + NOPQ][4 * zq + 4 * v]);
                             zw[4 * v] = t.x;
                             zw[4 * v + 1] = t.y;
                             zw[4 * v + 2] = t.z;
                             zw[4 * v + 3] = t.w;
                         }
-                        const int jc = (u + 1 + 4) % 9;  // queue slot of plane y: ((s - 8) + 4) % 9
+                        const int jc = (u + 1 + NOPQ) % Q;  // queue slot of plane y: (s - 2 NOPQ + NOPQ) % Q
                         float lap[4];
                         if constexpr (EXACT) {
 #pragma unroll
                             for (int i = 0; i < 4; i++) lap[i] = fmul<true>(zw[4 + i], p.c0);
 #pragma unroll
                             for (int k = 1; k <= NOPQ; k++) {
-                                const float4 xm = *reinterpret_cast<const float4 *>(&H[xi + HALO - k][4 * zq + HALO]);
-                                const float4 xp = *reinterpret_cast<const float4 *>(&H[xi + HALO + k][4 * zq + HALO]);
+                                const float4 xm = *reinterpret_cast<const float4 *>(&H[xi + NOPQ - k][4 * zq + HALO]);
+                                const float4 xp = *reinterpret_cast<const float4 *>(&H[xi + NOPQ + k][4 * zq + HALO]);
                                 const float xmv[4] = {xm.x, xm.y, xm.z, xm.w}, xpv[4] = {xp.x, xp.y, xp.z, xp.w};
 #pragma unroll
                                 for (int i = 0; i < 4; i++) {
                                     const float zp = fadd<true>(zw[4 + i - k], zw[4 + i + k]);
                                     const float xpair = fadd<true>(xmv[i], xpv[i]);
-                                    const float ypair = fadd<true>(q[(jc + 9 - k) % 9][i], q[(jc + k) % 9][i]);
+                                    const float ypair = fadd<true>(q[(jc + Q - k) % Q][i], q[(jc + k) % Q][i]);
                                     // ts_kernel.c:292-300 order: (z*cz + x*cx) + y*cy, then into lap
                                     float t = fadd<true>(fmul<true>(zp, p.cz[k]), fmul<true>(xpair, p.cx[k]));
                                     t = fadd<true>(t, fmul<true>(ypair, p.cy[k]));
@@ -226,8 +241,8 @@ __global__ void __launch_bounds__(s3::NTHREADS, 2)
                             float2 l23 = __fmul2_rn(make_float2(zw[6], zw[7]), make_float2(p.c0, p.c0));
 #pragma unroll
                             for (int k = 1; k <= NOPQ; k++) {
-                                const float4 xm = *reinterpret_cast<const float4 *>(&H[xi + HALO - k][4 * zq + HALO]);
-                                const float4 xp = *reinterpret_cast<const float4 *>(&H[xi + HALO + k][4 * zq + HALO]);
+                                const float4 xm = *reinterpret_cast<const float4 *>(&H[xi + NOPQ - k][4 * zq + HALO]);
+                                const float4 xp = *reinterpret_cast<const float4 *>(&H[xi + NOPQ + k][4 * zq + HALO]);
                                 float2 z01, z23;
                                 if (k % 2 == 0) {  // pairs aligned with the 16-byte loads
                                     z01 = __fadd2_rn(make_float2(zw[4 - k], zw[5 - k]), make_float2(zw[4 + k], zw[5 + k]));
@@ -238,7 +253,7 @@ __global__ void __launch_bounds__(s3::NTHREADS, 2)
                                 }
                                 const float2 x01 = __fadd2_rn(make_float2(xm.x, xm.y), make_float2(xp.x, xp.y));
                                 const float2 x23 = __fadd2_rn(make_float2(xm.z, xm.w), make_float2(xp.z, xp.w));
-                                const float *qa = q[(jc + 9 - k) % 9], *qb = q[(jc + k) % 9];
+                                const float *qa = q[(jc + Q - k) % Q], *qb = q[(jc + k) % Q];
                                 const float2 y01 = __fadd2_rn(make_float2(qa[0], qa[1]), make_float2(qb[0], qb[1]));
                                 const float2 y23 = __fadd2_rn(make_float2(qa[2], qa[3]), make_float2(qb[2], qb[3]));
                                 const float2 cz = make_float2(p.cz[k], p.cz[k]), cx = make_float2(p.cx[k], p.cx[k]);
@@ -385,10 +400,11 @@ static bool encode_fn() {
     return true;
 }
 
-bool make_tmap_3d(CUtensorMap *m, const float *base, int n1, int n2, int n3, int b1, int b2) {
+bool make_tmap_3d(CUtensorMap *m, const float *base, int n1, int n2, int n3, int b1, int b2, int p1) {
     if (!encode_fn()) return false;
     cuuint64_t dims[3] = {(cuuint64_t)n1, (cuuint64_t)n2, (cuuint64_t)n3};
-    cuuint64_t strides[2] = {(cuuint64_t)n1 * 4, (cuuint64_t)n1 * n2 * 4};
+    if (p1 == 0) p1 = n1;
+    cuuint64_t strides[2] = {(cuuint64_t)p1 * 4, (cuuint64_t)p1 * n2 * 4};
     cuuint32_t box[3] = {(cuuint32_t)b1, (cuuint32_t)b2, 1};
     cuuint32_t es[3] = {1, 1, 1};
     CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(base), dims, strides, box, es,
@@ -398,25 +414,26 @@ bool make_tmap_3d(CUtensorMap *m, const float *base, int n1, int n2, int n3, int
 }
 
 void stepB3_tma_boxes(int *halo1, int *halo2, int *tile1, int *tile2) {
-    *halo1 = s3::HZ;
-    *halo2 = s3::HX;
+    *halo1 = s3::HZ;  // (of the gradient's 8th-order path)
+    *halo2 = s3::Ring<4>::HX;
     *tile1 = s3::TZ;
     *tile2 = s3::TX;
 }
 
 bool stepB3_tma_eligible(int ndim, int nop, bool rho, const Grid &g) {
     // n3 <= 16384: the y sponge factors fit beside the rings in shared memory
-    return ndim == 3 && nop == 4 && !rho && g.n1 % 4 == 0 && g.n1 >= 16 && g.n2 >= 16 && g.n3 >= 9 && g.n3 <= 16384;
+    return ndim == 3 && nop <= 4 && !rho && g.p1 % 4 == 0 && g.n1 >= 16 && g.n2 >= 16 && g.n3 >= 9 && g.n3 <= 16384;
 }
 
 // tensor maps: [0] u[0] halo box, [1] u[1] halo box, [2] u[0] tile, [3] u[1] tile, [4] vel tile
-bool stepB3_tma_maps(CUtensorMap *maps, float *const u[2], const float *vel, const Grid &g) {
+bool stepB3_tma_maps(CUtensorMap *maps, float *const u[2], const float *vel, const Grid &g, int nop) {
     using namespace s3;
-    return make_tmap_3d(&maps[0], u[0], g.n1, g.n2, g.n3, HZ, HX) &&
-           make_tmap_3d(&maps[1], u[1], g.n1, g.n2, g.n3, HZ, HX) &&
-           make_tmap_3d(&maps[2], u[0], g.n1, g.n2, g.n3, TZ, TX) &&
-           make_tmap_3d(&maps[3], u[1], g.n1, g.n2, g.n3, TZ, TX) &&
-           make_tmap_3d(&maps[4], vel, g.n1, g.n2, g.n3, TZ, TX);
+    const int hx = TX + 2 * nop;
+    return make_tmap_3d(&maps[0], u[0], g.n1, g.n2, g.n3, HZ, hx, g.p1) &&
+           make_tmap_3d(&maps[1], u[1], g.n1, g.n2, g.n3, HZ, hx, g.p1) &&
+           make_tmap_3d(&maps[2], u[0], g.n1, g.n2, g.n3, TZ, TX, g.p1) &&
+           make_tmap_3d(&maps[3], u[1], g.n1, g.n2, g.n3, TZ, TX, g.p1) &&
+           make_tmap_3d(&maps[4], vel, g.n1, g.n2, g.n3, TZ, TX, g.p1);
 }
 
 // Planes per work item of the marching kernels.  An item of L planes takes
@@ -441,16 +458,17 @@ int march_planes(int n3, long long columns, int slots, int halo) {
     return best;
 }
 
-Step3Launch stepB3_tma_shape(const Grid &g, int num_sms, int L) {
+Step3Launch stepB3_tma_shape(const Grid &g, int num_sms, int L, int nop) {
     using namespace s3;
     Step3Launch s{};
     s.ntz = (g.n1 + TZ - 1) / TZ;
     s.ntx = (g.n2 + TX - 1) / TX;
-    s.L = L > 0 ? L : march_planes(g.n3, (long long)s.ntz * s.ntx, 2 * num_sms, 2 * NOPQ);
+    s.L = L > 0 ? L : march_planes(g.n3, (long long)s.ntz * s.ntx, 2 * num_sms, 2 * nop);
     s.nchunks = (g.n3 + s.L - 1) / s.L;
     s.items = s.ntz * s.ntx * s.nchunks;
     s.grid = std::min(s.items, 2 * num_sms);
-    s.smem = RING * sizeof(Stage) + TRING * sizeof(Tile) + (size_t)g.n3 * sizeof(float) + 128;
+    const size_t stage = ((size_t)HZ * (TX + 2 * nop) * sizeof(float) + 127) / 128 * 128;  // sizeof(Ring<nop>::Stage)
+    s.smem = (nop + AHEAD) * stage + TRING * sizeof(Tile) + (size_t)g.n3 * sizeof(float) + 128;
     return s;
 }
 
@@ -468,6 +486,7 @@ static Step3Params step3_params(const StepBParams &sp, const Step3Launch &sh, un
     p.n1 = sp.g.n1;
     p.n2 = sp.g.n2;
     p.n3 = sp.g.n3;
+    p.p1 = sp.g.p1;
     p.c0 = sp.k.c0;
     for (int k = 0; k <= 4; k++) {
         p.cz[k] = sp.k.c[0][k];
@@ -505,9 +524,21 @@ cudaError_t launch_stepB3_adj(const CUtensorMap &g_halo, const CUtensorMap &y_ti
     Step3Params p = step3_params(sp, sh, counter, base, err, Y);
     p.lap_v = lap_v;
     p.grad = grad;
-    cudaFuncSetAttribute(k_stepB3_o8<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
-    k_stepB3_o8<false, 2><<<sh.grid, s3::NTHREADS, sh.smem, s>>>(g_halo, y_tile, x_tile, p);
+    cudaFuncSetAttribute(k_stepB3<4, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+    k_stepB3<4, false, 2><<<sh.grid, s3::NTHREADS, sh.smem, s>>>(g_halo, y_tile, x_tile, p);
     return cudaGetLastError();
+}
+
+template <int NOP>
+static void launch_order(bool exact, const CUtensorMap &cur, const CUtensorMap &prv, const CUtensorMap &vel,
+                         const Step3Params &p, const Step3Launch &sh, cudaStream_t s) {
+    if (exact) {
+        cudaFuncSetAttribute(k_stepB3<NOP, true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+        k_stepB3<NOP, true, 0><<<sh.grid, s3::NTHREADS, sh.smem, s>>>(cur, prv, vel, p);
+    } else {
+        cudaFuncSetAttribute(k_stepB3<NOP, false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+        k_stepB3<NOP, false, 0><<<sh.grid, s3::NTHREADS, sh.smem, s>>>(cur, prv, vel, p);
+    }
 }
 
 // one step with explicit maps: cur halo-box map, prv tile-box map (the buffer
@@ -516,45 +547,19 @@ cudaError_t launch_stepB3_tma_with(bool exact, const CUtensorMap &cur, const CUt
                                    float *nxt, const StepBParams &sp, const Step3Launch &sh,
                                    unsigned long long *counter, unsigned long long base, int *err, cudaStream_t s,
                                    float *lap_out) {
-    Step3Params p{};
-    p.n1 = sp.g.n1;
-    p.n2 = sp.g.n2;
-    p.n3 = sp.g.n3;
-    p.c0 = sp.k.c0;
-    for (int k = 0; k <= 4; k++) {
-        p.cz[k] = sp.k.c[0][k];
-        p.cx[k] = sp.k.c[1][k];
-        p.cy[k] = sp.k.c[2][k];
-    }
-    p.w1 = sp.w1;
-    p.w2 = sp.w2;
-    p.w3 = sp.w3;
-    p.damp_prev = sp.damp_prev;
-    p.sponge_new = sp.sponge_new;
-    p.shell = sp.shell;
-    for (int a = 0; a < 3; a++) {
-        p.ilo[a] = sp.ilo[a];
-        p.ihi[a] = sp.ihi[a];
-    }
-    p.L = sh.L;
-    p.ntz = sh.ntz;
-    p.ntx = sh.ntx;
-    p.nchunks = sh.nchunks;
-    p.counter = counter;
-    p.base = base;
-    p.err = err;
-    p.nxt = nxt;
+    Step3Params p = step3_params(sp, sh, counter, base, err, nxt);
     p.lap_out = lap_out;
-    p.spin = sp.spin >= 0 ? sp.spin : s3::SPIN_LIMIT;
-    if (exact) {
-        cudaFuncSetAttribute(k_stepB3_o8<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
-        k_stepB3_o8<true, 0><<<sh.grid, s3::NTHREADS, sh.smem, s>>>(cur, prv, vel, p);
-    } else if (lap_out) {
-        cudaFuncSetAttribute(k_stepB3_o8<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
-        k_stepB3_o8<false, 1><<<sh.grid, s3::NTHREADS, sh.smem, s>>>(cur, prv, vel, p);
-    } else {
-        cudaFuncSetAttribute(k_stepB3_o8<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
-        k_stepB3_o8<false, 0><<<sh.grid, s3::NTHREADS, sh.smem, s>>>(cur, prv, vel, p);
+    switch (sp.nop) {
+        case 1: launch_order<1>(exact, cur, prv, vel, p, sh, s); break;
+        case 2: launch_order<2>(exact, cur, prv, vel, p, sh, s); break;
+        case 3: launch_order<3>(exact, cur, prv, vel, p, sh, s); break;
+        default:
+            if (lap_out) {
+                cudaFuncSetAttribute(k_stepB3<4, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+                k_stepB3<4, false, 1><<<sh.grid, s3::NTHREADS, sh.smem, s>>>(cur, prv, vel, p);
+            } else {
+                launch_order<4>(exact, cur, prv, vel, p, sh, s);
+            }
     }
     return cudaGetLastError();
 }

@@ -108,7 +108,7 @@ static awe_status grad_alloc(awe_plan *p, int T, int fmt) {
     st->fmt = fmt;
     st->nseg = (d.nt + T - 1) / T;
     const size_t es = fmt == AWE_CKPT_FP32 ? 4 : 2;
-    st->tma = p->use_tma && d.precision == AWE_FAST;
+    st->tma = p->tma_grad && d.precision == AWE_FAST;
     // 2D: two slots a step and two more levels, where memory allows them
     st->tb2 = p->tb2 && (long long)cells <= kFusedCells;
     if (st->tb2) {
@@ -212,13 +212,14 @@ static int grid_for(long long n) {
 
 static awe_status ckpt_store(awe_plan *p, int idx, const float *u, cudaStream_t s) {
     GradState *st = p->grad;
-    const long long cells = p->g.cells();
+    const Grid &g = p->g;
+    const long long cells = g.cells(), n = (long long)g.n1 * g.n2 * g.n3;  // n: without the lines' padding
     if (st->fmt == AWE_CKPT_BFP16) {
         short *q = (short *)st->ckpt + (size_t)idx * cells;
-        launch_ckpt_store_bfp(u, cells, q, st->scales + (size_t)idx * st->nblk, grid_for(cells), s);
+        launch_ckpt_store_bfp(u, n, q, st->scales + (size_t)idx * st->nblk, grid_for(n), s, g.n1, g.p1);
     } else if (st->fmt != AWE_CKPT_FP32) {
         void *q = (char *)st->ckpt + (size_t)idx * cells * 2;
-        launch_ckpt_store16(st->fmt == AWE_CKPT_FP16, u, cells, st->amax, q, st->scales + idx, grid_for(cells), s);
+        launch_ckpt_store16(st->fmt == AWE_CKPT_FP16, u, n, st->amax, q, st->scales + idx, grid_for(n), s, g.n1, g.p1);
     } else {
         float *q = (float *)st->ckpt + (size_t)idx * cells;
         CUDA_TRY(cudaMemcpyAsync(q, u, (size_t)cells * sizeof(float), cudaMemcpyDeviceToDevice, s));
@@ -228,13 +229,14 @@ static awe_status ckpt_store(awe_plan *p, int idx, const float *u, cudaStream_t 
 
 static awe_status ckpt_load(awe_plan *p, int idx, float *u, cudaStream_t s) {
     GradState *st = p->grad;
-    const long long cells = p->g.cells();
+    const Grid &g = p->g;
+    const long long cells = g.cells(), n = (long long)g.n1 * g.n2 * g.n3;  // n: without the lines' padding
     if (st->fmt == AWE_CKPT_BFP16) {
         const short *q = (const short *)st->ckpt + (size_t)idx * cells;
-        launch_ckpt_load_bfp(q, st->scales + (size_t)idx * st->nblk, cells, u, grid_for(cells), s);
+        launch_ckpt_load_bfp(q, st->scales + (size_t)idx * st->nblk, n, u, grid_for(n), s, g.n1, g.p1);
     } else if (st->fmt != AWE_CKPT_FP32) {
         const void *q = (const char *)st->ckpt + (size_t)idx * cells * 2;
-        launch_ckpt_load16(st->fmt == AWE_CKPT_FP16, q, cells, st->scales + idx, u, grid_for(cells), s);
+        launch_ckpt_load16(st->fmt == AWE_CKPT_FP16, q, n, st->scales + idx, u, grid_for(n), s, g.n1, g.p1);
     } else {
         const float *q = (const float *)st->ckpt + (size_t)idx * cells;
         CUDA_TRY(cudaMemcpyAsync(u, q, (size_t)cells * sizeof(float), cudaMemcpyDeviceToDevice, s));

@@ -92,8 +92,9 @@ struct awe_plan {
     float *d_snap_tmp = nullptr;
     long long launches = 0;
 
-    // TMA-staged 3D step (scheme CPU, 8th order)
-    bool use_tma = false;
+    // TMA-staged 3D step (scheme CPU, orders 2 to 8); tma_grad: the gradient's
+    // steps too (8th order, n1 % 4 == 0)
+    bool use_tma = false, tma_grad = false;
     CUtensorMap tmaps[5];
     awe::Step3Launch tma_shape{};
     unsigned long long *sched_counter = nullptr;

@@ -51,6 +51,19 @@ awe_status planA_init(awe_plan *p) {
     const int nb = d.nb < kNopA ? kNopA : d.nb;  // MAWEFDcart2Dgpu.cu:144
     p->nbd = nb;
     p->g = Grid{d.n[0] + 2 * nb, d.n[1] + 2 * nb, d.ndim == 3 ? d.n[2] + 2 * nb : 1};
+    // TMA-staged spherical step for AWE_FAST; AWE_STEP_KERNEL=simple keeps the
+    // register-march kernel (the tests compare both).  Lines of its levels
+    // start on 16-byte boundaries: n1 % 4 != 0 takes padded ones from 2^17
+    // cells on.  (A step of 185 x 122 x 122 ragged cells: 25 us against 33;
+    // below, launches bound both, 19 us against 25, and the plan stays with
+    // the kernels that step_kernel has always reported for such grids.)
+    const char *kern = std::getenv("AWE_STEP_KERNEL");
+    bool sph_tma = geom == 3 && d.precision == AWE_FAST && !(kern && std::strcmp(kern, "simple") == 0);
+    if (sph_tma) {
+        const Grid pitched(p->g.n1, p->g.n2, p->g.n3, (p->g.n1 + 3) / 4 * 4);
+        sph_tma = sphA_tma_eligible(pitched, nb) && (p->g.n1 % 4 == 0 || pitched.cells() >= 1 << 17);
+        if (sph_tma) p->g = pitched;
+    }
     const Grid &g = p->g;
     if (g.n1 < 12 || g.n2 < 12 || (d.ndim == 3 && g.n3 < 12)) {
         set_error("the GPU-program scheme needs at least 12 padded samples per axis");
@@ -141,15 +154,15 @@ awe_status planA_init(awe_plan *p) {
         pa.dd3 = 2 * dth;
         pa.dd4 = dth * dth;
         pa.dd5 = dph * dph;
-        std::vector<float> a2(g.n1), cr(g.n1), B((size_t)g.n1 * g.n2), D((size_t)g.n1 * g.n2);
+        std::vector<float> a2(g.p1), cr(g.p1), B((size_t)g.p1 * g.n2), D((size_t)g.p1 * g.n2);
         for (int ira = 0; ira < g.n1; ira++) {
             const float ra = dra * ira + ora;
             a2[ira] = (2 / ra);
             cr[ira] = (1 / (ra * ra));
             for (int ith = 0; ith < g.n2; ith++) {
                 const float th = dth * ith + oth;
-                B[(size_t)ith * g.n1 + ira] = (std::cos(th) / (ra * ra * std::sin(th)));
-                D[(size_t)ith * g.n1 + ira] = (1 / (ra * ra * std::sin(th) * std::sin(th)));
+                B[(size_t)ith * g.p1 + ira] = (std::cos(th) / (ra * ra * std::sin(th)));
+                D[(size_t)ith * g.p1 + ira] = (1 / (ra * ra * std::sin(th) * std::sin(th)));
             }
         }
         float *t0 = nullptr, *t1 = nullptr, *u0 = nullptr, *u1 = nullptr;
@@ -169,15 +182,10 @@ awe_status planA_init(awe_plan *p) {
 
     pa.nshot = 1;
     pa.shot_cells = g.cells();
-    // TMA-staged spherical step for AWE_FAST; AWE_STEP_KERNEL=simple keeps the
-    // register-march kernel (the tests compare both)
-    const char *kern = std::getenv("AWE_STEP_KERNEL");
-    const bool force_simple = kern && std::strcmp(kern, "simple") == 0;
     // (the TMA kernels' sponge index walks the axes in this grid's priority
     // order (r, phi, theta) = memory axes (1, 3, 2))
     const bool pri_rpt = pa.pri[0] == 0 && pa.pri[1] == 2 && pa.pri[2] == 1;
-    if (geom == 3 && d.precision == AWE_FAST && !force_simple && pri_rpt && sphA_tma_eligible(g, nb) &&
-        sphA_tma_maps(p->sph_maps, p->u, p->vel, g, 1)) {
+    if (sph_tma && pri_rpt && sphA_tma_maps(p->sph_maps, p->u, p->vel, g, 1)) {
         AWE_TRY(dev_alloc(p, (void **)&p->sched_counter, sizeof(unsigned long long)));
         AWE_TRY(dev_alloc(p, (void **)&p->d_err, sizeof(int)));
         CUDA_TRY(cudaMemset(p->sched_counter, 0, sizeof(unsigned long long)));
@@ -221,12 +229,14 @@ awe_status planA_model(awe_plan *p, const float *vel, const float *rfl) {
     const awe_desc &d = p->d;
     const Grid &g = p->g;
     StepAParams &pa = p->pa;
-    const size_t cells = (size_t)g.cells();
+    const size_t lines = (size_t)g.n2 * g.n3, cells = lines * g.n1;
     const int nb = p->nbd;
     p->inj_scale_ok = false;
     p->h_vel_raw.assign(cells, 0.f);
     expand_model(d.ndim, vel, p->h_vel_raw.data(), nb, d.n);
-    AWE_TRY(upload_t(p, &p->vel, p->h_vel_raw.data(), cells));
+    if (!p->vel) AWE_TRY(dev_alloc(p, (void **)&p->vel, (size_t)g.cells() * sizeof(float)));
+    CUDA_TRY(cudaMemcpy2D(p->vel, g.p1 * sizeof(float), p->h_vel_raw.data(), g.n1 * sizeof(float),
+                          g.n1 * sizeof(float), lines, cudaMemcpyHostToDevice));
     const std::vector<float> &v = p->h_vel_raw;
     const float dt = d.dt;
     auto coef = [](float q) { return (1 - q) / (1 + q); };

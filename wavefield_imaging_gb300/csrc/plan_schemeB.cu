@@ -224,6 +224,15 @@ awe_status planB_init(awe_plan *p) {
     p->nbd = nb;
     const int n3 = d.ndim == 3 ? d.n[2] : 1;
     p->g = Grid{d.n[0] + 2 * nb, d.n[1] + 2 * nb, d.ndim == 3 ? n3 + 2 * nb : 1};
+    // AWE_STEP_KERNEL=simple forces the one-thread-per-cell kernels (the tests
+    // compare both)
+    const char *kern = std::getenv("AWE_STEP_KERNEL");
+    const bool force_simple = kern && std::strcmp(kern, "simple") == 0;
+    {
+        // lines of a 3D level on 16-byte boundaries, so that the TMA step takes any n1
+        const Grid pitched(p->g.n1, p->g.n2, p->g.n3, (p->g.n1 + 3) / 4 * 4);
+        if (!force_simple && stepB3_tma_eligible(d.ndim, p->nop, false, pitched)) p->g = pitched;
+    }
     for (int a = 0; a < d.ndim; a++) p->opad[a] = d.o[a] - nb * d.d[a];  // fdutil_init
     float dd[3] = {d.d[0], d.d[1], d.ndim == 3 ? d.d[2] : 1.f};
     fd_coefficients(p->nop, d.ndim, dd, d.optfd, p->k);
@@ -246,6 +255,7 @@ awe_status planB_init(awe_plan *p) {
                     t[len[a] - 1 - i] = w[nb - i - 1];
                 }
             undamped_range(t, p->wlo[a], p->whi[a]);
+            t.resize((t.size() + 3) / 4 * 4, 1.f);  // read 4 at a time
             AWE_TRY(upload(p, &p->w[a], t.data(), t.size()));
         }
     }
@@ -255,21 +265,21 @@ awe_status planB_init(awe_plan *p) {
         AWE_TRY(upload(p, &p->damp, dm.data(), dm.size()));
     }
 
-    // TMA-staged step kernel for the 3D 8th-order case; AWE_STEP_KERNEL=simple
-    // forces the one-thread-per-cell kernel (used by the tests to compare both)
-    const char *kern = std::getenv("AWE_STEP_KERNEL");
-    const bool force_simple = kern && std::strcmp(kern, "simple") == 0;
+    // TMA-staged step kernel for 3D up to 8th order
     if (!force_simple && stepB3_tma_eligible(d.ndim, p->nop, false, p->g)) {
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
         const char *lenv = std::getenv("AWE_TMA_CHUNK");
-        p->tma_shape = stepB3_tma_shape(p->g, sms > 0 ? sms : 1, lenv ? std::atoi(lenv) : 0);
+        p->tma_shape = stepB3_tma_shape(p->g, sms > 0 ? sms : 1, lenv ? std::atoi(lenv) : 0, p->nop);
         AWE_TRY(dev_alloc(p, (void **)&p->sched_counter, sizeof(unsigned long long)));
         AWE_TRY(dev_alloc(p, (void **)&p->d_err, sizeof(int)));
         CUDA_TRY(cudaMemset(p->sched_counter, 0, sizeof(unsigned long long)));
         CUDA_TRY(cudaMemset(p->d_err, 0, sizeof(int)));
         p->sched_base = 0;
-        if (stepB3_tma_maps(p->tmaps, p->u, p->vel, p->g)) p->use_tma = true;
+        p->use_tma = stepB3_tma_maps(p->tmaps, p->u, p->vel, p->g, p->nop);
+        // the gradient's TMA steps (L(u) stored, adjoint) are of 8th order, and
+        // its FP64 result keeps the arithmetic of the kernels each grid has had
+        p->tma_grad = p->use_tma && p->nop == 4 && p->g.n1 % 4 == 0;
         const char *spin = std::getenv("AWE_PIPELINE_SPIN_LIMIT");
         if (spin && *spin) p->spin_limit = std::atoll(spin);
     }
@@ -405,7 +415,7 @@ awe_status set_geometry_common(awe_plan *p, int ns, const float *sou, int nr, co
     const awe_desc &d = p->d;
     const Grid &g = p->g;
     const int nd = d.ndim;
-    const long long s2 = g.n1, s3 = (long long)g.n1 * g.n2;
+    const long long s2 = g.s2(), s3 = g.s3();
     const bool spher = d.coords == AWE_SPHER;
     // reference fdm axes: cartesian z=axis1, x=axis2, y=axis3; spherical
     // programs map z=theta (axis 2), x=r (axis 1), y=phi (axis 3)
@@ -516,6 +526,7 @@ StepBParams stepB_params(const awe_plan *p) {
     StepBParams sp{};
     sp.g = g;
     sp.k = p->k;
+    sp.nop = p->nop;
     sp.w1 = p->w[0];
     sp.w2 = p->w[1];
     sp.w3 = p->w[2];
@@ -565,7 +576,7 @@ awe_status stepB_full(awe_plan *p, const StepBParams &sp0, const float *prv, con
         sp.ext_row = ext_row;
     }
     prof_begin(p, s);
-    if (p->use_tma && cur_map && prv_map) {
+    if (p->use_tma && (!p->den || p->tma_grad) && cur_map && prv_map) {
         cudaError_t e = launch_stepB3_tma_with(exact, *cur_map, *prv_map, p->tmaps[4], nxt, sp, p->tma_shape,
                                                p->sched_counter, p->sched_base, p->d_err, s, lap_out);
         p->sched_base += (unsigned long long)p->tma_shape.items + p->tma_shape.grid;
@@ -593,6 +604,7 @@ awe_status stepB_full(awe_plan *p, const StepBParams &sp0, const float *prv, con
     if (bnd) {
         Bnd3Params bp{};
         bp.g = g;
+        bp.nop = p->nop;
         bp.uo = nxt;
         bp.um = cur;
         bp.vel = p->vel;
@@ -728,12 +740,13 @@ awe_status planB_run_hooked(awe_plan *p, const float *d_wav, int ncs, float *d_d
         return flush_snapshots(p);
     }
     const bool fuse_rec = (d.ndim == 2 || stepB3_bnd(p)) && p->nr > 0;
+    const bool tma = p->use_tma && (!hook || p->tma_grad);
     for (int it = 0; it < d.nt; it++) {
         if (hook) AWE_TRY((*hook)(it, nxt, cur, s));
         const bool ext = fuse_rec && it % d.jdata == 0;
         const PointsAt pe = points_at(p, p->rec, p->nr, p->rec_rows, it);
-        AWE_TRY(stepB_full(p, sp, nxt, cur, nxt, it, d_wav, ncs, &p->tmaps[icur], &p->tmaps[2 + (1 - icur)], s,
-                           launches, nullptr, pe.pts, ext ? p->nr : 0, pe.stride,
+        AWE_TRY(stepB_full(p, sp, nxt, cur, nxt, it, d_wav, ncs, tma ? &p->tmaps[icur] : nullptr,
+                           tma ? &p->tmaps[2 + (1 - icur)] : nullptr, s, launches, nullptr, pe.pts, ext ? p->nr : 0, pe.stride,
                            ext ? d_dat + (size_t)row * p->nr : nullptr));
         std::swap(cur, nxt);  // nxt now holds the time level `it` (sponge pending)
         icur ^= 1;
