@@ -506,36 +506,117 @@ __device__ __forceinline__ int edge_axes(int j1, int j2, int j3, int m1, int m2,
     return (j1 == 0 || j1 == m1 - 1) + (j2 == 0 || j2 == m2 - 1) + (nd == 3 && (j3 == 0 || j3 == m3 - 1));
 }
 
-// skip_big: model cells on two or more edge axes (the model's edges and
-// corners, whose replicas span (nb+1)^2 or (nb+1)^3 padded cells) are left
-// to k_grad_fold_big
-// vel2 holds c = v^2 dt^2 per padded cell, or (cscale > 0) the velocity v with c = cscale v^2
-__device__ __forceinline__ double fold_c(const float *vel2, long long i, double cscale) {
-    const double v = vel2[i];
-    return cscale > 0 ? cscale * v * v : v;
+// Sum of the accumulators of the padded cells that replicate a model cell.
+// They all hold the cell's vel2 (the padding repeats it; a free surface zeroes
+// them together), so its factor is applied once, to the sum.  vel2 holds
+// c = v^2 dt^2 per padded cell, or (cscale > 0) the velocity v with c = cscale v^2.
+struct FoldParams {
+    const float2 *G;
+    const float *vel2;
+    double inv_dt2, cscale;
+    Grid g;
+    int nb, m1, m2, m3, nd;
+    int nbig, nends;  // blocks of the first two roles
+    double *out;
+};
+
+__device__ __forceinline__ void fold_store(const FoldParams &p, int j1, int j2, int j3, double acc) {
+    const int i3 = p.nd == 3 ? j3 + p.nb : 0;
+    const double v = p.vel2[((long long)i3 * p.g.n2 + j2 + p.nb) * p.g.p1 + j1 + p.nb];
+    const double c = p.cscale > 0 ? p.cscale * v * v : v;
+    p.out[((long long)j3 * p.m2 + j2) * p.m1 + j1] = acc * (-c * c * p.inv_dt2);
 }
 
-__global__ void k_grad_fold(const float2 *__restrict__ G, const float *__restrict__ vel2, double inv_dt2, Grid g,
-                            int nb, int m1, int m2, int m3, int nd, double *__restrict__ out, int skip_big,
-                            double cscale) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// The fold is bound by FP64 issue (GB300 converts and adds FP64 at 1/64 of the
+// FP32 rate, per warp whatever its active lanes), so a cell costs two
+// conversions and two adds, and cells with many replicas do not hold up a
+// warp of cells with one.  Three roles by block:
+//  1. the model's edges and corners ((nb+1)^2 or (nb+1)^3 replicas; 2D: the
+//     corners), one block each;
+//  2. the ends of every other axis-1 line (nb+1 contiguous replicas), 8 lanes each;
+//  3. the other cells, one thread each (lines along axis 1, so a warp's cells
+//     have 1 replica, or all nb+1 along axis 2 or 3).
+// 160 x 144 x 150 cells, nb = 24: one thread per cell and a second launch for
+// role 1 took 707 + 85 us, this 146 us; 512 x 512, nb = 40: 63 + 12 us, this 25 us.
+__global__ void __launch_bounds__(256) k_grad_fold(const FoldParams p) {
+    const int m1 = p.m1, m2 = p.m2, m3 = p.m3, nd = p.nd, tid = threadIdx.x;
+    long long b = blockIdx.x;
+    int j1, j2, j3 = 0, a1, b1, a2, b2, a3 = 0, b3 = 0;
+    if (b < p.nbig) {
+        if (nd == 2) {
+            j1 = (b & 1) ? m1 - 1 : 0;
+            j2 = (b & 2) ? m2 - 1 : 0;
+        } else if (b < 4LL * m1) {  // the edges along axis 1, the corners with them
+            const int e = (int)(b / m1);
+            j1 = (int)(b % m1);
+            j2 = (e & 1) ? m2 - 1 : 0;
+            j3 = (e & 2) ? m3 - 1 : 0;
+        } else if ((b -= 4LL * m1) < 4LL * (m2 - 2)) {
+            const int e = (int)(b / (m2 - 2));
+            j2 = 1 + (int)(b % (m2 - 2));
+            j1 = (e & 1) ? m1 - 1 : 0;
+            j3 = (e & 2) ? m3 - 1 : 0;
+        } else {
+            b -= 4LL * (m2 - 2);
+            const int e = (int)(b / (m3 - 2));
+            j3 = 1 + (int)(b % (m3 - 2));
+            j1 = (e & 1) ? m1 - 1 : 0;
+            j2 = (e & 2) ? m2 - 1 : 0;
+        }
+        fold_range(j1, m1, p.g.n1, p.nb, a1, b1);
+        fold_range(j2, m2, p.g.n2, p.nb, a2, b2);
+        if (nd == 3) fold_range(j3, m3, p.g.n3, p.nb, a3, b3);
+        const int w1 = b1 - a1 + 1, w2 = b2 - a2 + 1, vol = w1 * w2 * (b3 - a3 + 1);
+        double acc = 0;
+        for (int k = tid; k < vol; k += 256) {
+            const int i1 = a1 + k % w1, i2 = a2 + (k / w1) % w2, i3 = a3 + k / (w1 * w2);
+            acc += gsum_value(p.G[((long long)i3 * p.g.n2 + i2) * p.g.p1 + i1]);
+        }
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        __shared__ double part[8];
+        if ((tid & 31) == 0) part[tid >> 5] = acc;
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < 8; w++) acc += part[w];
+            fold_store(p, j1, j2, j3, acc);
+        }
+        return;
+    }
+    b -= p.nbig;
+    const bool split = p.nbig > 0;
+    if (b < p.nends) {
+        const long long u = b * 32 + tid / 8, line = u >> 1;
+        const bool hi = u & 1;
+        j2 = (int)(line % m2), j3 = (int)(line / m2);
+        j1 = hi ? m1 - 1 : 0;
+        const bool mine = line < (long long)m2 * m3 && !(hi && m1 == 1) &&
+                          !(split && edge_axes(j1, j2, j3, m1, m2, m3, nd) >= 2);
+        double acc = 0;
+        if (mine) {
+            fold_range(j1, m1, p.g.n1, p.nb, a1, b1);
+            fold_range(j2, m2, p.g.n2, p.nb, a2, b2);
+            if (nd == 3) fold_range(j3, m3, p.g.n3, p.nb, a3, b3);
+            for (int i3 = a3; i3 <= b3; i3++)
+                for (int i2 = a2; i2 <= b2; i2++)
+                    for (int i1 = a1 + (tid & 7); i1 <= b1; i1 += 8)
+                        acc += gsum_value(p.G[((long long)i3 * p.g.n2 + i2) * p.g.p1 + i1]);
+        }
+        for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (mine && (tid & 7) == 0) fold_store(p, j1, j2, j3, acc);
+        return;
+    }
+    const long long t = (b - p.nends) * 256 + tid;
     if (t >= (long long)m1 * m2 * m3) return;
-    const int j1 = (int)(t % m1), j2 = (int)((t / m1) % m2), j3 = (int)(t / ((long long)m1 * m2));
-    if (skip_big && edge_axes(j1, j2, j3, m1, m2, m3, nd) >= 2) return;
-    auto range = [&](int j, int m, int npad, int &lo, int &hi) { fold_range(j, m, npad, nb, lo, hi); };
-    int a1, b1, a2, b2, a3 = 0, b3 = 0;
-    range(j1, m1, g.n1, a1, b1);
-    range(j2, m2, g.n2, a2, b2);
-    if (nd == 3) range(j3, m3, g.n3, a3, b3);
+    j1 = (int)(t % m1), j2 = (int)((t / m1) % m2), j3 = (int)(t / ((long long)m1 * m2));
+    if (j1 == 0 || j1 == m1 - 1 || (split && edge_axes(j1, j2, j3, m1, m2, m3, nd) >= 2)) return;
+    fold_range(j2, m2, p.g.n2, p.nb, a2, b2);
+    if (nd == 3) fold_range(j3, m3, p.g.n3, p.nb, a3, b3);
     double acc = 0;
     for (int i3 = a3; i3 <= b3; i3++)
+#pragma unroll 4
         for (int i2 = a2; i2 <= b2; i2++)
-            for (int i1 = a1; i1 <= b1; i1++) {
-                const long long i = ((long long)i3 * g.n2 + i2) * g.p1 + i1;
-                const double v2 = fold_c(vel2, i, cscale);
-                acc += gsum_value(G[i]) * (-v2 * v2 * inv_dt2);
-            }
-    out[t] = acc;
+            acc += gsum_value(p.G[((long long)i3 * p.g.n2 + i2) * p.g.p1 + j1 + p.nb]);
+    fold_store(p, j1, j2, j3, acc);
 }
 
 __global__ void k_image_cut(const float2 *__restrict__ G, Grid g, int nb, int m1, int m2, int m3, int nd,
@@ -561,70 +642,23 @@ void launch_image_cut(const float2 *G, const Grid &g, int nb, const int *n, int 
     k_image_cut<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(G, g, nb, n[0], n[1], nd == 3 ? n[2] : 1, nd, out);
 }
 
-// The model's edge and corner cells, one block each: 2D the 4 corners; 3D
-// the 4 edges along each axis (corners counted with the axis-1 edges).
-__global__ void __launch_bounds__(256) k_grad_fold_big(const float2 *__restrict__ G, const float *__restrict__ vel2,
-                                                       double inv_dt2, Grid g, int nb, int m1, int m2, int m3, int nd,
-                                                       double *__restrict__ out, double cscale) {
-    long long b = blockIdx.x;
-    int j1, j2, j3 = 0;
-    if (nd == 2) {
-        j1 = (b & 1) ? m1 - 1 : 0;
-        j2 = (b & 2) ? m2 - 1 : 0;
-    } else if (b < 4LL * m1) {
-        const int e = (int)(b / m1);
-        j1 = (int)(b % m1);
-        j2 = (e & 1) ? m2 - 1 : 0;
-        j3 = (e & 2) ? m3 - 1 : 0;
-    } else if ((b -= 4LL * m1) < 4LL * (m2 - 2)) {
-        const int e = (int)(b / (m2 - 2));
-        j2 = 1 + (int)(b % (m2 - 2));
-        j1 = (e & 1) ? m1 - 1 : 0;
-        j3 = (e & 2) ? m3 - 1 : 0;
-    } else {
-        b -= 4LL * (m2 - 2);
-        const int e = (int)(b / (m3 - 2));
-        j3 = 1 + (int)(b % (m3 - 2));
-        j1 = (e & 1) ? m1 - 1 : 0;
-        j2 = (e & 2) ? m2 - 1 : 0;
-    }
-    int a1, b1, a2, b2, a3 = 0, b3 = 0;
-    fold_range(j1, m1, g.n1, nb, a1, b1);
-    fold_range(j2, m2, g.n2, nb, a2, b2);
-    if (nd == 3) fold_range(j3, m3, g.n3, nb, a3, b3);
-    const long long w1 = b1 - a1 + 1, w2 = b2 - a2 + 1, vol = w1 * w2 * (b3 - a3 + 1);
-    double acc = 0;
-    for (long long k = threadIdx.x; k < vol; k += blockDim.x) {
-        const long long i1 = a1 + k % w1, i2 = a2 + (k / w1) % w2, i3 = a3 + k / (w1 * w2);
-        const long long i = (i3 * g.n2 + i2) * g.p1 + i1;
-        const double v2 = fold_c(vel2, i, cscale);
-        acc += gsum_value(G[i]) * (-v2 * v2 * inv_dt2);
-    }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    __shared__ double part[8];
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += part[w];
-        out[((long long)j3 * m2 + j2) * m1 + j1] = t;
-    }
-}
-
 void launch_grad_fold(const float2 *G, const float *vel2, float dt, const Grid &g, int nb, const int *n, int nd,
                       double *out, cudaStream_t s, bool raw_v) {
-    const double cscale = raw_v ? (double)dt * (double)dt : 0.0;
-    const int m1 = n[0], m2 = n[1], m3 = nd == 3 ? n[2] : 1;
-    const long long m = (long long)m1 * m2 * m3;
-    const double inv = 1.0 / ((double)dt * (double)dt);
+    FoldParams p{};
+    p.G = G;
+    p.vel2 = vel2;
+    p.inv_dt2 = 1.0 / ((double)dt * (double)dt);
+    p.cscale = raw_v ? (double)dt * (double)dt : 0.0;
+    p.g = g;
+    p.nb = nb;
+    p.m1 = n[0], p.m2 = n[1], p.m3 = nd == 3 ? n[2] : 1;
+    p.nd = nd;
+    p.out = out;
     // edges and corners go to one block each when every model axis has an interior
-    const bool split = m1 >= 3 && m2 >= 3 && (nd == 2 || m3 >= 3);
-    k_grad_fold<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(G, vel2, inv, g, nb, m1, m2, m3, nd, out, split ? 1 : 0,
-                                                            cscale);
-    if (split) {
-        const long long nbig = nd == 2 ? 4 : 4LL * (m1 + m2 - 2 + m3 - 2);
-        k_grad_fold_big<<<(unsigned)nbig, 256, 0, s>>>(G, vel2, inv, g, nb, m1, m2, m3, nd, out, cscale);
-    }
+    if (p.m1 >= 3 && p.m2 >= 3 && (nd == 2 || p.m3 >= 3)) p.nbig = nd == 2 ? 4 : 4 * (p.m1 + p.m2 - 2 + p.m3 - 2);
+    p.nends = (int)((2LL * p.m2 * p.m3 + 31) / 32);
+    const long long cells = ((long long)p.m1 * p.m2 * p.m3 + 255) / 256;
+    k_grad_fold<<<(unsigned)(p.nbig + p.nends + cells), 256, 0, s>>>(p);
 }
 
 }  // namespace awe
