@@ -173,7 +173,7 @@ struct Bnd3Params {
     InjCells inj;  // fixed sources by cell (n = 0: walk src)
     const float *wav;
     int it, ncs, one_wavelet;
-    int n_int, nxr, nzr, rec_blocks;  // set by launch_bnd3
+    int n_int, nxr, nzr, end_blocks, rec_blocks;  // set by launch_bnd3
     int nop;                          // 1 .. 4
     // compact copies of the line ends ([n3][n2][16]: axis-1 cells 0..7, then
     // n1-8..n1-1) of um (em: written by the previous step's launch; null:
@@ -195,7 +195,7 @@ struct Bnd3AdjParams {
     const float *zl, *zh, *xl, *xh, *yl, *yh;
     const float *w1, *w2, *w3;  // sponge factors of the fold (null: weight 1)
     int top;                    // axis-1 low face (0 with a free surface)
-    int n_int, nxr, nzr;        // set by launch_bnd3_adj
+    int n_int, nxr, nzr, end_blocks;  // set by launch_bnd3_adj
 };
 void launch_bnd3_adj(Bnd3AdjParams p, cudaStream_t s);
 

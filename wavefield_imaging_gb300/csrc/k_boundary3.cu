@@ -9,15 +9,23 @@
 // lines, then axis-2 lines, then axis-3 lines, each an outward recurrence over
 // the nop outer cells from cell nop + 1), then the sponge.  The passes only
 // meet in the shell (cells within nop + 2 of a face), so the work splits into
-// blocks that each own a whole chain of dependencies:
-//  * a plane y in [nop+2, n3-nop-2) (no axis-3 face cell): its axis-1 line ends, then
-//    (after a barrier) its axis-2 line ends, each sponged once it is final;
-//  * a face block (the nop + 2 planes of a y face) x a 16-column x-range x a
-//    64-cell z-range: the axis-1 pass of its lines, the axis-2 pass of its
-//    z-range (x-ranges holding a face), the axis-3 pass of its columns, then
-//    the sponge of all its cells;
-//  * receiver blocks (256 receivers each) and one injection block, which read
-//    or write cells no pass touches.
+// roles, longest chain first, that each own whole chains of dependencies:
+//  * a plane y in [nop+2, n3-nop-2) (no axis-3 face cell), its axis-2 shell
+//    lines: their axis-1 ends, then (after a barrier) the axis-2 pass with the
+//    sponge, four z cells per thread;
+//  * a face block (the nop + 2 planes of a y face) x about 16 columns x about
+//    32 cells of axis 1: the axis-1 pass of its line ends, the axis-2 pass
+//    (x-ranges holding a face), then the axis-3 pass and the sponge of its
+//    columns together, four z cells per thread;
+//  * the axis-1 ends of every other line, one thread per end, sponged;
+//  * receiver blocks (256 receivers each) and the injection, which read or
+//    write cells no pass touches.
+// Latency bounds it but on the largest grids: every role is two or three
+// dependent rounds of loads, so they are kept short and the blocks many.  (A
+// block per plane for both its passes, and face blocks of up to 31 x 124
+// columns one cell at a time: 22.5 us for 251 x 223 x 199 cells at 4th order,
+// 52 us for 576^3 at 8th; so 11.8 us and 51 us, the scattered sectors of the
+// line ends.)
 // Every cell is written by one block only, so the result does not depend on
 // the order in which blocks run.
 //
@@ -36,7 +44,7 @@ namespace awe {
 
 namespace b3 {
 constexpr int SHELL = 6;  // the adjoint's nop + 2 (nop = 4): cells the ABC writes (1..4) or reads (5), and the face cell 0
-constexpr int XR = 16, ZR = 64;
+constexpr int XR = 16, ZQ = 8;  // face blocks: least columns and 4-cell groups of axis 1
 constexpr int NT = 256;
 }  // namespace b3
 
@@ -101,31 +109,65 @@ __device__ __forceinline__ void b3_damp8(float (&v)[8], const float *w, float wx
         if ((mask >> k) & 1u) v[k] = b3_damp<EXACT>(v[k], wz[k], wx, wy);
 }
 
-// one axis-2 face line (y, z): the NOP cells outward from xa, optionally
-// sponged (the NOP + 2 shell cells of the line)
-template <bool EXACT, int NOP>
-__device__ __forceinline__ void b3_xline(const Bnd3Params &p, long long c0, int y, int z, bool low, bool damp) {
-    constexpr int SHELL = NOP + 2;
-    const long long s2 = p.g.p1;
-    const int xa = low ? NOP + 1 : p.g.n2 - SHELL, dx = low ? -1 : 1;
-    const float b = __ldg((low ? p.xl : p.xh) + (long long)y * p.g.n1 + z);
-    float v[SHELL];  // cells xa .. the face cell 0 / n2-1
+// coefficients of cells z .. z+3 of a face line (cells past n1: 0)
+template <bool AL>
+__device__ __forceinline__ void b3_coef4(float (&b)[4], const float *row, int z, int n1) {
+    if constexpr (AL) {
+        const float4 x = __ldg(reinterpret_cast<const float4 *>(row + z));
+        b[0] = x.x, b[1] = x.y, b[2] = x.z, b[3] = x.w;
+    } else {
 #pragma unroll
-    for (int k = 0; k < SHELL; k++) v[k] = p.uo[c0 + (long long)(xa + k * dx) * s2];
-    float m[NOP + 1];
-#pragma unroll
-    for (int k = 0; k <= NOP; k++) m[k] = __ldg(p.um + c0 + (long long)(xa + k * dx) * s2);
-#pragma unroll
-    for (int k = 1; k <= NOP; k++) v[k] = b3_abc<EXACT>(m[k - 1], m[k], v[k - 1], b);
+        for (int i = 0; i < 4; i++) b[i] = z + i < n1 ? __ldg(row + z + i) : 0.f;
+    }
+}
+
+// Cells z .. z+3 of a face's recurrence along axis AXIS (2 or 3): NOP cells
+// outward (st) from the one at c0, all NOP + 2 shell cells sponged if damp.
+// wv: the sponge factors along AXIS at c0, dw their step; wc: the other one.
+template <bool EXACT, int NOP, int AXIS>
+__device__ __forceinline__ void b3_chain4(const Bnd3Params &p, long long c0, long long st, const float (&b)[4], int z,
+                                          bool damp, const float *wv, int dw, float wc) {
+    auto ld = [](float (&v)[4], const float *a) {
+        const float4 x = *reinterpret_cast<const float4 *>(a);
+        v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+    };
+    float v[4], f[4], m[NOP + 1][4], wz[4];
+    ld(v, p.uo + c0);
     if (damp) {
-        const float wz = __ldg(p.w1 + z), wy = __ldg(p.w3 + y);
-#pragma unroll
-        for (int k = 0; k < SHELL; k++) v[k] = b3_damp<EXACT>(v[k], wz, __ldg(p.w2 + xa + k * dx), wy);
-        p.uo[c0 + (long long)xa * s2] = v[0];
-        p.uo[c0 + (long long)(xa + (NOP + 1) * dx) * s2] = v[NOP + 1];
+        ld(f, p.uo + c0 + (NOP + 1) * st);
+        ld(wz, p.w1 + z);
     }
 #pragma unroll
-    for (int k = 1; k <= NOP; k++) p.uo[c0 + (long long)(xa + k * dx) * s2] = v[k];
+    for (int k = 0; k <= NOP; k++) ld(m[k], p.um + c0 + k * st);
+    auto put = [&](const float (&v)[4], int k) {
+        float o[4];
+        const float w = damp ? __ldg(wv + k * dw) : 1.f;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            o[i] = !damp ? v[i] : AXIS == 2 ? b3_damp<EXACT>(v[i], wz[i], w, wc) : b3_damp<EXACT>(v[i], wz[i], wc, w);
+        *reinterpret_cast<float4 *>(p.uo + c0 + k * st) = make_float4(o[0], o[1], o[2], o[3]);
+    };
+    if (damp) {
+        put(v, 0);
+        put(f, NOP + 1);
+    }
+#pragma unroll
+    for (int k = 1; k <= NOP; k++) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = b3_abc<EXACT>(m[k - 1][i], m[k][i], v[i], b[i]);
+        put(v, k);
+    }
+}
+
+// an axis-2 face of plane y, cells z .. z+3
+template <bool EXACT, int NOP, bool AL>
+__device__ __forceinline__ void b3_xchain(const Bnd3Params &p, int y, int z, bool low, bool damp) {
+    const long long s2 = p.g.p1;
+    const int xa = low ? NOP + 1 : p.g.n2 - NOP - 2, dx = low ? -1 : 1;
+    float b[4];
+    b3_coef4<AL>(b, (low ? p.xl : p.xh) + (long long)y * p.g.n1, z, p.g.n1);
+    b3_chain4<EXACT, NOP, 2>(p, ((long long)y * p.g.n2 + xa) * s2 + z, dx * s2, b, z, damp, p.w2 + xa, dx,
+                             damp ? __ldg(p.w3 + y) : 1.f);
 }
 
 // an end (0: cells 0..7, 1: cells n1-8..n1-1) of line `line` of the level the
@@ -150,61 +192,64 @@ __device__ __forceinline__ void b3_eput_from_uo(const Bnd3Params &p, long long l
     reinterpret_cast<float4 *>(p.eo)[line * 4 + part] = v;
 }
 
+// One end of line (y, x) (0: low, 1: high): the axis-1 recurrence and, with
+// damp, the sponge of its shell cells; the final values go to the compact copy
+// if put (without a sponge and with a free surface the low end is not read,
+// nor needed: the next step's low-end recurrence is off).
 template <bool EXACT, int NOP, bool AL>
-__global__ void __launch_bounds__(b3::NT, 4) k_bnd3(const Bnd3Params p) {
-    using b3::NT, b3::XR, b3::ZR;
+__device__ __forceinline__ void b3_end(const Bnd3Params &p, int y, int x, int end, bool damp, bool put) {
+    constexpr unsigned LOW = (1u << (NOP + 2)) - 1u, HIGH = LOW << (6 - NOP);  // of 8, those in the shell
+    const long long line = (long long)y * p.g.n2 + x;
+    float v[8] = {}, m[8];
+    const float wx = damp ? __ldg(p.w2 + x) : 1.f, wy = damp ? __ldg(p.w3 + y) : 1.f;
+    if (end == 0) {
+        if (p.top || damp) {
+            float *o = p.uo + line * p.g.p1;
+            b3_ld8<true>(v, o);
+            if (p.top) {
+                b3_mend<AL>(p, m, line, 0);
+                b3_zlow<EXACT, NOP>(v, m, __ldg(p.zl + line));
+            }
+            if (damp) b3_damp8<EXACT, true>(v, p.w1, wx, wy, LOW);
+            b3_st8<true>(o, v);
+        }
+    } else {
+        float *o = p.uo + line * p.g.p1 + p.g.n1 - 8;
+        b3_ld8<AL>(v, o);
+        b3_mend<AL>(p, m, line, 1);
+        b3_zhigh<EXACT, NOP>(v, m, __ldg(p.zh + line));
+        if (damp) b3_damp8<EXACT, AL>(v, p.w1 + p.g.n1 - 8, wx, wy, HIGH);
+        b3_st8<AL>(o, v);
+    }
+    if (put) b3_st8<true>(p.eo + line * 16 + 8 * end, v);
+}
+
+template <bool EXACT, int NOP, bool AL>
+__global__ void __launch_bounds__(b3::NT, 3) k_bnd3(const Bnd3Params p) {
+    using b3::NT;
     constexpr int SHELL = NOP + 2;
-    // elements of an end (of 8) that lie in the shell
-    constexpr unsigned LOW = (1u << SHELL) - 1u, HIGH = LOW << (8 - SHELL);
     const int tid = threadIdx.x;
-    const int n1 = p.g.n1, n2 = p.g.n2, n3 = p.g.n3;
+    const int n1 = p.g.n1, n2 = p.g.n2, n3 = p.g.n3, nq = (n1 + 3) / 4;
     const long long s2 = p.g.p1, s3 = s2 * n2;
+    const bool sponge = p.w1 != nullptr;
     int blk = blockIdx.x;
 
-    if (blk < p.n_int) {  // ---- one plane without axis-3 face cells
+    if (blk < p.n_int) {  // ---- the axis-2 shell of a plane without axis-3 face cells
         const int y = SHELL + blk;
-        const float wy = p.w3 ? __ldg(p.w3 + y) : 1.f;
-        for (int x = tid; x < n2; x += NT) {
-            const long long line = (long long)y * n2 + x;
-            float *o = p.uo + line * s2;
-            // lines in the axis-2 shell are sponged by the axis-2 pass below
-            const bool xshell = x < SHELL || x >= n2 - SHELL;
-            const bool damp = p.w1 && !xshell;
-            const float wx = damp ? __ldg(p.w2 + x) : 1.f;
-            float lo[8] = {}, hi[8], m[8];  // both ends as left
-            if (p.top || damp) {
-                b3_ld8<true>(lo, o);
-                if (p.top) {
-                    b3_mend<AL>(p, m, line, 0);
-                    b3_zlow<EXACT, NOP>(lo, m, __ldg(p.zl + line));
-                }
-                if (damp) b3_damp8<EXACT, true>(lo, p.w1, wx, wy, LOW);
-                b3_st8<true>(o, lo);
-            }
-            b3_ld8<AL>(hi, o + n1 - 8);
-            b3_mend<AL>(p, m, line, 1);
-            b3_zhigh<EXACT, NOP>(hi, m, __ldg(p.zh + line));
-            if (damp) b3_damp8<EXACT, AL>(hi, p.w1 + n1 - 8, wx, wy, HIGH);
-            b3_st8<AL>(o + n1 - 8, hi);
-            // final unless the axis-2 pass changes the line (the axis-2 shell);
-            // without a sponge and with a free surface the low end is not
-            // read (nor needed: the next step's low-end ABC is off)
-            if (p.eo && !xshell) {
-                b3_st8<true>(p.eo + line * 16, lo);
-                b3_st8<true>(p.eo + line * 16 + 8, hi);
-            }
+        if (tid < 4 * SHELL) {
+            const int k = tid >> 1;
+            b3_end<EXACT, NOP, AL>(p, y, k < SHELL ? k : n2 - 2 * SHELL + k, tid & 1, false, false);
         }
-        __syncthreads();  // the axis-2 pass reads the axis-1 results of lines x = 1..NOP+1
-        for (int z = tid; z < n1; z += NT) {
-            const long long c0 = (long long)y * s3 + z;
-            b3_xline<EXACT, NOP>(p, c0, y, z, true, p.w1 != nullptr);
-            b3_xline<EXACT, NOP>(p, c0, y, z, false, p.w1 != nullptr);
+        __syncthreads();
+        for (int l = tid; l < 2 * nq; l += NT) {
+            const bool low = l < nq;
+            b3_xchain<EXACT, NOP, AL>(p, y, 4 * (low ? l : l - nq), low, sponge);
         }
-        if (p.eo) {  // the axis-2 shell lines' ends, final now
+        if (p.eo) {
             __syncthreads();
-            for (int l = tid; l < 2 * SHELL * 4; l += NT) {
-                const int k = l >> 2, x = k < SHELL ? k : n2 - 2 * SHELL + k;
-                b3_eput_from_uo<AL>(p, (long long)y * n2 + x, l & 3);
+            if (tid < 8 * SHELL) {
+                const int k = tid >> 2, x = k < SHELL ? k : n2 - 2 * SHELL + k;
+                b3_eput_from_uo<AL>(p, (long long)y * n2 + x, tid & 3);
             }
         }
         return;
@@ -212,85 +257,56 @@ __global__ void __launch_bounds__(b3::NT, 4) k_bnd3(const Bnd3Params p) {
     blk -= p.n_int;
     if (blk < 2 * p.nxr * p.nzr) {  // ---- face block
         const int f = blk / (p.nxr * p.nzr), r = blk % (p.nxr * p.nzr), xr = r / p.nzr, zr = r % p.nzr;
-        const int xa = xr * XR, xb = xr == p.nxr - 1 ? n2 : xa + XR;
-        const int za = zr * ZR, zb = zr == p.nzr - 1 ? n1 : za + ZR;
+        const int xa = (int)((long long)n2 * xr / p.nxr), xb = (int)((long long)n2 * (xr + 1) / p.nxr);
+        const int qa = (int)((long long)nq * zr / p.nzr), qb = (int)((long long)nq * (zr + 1) / p.nzr);
         const int ya = f == 0 ? 0 : n3 - SHELL;  // planes [ya, ya + SHELL)
-        const int ncol = xb - xa, nz = zb - za;
+        const int ncol = xb - xa, nqz = qb - qa;
         // axis 1: the line ends inside this z-range
-        const bool zlo = zr == 0 && p.top, zhi = zr == p.nzr - 1;
-        if (zlo || zhi)
-            for (int l = tid; l < SHELL * ncol; l += NT) {
-                const int y = ya + l / ncol, x = xa + l % ncol;
-                const long long line = (long long)y * n2 + x;
-                float *o = p.uo + line * s2;
-                float v[8], m[8];
-                if (zlo) {
-                    b3_ld8<true>(v, o);
-                    b3_mend<AL>(p, m, line, 0);
-                    b3_zlow<EXACT, NOP>(v, m, __ldg(p.zl + line));
-                    b3_st8<true>(o, v);
-                }
-                if (zhi) {
-                    b3_ld8<AL>(v, o + n1 - 8);
-                    b3_mend<AL>(p, m, line, 1);
-                    b3_zhigh<EXACT, NOP>(v, m, __ldg(p.zh + line));
-                    b3_st8<AL>(o + n1 - 8, v);
-                }
+        const bool zlo = zr == 0, zhi = zr == p.nzr - 1;
+        if ((zlo && p.top) || zhi) {
+            for (int l = tid; l < 2 * SHELL * ncol; l += NT) {
+                const int k = l >> 1;
+                if (l & 1 ? zhi : zlo && p.top)
+                    b3_end<EXACT, NOP, AL>(p, ya + k / ncol, xa + k % ncol, l & 1, false, false);
             }
-        __syncthreads();
-        // axis 2: the x-ranges holding a face, lines (y, z) of this z-range
-        const bool xlo = xr == 0, xhi = xr == p.nxr - 1;
-        if (xlo || xhi)
-            for (int l = tid; l < SHELL * nz; l += NT) {
-                const int y = ya + l / nz, z = za + l % nz;
-                const long long c0 = (long long)y * s3 + z;
-                if (xlo) b3_xline<EXACT, NOP>(p, c0, y, z, true, false);
-                if (xhi) b3_xline<EXACT, NOP>(p, c0, y, z, false, false);
-            }
-        __syncthreads();
-        // axis 3: columns (x, z), planes NOP..1 from NOP+1 or n3-1-NOP..n3-2 from n3-2-NOP
-        for (int l = tid; l < ncol * nz; l += NT) {
-            const int x = xa + l / nz, z = za + l % nz;
-            const long long c0 = (long long)x * s2 + z;
-            const int y0 = f == 0 ? NOP + 1 : n3 - SHELL, dy = f == 0 ? -1 : 1;
-            const float b = __ldg((f == 0 ? p.yl : p.yh) + (long long)x * n1 + z);
-            float v = p.uo[c0 + (long long)y0 * s3], mprev = __ldg(p.um + c0 + (long long)y0 * s3);
-#pragma unroll
-            for (int k = 1; k <= NOP; k++) {
-                const long long c = c0 + (long long)(y0 + k * dy) * s3;
-                const float mc = __ldg(p.um + c);
-                v = b3_abc<EXACT>(mprev, mc, v, b);
-                p.uo[c] = v;
-                mprev = mc;
-            }
-        }
-        if (p.w1) {
             __syncthreads();
-            // sponge of every cell of the block (all lie in the axis-3 shell);
-            // the pad cells of a line hold 0, their factors 1
-            const int nq = (nz + 3) / 4;
-            for (int l = tid; l < SHELL * ncol * nq; l += NT) {
-                const int y = ya + l / (ncol * nq), k = l % (ncol * nq), x = xa + k / nq, z = za + 4 * (k % nq);
-                float4 *c = reinterpret_cast<float4 *>(p.uo + (long long)y * s3 + (long long)x * s2 + z);
-                float4 v = *c;
-                const float4 wz = __ldg(reinterpret_cast<const float4 *>(p.w1 + z));
-                const float wx = __ldg(p.w2 + x), wy = __ldg(p.w3 + y);
-                v = make_float4(b3_damp<EXACT>(v.x, wz.x, wx, wy), b3_damp<EXACT>(v.y, wz.y, wx, wy),
-                                b3_damp<EXACT>(v.z, wz.z, wx, wy), b3_damp<EXACT>(v.w, wz.w, wx, wy));
-                *c = v;
-            }
         }
-        if (p.eo && (zr == 0 || zr == p.nzr - 1)) {  // the line ends this block holds, final now
+        // axis 2: the x-ranges holding a face
+        const bool xlo = xr == 0, xhi = xr == p.nxr - 1;
+        if (xlo || xhi) {
+            for (int l = tid; l < SHELL * nqz; l += NT) {
+                const int y = ya + l / nqz, z = 4 * (qa + l % nqz);
+                if (xlo) b3_xchain<EXACT, NOP, AL>(p, y, z, true, false);
+                if (xhi) b3_xchain<EXACT, NOP, AL>(p, y, z, false, false);
+            }
+            __syncthreads();
+        }
+        // axis 3 and the sponge (all cells lie in the axis-3 shell; the pad cells of a line hold 0)
+        const int y0 = f == 0 ? NOP + 1 : n3 - SHELL, dy = f == 0 ? -1 : 1;
+        for (int l = tid; l < ncol * nqz; l += NT) {
+            const int x = xa + l / nqz, z = 4 * (qa + l % nqz);
+            float b[4];
+            b3_coef4<AL>(b, (f == 0 ? p.yl : p.yh) + (long long)x * n1, z, n1);
+            b3_chain4<EXACT, NOP, 3>(p, y0 * s3 + x * s2 + z, dy * s3, b, z, sponge, p.w3 + y0, dy,
+                                     sponge ? __ldg(p.w2 + x) : 1.f);
+        }
+        if (p.eo && (zlo || zhi)) {  // the line ends this block holds, final now
             __syncthreads();
             for (int l = tid; l < SHELL * ncol * 4; l += NT) {
                 const int k = l >> 2, part = l & 3;
-                if (part < 2 ? zr != 0 : zr != p.nzr - 1) continue;
-                b3_eput_from_uo<AL>(p, (long long)(ya + k / ncol) * n2 + xa + k % ncol, part);
+                if (part < 2 ? zlo : zhi)
+                    b3_eput_from_uo<AL>(p, (long long)(ya + k / ncol) * n2 + xa + k % ncol, part);
             }
         }
         return;
     }
     blk -= 2 * p.nxr * p.nzr;
+    if (blk < p.end_blocks) {  // ---- axis-1 ends of the other lines
+        const int ni = n2 - 2 * SHELL, t = blk * NT + tid, l = t >> 1;
+        if (l < ni * p.n_int) b3_end<EXACT, NOP, AL>(p, SHELL + l / ni, SHELL + l % ni, t & 1, sponge, p.eo != nullptr);
+        return;
+    }
+    blk -= p.end_blocks;
     if (blk < p.rec_blocks) {  // ---- receiver gather of um (its pending sponge applied)
         const int r = blk * NT + tid;
         if (r >= p.nr) return;
@@ -355,9 +371,10 @@ void launch_bnd3(bool exact, Bnd3Params p, cudaStream_t s) {
     using namespace b3;
     p.n_int = p.g.n3 - 2 * (p.nop + 2);
     p.nxr = p.g.n2 / XR > 0 ? p.g.n2 / XR : 1;
-    p.nzr = p.g.n1 / ZR > 0 ? p.g.n1 / ZR : 1;
+    p.nzr = (p.g.n1 + 3) / 4 / ZQ > 0 ? (p.g.n1 + 3) / 4 / ZQ : 1;
+    p.end_blocks = (int)((2LL * p.n_int * (p.g.n2 - 2 * (p.nop + 2)) + NT - 1) / NT);
     p.rec_blocks = p.rec_row ? (p.nr + NT - 1) / NT : 0;
-    const int grid = p.n_int + 2 * p.nxr * p.nzr + p.rec_blocks + (p.inj.n > 0 ? (p.inj.n + NT - 1) / NT : p.ns > 0 ? 1 : 0);
+    const int grid = p.n_int + 2 * p.nxr * p.nzr + p.end_blocks + p.rec_blocks + (p.inj.n > 0 ? (p.inj.n + NT - 1) / NT : p.ns > 0 ? 1 : 0);
     switch (p.nop) {
         case 1: return exact ? launch_bnd3_nop<true, 1>(p, grid, s) : launch_bnd3_nop<false, 1>(p, grid, s);
         case 2: return exact ? launch_bnd3_nop<true, 2>(p, grid, s) : launch_bnd3_nop<false, 2>(p, grid, s);
@@ -376,12 +393,14 @@ void launch_bnd3(bool exact, Bnd3Params p, cudaStream_t s) {
 //     kappa[b] += t; kappa[i] += c t (b the inward neighbour of i),
 //  3. g = I vel2 mu on every cell (I: at least nop from every face), the
 //     field the adjoint step's stencil reads.
-// Block roles as in k_bnd3, so each cell's chain runs in one block: a plane y
-// in [6, n3-6) folds its axis-2 bands, runs the axis-2 lines, then folds and
-// transposes its axis-1 line ends together, then forms g for the plane; a
-// face block (6 axis-3 face planes x 16 columns x 64 cells of axis 1) folds
-// all its cells, runs the axis-3, axis-2 and axis-1 lines it holds, then
-// forms g.  The result does not depend on block order.
+// Roles by block as in k_bnd3, so each cell's chain runs in one block: the
+// axis-2 shell of a plane y in [6, n3-6) (fold, axis-2 transpose, then its
+// lines' ends, then g); a face block (6 axis-3 face planes x about 16 columns
+// x about 32 cells: fold and axis-3 transpose, axis 2, line ends, g); the ends of
+// every other line with their g, one thread per end; and the g of all other
+// cells, which nothing changes.  The result does not depend on block order.
+// The g pass streams 12 bytes a cell and bounds it.  (A block per plane for all
+// of its work: 51 us for 208 x 192 x 198 cells; so 24.6 us.)
 namespace b3a {
 __device__ __forceinline__ void tcell(float &mi, float &mb, float &kb, float &ki, float c) {
     const float v = mi;
@@ -397,88 +416,81 @@ __device__ __forceinline__ float wcell3(const Bnd3AdjParams &p, int z, int x, in
 }
 
 // mu += W kappa, kappa = 0 (cells whose kappa is 0 keep their value)
-__device__ __forceinline__ void fold(const Bnd3AdjParams &p, long long i, int z, int x, int y) {
-    const float kv = p.kap[i];
-    if (kv != 0.f) {
-        p.mu[i] += wcell3(p, z, x, y) * kv;
-        p.kap[i] = 0.f;
+__device__ __forceinline__ void fold(const Bnd3AdjParams &p, float &m, float &k, int z, int x, int y) {
+    if (k != 0.f) {
+        m += wcell3(p, z, x, y) * k;
+        k = 0.f;
     }
 }
 
-// transpose of one line's ABC updates: cells base + j*st, j = 0..n-1;
-// high face i = n-2 .. n-5 (b = i-1), low face i = 1 .. 4 (b = i+1)
-__device__ __forceinline__ void tline(const Bnd3AdjParams &p, long long base, long long st, int n, float cl, float ch,
-                                      bool low) {
-    for (int i = n - 2; i >= n - 5; i--) {
-        const long long ci = base + i * st, cb = ci - st;
-        float mi = p.mu[ci], mb = p.mu[cb], kb = p.kap[cb], ki = p.kap[ci];
-        tcell(mi, mb, kb, ki, ch);
-        p.mu[ci] = mi;
-        p.mu[cb] = mb;
-        p.kap[cb] = kb;
-        p.kap[ci] = ki;
-    }
-    if (low)
-        for (int i = 1; i <= 4; i++) {
-            const long long ci = base + i * st, cb = ci + st;
-            float mi = p.mu[ci], mb = p.mu[cb], kb = p.kap[cb], ki = p.kap[ci];
-            tcell(mi, mb, kb, ki, cl);
-            p.mu[ci] = mi;
-            p.mu[cb] = mb;
-            p.kap[cb] = kb;
-            p.kap[ci] = ki;
-        }
+__device__ __forceinline__ void ld4(float (&v)[4], const float *a) {
+    const float4 t = *reinterpret_cast<const float4 *>(a);
+    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+}
+__device__ __forceinline__ void st4(float *a, const float (&v)[4]) {
+    *reinterpret_cast<float4 *>(a) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
-// axis-1 ends of line `line` (n1 % 4 == 0): optionally fold cells 0..5 and
-// n1-6..n1-1 first, then the transposed updates, in registers
-__device__ __forceinline__ void zends(const Bnd3AdjParams &p, long long line, int x, int y, bool dofold) {
-    const int n1 = p.g.n1, q = n1 / 4;
-    float4 *M = reinterpret_cast<float4 *>(p.mu + line * n1);
-    float4 *K = reinterpret_cast<float4 *>(p.kap + line * n1);
-    auto fold4 = [&](float4 &m, float4 &k, int z0, unsigned mask) {
-        float *mv = &m.x, *kv = &k.x;
+// Cells z .. z+3 of a face along axis AXIS (2 or 3): the six shell cells from
+// the face cell at c0 inward (st); optional fold, then the transposed updates
+// of cells 4 .. 1 (high face: the one next to the face first) in registers.
+// (x, y) is the face cell, d the step inward; row the face's coefficients.
+template <int AXIS>
+__device__ __forceinline__ void face4(const Bnd3AdjParams &p, long long c0, long long st, const float *row, int z, int x,
+                                      int y, int d, bool dofold) {
+    float m[6][4], k[6][4], c[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-            if (((mask >> j) & 1u) && kv[j] != 0.f) {
-                mv[j] += wcell3(p, z0 + j, x, y) * kv[j];
-                kv[j] = 0.f;
-            }
-    };
-    {  // high end: cells n1-8 .. n1-1
-        float4 ma = M[q - 2], mb = M[q - 1], ka = K[q - 2], kb = K[q - 1];
-        if (dofold) {
-            fold4(ma, ka, n1 - 8, 12u);
-            fold4(mb, kb, n1 - 4, 15u);
+    for (int j = 0; j < 6; j++) {
+        ld4(m[j], p.mu + c0 + j * st);
+        ld4(k[j], p.kap + c0 + j * st);
+    }
+    {
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(row + z));
+        c[0] = t.x, c[1] = t.y, c[2] = t.z, c[3] = t.w;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        if (dofold)
+#pragma unroll
+            for (int j = 0; j < 6; j++)
+                fold(p, m[j][i], k[j][i], z + i, AXIS == 2 ? x + j * d : x, AXIS == 3 ? y + j * d : y);
+#pragma unroll
+        for (int j = 1; j <= 4; j++) tcell(m[j][i], m[j + 1][i], k[j + 1][i], k[j][i], c[i]);
+    }
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+        st4(p.mu + c0 + j * st, m[j]);
+        st4(p.kap + c0 + j * st, k[j]);
+    }
+}
+
+// one end of line (y, x) (0: cells 0..7, 1: n1-8..n1-1; n1 % 4 == 0): optional
+// fold of the shell cells, then the transposed updates, in registers (m: as left)
+__device__ __forceinline__ void lend(const Bnd3AdjParams &p, int y, int x, int end, bool dofold, float (&m)[8]) {
+    const long long line = (long long)y * p.g.n2 + x;
+    const int z0 = end ? p.g.n1 - 8 : 0;
+    float *M = p.mu + line * p.g.n1 + z0, *K = p.kap + line * p.g.n1 + z0;
+    float k[8];
+    b3_ld8<true>(m, M);
+    b3_ld8<true>(k, K);
+    if (dofold)
+#pragma unroll
+        for (int j = 0; j < 6; j++) {  // the shell: elements 0..5 or 2..7
+            const int e = end ? j + 2 : j;
+            if (end) fold(p, m[j + 2], k[j + 2], z0 + e, x, y);
+            else fold(p, m[j], k[j], z0 + e, x, y);
         }
+    if (end) {
         const float h = __ldg(p.zh + line);
-        tcell(mb.z, mb.y, kb.y, kb.z, h);
-        tcell(mb.y, mb.x, kb.x, kb.y, h);
-        tcell(mb.x, ma.w, ka.w, kb.x, h);
-        tcell(ma.w, ma.z, ka.z, ka.w, h);
-        M[q - 2] = ma;
-        M[q - 1] = mb;
-        K[q - 2] = ka;
-        K[q - 1] = kb;
+#pragma unroll
+        for (int j = 1; j <= 4; j++) tcell(m[7 - j], m[6 - j], k[6 - j], k[7 - j], h);
+    } else if (p.top) {
+        const float l = __ldg(p.zl + line);
+#pragma unroll
+        for (int j = 1; j <= 4; j++) tcell(m[j], m[j + 1], k[j + 1], k[j], l);
     }
-    {  // low end: cells 0 .. 7
-        float4 ma = M[0], mb = M[1], ka = K[0], kb = K[1];
-        if (dofold) {
-            fold4(ma, ka, 0, 15u);
-            fold4(mb, kb, 4, 3u);
-        }
-        if (p.top) {
-            const float l = __ldg(p.zl + line);
-            tcell(ma.y, ma.z, ka.z, ka.y, l);
-            tcell(ma.z, ma.w, ka.w, ka.z, l);
-            tcell(ma.w, mb.x, kb.x, ka.w, l);
-            tcell(mb.x, mb.y, kb.y, kb.x, l);
-        }
-        M[0] = ma;
-        M[1] = mb;
-        K[0] = ka;
-        K[1] = kb;
-    }
+    b3_st8<true>(M, m);
+    b3_st8<true>(K, k);
 }
 
 // g = I vel2 mu on the 4 cells z .. z+3 of line (y, x) (z % 4 == 0), from
@@ -500,165 +512,120 @@ __device__ __forceinline__ void gcells(const Bnd3AdjParams &p, int y, int z, int
     gstore(p, y, z, x, *reinterpret_cast<const float4 *>(p.mu + c), __ldg(reinterpret_cast<const float4 *>(p.vel2 + c)));
 }
 
-// g of a whole plane y, four groups of 4 cells per thread in flight
-__device__ __forceinline__ void gplane(const Bnd3AdjParams &p, int y, int tid) {
-    const int n1 = p.g.n1, n2 = p.g.n2, nq = n1 / 4, total = n2 * nq;
-    const long long base = (long long)y * n2 * n1;
-    for (int l0 = tid; l0 < total; l0 += 4 * b3::NT) {
-        float4 m[4], v[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int l = l0 + u * b3::NT;
-            if (l < total) {
-                const long long c = base + 4LL * l;  // line l / nq, cells 4 (l % nq) ..: contiguous in the plane
-                m[u] = *reinterpret_cast<const float4 *>(p.mu + c);
-                v[u] = __ldg(reinterpret_cast<const float4 *>(p.vel2 + c));
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int l = l0 + u * b3::NT;
-            if (l < total) gstore(p, y, 4 * (l % nq), l / nq, m[u], v[u]);
-        }
-    }
-}
 }  // namespace b3a
 
-__global__ void __launch_bounds__(b3::NT) k_bnd3_adj(const Bnd3AdjParams p) {
+__global__ void __launch_bounds__(b3::NT, 2) k_bnd3_adj(const Bnd3AdjParams p) {
     using namespace b3;
     using namespace b3a;
     const int tid = threadIdx.x;
-    const int n1 = p.g.n1, n2 = p.g.n2, n3 = p.g.n3;
+    const int n1 = p.g.n1, n2 = p.g.n2, n3 = p.g.n3, nq = n1 / 4;
     const long long s2 = n1, s3 = (long long)n1 * n2;
     int blk = blockIdx.x;
+    float m[8];
 
-    if (blk < p.n_int) {  // ---- one plane without axis-3 face cells
+    if (blk < p.n_int) {  // ---- the axis-2 shell of a plane without axis-3 face cells
         const int y = SHELL + blk;
-        // fold the axis-2 bands (x < 6, x >= n2-6), every z
-        for (int l = tid; l < 2 * SHELL * n1; l += NT) {
-            const int k = l / n1, z = l % n1, x = k < SHELL ? k : n2 - 2 * SHELL + k;
-            fold(p, (long long)y * s3 + (long long)x * s2 + z, z, x, y);
+        for (int l = tid; l < 2 * nq; l += NT) {
+            const bool low = l < nq;
+            const int z = 4 * (low ? l : l - nq), x = low ? 0 : n2 - 1, d = low ? 1 : -1;
+            face4<2>(p, (long long)y * s3 + x * s2 + z, d * s2, (low ? p.xl : p.xh) + (long long)y * n1, z, x, y, d, true);
         }
         __syncthreads();
-        // axis-2 lines (y, z)
-        for (int z = tid; z < n1; z += NT) {
-            const long long line = (long long)y * n1 + z;
-            tline(p, (long long)y * s3 + z, s2, n2, __ldg(p.xl + line), __ldg(p.xh + line), true);
+        if (tid < 4 * SHELL) {
+            const int k = tid >> 1;
+            lend(p, y, k < SHELL ? k : n2 - 2 * SHELL + k, tid & 1, false, m);
         }
         __syncthreads();
-        // axis-1 ends, folded here for the lines outside the axis-2 bands
-        for (int x = tid; x < n2; x += NT) zends(p, (long long)y * n2 + x, x, y, x >= SHELL && x < n2 - SHELL);
-        __syncthreads();
-        gplane(p, y, tid);
+        for (int l = tid; l < 2 * SHELL * nq; l += NT) {
+            const int k = l / nq;
+            gcells(p, y, 4 * (l % nq), k < SHELL ? k : n2 - 2 * SHELL + k);
+        }
         return;
     }
     blk -= p.n_int;
     if (blk < 2 * p.nxr * p.nzr) {  // ---- face block
         const int f = blk / (p.nxr * p.nzr), r = blk % (p.nxr * p.nzr), xr = r / p.nzr, zr = r % p.nzr;
-        const int xa = xr * XR, xb = xr == p.nxr - 1 ? n2 : xa + XR;
-        const int za = zr * ZR, zb = zr == p.nzr - 1 ? n1 : za + ZR;
+        const int xa = (int)((long long)n2 * xr / p.nxr), xb = (int)((long long)n2 * (xr + 1) / p.nxr);
+        const int qa = (int)((long long)nq * zr / p.nzr), qb = (int)((long long)nq * (zr + 1) / p.nzr);
         const int ya = f == 0 ? 0 : n3 - SHELL;
-        const int ncol = xb - xa, nz = zb - za;
-        for (int l = tid; l < SHELL * ncol * nz; l += NT) {  // fold every cell (all in the axis-3 shell)
-            const int y = ya + l / (ncol * nz), k = l % (ncol * nz), x = xa + k / nz, z = za + k % nz;
-            fold(p, (long long)y * s3 + (long long)x * s2 + z, z, x, y);
+        const int ncol = xb - xa, nqz = qb - qa;
+        // fold (every cell lies in the axis-3 shell) and axis 3
+        const int yf = f == 0 ? 0 : n3 - 1, dy = f == 0 ? 1 : -1;
+        for (int l = tid; l < ncol * nqz; l += NT) {
+            const int x = xa + l / nqz, z = 4 * (qa + l % nqz);
+            face4<3>(p, yf * s3 + x * s2 + z, dy * s3, (f == 0 ? p.yl : p.yh) + (long long)x * n1, z, x, yf, dy, true);
         }
         __syncthreads();
-        // axis 3: columns (x, z) of this block, the face planes only
-        for (int l = tid; l < ncol * nz; l += NT) {
-            const int x = xa + l / nz, z = za + l % nz;
-            const long long c0 = (long long)x * s2 + z;
-            const float b = __ldg((f == 0 ? p.yl : p.yh) + (long long)x * n1 + z);
-            if (f == 0) {
-                for (int i = 1; i <= 4; i++) {
-                    const long long ci = c0 + i * s3, cb = ci + s3;
-                    float mi = p.mu[ci], mb = p.mu[cb], kb = p.kap[cb], ki = p.kap[ci];
-                    tcell(mi, mb, kb, ki, b);
-                    p.mu[ci] = mi;
-                    p.mu[cb] = mb;
-                    p.kap[cb] = kb;
-                    p.kap[ci] = ki;
-                }
-            } else {
-                for (int i = n3 - 2; i >= n3 - 5; i--) {
-                    const long long ci = c0 + i * s3, cb = ci - s3;
-                    float mi = p.mu[ci], mb = p.mu[cb], kb = p.kap[cb], ki = p.kap[ci];
-                    tcell(mi, mb, kb, ki, b);
-                    p.mu[ci] = mi;
-                    p.mu[cb] = mb;
-                    p.kap[cb] = kb;
-                    p.kap[ci] = ki;
-                }
-            }
-        }
-        __syncthreads();
-        // axis 2: the x-ranges holding a face, lines (y, z) of this z-range
+        // axis 2: the x-ranges holding a face
         const bool xlo = xr == 0, xhi = xr == p.nxr - 1;
-        if (xlo || xhi)
-            for (int l = tid; l < SHELL * nz; l += NT) {
-                const int y = ya + l / nz, z = za + l % nz;
-                const long long line = (long long)y * n1 + z, c0 = (long long)y * s3 + z;
-                // a line's two faces belong to the first and the last x-range
-                if (xlo && xhi) {
-                    tline(p, c0, s2, n2, __ldg(p.xl + line), __ldg(p.xh + line), true);
-                } else if (xhi) {
-                    tline(p, c0, s2, n2, 0.f, __ldg(p.xh + line), false);
-                } else {  // low face only: i = 1 .. 4
-                    const float cl = __ldg(p.xl + line);
-                    for (int i = 1; i <= 4; i++) {
-                        const long long ci = c0 + i * s2, cb = ci + s2;
-                        float mi = p.mu[ci], mb = p.mu[cb], kb = p.kap[cb], ki = p.kap[ci];
-                        tcell(mi, mb, kb, ki, cl);
-                        p.mu[ci] = mi;
-                        p.mu[cb] = mb;
-                        p.kap[cb] = kb;
-                        p.kap[ci] = ki;
-                    }
-                }
+        if (xlo || xhi) {
+            for (int l = tid; l < SHELL * nqz; l += NT) {
+                const int y = ya + l / nqz, z = 4 * (qa + l % nqz);
+                const long long c = (long long)y * s3 + z, row = (long long)y * n1;
+                if (xhi) face4<2>(p, c + (n2 - 1) * s2, -s2, p.xh + row, z, n2 - 1, y, -1, false);
+                if (xlo) face4<2>(p, c, s2, p.xl + row, z, 0, y, 1, false);
             }
-        __syncthreads();
-        // axis 1: the line ends inside this z-range (already folded)
+            __syncthreads();
+        }
+        // axis 1: the line ends inside this z-range
         const bool zlo = zr == 0, zhi = zr == p.nzr - 1;
-        if (zlo && zhi) {
-            for (int l = tid; l < SHELL * ncol; l += NT) {
-                const int y = ya + l / ncol, x = xa + l % ncol;
-                zends(p, (long long)y * n2 + x, x, y, false);
+        if (zlo || zhi) {
+            for (int l = tid; l < 2 * SHELL * ncol; l += NT) {
+                const int k = l >> 1;
+                if (l & 1 ? zhi : zlo && p.top) lend(p, ya + k / ncol, xa + k % ncol, l & 1, false, m);
             }
-        } else if (zlo || zhi) {
-            for (int l = tid; l < SHELL * ncol; l += NT) {
-                const int y = ya + l / ncol, x = xa + l % ncol;
-                const long long line = (long long)y * n2 + x;
-                if (zhi) {
-                    tline(p, line * n1, 1, n1, 0.f, __ldg(p.zh + line), false);
-                } else if (p.top) {
-                    const float cl = __ldg(p.zl + line);
-                    for (int i = 1; i <= 4; i++) {
-                        const long long ci = line * n1 + i, cb = ci + 1;
-                        float mi = p.mu[ci], mb = p.mu[cb], kb = p.kap[cb], ki = p.kap[ci];
-                        tcell(mi, mb, kb, ki, cl);
-                        p.mu[ci] = mi;
-                        p.mu[cb] = mb;
-                        p.kap[cb] = kb;
-                        p.kap[ci] = ki;
-                    }
-                }
-            }
+            __syncthreads();
         }
-        __syncthreads();
-        const int nq = nz / 4;
-        for (int l = tid; l < SHELL * ncol * nq; l += NT) {
-            const int y = ya + l / (ncol * nq), k = l % (ncol * nq);
-            gcells(p, y, za + 4 * (k % nq), xa + k / nq);
+        for (int l = tid; l < SHELL * ncol * nqz; l += NT) {
+            const int k = l / nqz;
+            gcells(p, ya + k / ncol, 4 * (qa + l % nqz), xa + k % ncol);
         }
+        return;
+    }
+    blk -= 2 * p.nxr * p.nzr;
+    const int ni = n2 - 2 * SHELL;
+    if (blk < p.end_blocks) {  // ---- axis-1 ends of the other lines, and their g
+        const int t = blk * NT + tid, l = t >> 1, end = t & 1;
+        if (l >= ni * p.n_int) return;
+        const int y = SHELL + l / ni, x = SHELL + l % ni, z = end ? n1 - 8 : 0;
+        float v[8];
+        b3_ld8<true>(v, p.vel2 + ((long long)y * n2 + x) * n1 + z);
+        lend(p, y, x, end, true, m);
+        gstore(p, y, z, x, make_float4(m[0], m[1], m[2], m[3]), make_float4(v[0], v[1], v[2], v[3]));
+        gstore(p, y, z + 4, x, make_float4(m[4], m[5], m[6], m[7]), make_float4(v[4], v[5], v[6], v[7]));
+        return;
+    }
+    blk -= p.end_blocks;
+    // ---- g of the cells no transposed update touches, four groups of 4 cells per thread in flight
+    const int per = (ni * nq + 4 * NT - 1) / (4 * NT), y = SHELL + blk / per, l0 = blk % per * 4 * NT + tid;
+    const long long base = ((long long)y * n2 + SHELL) * n1;
+    float4 a[4], v[4];
+    bool in[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int l = l0 + u * NT, q = l % nq;
+        in[u] = l < ni * nq && q >= 2 && q < nq - 2;
+        if (in[u]) {
+            a[u] = *reinterpret_cast<const float4 *>(p.mu + base + 4LL * l);
+            v[u] = __ldg(reinterpret_cast<const float4 *>(p.vel2 + base + 4LL * l));
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int l = l0 + u * NT;
+        if (in[u]) gstore(p, y, 4 * (l % nq), SHELL + l / nq, a[u], v[u]);
     }
 }
 
 void launch_bnd3_adj(Bnd3AdjParams p, cudaStream_t s) {
     using namespace b3;
+    const int nq = p.g.n1 / 4, ni = p.g.n2 - 2 * SHELL;
     p.n_int = p.g.n3 - 2 * SHELL;
     p.nxr = p.g.n2 / XR > 0 ? p.g.n2 / XR : 1;
-    p.nzr = p.g.n1 / ZR > 0 ? p.g.n1 / ZR : 1;
-    k_bnd3_adj<<<p.n_int + 2 * p.nxr * p.nzr, NT, 0, s>>>(p);
+    p.nzr = nq / ZQ > 0 ? nq / ZQ : 1;
+    p.end_blocks = (int)((2LL * p.n_int * ni + NT - 1) / NT);
+    const int inner = p.n_int * ((ni * nq + 4 * NT - 1) / (4 * NT));
+    k_bnd3_adj<<<p.n_int + 2 * p.nxr * p.nzr + p.end_blocks + inner, NT, 0, s>>>(p);
 }
 
 }  // namespace awe
