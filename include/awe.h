@@ -325,7 +325,7 @@ typedef struct {
     long long cells;         /* padded cells of all shots */
     int tile_z, tile_x, grid; /* forward kernel: tile, or (n1, columns per item) of the column march */
     int work_items;           /* (shot, tile or column chunk) + (shot, receiver block) items per launch */
-    int launches_per_forward; /* = nt */
+    int launches_per_forward; /* nt, less where a launch takes several steps */
 } awe_batch_info_t;
 
 /* desc: the whole model (n[0] = nz, n[1] = model columns), nb, fdorder,
@@ -339,14 +339,16 @@ awe_status awe_batch_set_model(awe_batch *batch, const float *vel);
 awe_status awe_batch_forward(awe_batch *batch, const float *wav, float *dat);
 awe_status awe_batch_forward_device(awe_batch *batch, const float *d_wav, float *d_dat, void *stream);
 /* Autotuner: times `steps` time steps of every tile shape and grid size,
- * and of the column-march kernel (8th order: whole columns streamed by bulk
- * copies, chunks of 16/32/64 columns) on the current model and keeps the
- * fastest for the forward (the next forward recaptures); the gradient keeps
- * the fastest tile shape.  tile_out: the tile index, or 4 for the column
- * march; grid_out: the forward's grid. */
+ * of the column-march kernel (8th order: whole columns streamed by bulk
+ * copies, several chunk lengths) and of the kernel that takes several steps a
+ * launch (up to 8th order; the default) on the current model and keeps the
+ * fastest for the forward (the next forward recaptures); the gradient's sweeps
+ * take several steps a launch where they can, else the fastest tile shape.
+ * tile_out: the tile index, 4 for the column march, 5 for several steps a
+ * launch; grid_out: the forward's grid. */
 awe_status awe_batch_tune(awe_batch *batch, int steps, int *tile_out, int *grid_out);
 awe_status awe_batch_info(const awe_batch *batch, awe_batch_info_t *info);
-/* Picks the forward kernel without timing: kernel 0-3 = the tile shapes,
+/* Picks a one-step kernel without timing: kernel 0-3 = the tile shapes,
  * 4 = the column march with `chunk` columns per item (8th order only);
  * grid <= 0 = the default (4 CTAs per SM for tiles, every resident CTA for
  * the column march). */

@@ -83,3 +83,47 @@ def test_gradient_and_image_equal_the_one_step_kernels(n, nb, order, nt, ns, nr,
     for a, b in zip(ours, run()):
         np.testing.assert_array_equal(a, b)
     assert nr == 0 or np.abs(ours[0]).max() > 0
+
+
+@pytest.mark.parametrize("nz,nb,order,windows,jdata,fsrf", [
+    (12, 4, 2, [(0, 5), (3, 1)], 1, 0),            # windows narrower than a tile's strips
+    (60, 10, 8, [(0, 47), (20, 90), (101, 33)], 3, 1),
+    (120, 8, 4, [(0, 131), (7, 64), (7, 64)], 2, 0),  # two shots on one window
+    (200, 20, 6, [(0, 129)], 1, 0)])
+def test_batch_equals_the_tile_kernels(nz, nb, order, windows, jdata, fsrf):
+    """Traces, misfit and gradient of several steps a launch over windows of
+    several widths, against the one-step tile kernels (select(0)) bit for bit;
+    segments and traces that end inside a launch."""
+    import wavefield_imaging_gb300 as awe
+
+    rng = np.random.default_rng(nz)
+    nt, nxm = 53, max(x0 + nx for x0, nx in windows)
+    vel = (150 + 30 * rng.random((nxm, nz))).astype(np.float32)
+    shots = []
+    for k, (x0, nx) in enumerate(windows):
+        sou = np.stack([(x0 + rng.uniform(0.1, 0.9, k + 1) * (nx - 1)) * 5.0, rng.uniform(0.45, 0.6, k + 1) * (nz - 1) * 5.0], 1)
+        rec = np.stack([(x0 + np.linspace(0, nx - 1, 9)) * 5.0, np.full(9, 0.5 * (nz - 1) * 5.0)], 1)
+        shots.append((x0, nx, sou.astype(np.float32), rec.astype(np.float32)))
+    desc = awe.make_desc(2, (nz, nxm), (5.0, 5.0), (0.0, 0.0), nt, 0.005, nb=nb, fdorder=order, dabc=1, expl=1,
+                         jdata=jdata, fsrf=fsrf, precision=awe.FAST)
+    wav, out = ricker(nt, 0.005), []
+    # residuals at every receiver and step, whether the wave has come or not
+    obs = [rng.standard_normal(((nt - 1) // jdata + 1, 9)).astype(np.float32) for _ in windows]
+    with awe.Batch(desc, shots) as b:
+        b.set_model(vel)
+        assert b.info.launches_per_forward < nt
+        for sel in (False, True):
+            if sel:
+                b.select(0)
+                assert b.info.launches_per_forward == nt
+            d = b.forward(wav)
+            d2 = b.forward(wav)  # replayed
+            g, J = b.gradient(wav, obs, ckpt_every=7, ckpt_format=awe.CKPT_FP32)
+            out.append((d, d2, g, J))
+    (d0, e0, g0, J0), (d1, e1, g1, J1) = out
+    assert np.abs(g1).max() > 0 and J0 == J1
+    for a, b_, c, e in zip(d0, d1, e0, e1):
+        np.testing.assert_array_equal(a, b_)
+        np.testing.assert_array_equal(c, e)
+    # FP64 sums of the fold run in one order; the accumulators are the same bits
+    np.testing.assert_array_equal(g0, g1)

@@ -88,13 +88,22 @@ void launch_stepB(int ndim, int nop, bool exact, bool rho, const float *cur, flo
                   const float *den, const StepBParams &p, cudaStream_t s);
 
 // ---- several 2D steps in one launch (k_tb2d.cu) ----
-constexpr int kTb2Threads = 512;
+constexpr int kTb2Threads = 512, kTb2BatchThreads = 256;
 constexpr size_t kTb2SmemMax = 200 * 1024;
 // tile of tz x tx cells, k steps a launch, region of the tile and its halos
 // (rz x rx; hz >= nop k a multiple of 4, hx = nop k), cx columns a thread
 struct Tb2Shape {
     int k, tz, tx, hz, hx, rz, rx, ntz, ntx, cx;
 };
+// a tile of a batch: its window and its points in the lists (read at once, so
+// that the loads of its cells are not behind a chain of small ones)
+struct __align__(16) Tb2Tile {
+    long long off, dat_off;  // first cell and first trace sample of the window
+    int n2, wx_off, nr;      // its columns, first axis-2 sponge factor, receivers
+    int z0, x0;              // first cell of the tile
+    int rec0, nrec, cell0, ncell, ent0, nent, pad;
+};
+struct BatchShot;
 struct Tb2Params {
     int n1, n2, k, it;
     int tz, tx, hz, hx, rz, rx;
@@ -119,7 +128,33 @@ struct Tb2Params {
     const float *wav;
     int ncs, jdata, nr;
     float *dat;
+    const Tb2Tile *tiles;  // a batch: one block each (n2, nr, w2, wav of the adjoint and dat are per window)
 };
+// the lists of one grid's points (its tiles from tile0 on, ntx columns of them)
+struct Tb2Grid {
+    int n1, n2, ntx, tile0;
+    const GeoPoint *inj;
+    int ninj;
+    const GeoPoint *rec;
+    int nrec;
+};
+struct Tb2HostLists {
+    std::vector<int> buf;
+    size_t off[7];  // of Tb2Params' lists, in their order
+    int most[3];    // max_rec, max_cell, max_ent
+};
+// false: points on a grid's last line, or more in a tile than fit
+bool tb2_host_lists(const Tb2Shape &sh, const std::vector<Tb2Grid> &grids, int ntile, Tb2HostLists &out);
+size_t tb2_smem(const Tb2Shape &sh, const int *most);
+// points, lists and their sizes of a launch (buf: the lists on the device)
+void tb2_set_lists(Tb2Params &q, const int *buf, const size_t *off, const int *most, bool inj, bool rec);
+// the batch: ntile blocks; mode 0, 2 or 3, cx = 4
+void launch_tb2_batch(int nop, int mode, const Tb2Params &p, const Tb2Shape &sh, int ntile, size_t smem,
+                      cudaStream_t s);
+// imaging condition of a segment of the batch (k_tb2_image); cols: (shot, first of 4 columns)
+void launch_batch_image(float2 *G, const float *lap, const float *nu, long long stride, const BatchShot *shots,
+                        const int2 *cols, int ncols, int n1, int nop, const GeoPoint *src, const float *wav, int k0,
+                        int k1, cudaStream_t s);
 // mode 0: AWE_FAST, 1: AWE_EXACT, 2: the adjoint step, 3: AWE_FAST with slots
 void launch_tb2(int nop, int mode, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s);
 

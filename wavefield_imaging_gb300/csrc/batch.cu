@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <vector>
@@ -61,6 +62,22 @@ struct awe_batch {
     int4 *d_col_items = nullptr;
     int *d_err = nullptr;  // set by a bulk-copy wait that timed out
     int col_adj_grid = 0;  // column-march adjoint's grid (0: the tile adjoint)
+    // several steps a launch (k_tb2d.cu): possible for these points, the forward's; two more
+    // levels, the tiles, the point lists of the forward and of the adjoint
+    bool tb2_ok = false, tb2 = false, selected = false;  // selected: a kernel by awe_batch_select
+    Tb2Shape tb2_shape{};
+    std::vector<Tb2Grid> tb2_grids;
+    int tb2_tiles = 0, tb2_ncols = 0;
+    float *tb2_u = nullptr, *tb2_xy = nullptr;
+    int2 *d_tb2_cols = nullptr;
+    struct Lists {
+        int *buf = nullptr;
+        Tb2Tile *tiles = nullptr;
+        size_t off[7] = {};
+        int most[3] = {};
+    } tb2_fwd, tb2_adj;
+    bool tb2_grad = false, tb2_tried = false;  // the gradient's slots hold both sweeps of a segment; asked for
+    std::vector<GeoPoint> h_src;
 };
 
 #define CUDA_TRY(expr)                                                                            \
@@ -133,6 +150,132 @@ static awe_status build_col_items(awe_batch *b, int L) {
     return AWE_OK;
 }
 
+// Tile of k_tb2d.cu for all windows: 4 columns a thread, up to 256 threads, two
+// blocks per SM (one loads while the other steps).  A tile of r cells with its
+// halos takes about 2 us a launch and 0.25 us + 0.15 ns r a step alone on an SM,
+// 1.2 times as long beside another; lines of a multiple of 8 strips read shared
+// memory without bank conflicts (5 %).  Fitted to 12 windows of 592 x 580 cells at
+// 8th order, where 48 x 48 cells took 14.3 us a step with 2 steps a launch, 18.1
+// with one (56 x 56), 15.5 with three (40 x 40), and the one-step kernels 17.8.
+static bool tb2_batch_shape(const std::vector<BatchShot> &shots, int n1, int nop, int sms, Tb2Shape &best) {
+    double cost = 1e30;
+    for (int tz0 = 8; tz0 <= 120; tz0 += 4)
+        for (int tx = 8; tx <= 120; tx += 4)
+            for (int k = 1; k <= 12; k++) {
+                Tb2Shape s{};
+                s.k = k;
+                s.cx = 4;
+                s.ntz = (n1 + tz0 - 1) / tz0;
+                s.tz = ((n1 + s.ntz - 1) / s.ntz + 3) / 4 * 4;
+                s.ntz = (n1 + s.tz - 1) / s.tz;
+                s.tx = tx;
+                s.hx = nop * k;
+                s.hz = (s.hx + 3) / 4 * 4;
+                s.rz = s.tz + 2 * s.hz;
+                s.rx = (s.tx + 2 * s.hx + 3) / 4 * 4;
+                if ((s.rz / 4) * (s.rx / 4) > kTb2BatchThreads) break;
+                long long tiles = 0;
+                for (const BatchShot &sh : shots) tiles += (long long)s.ntz * ((sh.n2 + tx - 1) / tx);
+                const double r = (double)s.rz * s.rx;
+                const double rounds = tiles <= sms ? 1.0 : std::max(1.0, 0.6 * tiles / sms);
+                const double c = rounds * (2.0 / k + 0.25 + 1.5e-4 * r) * (s.rz % 32 ? 1.05 : 1.0);
+                if (c < cost) {
+                    cost = c;
+                    best = s;
+                }
+            }
+    return cost < 1e30;
+}
+
+static awe_status upload_lists(awe_batch *b, awe_batch::Lists &l, const Tb2HostLists &h) {
+    const Tb2Shape &sh = b->tb2_shape;
+    std::vector<Tb2Tile> tiles;
+    for (size_t s = 0; s < b->shots.size(); s++)
+        for (int k = 0; k < b->tb2_grids[s].ntx * sh.ntz; k++) {
+            const BatchShot &q = b->shots[s];
+            const int n = (int)tiles.size();
+            const int *c = &h.buf[h.off[0] + n], *e = &h.buf[h.off[1] + n], *r = &h.buf[h.off[2] + n];
+            tiles.push_back({q.off, q.dat_off, q.n2, q.wx_off, q.nr, k % sh.ntz * sh.tz, k / sh.ntz * sh.tx, r[0],
+                             r[1] - r[0], c[0], c[1] - c[0], e[0], e[1] - e[0], 0});
+        }
+    awe_status st = balloc(b, (void **)&l.buf, h.buf.size() * sizeof(int));
+    if (st == AWE_OK) st = balloc(b, (void **)&l.tiles, tiles.size() * sizeof(Tb2Tile));
+    if (st != AWE_OK) return st;
+    CUDA_TRY(cudaMemcpy(l.tiles, tiles.data(), tiles.size() * sizeof(Tb2Tile), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(l.buf, h.buf.data(), h.buf.size() * sizeof(int), cudaMemcpyHostToDevice));
+    std::copy(h.off, h.off + 7, l.off);
+    std::copy(h.most, h.most + 3, l.most);
+    return AWE_OK;
+}
+
+// tiles and point lists of k_tb2d.cu; b->tb2_ok stays false where it does not
+// apply (order above 8, a source in the sponge, points on a window's last
+// line, too many in a tile, no memory for two more levels)
+static awe_status set_tb2(awe_batch *b) {
+    const char *kern = std::getenv("AWE_STEP_KERNEL");
+    if (b->nop > 4 || (kern && std::strcmp(kern, "simple") == 0)) return AWE_OK;
+    for (const BatchShot &sh : b->shots)
+        for (int k = 0; k < sh.ns; k++) {
+            const GeoPoint &g = b->h_src[sh.src0 + k];
+            for (int c = 0; c < 4; c++) {
+                const long long n = g.base + (c & 1) + (c >> 1) * (long long)b->n1;
+                if (g.w[c] == 0.f || n >= (long long)sh.n2 * b->n1) continue;
+                if (b->h_wz[n % b->n1] != 1.f || b->h_wx[sh.wx_off + n / b->n1] != 1.f) return AWE_OK;
+            }
+        }
+    if (!tb2_batch_shape(b->shots, b->n1, b->nop, std::max(b->sms, 1), b->tb2_shape)) return AWE_OK;
+    const Tb2Shape &sh = b->tb2_shape;
+    std::vector<int2> cols;
+    for (int s = 0; s < (int)b->shots.size(); s++) {
+        const BatchShot &q = b->shots[s];
+        const int ntx = (q.n2 + sh.tx - 1) / sh.tx;
+        b->tb2_grids.push_back({b->n1, q.n2, ntx, b->tb2_tiles, b->h_src.data() + q.src0, q.ns,
+                                b->h_rec.data() + q.rec0, q.nr});
+        b->tb2_tiles += ntx * sh.ntz;
+        for (int x = 0; x < q.n2; x += 4) cols.push_back(make_int2(s, x));
+    }
+    b->tb2_ncols = (int)cols.size();
+    if (b->tb2_ncols > 65535) return AWE_OK;  // (rows of k_batch_image's grid)
+    Tb2HostLists h;
+    if (!tb2_host_lists(sh, b->tb2_grids, b->tb2_tiles, h)) return AWE_OK;
+    awe_status st = upload_lists(b, b->tb2_fwd, h);
+    if (st == AWE_OK) st = balloc(b, (void **)&b->d_tb2_cols, cols.size() * sizeof(int2));
+    if (st != AWE_OK) return st;
+    CUDA_TRY(cudaMemcpy(b->d_tb2_cols, cols.data(), cols.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    b->tb2_ok = balloc(b, (void **)&b->tb2_u, (size_t)2 * b->cells * sizeof(float)) == AWE_OK;
+    cudaGetLastError();
+    b->tb2 = b->tb2_ok;
+    return AWE_OK;
+}
+
+// k steps of every window from levels prv, cur: it .. it + k - 1 forward, it ..
+// it - k + 1 of the adjoint; slots: L of the levels read (adjoint: nu)
+static void tb2_steps(awe_batch *b, bool adj, const float *prv, const float *cur, float *oprv, float *ocur,
+                      float *slots, int it, int k, bool receivers, cudaStream_t s) {
+    const Tb2Shape &sh = b->tb2_shape;
+    const awe_batch::Lists &l = adj ? b->tb2_adj : b->tb2_fwd;
+    Tb2Params q{};
+    q.n1 = b->n1;
+    q.k = k;
+    q.it = it;
+    q.tz = sh.tz, q.tx = sh.tx, q.hz = sh.hz, q.hx = sh.hx, q.rz = sh.rz, q.rx = sh.rx;
+    q.c0 = b->k.c0;
+    for (int i = 0; i <= b->nop; i++) q.cz[i] = b->k.c[0][i], q.cx[i] = b->k.c[1][i];
+    q.cur = cur, q.prv = prv, q.vel = b->vel, q.ocur = ocur, q.oprv = oprv;
+    q.slots = slots;
+    q.slot_stride = b->cells;
+    if (b->d.dabc) q.w1 = b->wz, q.w2 = b->wx;
+    undamped_range(b->h_wz, q.ilo1, q.ihi1);
+    q.ilo2 = q.ilo1;  // (a window's axis-2 factors mirror the same profile: its high end is n2 - ilo2)
+    tb2_set_lists(q, l.buf, l.off, l.most, true, receivers);
+    q.wav = adj ? b->res : b->wav;
+    q.ncs = 1;
+    q.jdata = b->d.jdata;
+    q.dat = receivers ? b->dat : nullptr;
+    q.tiles = l.tiles;
+    launch_tb2_batch(b->nop, adj ? 2 : slots ? 3 : 0, q, sh, b->tb2_tiles, tb2_smem(sh, l.most), s);
+}
+
 static BatchStep step_params(const awe_batch *b, int it) {
     BatchStep p{};
     // level it lives in u[it & 1] (cur); the new level overwrites u[(it + 1) & 1]
@@ -168,7 +311,26 @@ static void launch_fwd(awe_batch *b, const BatchStep &p, cudaStream_t s, bool re
                        b->grid, p, s);
 }
 
+// steps it0 .. it1 - 1; hook(it, prv, cur) sees the levels before every step it % every == 0
+template <class Hook>
+static void tb2_range(awe_batch *b, int it0, int it1, cudaStream_t s, int every, const Hook &hook) {
+    float *prv = b->u[(it0 + 1) & 1], *cur = b->u[it0 & 1];
+    float *prv2 = b->tb2_u, *cur2 = b->tb2_u + b->cells;
+    for (int it = it0; it < it1;) {
+        int k = std::min(b->tb2_shape.k, it1 - it);
+        if (every > 0) {
+            if (it % every == 0) hook(it, prv, cur);
+            k = std::min(k, every - it % every);
+        }
+        tb2_steps(b, false, prv, cur, prv2, cur2, nullptr, it, k, b->ndat > 0, s);
+        std::swap(prv, prv2);
+        std::swap(cur, cur2);
+        it += k;
+    }
+}
+
 static void launch_range(awe_batch *b, int it0, int it1, cudaStream_t s) {
+    if (b->tb2) return tb2_range(b, it0, it1, s, 0, [](int, float *, float *) {});
     for (int it = it0; it < it1; it++) {
         const BatchStep p = step_params(b, it);
         if (b->colL > 0)
@@ -202,7 +364,7 @@ static awe_status run_all(awe_batch *b, cudaStream_t s) {
         }
     }
     CUDA_TRY(cudaGraphLaunch(b->exec, s));
-    b->launches = b->d.nt;
+    b->launches = b->tb2 ? (b->d.nt + b->tb2_shape.k - 1) / b->tb2_shape.k : b->d.nt;
     return AWE_OK;
 }
 
@@ -308,6 +470,7 @@ awe_status awe_batch_create(const awe_desc *desc, int nshots, const awe_shot *sh
     b->cells = off;
     b->ndat = doff;
     b->h_rec = hr;
+    b->h_src = hs;
     awe_status st = AWE_OK;
     const size_t cb = (size_t)off * sizeof(float);
     for (void **p : {(void **)&b->u[0], (void **)&b->u[1], (void **)&b->vel})
@@ -337,6 +500,7 @@ awe_status awe_batch_create(const awe_desc *desc, int nshots, const awe_shot *sh
         build_items(b);
         st = upload_items(b);
     }
+    if (st == AWE_OK) st = set_tb2(b);
     if (st != AWE_OK) {
         awe_batch_destroy(b);
         return st;
@@ -439,9 +603,24 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
     CUDA_TRY(cudaEventCreate(&e1));
-    float best = 1e30f;
+    float best = 1e30f, tb2_ms = 1e30f;
     int best_tile = b->tile, best_grid = b->grid;
     const size_t bytes = (size_t)b->cells * sizeof(float);
+    b->colL = 0;
+    if (b->tb2_ok) {
+        const int n = std::min((steps + b->tb2_shape.k - 1) / b->tb2_shape.k * b->tb2_shape.k, b->d.nt);
+        b->tb2 = true;
+        cudaMemsetAsync(b->u[0], 0, bytes, b->stream);
+        cudaMemsetAsync(b->u[1], 0, bytes, b->stream);
+        launch_range(b, 0, std::min(n, b->tb2_shape.k), b->stream);  // warm
+        cudaEventRecord(e0, b->stream);
+        launch_range(b, 0, n, b->stream);
+        cudaEventRecord(e1, b->stream);
+        CUDA_TRY(cudaEventSynchronize(e1));
+        cudaEventElapsedTime(&tb2_ms, e0, e1);
+        tb2_ms *= (float)steps / n;
+        b->tb2 = false;
+    }
     for (int t = 0; t < kBatchNumTiles; t++) {
         b->tile = t;
         build_items(b);
@@ -470,7 +649,18 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
     b->grid = best_grid;
     int best_col = 0, best_col_grid = 0;
     const int cpsm = batch2d_col_shape(b->nop, b->n1, nullptr) ? batch2d_col_ctas_per_sm(b->n1) : 0;
-    for (int L : {16, 32, 64}) {
+    // and the chunk length whose items take the fewest column times in whole
+    // waves (L + 8 a chunk): 48 windows of 592 x 580 had 484 items of 64 columns
+    // on 608 slots
+    int Lw = 64;
+    long long cols_best = -1;
+    for (int L = 12; cpsm > 0 && L <= 128; L++) {
+        long long items = 0;
+        for (const BatchShot &sh : b->shots) items += (sh.n2 + L - 1) / L;
+        const long long t = (items + (long long)cpsm * b->sms - 1) / ((long long)cpsm * b->sms) * (L + 8);
+        if (cols_best < 0 || t < cols_best) cols_best = t, Lw = L;
+    }
+    for (int L : {16, 32, 64, Lw}) {
         if (cpsm <= 0) break;
         awe_status st = build_col_items(b, L);
         if (st != AWE_OK) return st;
@@ -500,6 +690,8 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
         if (st != AWE_OK) return st;
         b->col_grid = best_col_grid;
     }
+    b->tb2 = tb2_ms < best;
+    b->selected = false;
     int bad = 0;
     CUDA_TRY(cudaMemcpy(&bad, b->d_err, sizeof bad, cudaMemcpyDeviceToHost));
     if (bad) {
@@ -511,8 +703,8 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
     if (st != AWE_OK) return st;
     drop_graph(b);  // recaptured with the chosen shape on the next forward
     CUDA_TRY(cudaGetLastError());
-    if (tile_out) *tile_out = b->colL > 0 ? kBatchNumTiles : best_tile;
-    if (grid_out) *grid_out = b->colL > 0 ? b->col_grid : best_grid;
+    if (tile_out) *tile_out = b->tb2 ? kBatchNumTiles + 1 : b->colL > 0 ? kBatchNumTiles : best_tile;
+    if (grid_out) *grid_out = b->tb2 ? b->tb2_tiles : b->colL > 0 ? b->col_grid : best_grid;
     return AWE_OK;
 }
 
@@ -558,7 +750,9 @@ static awe_status build_rec_cells(awe_batch *b) {
 }
 
 static awe_status grad_alloc(awe_batch *b, int T, int fmt) {
-    if (b->gT == T && b->gfmt == fmt) return AWE_OK;
+    const bool want = b->tb2_ok && !b->selected;
+    if (b->gT == T && b->gfmt == fmt && (b->tb2_grad || b->tb2_tried || !want)) return AWE_OK;
+    b->gT = 0;
     for (void *q : {(void *)b->slots, b->ckpt, (void *)b->scales}) {
         if (!q) continue;
         cudaFree(q);
@@ -569,7 +763,28 @@ static awe_status grad_alloc(awe_batch *b, int T, int fmt) {
     b->scales = nullptr;
     const int nseg = (b->d.nt + T - 1) / T;
     const size_t es = fmt == AWE_CKPT_FP32 ? 4 : 2;
-    awe_status st = balloc(b, (void **)&b->slots, (size_t)(T + 1) * b->cells * sizeof(float));
+    // several steps a launch: both sweeps of a segment and two more levels, where memory allows them
+    b->tb2_grad = false;
+    b->tb2_tried = want;
+    if (want) {
+        if (!b->tb2_adj.buf) {
+            std::vector<Tb2Grid> grids = b->tb2_grids;
+            for (Tb2Grid &g : grids) g.inj = g.rec, g.ninj = g.nrec, g.rec = nullptr, g.nrec = 0;
+            Tb2HostLists h;
+            if (tb2_host_lists(b->tb2_shape, grids, b->tb2_tiles, h)) {
+                const awe_status ls = upload_lists(b, b->tb2_adj, h);
+                if (ls != AWE_OK) return ls;
+            }
+        }
+        if (!b->tb2_xy && balloc(b, (void **)&b->tb2_xy, (size_t)2 * b->cells * sizeof(float)) != AWE_OK)
+            b->tb2_xy = nullptr;
+        b->tb2_grad = b->tb2_adj.buf && b->tb2_xy &&
+                      balloc(b, (void **)&b->slots, (size_t)std::max(2 * T, T + 1) * b->cells * sizeof(float)) == AWE_OK;
+        if (!b->tb2_grad) b->slots = nullptr;
+        cudaGetLastError();
+    }
+    awe_status st = AWE_OK;
+    if (!b->tb2_grad) st = balloc(b, (void **)&b->slots, (size_t)(T + 1) * b->cells * sizeof(float));
     if (st == AWE_OK) st = balloc(b, &b->ckpt, (size_t)2 * nseg * b->cells * es);
     b->gscale_per = fmt == AWE_CKPT_BFP16 ? (b->cells + kBfpBlock - 1) / kBfpBlock : (long long)b->shots.size();
     if (st == AWE_OK) st = balloc(b, (void **)&b->scales, (size_t)2 * nseg * b->gscale_per * sizeof(float));
@@ -623,6 +838,7 @@ static awe_status grad_sequence(awe_batch *b, cudaStream_t s) {
     const long long cells = b->cells;
     const size_t cb = (size_t)cells * sizeof(float);
     const int T = b->gT, ns = (int)b->shots.size();
+    const bool tb2 = b->tb2_grad && !b->selected;
     const size_t es = b->gfmt == AWE_CKPT_FP32 ? 4 : 2;
     auto ck = [&](int idx) { return (void *)((char *)b->ckpt + (size_t)idx * cells * es); };
     auto sc = [&](int idx) { return b->scales + (size_t)idx * b->gscale_per; };
@@ -630,24 +846,50 @@ static awe_status grad_sequence(awe_batch *b, cudaStream_t s) {
     CUDA_TRY(cudaMemsetAsync(b->d_err, 0, sizeof(int), s));
     CUDA_TRY(cudaMemsetAsync(b->u[0], 0, cb, s));
     CUDA_TRY(cudaMemsetAsync(b->u[1], 0, cb, s));
-    for (int it = 0; it < b->d.nt; it++) {
-        BatchStep p = step_params(b, it);
-        if (it % T == 0) {
-            const int seg = it / T;
-            launch_batch_ckpt(true, b->gfmt, b->d_shots, ns, p.nxt, ck(2 * seg), sc(2 * seg), b->n1, cells, s);
-            launch_batch_ckpt(true, b->gfmt, b->d_shots, ns, (float *)p.cur, ck(2 * seg + 1), sc(2 * seg + 1), b->n1,
-                              cells, s);
+    auto store = [&](int it, float *prv, float *cur) {
+        const int seg = it / T;
+        launch_batch_ckpt(true, b->gfmt, b->d_shots, ns, prv, ck(2 * seg), sc(2 * seg), b->n1, cells, s);
+        launch_batch_ckpt(true, b->gfmt, b->d_shots, ns, cur, ck(2 * seg + 1), sc(2 * seg + 1), b->n1, cells, s);
+    };
+    if (b->tb2) tb2_range(b, 0, b->d.nt, s, T, store);
+    else
+        for (int it = 0; it < b->d.nt; it++) {
+            BatchStep p = step_params(b, it);
+            if (it % T == 0) store(it, p.nxt, (float *)p.cur);
+            launch_fwd(b, p, s, true);
         }
-        launch_fwd(b, p, s, true);
-    }
     launch_residual_flat(b->dat, b->dobs, b->res, b->ndat, b->part, s);
     // adjoint sweep, last segment first
     CUDA_TRY(cudaMemsetAsync(b->gX, 0, cb, s));
     CUDA_TRY(cudaMemsetAsync(b->gY, 0, cb, s));
     CUDA_TRY(cudaMemsetAsync(b->G, 0, (size_t)cells * sizeof(float2), s));
     float *X = b->gX, *Y = b->gY;
+    float *X2 = b->tb2_xy, *Y2 = X2 + cells;  // (tb2)
     for (int seg = b->gseg - 1; seg >= 0; seg--) {
         const int k0 = seg * T, k1 = std::min(k0 + T, b->d.nt);
+        if (tb2) {
+            // both sweeps of the segment, several steps a launch, then its imaging condition at once
+            const int K = b->tb2_shape.k;
+            float *nu0 = b->slots + (size_t)T * cells;
+            float *A = b->u[0], *B = b->u[1], *A2 = b->tb2_u, *B2 = b->tb2_u + cells;
+            launch_batch_ckpt(false, b->gfmt, b->d_shots, ns, A, ck(2 * seg), sc(2 * seg), b->n1, cells, s);
+            launch_batch_ckpt(false, b->gfmt, b->d_shots, ns, B, ck(2 * seg + 1), sc(2 * seg + 1), b->n1, cells, s);
+            for (int k = k0; k < k1; k += K) {
+                tb2_steps(b, false, A, B, A2, B2, b->slots + (size_t)(k - k0) * cells, k, std::min(K, k1 - k), false, s);
+                std::swap(A, A2);
+                std::swap(B, B2);
+            }
+            for (int k = k1 - 1; k >= k0;) {
+                const int n = std::min(K, k - k0 + 1);
+                tb2_steps(b, true, Y, X, Y2, X2, nu0 + (size_t)(k1 - 1 - k) * cells, k, n, false, s);
+                std::swap(X, X2);
+                std::swap(Y, Y2);
+                k -= n;
+            }
+            launch_batch_image(b->G, b->slots, nu0, cells, b->d_shots, b->d_tb2_cols, b->tb2_ncols, b->n1, b->nop,
+                               b->src, b->wav, k0, k1, s);
+            continue;
+        }
         launch_batch_ckpt(false, b->gfmt, b->d_shots, ns, b->slots, ck(2 * seg), sc(2 * seg), b->n1, cells, s);
         launch_batch_ckpt(false, b->gfmt, b->d_shots, ns, b->slots + cells, ck(2 * seg + 1), sc(2 * seg + 1), b->n1,
                           cells, s);
@@ -737,6 +979,8 @@ awe_status awe_batch_select(awe_batch *b, int kernel, int chunk, int grid) {
     CUDA_TRY(cudaSetDevice(b->device));
     drop_graph(b);
     if (kernel < kBatchNumTiles) {
+        b->tb2 = false;
+        b->selected = true;
         b->tile = kernel;
         b->grid = grid > 0 ? grid : 4 * std::max(b->sms, 1);
         b->colL = 0;
@@ -752,6 +996,8 @@ awe_status awe_batch_select(awe_batch *b, int kernel, int chunk, int grid) {
         set_error("awe_batch_select: the column march does not fit on this device");
         return AWE_ERR_UNSUPPORTED;
     }
+    b->tb2 = false;
+    b->selected = true;
     awe_status st = build_col_items(b, chunk);
     if (st != AWE_OK) return st;
     b->col_grid = grid > 0 ? grid : cpsm * b->sms;
@@ -767,7 +1013,12 @@ awe_status awe_batch_info(const awe_batch *b, awe_batch_info_t *info) {
     info->nsmp = b->nsmp;
     info->total_samples = b->ndat;
     info->cells = b->cells;
-    if (b->colL > 0) {  // column march: whole columns, chunks of colL
+    if (b->tb2) {
+        info->tile_z = b->tb2_shape.tz;
+        info->tile_x = b->tb2_shape.tx;
+        info->grid = b->tb2_tiles;
+        info->work_items = b->tb2_tiles;
+    } else if (b->colL > 0) {  // column march: whole columns, chunks of colL
         info->tile_z = b->n1;
         info->tile_x = b->colL;
         info->grid = b->col_grid;
@@ -778,7 +1029,7 @@ awe_status awe_batch_info(const awe_batch *b, awe_batch_info_t *info) {
         info->grid = b->grid;
         info->work_items = (int)b->items.size();
     }
-    info->launches_per_forward = b->d.nt;
+    info->launches_per_forward = b->tb2 ? (b->d.nt + b->tb2_shape.k - 1) / b->tb2_shape.k : b->d.nt;
     return AWE_OK;
 }
 

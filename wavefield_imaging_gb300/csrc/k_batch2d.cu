@@ -1,4 +1,5 @@
-// Batched 2D forward of the CPU-program scheme: many shots, each on its own
+// Batched 2D forward of the CPU-program scheme, one step a launch (orders above
+// 8, points that k_tb2d.cu does not take, or selected): many shots, each on its own
 // window of one model, advanced one time step by one launch.
 //
 // A launch walks a flat list of work items: every (shot, tile) of the shots'

@@ -15,6 +15,12 @@
 // 592 x 592 8th order 4.35, 1.91; 141 x 183 4th order 2.45, 0.79; 1480 x 1480
 // 8th order 16.4, 8.6.  What bounds it now is the latency of a step in one
 // block per SM (0.4 of the issue slots), then shared-memory reads.
+//
+// A batch of shots takes its windows' tiles in one launch, two smaller blocks
+// per SM: 12 windows of 592 x 580 at 8th order 17.8 us a step with the one-step
+// kernels, 14.3 so; their gradient (recompute and adjoint sweep of a segment,
+// then its imaging condition at once) 102 us a step, 68 so.  48 such windows
+// stream from HBM, where the column march (52 us) is ahead of this (60).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,8 +37,10 @@ namespace {
 // MODE 0: AWE_FAST, 1: AWE_EXACT, 3: AWE_FAST storing slots (the gradient's recompute),
 // 2 (ADJ): the adjoint step (k_adjB): cur = nu_k, prv = nu_{k+1}, shared memory holds
 // I vel2 nu; step j is time step it - j; the cells' entries are receiver residuals
-template <int NOP, int MODE, int CX>
-__global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
+// BATCH: tiles of many shots' windows (p.tiles), with the operations of k_batch2d and
+// k_batch2d_adj, whose Laplacian is one chain of fused multiply-adds
+template <int NOP, int MODE, int CX, bool BATCH>
+__global__ void __launch_bounds__(BATCH ? kTb2BatchThreads : kTb2Threads, BATCH ? 2 : 1) k_tb2(const Tb2Params p) {
     constexpr bool EXACT = MODE == 1, ADJ = MODE == 2, SLOTS = MODE >= 2;
     extern __shared__ float smem[];
     const int zt = p.rz / 4, rz = p.rz, tid = threadIdx.x;
@@ -40,71 +48,97 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
     // four columns of padding on either side: outer halo strips read past the region
     const int plane = (p.rx + 8) * rz;
     float *S0 = smem + 4 * rz, *S1 = S0 + plane;
-    const int tz0 = blockIdx.x * p.tz, tx0 = blockIdx.y * p.tx;
+    int tz0 = blockIdx.x * p.tz, tx0 = blockIdx.y * p.tx, tile = blockIdx.y * gridDim.x + blockIdx.x;
+    int n2 = p.n2, nr = p.nr, ncs = p.ncs, ihi2 = p.ihi2;
+    int rec0, nrec, cell0, ncell, ent0, nent;  // the tile's points in the lists
+    long long off = 0;
+    const float *w2 = p.w2, *wav = p.wav;
+    float *dat = p.dat;
+    if constexpr (BATCH) {
+        tile = blockIdx.x;
+        const Tb2Tile t = p.tiles[tile];
+        tz0 = t.z0, tx0 = t.x0;
+        n2 = t.n2, nr = t.nr, ihi2 = n2 - p.ilo2;
+        off = t.off;
+        if (w2) w2 += t.wx_off;
+        if (dat) dat += t.dat_off;
+        if (ADJ) ncs = nr, wav += t.dat_off;
+        rec0 = t.rec0, nrec = p.rec_start ? t.nrec : 0, cell0 = t.cell0, ncell = t.ncell, ent0 = t.ent0, nent = t.nent;
+    } else {
+        rec0 = p.rec_start ? p.rec_start[tile] : 0, nrec = p.rec_start ? p.rec_start[tile + 1] - rec0 : 0;
+        cell0 = p.inj_start ? p.inj_start[tile] : 0, ncell = p.inj_start ? p.inj_start[tile + 1] - cell0 : 0;
+        ent0 = p.inj_start ? p.ent_start[tile] : 0, nent = p.inj_start ? p.ent_start[tile + 1] - ent0 : 0;
+    }
     const int z0 = tz0 - p.hz + 4 * zs, x0 = tx0 - p.hx + CX * xg;  // the thread's first cell
-    const int n1 = p.n1, n2 = p.n2, tz1 = min(tz0 + p.tz, n1), tx1 = min(tx0 + p.tx, n2);
+    const int n1 = p.n1, tz1 = min(tz0 + p.tz, n1), tx1 = min(tx0 + p.tx, n2);
     const int own = CX * xg * rz + 4 * zs;
-    const bool vec = (n1 & 3) == 0;
+    const bool vec = BATCH || (n1 & 3) == 0;
 
     // cells outside the grid take the nearest one's values: nothing a step keeps depends on them
     const int zc[4] = {min(max(z0, 0), vec ? n1 - 4 : n1 - 1), min(max(z0 + 1, 0), n1 - 1), min(max(z0 + 2, 0), n1 - 1),
                        min(max(z0 + 3, 0), n1 - 1)};
     auto load = [&](const float *src, int c) {
-        const float *q = src + (long long)min(max(x0 + c, 0), n2 - 1) * n1;
+        const float *q = src + off + (long long)min(max(x0 + c, 0), n2 - 1) * n1;
         return vec ? *reinterpret_cast<const float4 *>(q + zc[0]) : make_float4(q[zc[0]], q[zc[1]], q[zc[2]], q[zc[3]]);
     };
     float4 cur[CX], prv[CX], vel[CX];
     float wz[4], wx[CX];
+    // a batch has rounds of tiles: all loads of a tile go out first
+    if constexpr (BATCH) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;");
+#pragma unroll
+        for (int c = 0; c < CX; c++) {
+            cur[c] = load(p.cur, c);
+            prv[c] = load(p.prv, c);
+        }
+    }
     // what no step writes, before the wait for the previous launch
 #pragma unroll
     for (int c = 0; c < CX; c++) {
         vel[c] = load(p.vel, c);
-        wx[c] = p.w2 ? __ldg(p.w2 + min(max(x0 + c, 0), n2 - 1)) : 1.f;
+        wx[c] = w2 ? __ldg(w2 + min(max(x0 + c, 0), n2 - 1)) : 1.f;
     }
 #pragma unroll
     for (int i = 0; i < 4; i++) wz[i] = p.w1 ? __ldg(p.w1 + min(max(z0 + i, 0), n1 - 1)) : 1.f;
     // The tile's receivers and sources, with the wavelet samples of the launch's
     // steps, go to shared memory here: read from global memory in every step,
     // the chain of their loads made the tiles that hold them twice as slow.
-    const int tile = blockIdx.y * gridDim.x + blockIdx.x;
-    const int nrec = p.rec_start ? p.rec_start[tile + 1] - p.rec_start[tile] : 0;
-    const int ncell = p.inj_start ? p.inj_start[tile + 1] - p.inj_start[tile] : 0;
     float4 *rec_w = reinterpret_cast<float4 *>(smem + 2 * plane), *rec_d = rec_w + p.max_rec;
     int4 *cells = reinterpret_cast<int4 *>(rec_d + p.max_rec);  // cell, first and last entry, v^2 dt^2 (ADJ: sponge)
     int2 *rec_l = reinterpret_cast<int2 *>(cells + p.max_cell);  // cell, receiver
     int *mine = reinterpret_cast<int *>(rec_l + p.max_rec);      // per thread: first cell * 65536 + cells
     float *ent_w = reinterpret_cast<float *>(mine + kTb2Threads), *ent_d = ent_w + p.max_ent;
     for (int r = tid; r < nrec; r += blockDim.x) {
-        const int4 q = p.rec_pt[p.rec_start[tile] + r];  // z, x, receiver
+        const int4 q = p.rec_pt[rec0 + r];  // z, x, receiver
         rec_l[r] = make_int2((q.y - tx0 + p.hx) * rz + q.x - tz0 + p.hz, q.z);
-        rec_w[r] = *reinterpret_cast<const float4 *>(p.rec_wt + 4 * (p.rec_start[tile] + r));
-        if (p.w1) rec_d[r] = make_float4(p.w1[q.x], p.w1[q.x + 1], p.w2[q.y], p.w2[q.y + 1]);
+        rec_w[r] = *reinterpret_cast<const float4 *>(p.rec_wt + 4 * (rec0 + r));
+        if (p.w1) rec_d[r] = make_float4(p.w1[q.x], p.w1[q.x + 1], w2[q.y], w2[q.y + 1]);
     }
     if (ADJ) mine[tid] = 0;
     if (ncell > 0) {
-        const int i0 = p.inj_start[tile], e0 = p.ent_start[tile], nent = p.ent_start[tile + 1] - e0;
         if (ADJ) __syncthreads();
         auto owner = [&](const int4 &q) { return (q.y - tx0 + p.hx) / CX * zt + (q.x - tz0 + p.hz) / 4; };
         for (int s = tid; s < ncell; s += blockDim.x) {
-            const int4 q = p.inj_cell[i0 + s];  // z, x, first and last entry, a thread's cells one after the other
-            float f = ADJ ? 1.f : p.vel[(long long)q.y * n1 + q.x];
-            if (ADJ && p.w1) f = __fmul_rn(p.w1[q.x], p.w2[q.y]);
-            cells[s] = make_int4((q.y - tx0 + p.hx) * rz + q.x - tz0 + p.hz, q.z - e0, q.w - e0, __float_as_int(f));
+            const int4 q = p.inj_cell[cell0 + s];  // z, x, first and last entry, a thread's cells one after the other
+            float f = ADJ ? 1.f : p.vel[off + (long long)q.y * n1 + q.x];
+            if (ADJ && p.w1) f = __fmul_rn(p.w1[q.x], w2[q.y]);
+            cells[s] = make_int4((q.y - tx0 + p.hx) * rz + q.x - tz0 + p.hz, q.z - ent0, q.w - ent0, __float_as_int(f));
             const int o = owner(q);
-            if (ADJ && (s == 0 || owner(p.inj_cell[i0 + s - 1]) != o)) {
+            if (ADJ && (s == 0 || owner(p.inj_cell[cell0 + s - 1]) != o)) {
                 int n = 1;
-                while (s + n < ncell && owner(p.inj_cell[i0 + s + n]) == o) n++;
+                while (s + n < ncell && owner(p.inj_cell[cell0 + s + n]) == o) n++;
                 mine[o] = s * 65536 + n;
             }
         }
         for (int e = tid; e < nent; e += blockDim.x) {
-            const int2 en = p.inj_ent[e0 + e];
+            const int2 en = p.inj_ent[ent0 + e];
             ent_w[e] = __int_as_float(en.y);
             for (int j = 0; j < p.k; j++) {
                 const int it = ADJ ? p.it - j : p.it + j;
                 float d = 0.f;
-                if (!ADJ) d = p.wav[(long long)it * p.ncs + (p.ncs == 1 ? 0 : en.x >> 3)];
-                else if (it % p.jdata == 0) d = p.wav[(long long)(it / p.jdata) * p.ncs + (en.x >> 3)];
+                if (!ADJ) d = wav[(long long)it * ncs + (ncs == 1 ? 0 : en.x >> 3)];
+                else if (it % p.jdata == 0) d = wav[(long long)(it / p.jdata) * ncs + (en.x >> 3)];
                 ent_d[j * p.max_ent + e] = d;
             }
         }
@@ -121,7 +155,7 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
     auto store = [&](float *dst, int c, const float4 &v) {
         const int x = x0 + c;
         if (z0 < tz0 || z0 >= tz1 || x < tx0 || x >= tx1) return;
-        float *d = dst + (long long)x * n1 + z0;
+        float *d = dst + off + (long long)x * n1 + z0;
         if (vec) {
             *reinterpret_cast<float4 *>(d) = v;
         } else {
@@ -131,12 +165,17 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
             if (z0 + 3 < tz1) d[3] = v.w;
         }
     };
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;");
+    if constexpr (!BATCH) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;");
+#pragma unroll
+        for (int c = 0; c < CX; c++) {
+            cur[c] = load(p.cur, c);
+            prv[c] = load(p.prv, c);
+        }
+    }
 #pragma unroll
     for (int c = 0; c < CX; c++) {
-        cur[c] = load(p.cur, c);
-        prv[c] = load(p.prv, c);
         *reinterpret_cast<float4 *>(S0 + own + c * rz) = ADJ ? weighted(cur[c], c) : cur[c];
     }
     __syncthreads();
@@ -146,7 +185,7 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
     // uniform: every cell the steps compute is interior / keeps its value under the sponge
     const int e0 = NOP * (p.k - 1);
     const bool inner = tz0 - e0 - 3 >= NOP && tz1 + e0 + 3 <= n1 - NOP && tx0 - e0 - 3 >= NOP && tx1 + e0 + 3 <= n2 - NOP;
-    const bool damp = p.w1 && !(tz0 - e0 >= p.ilo1 && tz1 + e0 <= p.ihi1 && tx0 - e0 >= p.ilo2 && tx1 + e0 <= p.ihi2);
+    const bool damp = p.w1 && !(tz0 - e0 >= p.ilo1 && tz1 + e0 <= p.ihi1 && tx0 - e0 >= p.ilo2 && tx1 + e0 <= ihi2);
 
     // the thread's cells are within `need` of the tile: computed while the later
     // steps of the launch still need them
@@ -158,7 +197,8 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
 #pragma unroll 1
         for (int e = q.y; e < q.z; e++) {
             if constexpr (ADJ) {
-                v = __fadd_rn(v, __fmul_rn(f, __fmul_rn(f, __fmul_rn(ent_w[e], dd[e]))));
+                const float r = __fmul_rn(f, __fmul_rn(ent_w[e], dd[e]));
+                v = BATCH ? fmaf(f, r, v) : __fadd_rn(v, __fmul_rn(f, r));
             } else {
                 const float a = __fmul_rn(dd[e], ent_w[e]);
                 v = EXACT ? __fadd_rn(v, __fmul_rn(a, f)) : fmaf(a, f, v);
@@ -260,9 +300,14 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
                             }
                             const float2 x0p = __fadd2_rn(make_float2(xm.x, xm.y), make_float2(xp.x, xp.y));
                             const float2 x1p = __fadd2_rn(make_float2(xm.z, xm.w), make_float2(xp.z, xp.w));
+                            const float2 c0 = make_float2(p.c0, p.c0);
+                            if constexpr (BATCH) {
+                                l0 = __ffma2_rn(x0p, cx, __ffma2_rn(z0p, cz, k == 1 ? __fmul2_rn(u0, c0) : l0));
+                                l1 = __ffma2_rn(x1p, cx, __ffma2_rn(z1p, cz, k == 1 ? __fmul2_rn(u1, c0) : l1));
+                                continue;
+                            }
                             const float2 t0 = __ffma2_rn(z0p, cz, __fmul2_rn(x0p, cx));
                             const float2 t1 = __ffma2_rn(z1p, cz, __fmul2_rn(x1p, cx));
-                            const float2 c0 = make_float2(p.c0, p.c0);
                             l0 = k == 1 ? __ffma2_rn(u0, c0, t0) : __fadd2_rn(l0, t0);
                             l1 = k == 1 ? __ffma2_rn(u1, c0, t1) : __fadd2_rn(l1, t1);
                         }
@@ -304,7 +349,7 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
             }
             // receivers of the level this step reads, pending sponge applied (lint2d_extract)
             if (!ADJ && nrec > 0 && (p.jdata == 1 || it % p.jdata == 0)) {
-                float *row = p.dat + (long long)(it / p.jdata) * p.nr;
+                float *row = dat + (long long)(it / p.jdata) * nr;
                 for (int r = tid; r < nrec; r += blockDim.x) {
                     const int2 li = rec_l[r];
                     const float4 w = rec_w[r], d = rec_d[r];
@@ -347,10 +392,10 @@ __global__ void __launch_bounds__(kTb2Threads, 1) k_tb2(const Tb2Params p) {
     }
 }
 
-template <int NOP, int MODE, int CX>
-static void launch_cx(const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
+template <int NOP, int MODE, int CX, bool BATCH = false>
+static void launch_cx(const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s, int ntile = 0) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(sh.ntz, sh.ntx);
+    cfg.gridDim = BATCH ? dim3(ntile) : dim3(sh.ntz, sh.ntx);
     cfg.blockDim = dim3((sh.rz / 4) * (sh.rx / CX));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -359,8 +404,8 @@ static void launch_cx(const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaS
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaFuncSetAttribute(k_tb2<NOP, MODE, CX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTb2SmemMax);
-    cudaLaunchKernelEx(&cfg, k_tb2<NOP, MODE, CX>, p);
+    cudaFuncSetAttribute(k_tb2<NOP, MODE, CX, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTb2SmemMax);
+    cudaLaunchKernelEx(&cfg, k_tb2<NOP, MODE, CX, BATCH>, p);
 }
 
 template <int NOP, int CX>
@@ -380,7 +425,24 @@ static void launch_nop(int mode, const Tb2Params &p, const Tb2Shape &sh, size_t 
     else launch_mode<NOP, 4>(mode, p, sh, smem, s);
 }
 
+template <int NOP>
+static void launch_batch(int mode, const Tb2Params &p, const Tb2Shape &sh, int ntile, size_t smem, cudaStream_t s) {
+    if (mode == 0) launch_cx<NOP, 0, 4, true>(p, sh, smem, s, ntile);
+    else if (mode == 2) launch_cx<NOP, 2, 4, true>(p, sh, smem, s, ntile);
+    else launch_cx<NOP, 3, 4, true>(p, sh, smem, s, ntile);
+}
+
 }  // namespace
+
+void launch_tb2_batch(int nop, int mode, const Tb2Params &p, const Tb2Shape &sh, int ntile, size_t smem,
+                      cudaStream_t s) {
+    switch (nop) {
+        case 1: launch_batch<1>(mode, p, sh, ntile, smem, s); break;
+        case 2: launch_batch<2>(mode, p, sh, ntile, smem, s); break;
+        case 3: launch_batch<3>(mode, p, sh, ntile, smem, s); break;
+        default: launch_batch<4>(mode, p, sh, ntile, smem, s); break;
+    }
+}
 
 void launch_tb2(int nop, int mode, const Tb2Params &p, const Tb2Shape &sh, size_t smem, cudaStream_t s) {
     switch (nop) {
@@ -427,6 +489,66 @@ __global__ void __launch_bounds__(256) k_tb2_image(float2 *__restrict__ G, const
 void launch_tb2_image(float2 *G, const float *lap, const float *nu, long long stride, const AdjParams &p, int k0,
                       int k1, cudaStream_t s) {
     k_tb2_image<<<dim3((p.g.n1 + 63) / 64, (p.g.n2 + 3) / 4), dim3(64, 4), 0, s>>>(G, lap, nu, stride, p, k0, k1);
+}
+
+// The same for a batch: four cells of axis 1 per thread; a shot's few sources
+// are matched to the thread's cells once.
+__global__ void __launch_bounds__(128) k_batch_image(float2 *__restrict__ G, const float *__restrict__ lap,
+                                                     const float *__restrict__ nu, long long stride,
+                                                     const BatchShot *__restrict__ shots,
+                                                     const int2 *__restrict__ cols, int n1, int nop,
+                                                     const GeoPoint *__restrict__ src, const float *__restrict__ wav,
+                                                     int k0, int k1) {
+    const int2 item = cols[blockIdx.y];
+    const BatchShot sh = shots[item.x];
+    const int z = 4 * (blockIdx.x * 32 + threadIdx.x), x = item.y + threadIdx.y;
+    if (z >= n1 || x >= sh.n2) return;
+    const long long cell = (long long)x * n1 + z, i = sh.off + cell;
+    bool in[4], src_here = false;
+#pragma unroll
+    for (int c = 0; c < 4; c++) in[c] = x >= nop && x < sh.n2 - nop && z + c >= nop && z + c < n1 - nop;
+    for (int q = 0; q < sh.ns; q++) {  // corners lie within n1 + 1 of the base index
+        const long long b = src[sh.src0 + q].base - cell;
+        src_here = src_here || (b >= -(long long)n1 - 1 && b <= 3);
+    }
+    float4 *g = reinterpret_cast<float4 *>(G + i);
+    const float4 g0 = g[0], g1 = g[1];
+    float2 a[4] = {make_float2(g0.x, g0.y), make_float2(g0.z, g0.w), make_float2(g1.x, g1.y), make_float2(g1.z, g1.w)};
+    const float *l = lap + i + (k1 - k0) * stride;  // slot k - k0: L(V_k)
+    const float *n = nu + i;                        // slot k1 - 1 - k: nu_k
+#pragma unroll 4
+    for (int k = k1 - 1; k >= k0; k--) {
+        l -= stride;
+        const float4 lv = __ldcs(reinterpret_cast<const float4 *>(l)), nv = __ldcs(reinterpret_cast<const float4 *>(n));
+        n += stride;
+        const float lf[4] = {lv.x, lv.y, lv.z, lv.w}, nf[4] = {nv.x, nv.y, nv.z, nv.w};
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            if (in[c]) a[c] = gsum_add(a[c], __fmul_rn(nf[c], lf[c]));
+        if (src_here) {
+            const float dd = wav[k];
+#pragma unroll 1
+            for (int q = 0; q < sh.ns; q++) {
+                const GeoPoint gp = src[sh.src0 + q];
+#pragma unroll
+                for (int cc = 0; cc < 4; cc++) {
+                    const long long d = gp.base + (cc & 1) + (cc >> 1) * (long long)n1 - cell;
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        if (d == c) a[c] = gsum_add_prod(a[c], nf[c], __fmul_rn(dd, gp.w[cc]));
+                }
+            }
+        }
+    }
+    g[0] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);
+    g[1] = make_float4(a[2].x, a[2].y, a[3].x, a[3].y);
+}
+
+void launch_batch_image(float2 *G, const float *lap, const float *nu, long long stride, const BatchShot *shots,
+                        const int2 *cols, int ncols, int n1, int nop, const GeoPoint *src, const float *wav, int k0,
+                        int k1, cudaStream_t s) {
+    k_batch_image<<<dim3((n1 / 4 + 31) / 32, ncols), dim3(32, 4), 0, s>>>(G, lap, nu, stride, shots, cols, n1, nop, src,
+                                                                         wav, k0, k1);
 }
 
 }  // namespace awe

@@ -73,48 +73,55 @@ static Tb2Shape tb2_shape(const Grid &g, int nop, int sms) {
 }
 
 // two level buffers with their padding columns, the longest lists of a tile, a word per thread
-static size_t tb2_smem(const Tb2Shape &sh, const int *most) {
+size_t tb2_smem(const Tb2Shape &sh, const int *most) {
     return (size_t)2 * (sh.rx + 8) * sh.rz * 4 + (size_t)most[0] * 40 + (size_t)most[1] * 16 + kTb2Threads * 4 +
            (size_t)most[2] * 4 * (1 + sh.k);
 }
 
-awe_status set_tb2_lists(awe_plan *p, Tb2Lists &t, const std::vector<GeoPoint> &inj, const std::vector<GeoPoint> *rec) {
-    t.ok = false;
-    if (!p->tb2 || p->move_mode >= 0 || p->sponge_deferred) return AWE_OK;
-    const Grid &g = p->g;
-    const Tb2Shape &sh = p->tb2_shape;
-    const int ntile = sh.ntz * sh.ntx;
+bool tb2_host_lists(const Tb2Shape &sh, const std::vector<Tb2Grid> &grids, int ntile, Tb2HostLists &out) {
     struct Cell {
         int tile, owner;  // owner: the thread that holds the cell
         int4 q;
     };
-    // receivers by the tile of their base cell (all four corners are in its region)
-    std::vector<Cell> rc;
-    for (int r = 0; rec && r < (int)rec->size(); r++) {
-        const int z = (int)((*rec)[r].base % g.n1), x = (int)((*rec)[r].base / g.n1);
-        if (z >= g.n1 - 1 || x >= g.n2 - 1) return AWE_OK;
-        rc.push_back({(x / sh.tx) * sh.ntz + z / sh.tz, 0, make_int4(z, x, r, 0)});
-    }
-    // cells that points inject into, each with its entries in (point, corner)
-    // order, in every tile whose region holds the cell
-    std::vector<std::pair<long long, int>> e;
-    for (int s = 0; s < (int)inj.size(); s++)
-        for (int c = 0; c < 4; c++) {
-            const long long n = inj[s].base + p->h_corner_off[c];
-            if (n >= g.cells()) return AWE_OK;
-            e.push_back({n, 8 * s + c});
+    std::vector<Cell> rc, cell;
+    std::vector<const float *> rw;  // weights of the receivers in rc's first order
+    std::vector<int2> ea;           // entries of the grids' cells, in (point, corner) order per cell
+    size_t ns = 0;
+    for (const Tb2Grid &g : grids) {
+        // receivers by the tile of their base cell (all four corners are in its region)
+        for (int r = 0; r < g.nrec; r++) {
+            const int z = (int)(g.rec[r].base % g.n1), x = (int)(g.rec[r].base / g.n1);
+            if (z >= g.n1 - 1 || x >= g.n2 - 1) return false;
+            rc.push_back({g.tile0 + (x / sh.tx) * sh.ntz + z / sh.tz, (int)rw.size(), make_int4(z, x, r, 0)});
+            rw.push_back(g.rec[r].w);
         }
-    std::sort(e.begin(), e.end());
-    std::vector<Cell> cell;
-    for (size_t k = 0, k1; k < e.size(); k = k1) {
-        for (k1 = k; k1 < e.size() && e[k1].first == e[k].first;) k1++;
-        const int z = (int)(e[k].first % g.n1), x = (int)(e[k].first / g.n1);
-        for (int bx = std::max(0, (x - sh.hx) / sh.tx - 1); bx < sh.ntx && bx * sh.tx - sh.hx <= x; bx++)
-            for (int bz = std::max(0, (z - sh.hz) / sh.tz - 1); bz < sh.ntz && bz * sh.tz - sh.hz <= z; bz++) {
-                const int lx = x - bx * sh.tx + sh.hx, lz = z - bz * sh.tz + sh.hz;
-                if (lx < sh.rx && lz < sh.rz)
-                    cell.push_back({bx * sh.ntz + bz, lx / sh.cx * (sh.rz / 4) + lz / 4, make_int4(z, x, (int)k, (int)k1)});
+        // cells that points inject into, each with its entries, in every tile whose region holds the cell
+        ns += g.ninj;
+        std::vector<std::pair<long long, int>> e;
+        for (int s = 0; s < g.ninj; s++)
+            for (int c = 0; c < 4; c++) {
+                const long long n = g.inj[s].base + (c & 1) + (c >> 1) * (long long)g.n1;
+                if (n >= (long long)g.n1 * g.n2) return false;
+                e.push_back({n, 8 * s + c});
             }
+        std::sort(e.begin(), e.end());
+        const int ea0 = (int)ea.size();
+        for (const auto &v : e) {
+            int w;
+            std::memcpy(&w, &g.inj[v.second >> 3].w[v.second & 7], sizeof w);
+            ea.push_back(make_int2(v.second, w));
+        }
+        for (size_t k = 0, k1; k < e.size(); k = k1) {
+            for (k1 = k; k1 < e.size() && e[k1].first == e[k].first;) k1++;
+            const int z = (int)(e[k].first % g.n1), x = (int)(e[k].first / g.n1);
+            for (int bx = std::max(0, (x - sh.hx) / sh.tx - 1); bx < g.ntx && bx * sh.tx - sh.hx <= x; bx++)
+                for (int bz = std::max(0, (z - sh.hz) / sh.tz - 1); bz < sh.ntz && bz * sh.tz - sh.hz <= z; bz++) {
+                    const int lx = x - bx * sh.tx + sh.hx, lz = z - bz * sh.tz + sh.hz;
+                    if (lx < sh.rx && lz < sh.rz)
+                        cell.push_back({g.tile0 + bx * sh.ntz + bz, lx / sh.cx * (sh.rz / 4) + lz / 4,
+                                        make_int4(z, x, ea0 + (int)k, ea0 + (int)k1)});
+                }
+        }
     }
     auto order = [](const Cell &a, const Cell &b) { return a.tile != b.tile ? a.tile < b.tile : a.owner < b.owner; };
     std::stable_sort(rc.begin(), rc.end(), order);
@@ -125,11 +132,7 @@ awe_status set_tb2_lists(awe_plan *p, Tb2Lists &t, const std::vector<GeoPoint> &
     for (Cell &c : cell) {
         const int k0 = c.q.z, k1 = c.q.w;
         c.q.z = (int)ent.size();
-        for (int k = k0; k < k1; k++) {
-            int w;
-            std::memcpy(&w, &inj[e[k].second >> 3].w[e[k].second & 7], sizeof w);
-            ent.push_back(make_int2(e[k].second, w));
-        }
+        ent.insert(ent.end(), ea.begin() + k0, ea.begin() + k1);
         c.q.w = (int)ent.size();
         start[0][c.tile + 1]++;
         start[1][c.tile + 1] += k1 - k0;
@@ -141,15 +144,15 @@ awe_status set_tb2_lists(awe_plan *p, Tb2Lists &t, const std::vector<GeoPoint> &
             most[k] = std::max(most[k], start[k][q + 1]);
             start[k][q + 1] += start[k][q];
         }
-    t.most[0] = most[2];
-    t.most[1] = most[0];
-    t.most[2] = most[1];
-    if (most[0] >= 32768 || tb2_smem(sh, t.most) > kTb2SmemMax) return AWE_OK;  // one tile's points do not fit
-    // one buffer and one copy; sized for injected corners in four tiles each, so
-    // that points that only move keep it (a captured time loop reads it)
-    const size_t nst = (size_t)(ntile + 4) / 4 * 4 + 4, ns = inj.size(), nr = rc.size();
+    out.most[0] = most[2];
+    out.most[1] = most[0];
+    out.most[2] = most[1];
+    if (most[0] >= 32768 || tb2_smem(sh, out.most) > kTb2SmemMax) return false;  // one tile's points do not fit
+    // one buffer; sized for injected corners in four tiles each, so that points
+    // that only move keep it (a captured time loop reads it)
+    const size_t nst = (size_t)(ntile + 4) / 4 * 4 + 4, nr = rc.size();
     const size_t ncell = std::max(cell.size(), 16 * ns), nent = std::max(ent.size() + 1, 16 * ns + 1) / 2 * 2;
-    size_t *off = t.off;
+    size_t *off = out.off;
     off[0] = 0;
     off[1] = off[0] + nst;
     off[2] = off[1] + nst;
@@ -157,15 +160,29 @@ awe_status set_tb2_lists(awe_plan *p, Tb2Lists &t, const std::vector<GeoPoint> &
     off[4] = off[3] + 4 * ncell;    // rec_pt
     off[5] = off[4] + 4 * nr;       // inj_ent
     off[6] = off[5] + 2 * nent;     // rec_wt
-    const size_t total = off[6] + 4 * nr;
-    std::vector<int> buf(total, 0);
+    std::vector<int> &buf = out.buf;
+    buf.assign(off[6] + 4 * nr, 0);
     for (int k = 0; k < 3; k++) std::copy(start[k].begin(), start[k].end(), buf.begin() + off[k]);
     for (size_t k = 0; k < cell.size(); k++) std::memcpy(&buf[off[3] + 4 * k], &cell[k].q, sizeof(int4));
     if (!ent.empty()) std::memcpy(&buf[off[5]], ent.data(), ent.size() * sizeof(int2));
     for (size_t k = 0; k < rc.size(); k++) {
         std::memcpy(&buf[off[4] + 4 * k], &rc[k].q, sizeof(int4));
-        std::memcpy(&buf[off[6] + 4 * k], (*rec)[rc[k].q.z].w, 4 * sizeof(float));
+        std::memcpy(&buf[off[6] + 4 * k], rw[rc[k].owner], 4 * sizeof(float));
     }
+    return true;
+}
+
+awe_status set_tb2_lists(awe_plan *p, Tb2Lists &t, const std::vector<GeoPoint> &inj, const std::vector<GeoPoint> *rec) {
+    t.ok = false;
+    if (!p->tb2 || p->move_mode >= 0 || p->sponge_deferred) return AWE_OK;
+    const Tb2Shape &sh = p->tb2_shape;
+    const Tb2Grid grid{p->g.n1, p->g.n2, sh.ntx, 0, inj.data(), (int)inj.size(), rec ? rec->data() : nullptr,
+                       rec ? (int)rec->size() : 0};
+    Tb2HostLists h;
+    if (!tb2_host_lists(sh, {grid}, sh.ntz * sh.ntx, h)) return AWE_OK;
+    const size_t total = h.buf.size();
+    std::copy(h.off, h.off + 7, t.off);
+    std::copy(h.most, h.most + 3, t.most);
     if (t.cap < total) {
         dev_free(p, t.buf);
         t.buf = nullptr;
@@ -173,9 +190,20 @@ awe_status set_tb2_lists(awe_plan *p, Tb2Lists &t, const std::vector<GeoPoint> &
         AWE_TRY(dev_alloc(p, (void **)&t.buf, total * sizeof(int)));
         t.cap = total;
     }
-    CUDA_TRY(cudaMemcpy(t.buf, buf.data(), total * sizeof(int), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(t.buf, h.buf.data(), total * sizeof(int), cudaMemcpyHostToDevice));
     t.ok = true;
     return AWE_OK;
+}
+
+void tb2_set_lists(Tb2Params &q, const int *buf, const size_t *off, const int *most, bool inj, bool rec) {
+    if (most[1] > 0 && inj) q.inj_start = buf + off[0];
+    q.ent_start = buf + off[1];
+    if (most[0] > 0 && rec) q.rec_start = buf + off[2];
+    q.inj_cell = (const int4 *)(buf + off[3]);
+    q.rec_pt = (const int4 *)(buf + off[4]);
+    q.inj_ent = (const int2 *)(buf + off[5]);
+    q.rec_wt = (const float *)(buf + off[6]);
+    q.max_rec = most[0], q.max_cell = most[1], q.max_ent = most[2];
 }
 
 void tb2_launch(awe_plan *p, bool adj, const float *prv, const float *cur, float *oprv, float *ocur, float *slots,
@@ -197,14 +225,7 @@ void tb2_launch(awe_plan *p, bool adj, const float *prv, const float *cur, float
     q.slot_level = slot_level;
     if (d.dabc && !d.hybrid) q.w1 = p->w[0], q.w2 = p->w[1];
     q.ilo1 = p->wlo[0], q.ihi1 = p->whi[0], q.ilo2 = p->wlo[1], q.ihi2 = p->whi[1];
-    if (t.most[1] > 0 && d_wav) q.inj_start = t.buf + t.off[0];
-    q.ent_start = t.buf + t.off[1];
-    if (t.most[0] > 0 && d_dat) q.rec_start = t.buf + t.off[2];
-    q.inj_cell = (const int4 *)(t.buf + t.off[3]);
-    q.rec_pt = (const int4 *)(t.buf + t.off[4]);
-    q.inj_ent = (const int2 *)(t.buf + t.off[5]);
-    q.rec_wt = (const float *)(t.buf + t.off[6]);
-    q.max_rec = t.most[0], q.max_cell = t.most[1], q.max_ent = t.most[2];
+    tb2_set_lists(q, t.buf, t.off, t.most, d_wav != nullptr, d_dat != nullptr);
     q.wav = d_wav;
     q.ncs = ncs;
     q.jdata = d.jdata;
