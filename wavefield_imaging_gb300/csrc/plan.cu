@@ -590,14 +590,14 @@ awe_status awe_forward_device(awe_plan *p, const float *d_wav, int ncs, float *d
     }
     CUDA_TRY(cudaSetDevice(p->device));
     cudaStream_t s = stream ? (cudaStream_t)stream : p->stream;
-    // the loops of the CPU-program scheme and of the cartesian and polar
-    // GPU-program ones are pure stream
-    // work without a frame callback and profiling.  The first run with its
-    // pointers launches it directly (300 captured and instantiated steps cost
-    // 0.9 ms before the first one runs); a second one captures it as a CUDA
-    // graph, replayed from then on (what matters for small 2D grids).
+    // The time loop is pure stream work without a frame callback and profiling
+    // (a run restarts the work counter of the TMA kernels, so the bases in its
+    // launches hold for every replay).  The first run with its pointers launches
+    // it directly (300 captured and instantiated steps cost 0.9 ms before the
+    // first one runs); a second one captures it as a CUDA graph, replayed from
+    // then on (what matters for small grids).
     const bool cpu = p->d.scheme == AWE_SCHEME_CPU;
-    const bool graph = (cpu || p->pa.geom != 3) && !(p->nsnap > 0 && p->snap_cb) && !p->profile;
+    const bool graph = !(p->nsnap > 0 && p->snap_cb) && !p->profile;
     awe_status st = AWE_OK;
     if (!cpu) st = planA_prepare(p);  // uploads: not inside a capture
     if (st != AWE_OK) return st;

@@ -732,11 +732,11 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
     return AWE_OK;
     };  // seq
 
-    // Without the TMA path (whose work-counter bases are host state) and
-    // without snapshot delivery or profiling, the sequence is captured once as
+    // Without snapshot delivery or profiling, the sequence is captured once as
     // a CUDA graph and replayed while its buffers and settings stay the same
-    // (what matters for launch-bound 2D grids).
-    const bool graph = !st->tma && !p->snap_cb && !p->profile;
+    // (its forward run restarts the TMA kernels' work counter, so the bases in
+    // the captured launches hold for every replay).
+    const bool graph = !p->snap_cb && !p->profile;
     long long launches = 0;
     const void *key[4] = {d_wav, d_dobs, d_grad, dat};
     bool same = st->g_ncs == ncs && st->g_image == image;
