@@ -355,10 +355,10 @@ void launch_tb2_image(float2 *G, const float *lap, const float *nu, long long st
                       int k1, cudaStream_t s);
 void launch_abc_adjB(int nop, int fsrf, float *mu, float *kap, const AbcB &a, const Grid &g, cudaStream_t s);
 void launch_kap_fold(float *mu, float *kap, const AdjParams &p, cudaStream_t s);
-void launch_rec_adj(float *mu, const GeoPoint *pts, int nr, const float *r, const AdjParams &p, const long long *off,
-                    cudaStream_t s);
-void launch_src_grad_cells(float2 *G, const float *nu, const InjCells &c, const float *wav, int it, int ncs,
-                           bool one_wavelet, cudaStream_t s);
+// receiver residuals into mu and the source term of the gradient (c.n = 0: none)
+void launch_points_adj(float *mu, const GeoPoint *pts, int nr, const float *r, const AdjParams &p, const long long *off,
+                       float2 *G, const float *nu, const InjCells &c, const float *wav, int it, int ncs,
+                       bool one_wavelet, cudaStream_t s);
 void launch_residual(const float *d, const float *dobs, float *r, int nrows, int nr, double *row_sum, cudaStream_t s);
 // n1, p1: checkpoints hold the n cells of the levels' lines without their padding
 void launch_ckpt_store16(bool fp16, const float *u, long long n, unsigned int *amax, void *q, float *scale, int grid,

@@ -318,35 +318,38 @@ void launch_kap_fold(float *mu, float *kap, const AdjParams &p, cudaStream_t s) 
     k_kap_fold<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(mu, kap, p, W);
 }
 
-// W R^T r: receiver residuals into mu (scaled by W twice: once from the
-// gather of W V, once from mu = W lambda).  Coincident corners add atomically.
-__global__ void k_rec_adj(float *mu, const GeoPoint *__restrict__ pts, int nr, const float *__restrict__ r,
-                          AdjParams p, const long long *__restrict__ off) {
-    const int ir = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ir >= nr) return;
-    const GeoPoint pt = pts[ir];
-    const float rv = r[ir];
-    const Grid g = p.g;
-    const int nc = p.nd == 3 ? 8 : 4;
-    for (int c = 0; c < nc; c++) {
-        const long long n = pt.base + off[c];
-        const int i1 = (int)(n % g.p1), i2 = (int)((n / g.p1) % g.n2), i3 = (int)(n / ((long long)g.p1 * g.n2));
-        const float w = wcell(p, i1, i2, i3);
-        atomicAdd(mu + n, w * (w * (pt.w[c] * rv)));
+// The points' part of an adjoint step, one launch of two roles that share no
+// data.  W R^T r: receiver residuals into mu (scaled by W twice: once from the
+// gather of W V, once from mu = W lambda), one thread per receiver, its corners'
+// loads in flight together; coincident corners add atomically.  Source term of the gradient: dJ/dvel2[node] +=
+// nu[node] * wav * w, one thread per cell, its (source, corner) entries in
+// order.  Latency bounds it (1024 receivers, one source: two launches of 6.9 and
+// 3.1 us, this 6.8 us).
+template <int NC>
+__global__ void __launch_bounds__(128) k_points_adj(float *mu, const GeoPoint *__restrict__ pts, int nr,
+                                                    const float *__restrict__ r, AdjParams p,
+                                                    const long long *__restrict__ off, int rec_blocks, float2 *G,
+                                                    const float *__restrict__ nu, const InjCells c,
+                                                    const float *__restrict__ wav, int it, int ncs, int one_wavelet) {
+    if ((int)blockIdx.x < rec_blocks) {
+        const int ir = blockIdx.x * 128 + threadIdx.x;
+        if (ir >= nr) return;
+        const GeoPoint pt = pts[ir];
+        const float rv = r[ir];
+        const Grid g = p.g;
+        float v[NC];
+#pragma unroll
+        for (int k = 0; k < NC; k++) {
+            const long long n = pt.base + off[k];
+            const int i1 = (int)(n % g.p1), i2 = (int)((n / g.p1) % g.n2), i3 = (int)(n / ((long long)g.p1 * g.n2));
+            const float w = wcell(p, i1, i2, i3);
+            v[k] = w * (w * (pt.w[k] * rv));
+        }
+#pragma unroll
+        for (int k = 0; k < NC; k++) atomicAdd(mu + pt.base + off[k], v[k]);
+        return;
     }
-}
-
-void launch_rec_adj(float *mu, const GeoPoint *pts, int nr, const float *r, const AdjParams &p, const long long *off,
-                    cudaStream_t s) {
-    if (nr > 0) k_rec_adj<<<(nr + 127) / 128, 128, 0, s>>>(mu, pts, nr, r, p, off);
-}
-
-// source term of the gradient: dJ/dvel2[node] += nu[node] * wav * w, one thread
-// per cell, its (source, corner) entries in order
-__global__ void __launch_bounds__(128) k_src_grad_cells(float2 *G, const float *__restrict__ nu, const InjCells c,
-                                                        const float *__restrict__ wav, int it, int ncs,
-                                                        int one_wavelet) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (blockIdx.x - rec_blocks) * 128 + threadIdx.x;
     if (k >= c.n) return;
     const long long n = c.cell[k];
     float2 g = G[n];
@@ -359,9 +362,15 @@ __global__ void __launch_bounds__(128) k_src_grad_cells(float2 *G, const float *
     G[n] = g;
 }
 
-void launch_src_grad_cells(float2 *G, const float *nu, const InjCells &c, const float *wav, int it, int ncs,
-                           bool one_wavelet, cudaStream_t s) {
-    if (c.n > 0) k_src_grad_cells<<<(c.n + 127) / 128, 128, 0, s>>>(G, nu, c, wav, it, ncs, one_wavelet ? 1 : 0);
+void launch_points_adj(float *mu, const GeoPoint *pts, int nr, const float *r, const AdjParams &p, const long long *off,
+                       float2 *G, const float *nu, const InjCells &c, const float *wav, int it, int ncs,
+                       bool one_wavelet, cudaStream_t s) {
+    const int rec_blocks = (nr + 127) / 128, blocks = rec_blocks + (c.n + 127) / 128;
+    if (blocks == 0) return;
+    if (p.nd == 3)
+        k_points_adj<8><<<blocks, 128, 0, s>>>(mu, pts, nr, r, p, off, rec_blocks, G, nu, c, wav, it, ncs, one_wavelet);
+    else
+        k_points_adj<4><<<blocks, 128, 0, s>>>(mu, pts, nr, r, p, off, rec_blocks, G, nu, c, wav, it, ncs, one_wavelet);
 }
 
 // ---------------------------------------------------------------------------

@@ -714,12 +714,10 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
                 launch_kap_fold(Y, st->kap, ap, s);
                 launches++;
             }
-            if (k % d.jdata == 0 && p->nr > 0 && !fuse_pts) {
-                launch_rec_adj(Y, p->rec, p->nr, st->r + (size_t)(k / d.jdata) * p->nr, ap, p->corner_off, s);
-                launches++;
-            }
-            if (p->ns > 0 && !xcorr && !fuse_pts) {
-                launch_src_grad_cells(st->G, X, p->inj, d_wav, k, ncs, ncs == 1, s);
+            const bool rec = k % d.jdata == 0 && p->nr > 0, src = p->ns > 0 && !xcorr;
+            if (!fuse_pts && (rec || src)) {
+                launch_points_adj(Y, p->rec, rec ? p->nr : 0, rec ? st->r + (size_t)(k / d.jdata) * p->nr : nullptr, ap,
+                                  p->corner_off, st->G, X, src ? p->inj : InjCells{}, d_wav, k, ncs, ncs == 1, s);
                 launches++;
             }
             std::swap(X, Y);
