@@ -235,7 +235,6 @@ static awe_status set_tb2(awe_batch *b) {
         for (int x = 0; x < q.n2; x += 4) cols.push_back(make_int2(s, x));
     }
     b->tb2_ncols = (int)cols.size();
-    if (b->tb2_ncols > 65535) return AWE_OK;  // (rows of k_batch_image's grid)
     Tb2HostLists h;
     if (!tb2_host_lists(sh, b->tb2_grids, b->tb2_tiles, h)) return AWE_OK;
     awe_status st = upload_lists(b, b->tb2_fwd, h);

@@ -499,9 +499,9 @@ __global__ void __launch_bounds__(128) k_batch_image(float2 *__restrict__ G, con
                                                      const int2 *__restrict__ cols, int n1, int nop,
                                                      const GeoPoint *__restrict__ src, const float *__restrict__ wav,
                                                      int k0, int k1) {
-    const int2 item = cols[blockIdx.y];
+    const int2 item = cols[blockIdx.x];
     const BatchShot sh = shots[item.x];
-    const int z = 4 * (blockIdx.x * 32 + threadIdx.x), x = item.y + threadIdx.y;
+    const int z = 4 * (blockIdx.y * 32 + threadIdx.x), x = item.y + threadIdx.y;
     if (z >= n1 || x >= sh.n2) return;
     const long long cell = (long long)x * n1 + z, i = sh.off + cell;
     bool in[4], src_here = false;
@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(128) k_batch_image(float2 *__restrict__ G, con
 void launch_batch_image(float2 *G, const float *lap, const float *nu, long long stride, const BatchShot *shots,
                         const int2 *cols, int ncols, int n1, int nop, const GeoPoint *src, const float *wav, int k0,
                         int k1, cudaStream_t s) {
-    k_batch_image<<<dim3((n1 / 4 + 31) / 32, ncols), dim3(32, 4), 0, s>>>(G, lap, nu, stride, shots, cols, n1, nop, src,
+    k_batch_image<<<dim3(ncols, (n1 / 4 + 31) / 32), dim3(32, 4), 0, s>>>(G, lap, nu, stride, shots, cols, n1, nop, src,
                                                                          wav, k0, k1);
 }
 
