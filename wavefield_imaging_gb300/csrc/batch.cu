@@ -762,29 +762,7 @@ static awe_status grad_alloc(awe_batch *b, int T, int fmt) {
     b->scales = nullptr;
     const int nseg = (b->d.nt + T - 1) / T;
     const size_t es = fmt == AWE_CKPT_FP32 ? 4 : 2;
-    // several steps a launch: both sweeps of a segment and two more levels, where memory allows them
-    b->tb2_grad = false;
-    b->tb2_tried = want;
-    if (want) {
-        if (!b->tb2_adj.buf) {
-            std::vector<Tb2Grid> grids = b->tb2_grids;
-            for (Tb2Grid &g : grids) g.inj = g.rec, g.ninj = g.nrec, g.rec = nullptr, g.nrec = 0;
-            Tb2HostLists h;
-            if (tb2_host_lists(b->tb2_shape, grids, b->tb2_tiles, h)) {
-                const awe_status ls = upload_lists(b, b->tb2_adj, h);
-                if (ls != AWE_OK) return ls;
-            }
-        }
-        if (!b->tb2_xy && balloc(b, (void **)&b->tb2_xy, (size_t)2 * b->cells * sizeof(float)) != AWE_OK)
-            b->tb2_xy = nullptr;
-        b->tb2_grad = b->tb2_adj.buf && b->tb2_xy &&
-                      balloc(b, (void **)&b->slots, (size_t)std::max(2 * T, T + 1) * b->cells * sizeof(float)) == AWE_OK;
-        if (!b->tb2_grad) b->slots = nullptr;
-        cudaGetLastError();
-    }
-    awe_status st = AWE_OK;
-    if (!b->tb2_grad) st = balloc(b, (void **)&b->slots, (size_t)(T + 1) * b->cells * sizeof(float));
-    if (st == AWE_OK) st = balloc(b, &b->ckpt, (size_t)2 * nseg * b->cells * es);
+    awe_status st = balloc(b, &b->ckpt, (size_t)2 * nseg * b->cells * es);
     b->gscale_per = fmt == AWE_CKPT_BFP16 ? (b->cells + kBfpBlock - 1) / kBfpBlock : (long long)b->shots.size();
     if (st == AWE_OK) st = balloc(b, (void **)&b->scales, (size_t)2 * nseg * b->gscale_per * sizeof(float));
     if (st != AWE_OK) return st;
@@ -804,6 +782,37 @@ static awe_status grad_alloc(awe_batch *b, int T, int fmt) {
         for (size_t s = 0; s < w.size(); s++) w[s] = make_int2(b->shots_in[s].x0, b->shots_in[s].nx);
         CUDA_TRY(cudaMemcpy(b->win, w.data(), w.size() * sizeof(int2), cudaMemcpyHostToDevice));
     }
+    // several steps a launch: slots for both sweeps of a segment and two more
+    // levels, where memory is left for them when all else is allocated
+    b->tb2_grad = false;
+    b->tb2_tried = want;
+    if (want) {
+        if (!b->tb2_adj.buf) {
+            std::vector<Tb2Grid> grids = b->tb2_grids;
+            for (Tb2Grid &g : grids) g.inj = g.rec, g.ninj = g.nrec, g.rec = nullptr, g.nrec = 0;
+            Tb2HostLists h;
+            if (tb2_host_lists(b->tb2_shape, grids, b->tb2_tiles, h)) {
+                st = upload_lists(b, b->tb2_adj, h);
+                if (st != AWE_OK) return st;
+            }
+        }
+        if (b->tb2_adj.buf && !b->tb2_xy &&
+            balloc(b, (void **)&b->tb2_xy, (size_t)2 * b->cells * sizeof(float)) != AWE_OK)
+            b->tb2_xy = nullptr;
+        b->tb2_grad = b->tb2_adj.buf && b->tb2_xy &&
+                      balloc(b, (void **)&b->slots, (size_t)std::max(2 * T, T + 1) * b->cells * sizeof(float)) == AWE_OK;
+        if (!b->tb2_grad) {
+            b->slots = nullptr;
+            if (b->tb2_xy) {
+                cudaFree(b->tb2_xy);
+                b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), (void *)b->tb2_xy));
+                b->tb2_xy = nullptr;
+            }
+        }
+        cudaGetLastError();
+    }
+    if (!b->tb2_grad) st = balloc(b, (void **)&b->slots, (size_t)(T + 1) * b->cells * sizeof(float));
+    if (st != AWE_OK) return st;
     b->gT = T;
     b->gfmt = fmt;
     b->gseg = nseg;
