@@ -1007,7 +1007,7 @@ def run_batch(args):
            "achieved_GBps": 16.0 * cells * nt / (ms / 1e3) / 1e9,
            "plain": {"ms": plain_ms, "shots_per_s": nshots / (plain_ms / 1e3), "launches": plain_launches},
            "speedup_vs_plain": plain_ms / ms, "max_rel_l2_vs_plain": worst,
-           "gpu_launches": nt * args.steps, "clocks": clocks}
+           "gpu_launches": batch.info.launches_per_forward * args.steps, "clocks": clocks}
     print(json.dumps(out))
     batch.close()
 
