@@ -190,8 +190,10 @@ void launch_model_abc(const float *raw, const ModelPrep &m, float *const abc[6],
 // The boundary work of a 3D step in one launch (k_boundary3.cu): one-way ABC
 // of the six faces, sponge of the shell the step kernel left unsponged
 // (cells within nop + 2 of a face), the receiver gather of the level the step
-// read, and the injection (ns > 0; only when no source corner lies in that
-// shell, whose cells the ABC reads).
+// read, and the injection (ns > 0; only when no source corner lies on a cell
+// that the launch's other blocks store: that shell, and the kBndEnd cells at
+// each end of a line, which are loaded and stored together).
+constexpr int kBndEnd = 8;
 struct Bnd3Params {
     Grid g;
     float *uo;        // the new level

@@ -2,8 +2,9 @@
 // the one-way ABC of the six faces (abcone3d_apply, fdutil.c:2085-2177), the
 // sponge of the shell the step kernel left unsponged (sponge3d_apply,
 // fdutil.c:2248-2310), the receiver gather of the level the step read
-// (lint3d_extract, fdutil.c:1653-1670) and, when no source touches the shell,
-// the injection (lint3d_inject1_with_vv, fdutil.c:1723-1740).
+// (lint3d_extract, fdutil.c:1653-1670) and, when no source touches a cell that
+// another role stores, the injection (lint3d_inject1_with_vv,
+// fdutil.c:1723-1740).
 //
 // The reference applies the ABC as three passes over the whole grid (axis-1
 // lines, then axis-2 lines, then axis-3 lines, each an outward recurrence over
@@ -46,6 +47,7 @@ namespace b3 {
 constexpr int SHELL = 6;  // the adjoint's nop + 2 (nop = 4): cells the ABC writes (1..4) or reads (5), and the face cell 0
 constexpr int XR = 16, ZQ = 8;  // face blocks: least columns and 4-cell groups of axis 1
 constexpr int NT = 256;
+static_assert(kBndEnd == 8, "b3_ld8, b3_st8: the cells of a line end");
 }  // namespace b3
 
 template <bool EXACT>
@@ -193,7 +195,8 @@ __device__ __forceinline__ void b3_eput_from_uo(const Bnd3Params &p, long long l
 }
 
 // One end of line (y, x) (0: low, 1: high): the axis-1 recurrence and, with
-// damp, the sponge of its shell cells; the final values go to the compact copy
+// damp, the sponge of its shell cells; all eight cells are stored, so no source
+// of this launch lies on them; the final values go to the compact copy
 // if put (without a sponge and with a free surface the low end is not read,
 // nor needed: the next step's low-end recurrence is off).
 template <bool EXACT, int NOP, bool AL>

@@ -57,7 +57,7 @@ struct awe_plan {
     std::vector<awe::GeoPoint> h_src, h_rec;
     std::vector<awe::Lint> h_src_lint;  // source corner indices in the reference's fdm axes
     bool sponge_deferred = false;  // a source node lies in the sponge band outside the boundary shell
-    bool src_in_shell = false;     // a source node lies within nop + 2 of a face (3D)
+    bool src_in_shell = false;     // a source corner lies on a cell that the 3D boundary launch stores
     int src_cap = 0, rec_cap = 0;  // points the src / rec device buffers hold
     // fixed sources by cell (set_inj_cells): one buffer, kept while large enough
     awe::InjCells inj{};

@@ -508,26 +508,29 @@ awe_status set_geometry_common(awe_plan *p, int ns, const float *sou, int nr, co
 
     // scheme CPU: a source node inside the sponge band but outside the
     // boundary shell would be sponged before its injection by the fused
-    // step; such runs defer the whole sponge to after the injection
+    // step; such runs defer the whole sponge to after the injection.
+    // src_in_shell: a corner lies on a cell that the 3D boundary launch stores
+    // (the shell, and the eight cells it rewrites at each end of a line).  A
+    // corner of weight 0 counts: its cell is read and stored all the same.
     p->sponge_deferred = false;
     p->src_in_shell = false;
     if (d.scheme == AWE_SCHEME_CPU && d.dabc && !d.hybrid) {
-        const int shell = (nd == 3) ? p->nop + 2 : 0;
+        const int shell = (nd == 3) ? p->nop + 2 : 0, ends = (nd == 3) ? std::max(shell, kBndEnd) : 0;
         const int nc = nd == 3 ? 8 : 4;
         for (const GeoPoint &gp : p->h_src)
             for (int c = 0; c < nc; c++) {
-                if (gp.w[c] == 0.f) continue;
                 const long long n = gp.base + off[c];
                 const int i3 = (int)(n / s3), i2 = (int)((n % s3) / s2), i1 = (int)(n % s2);
                 const int ii[3] = {i1, i2, i3}, nn[3] = {g.n1, g.n2, g.n3};
-                bool band = false, inshell = false;
+                bool band = false, inshell = false, stored = false;
                 for (int a = 0; a < nd; a++) {
                     const int dist = std::min(ii[a], nn[a] - 1 - ii[a]);
                     band = band || dist < p->nbd;
                     inshell = inshell || dist < shell;
+                    stored = stored || dist < (a == 0 ? ends : shell);
                 }
-                if (band && !inshell) p->sponge_deferred = true;
-                if (inshell) p->src_in_shell = true;
+                if (gp.w[c] != 0.f && band && !inshell) p->sponge_deferred = true;
+                if (stored) p->src_in_shell = true;
             }
     }
     return AWE_OK;
