@@ -108,7 +108,8 @@ typedef struct {
     int nsnap;         /* snapshots written by awe_forward */
     size_t snap_elems; /* floats per snapshot */
     size_t device_bytes; /* device memory held by the plan */
-    int step_kernel;     /* 0: register kernels; 1: TMA-staged 3D 8th-order kernel; 2: TMA-staged spherical kernel */
+    int step_kernel;     /* of the next run: 0 register kernels, 1 TMA-staged 3D kernel (orders 2 to 8, constant
+                          density), 2 TMA-staged spherical kernel */
 } awe_info;
 
 typedef struct awe_plan awe_plan;
@@ -124,7 +125,8 @@ awe_status awe_plan_create(const awe_desc *desc, int device, awe_plan **out);
 awe_status awe_plan_destroy(awe_plan *plan);
 awe_status awe_plan_info(const awe_plan *plan, awe_info *info);
 
-/* vel, den, rfl: host [n3][n2][n1] unpadded; den and rfl may be NULL. */
+/* vel, den, rfl: host [n3][n2][n1] unpadded; den (NULL: constant density, also
+ * after a model that had one) and rfl may be NULL. */
 awe_status awe_set_model(awe_plan *plan, const float *vel, const float *den, const float *rfl);
 
 /* Source and receiver coordinates, host, ndim floats per point in the

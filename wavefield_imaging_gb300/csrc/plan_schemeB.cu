@@ -381,6 +381,9 @@ awe_status planB_model(awe_plan *p, const float *vel, const float *den) {
         CUDA_TRY(cudaMemcpyAsync(stage, den, raw * sizeof(float), cudaMemcpyHostToDevice, s));
         if (!p->den) AWE_TRY(dev_alloc(p, (void **)&p->den, cells * sizeof(float)));
         launch_model_pad(stage, p->den, m, false, s);
+    } else if (p->den) {  // back to constant density
+        dev_free(p, p->den);
+        p->den = nullptr;
     }
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(s));
@@ -600,7 +603,7 @@ awe_status stepB_full(awe_plan *p, const StepBParams &sp0, const float *prv, con
         sp.ext_row = ext_row;
     }
     prof_begin(p, s);
-    if (p->use_tma && (!p->den || p->tma_grad) && cur_map && prv_map) {
+    if (p->use_tma && !p->den && cur_map && prv_map) {  // (no density term there)
         cudaError_t e = launch_stepB3_tma_with(exact, *cur_map, *prv_map, p->tmaps[4], nxt, sp, p->tma_shape,
                                                p->sched_counter, p->sched_base, p->d_err, s, lap_out);
         p->sched_base += (unsigned long long)p->tma_shape.items + p->tma_shape.grid;

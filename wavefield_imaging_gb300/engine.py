@@ -162,6 +162,9 @@ def make_desc(ndim, n, d, o, nt, dt, coords=CART, scheme=SCHEME_CPU, nb=-1, fdor
     return q
 
 
+_STEP_KERNELS = {1: "tma3d", 2: "tma_sph"}
+
+
 class Plan:
     """One modelling set-up on one GPU: padded grid, model, geometry."""
 
@@ -169,14 +172,13 @@ class Plan:
         self._h = C.c_void_p()
         _check(lib().awe_plan_create(C.byref(desc), device, C.byref(self._h)))
         self.desc = desc
-        info = Info()
-        _check(lib().awe_plan_info(self._h, C.byref(info)))
+        info = self._info()
         self.npad = tuple(info.npad)
         self.nbpad = info.nbpad
         self.nsmp = info.nsmp
         self.nsnap = info.nsnap
         self.snap_elems = info.snap_elems
-        self.step_kernel = {1: "tma3d", 2: "tma_sph"}.get(info.step_kernel, "simple")
+        self.step_kernel = _STEP_KERNELS.get(info.step_kernel, "simple")
         self._cb = None
         self.ns = self.nr = 0
 
@@ -184,16 +186,20 @@ class Plan:
     def handle(self):
         return self._h
 
-    def device_bytes(self) -> int:
+    def _info(self) -> Info:
         info = Info()
         _check(lib().awe_plan_info(self._h, C.byref(info)))
-        return info.device_bytes
+        return info
+
+    def device_bytes(self) -> int:
+        return self._info().device_bytes
 
     def set_model(self, vel, den=None, rfl=None):
         vel = np.ascontiguousarray(vel, np.float32)
         den = None if den is None else np.ascontiguousarray(den, np.float32)
         rfl = None if rfl is None else np.ascontiguousarray(rfl, np.float32)
         _check(lib().awe_set_model(self._h, _fp(vel), _fp(den), _fp(rfl)))
+        self.step_kernel = _STEP_KERNELS.get(self._info().step_kernel, "simple")  # (a density changes it)
 
     def set_geometry(self, sou, rec):
         nd = self.desc.ndim
