@@ -111,7 +111,12 @@ __global__ void __launch_bounds__(256) k_stepA_sph_march(const float *__restrict
     const Grid g = p.g;
     if (i1 >= g.n1 || i2 >= g.n2) return;
     const long long s2 = g.n1, s3 = (long long)g.n1 * g.n2;
-    const int p0 = blockIdx.z * kSphChunk, p1 = min(p0 + kSphChunk, g.n3);
+    // blockIdx.z enumerates (shot, phi chunk); shots' fields lie back to back
+    const int nchunk = (g.n3 + kSphChunk - 1) / kSphChunk, shot = blockIdx.z / nchunk;
+    cur += shot * p.shot_cells;
+    prv += shot * p.shot_cells;
+    nxt += shot * p.shot_cells;
+    const int p0 = (blockIdx.z % nchunk) * kSphChunk, p1 = min(p0 + kSphChunk, g.n3);
     const bool in12 = i1 >= 4 && i1 < g.n1 - 4 && i2 >= 4 && i2 < g.n2 - 4;
     const long long t = (long long)i2 * g.n1 + i1;
     const float A2 = __ldg(p.tr0 + i1), Cr = __ldg(p.tr1 + i1), B = __ldg(p.tt0 + t), D = __ldg(p.tt1 + t);
@@ -156,9 +161,7 @@ __global__ void __launch_bounds__(256) k_stepA_sph_march2(const float *__restric
     const Grid g = p.g;
     if (i1 >= g.n1 || i2 >= g.n2) return;
     const long long s2 = g.n1, s3 = (long long)g.n1 * g.n2;
-    // blockIdx.z enumerates (shot, phi chunk); shots' fields lie back to back
-    const int nchunk = (g.n3 + kSphChunk - 1) / kSphChunk;
-    const int shot = blockIdx.z / nchunk;
+    const int nchunk = (g.n3 + kSphChunk - 1) / kSphChunk, shot = blockIdx.z / nchunk;
     cur += shot * p.shot_cells;
     prv += shot * p.shot_cells;
     nxt += shot * p.shot_cells;
@@ -218,9 +221,9 @@ __global__ void __launch_bounds__(256) k_stepA_sph_march2(const float *__restric
 
 static void step_fast(const float *cur, const float *prv, float *nxt, const float *vel, const StepAParams &p,
                       cudaStream_t s) {
-    const int nchunk = (p.g.n3 + kSphChunk - 1) / kSphChunk;
+    const int nchunk = (p.g.n3 + kSphChunk - 1) / kSphChunk * (p.nshot > 0 ? p.nshot : 1);
     if (p.g.n1 % 2 == 0) {
-        dim3 block(32, 8, 1), grid((p.g.n1 / 2 + 31) / 32, (p.g.n2 + 7) / 8, nchunk * (p.nshot > 0 ? p.nshot : 1));
+        dim3 block(32, 8, 1), grid((p.g.n1 / 2 + 31) / 32, (p.g.n2 + 7) / 8, nchunk);
         k_stepA_sph_march2<<<grid, block, 0, s>>>(cur, prv, nxt, vel, p);
     } else {
         dim3 block(64, 4, 1), grid((p.g.n1 + 63) / 64, (p.g.n2 + 3) / 4, nchunk);
