@@ -190,7 +190,16 @@ __global__ void __launch_bounds__(BATCH ? kTb2BatchThreads : kTb2Threads, BATCH 
     // the thread's cells are within `need` of the tile: computed while the later
     // steps of the launch still need them
     int need = max(max(max(tz0 - (z0 + 3), z0 - (tz1 - 1)), max(tx0 - (x0 + CX - 1), x0 - (tx1 - 1))), 0);
-    if (z0 + 3 < 0 || z0 >= n1 || x0 + CX - 1 < 0 || x0 >= n2) need = 1 << 30;
+    if (z0 + 3 < 0 || z0 >= n1 || x0 + CX - 1 < 0 || x0 >= n2) {
+        need = 1 << 30;
+        // I vel2 nu outside the grid in the second buffer too: no step stores it there, and the cells within NOP
+        // of an edge, whose nu the sources' term of the gradient takes, read it
+        if constexpr (ADJ) {
+#pragma unroll
+            for (int c = 0; c < CX; c++)
+                *reinterpret_cast<float4 *>(S1 + own + c * rz) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
     // v with its cell's entries of step j added, in (point, corner) order
     auto with_entries = [&](float v, const int4 &q, int j) {
         const float f = __int_as_float(q.w), *dd = ent_d + j * p.max_ent;
