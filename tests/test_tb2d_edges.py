@@ -44,3 +44,24 @@ def test_gradient_of_sources_at_the_edge(n, nb, order, dabc, monkeypatch):
     for a, b in zip(out[0][:-1], out[1][:-1]):
         assert np.isfinite(b).all() and np.abs(b).max() > 0
         np.testing.assert_array_equal(a, b)
+
+
+def test_batch_gradient_of_sources_at_the_edge():
+    import wavefield_imaging_gb300 as awe
+
+    rng = np.random.default_rng(3)
+    nz, nb, nt, windows, shots, obs = 72, 4, 50, [(0, 47), (20, 61)], [], []
+    for x0, nx in windows:
+        sou = np.array([(x + x0 * D, z) for x, z in _points((nz, nx), nb)], np.float32)
+        rec = np.stack([(x0 + rng.uniform(0, nx - 1, 20)) * D, rng.uniform(0, nz - 1, 20) * D], 1).astype(np.float32)
+        shots.append((x0, nx, sou, rec))
+        obs.append(rng.standard_normal((nt, 20)).astype(np.float32))
+    desc = awe.make_desc(2, (nz, 81), (D, D), (0.0, 0.0), nt, 0.005, nb=nb, fdorder=8, expl=1, precision=awe.FAST)
+    with awe.Batch(desc, shots) as b:
+        b.set_model((150 + 30 * rng.random((81, nz))).astype(np.float32))
+        assert b.info.launches_per_forward < nt
+        g0, _ = b.gradient(ricker(nt, 0.005), obs, ckpt_every=11, ckpt_format=awe.CKPT_FP32)
+        b.select(0)
+        g1, _ = b.gradient(ricker(nt, 0.005), obs, ckpt_every=11, ckpt_format=awe.CKPT_FP32)
+    assert np.isfinite(g1).all() and np.abs(g1).max() > 0
+    np.testing.assert_array_equal(g0, g1)

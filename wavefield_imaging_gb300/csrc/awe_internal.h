@@ -115,7 +115,7 @@ struct Tb2Params {
     float *slots;
     long long slot_stride;
     int slot_level;
-    const float *w1, *w2;            // sponge factors (null: no sponge)
+    const float *w1, *w2;            // sponge factors (null: no sponge; a batch: never null)
     int ilo1, ihi1, ilo2, ihi2;      // every factor in the range is 1
     // per tile: source cells of its region (z, x, first and last entry) with
     // their entries (source * 8 + corner, weight bits), and the receivers of its

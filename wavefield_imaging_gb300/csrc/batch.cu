@@ -263,14 +263,14 @@ static void tb2_steps(awe_batch *b, bool adj, const float *prv, const float *cur
     q.cur = cur, q.prv = prv, q.vel = b->vel, q.ocur = ocur, q.oprv = oprv;
     q.slots = slots;
     q.slot_stride = b->cells;
-    if (b->d.dabc) q.w1 = b->wz, q.w2 = b->wx;
+    q.w1 = b->wz, q.w2 = b->wx;  // (all 1 without a sponge)
     undamped_range(b->h_wz, q.ilo1, q.ihi1);
     q.ilo2 = q.ilo1;  // (a window's axis-2 factors mirror the same profile: its high end is n2 - ilo2)
     tb2_set_lists(q, l.buf, l.off, l.most, true, receivers);
     q.wav = adj ? b->res : b->wav;
     q.ncs = 1;
     q.jdata = b->d.jdata;
-    q.dat = receivers ? b->dat : nullptr;
+    q.dat = b->dat;  // (read with q.rec_start only)
     q.tiles = l.tiles;
     launch_tb2_batch(b->nop, adj ? 2 : slots ? 3 : 0, q, sh, b->tb2_tiles, tb2_smem(sh, l.most), s);
 }

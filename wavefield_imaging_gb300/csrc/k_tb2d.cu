@@ -60,8 +60,7 @@ __global__ void __launch_bounds__(BATCH ? kTb2BatchThreads : kTb2Threads, BATCH 
         tz0 = t.z0, tx0 = t.x0;
         n2 = t.n2, nr = t.nr, ihi2 = n2 - p.ilo2;
         off = t.off;
-        if (w2) w2 += t.wx_off;
-        if (dat) dat += t.dat_off;
+        w2 += t.wx_off, dat += t.dat_off;
         if (ADJ) ncs = nr, wav += t.dat_off;
         rec0 = t.rec0, nrec = p.rec_start ? t.nrec : 0, cell0 = t.cell0, ncell = t.ncell, ent0 = t.ent0, nent = t.nent;
     } else {
