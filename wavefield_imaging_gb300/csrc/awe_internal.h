@@ -377,9 +377,10 @@ void launch_ckpt_load_bfp(const short *q, const float *scale, long long n, float
 // image on the model grid: the padded grid's model window of G
 void launch_add_f64(double *dst, const double *src, long long n, cudaStream_t s);
 void launch_image_cut(const float2 *G, const Grid &g, int nb, const int *n, int nd, double *out, cudaStream_t s);
-// vel2: v^2 dt^2 per padded cell, or the velocity itself (raw_v: c = dt^2 v^2)
+// vel2: v^2 dt^2 per padded cell, or the velocity itself (raw_v: c = dt^2 v^2);
+// zero1: samples of every line that a free surface sets to 0
 void launch_grad_fold(const float2 *G, const float *vel2, float dt, const Grid &g, int nb, const int *n, int nd,
-                      double *out, cudaStream_t s, bool raw_v = false);
+                      double *out, cudaStream_t s, bool raw_v = false, int zero1 = 0);
 
 // ---- batched 2D forward (k_batch2d.cu) ----
 struct BatchShot {

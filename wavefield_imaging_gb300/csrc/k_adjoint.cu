@@ -516,22 +516,25 @@ __device__ __forceinline__ int edge_axes(int j1, int j2, int j3, int m1, int m2,
 }
 
 // Sum of the accumulators of the padded cells that replicate a model cell.
-// They all hold the cell's vel2 (the padding repeats it; a free surface zeroes
-// them together), so its factor is applied once, to the sum.  vel2 holds
-// c = v^2 dt^2 per padded cell, or (cscale > 0) the velocity v with c = cscale v^2.
+// They hold the cell's vel2 (the padding repeats it), so its factor is applied
+// once, to the sum; those of the first zero1 samples of a line, which a free
+// surface sets to 0, add nothing and are left out (they are all the replicas of
+// the first cell of a line, or some of the only one's).  vel2 holds c = v^2 dt^2
+// per padded cell, or (cscale > 0) the velocity v with c = cscale v^2.
 struct FoldParams {
     const float2 *G;
     const float *vel2;
     double inv_dt2, cscale;
     Grid g;
-    int nb, m1, m2, m3, nd;
+    int nb, m1, m2, m3, nd, zero1;
     int nbig, nends;  // blocks of the first two roles
     double *out;
 };
 
-__device__ __forceinline__ void fold_store(const FoldParams &p, int j1, int j2, int j3, double acc) {
+// i1: the last replica along axis 1
+__device__ __forceinline__ void fold_store(const FoldParams &p, int i1, int j1, int j2, int j3, double acc) {
     const int i3 = p.nd == 3 ? j3 + p.nb : 0;
-    const double v = p.vel2[((long long)i3 * p.g.n2 + j2 + p.nb) * p.g.p1 + j1 + p.nb];
+    const double v = p.vel2[((long long)i3 * p.g.n2 + j2 + p.nb) * p.g.p1 + i1];
     const double c = p.cscale > 0 ? p.cscale * v * v : v;
     p.out[((long long)j3 * p.m2 + j2) * p.m1 + j1] = acc * (-c * c * p.inv_dt2);
 }
@@ -575,7 +578,8 @@ __global__ void __launch_bounds__(256) k_grad_fold(const FoldParams p) {
         fold_range(j1, m1, p.g.n1, p.nb, a1, b1);
         fold_range(j2, m2, p.g.n2, p.nb, a2, b2);
         if (nd == 3) fold_range(j3, m3, p.g.n3, p.nb, a3, b3);
-        const int w1 = b1 - a1 + 1, w2 = b2 - a2 + 1, vol = w1 * w2 * (b3 - a3 + 1);
+        a1 = max(a1, p.zero1);
+        const int w1 = max(b1 - a1 + 1, 0), w2 = b2 - a2 + 1, vol = w1 * w2 * (b3 - a3 + 1);
         double acc = 0;
         for (int k = tid; k < vol; k += 256) {
             const int i1 = a1 + k % w1, i2 = a2 + (k / w1) % w2, i3 = a3 + k / (w1 * w2);
@@ -587,7 +591,7 @@ __global__ void __launch_bounds__(256) k_grad_fold(const FoldParams p) {
         __syncthreads();
         if (tid == 0) {
             for (int w = 1; w < 8; w++) acc += part[w];
-            fold_store(p, j1, j2, j3, acc);
+            fold_store(p, b1, j1, j2, j3, acc);
         }
         return;
     }
@@ -607,11 +611,11 @@ __global__ void __launch_bounds__(256) k_grad_fold(const FoldParams p) {
             if (nd == 3) fold_range(j3, m3, p.g.n3, p.nb, a3, b3);
             for (int i3 = a3; i3 <= b3; i3++)
                 for (int i2 = a2; i2 <= b2; i2++)
-                    for (int i1 = a1 + (tid & 7); i1 <= b1; i1 += 8)
+                    for (int i1 = max(a1, p.zero1) + (tid & 7); i1 <= b1; i1 += 8)
                         acc += gsum_value(p.G[((long long)i3 * p.g.n2 + i2) * p.g.p1 + i1]);
         }
         for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (mine && (tid & 7) == 0) fold_store(p, j1, j2, j3, acc);
+        if (mine && (tid & 7) == 0) fold_store(p, b1, j1, j2, j3, acc);
         return;
     }
     const long long t = (b - p.nends) * 256 + tid;
@@ -625,7 +629,7 @@ __global__ void __launch_bounds__(256) k_grad_fold(const FoldParams p) {
 #pragma unroll 4
         for (int i2 = a2; i2 <= b2; i2++)
             acc += gsum_value(p.G[((long long)i3 * p.g.n2 + i2) * p.g.p1 + j1 + p.nb]);
-    fold_store(p, j1, j2, j3, acc);
+    fold_store(p, j1 + p.nb, j1, j2, j3, acc);
 }
 
 __global__ void k_image_cut(const float2 *__restrict__ G, Grid g, int nb, int m1, int m2, int m3, int nd,
@@ -652,8 +656,9 @@ void launch_image_cut(const float2 *G, const Grid &g, int nb, const int *n, int 
 }
 
 void launch_grad_fold(const float2 *G, const float *vel2, float dt, const Grid &g, int nb, const int *n, int nd,
-                      double *out, cudaStream_t s, bool raw_v) {
+                      double *out, cudaStream_t s, bool raw_v, int zero1) {
     FoldParams p{};
+    p.zero1 = zero1;
     p.G = G;
     p.vel2 = vel2;
     p.inv_dt2 = 1.0 / ((double)dt * (double)dt);

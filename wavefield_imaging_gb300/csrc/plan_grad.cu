@@ -725,7 +725,7 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
         }
     }
     if (xcorr) launch_image_cut(st->G, g, p->nbd, d.n, d.ndim, d_grad, s);
-    else launch_grad_fold(st->G, p->vel, d.dt, g, p->nbd, d.n, d.ndim, d_grad, s);
+    else launch_grad_fold(st->G, p->vel, d.dt, g, p->nbd, d.n, d.ndim, d_grad, s, false, d.fsrf ? p->nbd + 1 : 0);
     launches++;
     return AWE_OK;
     };  // seq
