@@ -1,0 +1,85 @@
+"""Memory that a plan can do without (the levels, slots and lists of several
+steps a launch, the line-end copies and padded lines of a 3D level) is given back
+when something else needs it: whatever fits with the one-step kernels fits, with
+the same results.  Every limit in a process of its own (it is read once)."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+_CODE = r'''
+import sys; sys.path.insert(0, "."); sys.path.insert(0, "tests")
+import hashlib
+import numpy as np, wavefield_imaging_gb300 as awe
+from helpers import ricker
+kind = sys.argv[1]
+n = dict(grad2d=(300, 290), frames2d=(300, 290), fwd3d=(70, 60, 52))[kind]
+nt, d = 60, (5.0,) * len(n)
+rng = np.random.default_rng(1)
+vel = (150 + 30 * rng.random(n[::-1])).astype(np.float32)
+axes = (1, 0) if len(n) == 2 else (1, 2, 0)
+sou = np.array([[0.5 * (n[a] - 1) * 5.0 for a in axes]], np.float32)
+rec = np.stack([rng.uniform(0, (n[a] - 1) * 5.0, 40) for a in axes], 1).astype(np.float32)
+desc = awe.make_desc(len(n), n, d, (0.0,) * len(n), nt, 0.005, nb=10, fdorder=4, dabc=1, expl=1,
+                     jsnap=10 if kind == "frames2d" else 0, precision=awe.EXACT if kind == "fwd3d" else awe.FAST)
+res = []
+def h(*a):
+    return hashlib.sha1(b"".join(np.ascontiguousarray(x).tobytes() for x in a)).hexdigest()[:12]
+def call(f):
+    try:
+        res.append(f())
+    except awe.AweError as e:
+        res.append("E%d" % e.status)
+wav, obs = ricker(nt, 0.005), rng.standard_normal((nt, 40)).astype(np.float32)
+held = launches = 0
+try:
+    p = awe.Plan(desc)
+    p.set_model(vel); p.set_geometry(sou, rec)
+    for _ in range(3):  # launched, captured, replayed
+        if kind != "fwd3d":
+            call(lambda: h(p.gradient(wav, obs, ckpt_every=5)[0]))
+            launches = p.last_launch_count()
+        if kind == "frames2d":
+            call(lambda: h(*p.forward(wav, snapshots=True)))
+        if kind == "fwd3d":
+            call(lambda: h(p.forward(wav)))
+            launches = p.last_launch_count()
+    held = p.device_bytes()
+except awe.AweError as e:
+    res.append("C%d" % e.status)
+print(held, launches, " ".join(res))
+'''
+
+
+def _run(kind, limit=0, kernel=""):
+    env = dict(os.environ, AWE_DEVICE_BYTES_LIMIT=str(limit) if limit else "", AWE_STEP_KERNEL=kernel)
+    r = subprocess.run([sys.executable, "-c", _CODE, kind], cwd=ROOT, env=env, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    held, launches, *res = r.stdout.strip().splitlines()[-1].split()
+    return int(held), int(launches), res
+
+
+@pytest.mark.parametrize("kind", ["grad2d", "frames2d", "fwd3d"])
+def test_what_fits_one_step_a_launch_fits(kind):
+    need, many, want = _run(kind, kernel="simple")
+    level = {2: 320 * 310, 3: 90 * 80 * 72}[3 if kind == "fwd3d" else 2] * 4
+    if kind == "frames2d":
+        need += 6 * 300 * 290 * 4  # the frames' buffer of the call
+    free, few, res = _run(kind)
+    assert res == want and few < many and free > need - 2 * level
+    top = max(free, need)
+    for limit in (need, need + level // 2, need + 2 * level, need + 4 * level, (need + top) // 2, top + 8 * level):
+        held, _, res = _run(kind, limit)
+        assert res == want and held <= limit
+
+
+def test_too_little_memory_is_an_error_every_time():
+    need, _, want = _run("grad2d", kernel="simple")
+    _, _, res = _run("grad2d", need - (1 << 19))
+    assert set(res) == {"E3"} or res[0].startswith("C3")  # AWE_ERR_NOMEM
+    assert len(want) == 3

@@ -72,23 +72,54 @@ static size_t device_bytes_limit() {
     return lim;
 }
 
-awe_status dev_alloc(awe_plan *p, void **ptr, size_t bytes) {
+// memory the plan can do without; null and AWE_ERR_NOMEM where there is none left
+awe_status dev_alloc_extra(awe_plan *p, void **ptr, size_t bytes) {
+    *ptr = nullptr;
     if (bytes == 0) bytes = 16;
     const size_t lim = device_bytes_limit();
     if (lim && p->device_bytes + bytes > lim) {
-        *ptr = nullptr;
         set_error("device memory limit: %zu bytes held + %zu requested > AWE_DEVICE_BYTES_LIMIT %zu",
                   p->device_bytes, bytes, lim);
         return AWE_ERR_NOMEM;
     }
     cudaError_t e = cudaMalloc(ptr, bytes);
     if (e != cudaSuccess) {
+        cudaGetLastError();
+        *ptr = nullptr;
         set_error("cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
         return AWE_ERR_NOMEM;
     }
     p->allocs.push_back({*ptr, bytes});
     p->device_bytes += bytes;
     return AWE_OK;
+}
+
+// Gives back one of the things the plan can do without, the largest first: a
+// gradient kept for the next call in its form for several steps a launch (the
+// next call allocates what then fits), the two levels of k_tb2d.cu with their
+// lists, the line-end copies of k_bnd3.  Captured loops that read them go too.
+static bool release_extra(awe_plan *p) {
+    if (plan_gradient_release(p)) return true;
+    std::vector<void *> give;
+    if (p->tb2) {
+        give = {p->tb2_u, p->tb2_fwd.buf, p->tb2_adj.buf};
+        p->tb2 = false;
+        p->tb2_u = nullptr;
+        p->tb2_fwd = p->tb2_adj = Tb2Lists{};
+    } else if (p->ends[0]) {
+        give = {p->ends[0], p->ends[1]};
+        p->ends[0] = p->ends[1] = nullptr;
+    }
+    if (give.empty()) return false;
+    plan_graph_drop(p);
+    for (void *q : give) dev_free(p, q);
+    return true;
+}
+
+awe_status dev_alloc(awe_plan *p, void **ptr, size_t bytes) {
+    awe_status st = dev_alloc_extra(p, ptr, bytes);
+    while (st != AWE_OK && release_extra(p)) st = dev_alloc_extra(p, ptr, bytes);
+    return st;
 }
 
 void dev_free(awe_plan *p, void *ptr) {

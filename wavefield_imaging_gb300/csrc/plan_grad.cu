@@ -59,8 +59,9 @@ struct GradState {
     size_t nd_cap = 0;      // trace samples dat and r hold
     // 2D, several steps a launch (k_tb2d.cu): slots hold T levels of L(V_k) and
     // T of nu_k, xy2 two more levels for the adjoint sweep
-    bool tb2 = false;
+    bool tb2 = false, tb2_tried = false;  // tried: no memory for it
     float *xy2 = nullptr;
+    bool busy = false;  // a call uses it
     // misfit rows (pinned, written by the stream) and the captured gradient
     double *h_rows = nullptr;
     size_t h_rows_n = 0;
@@ -96,12 +97,18 @@ void plan_gradient_free(awe_plan *p) {
     p->grad = nullptr;
 }
 
-static awe_status grad_alloc(awe_plan *p, int T, int fmt) {
-    const size_t nd = (size_t)p->nsmp * (p->nr > 0 ? p->nr : 1);
-    if (p->grad && p->grad->T == T && p->grad->fmt == fmt && p->grad->nd_cap >= nd) return AWE_OK;
+bool plan_gradient_release(awe_plan *p) {
+    if (!p->grad || !p->grad->tb2 || p->grad->busy) return false;
     plan_gradient_free(p);
-    GradState *st = new GradState();
-    p->grad = st;
+    return true;
+}
+
+// several steps a launch apply to the gradient of this plan and its points
+static bool want_tb2(const awe_plan *p) {
+    return p->tb2 && p->tb2_fwd.ok && p->g.cells() <= kFusedCells;
+}
+
+static awe_status grad_buffers(awe_plan *p, GradState *st, int T, int fmt, size_t nd) {
     const awe_desc &d = p->d;
     const size_t cells = (size_t)p->g.cells();
     st->T = T;
@@ -109,18 +116,6 @@ static awe_status grad_alloc(awe_plan *p, int T, int fmt) {
     st->nseg = (d.nt + T - 1) / T;
     const size_t es = fmt == AWE_CKPT_FP32 ? 4 : 2;
     st->tma = p->tma_grad && d.precision == AWE_FAST;
-    // 2D: two slots a step and two more levels, where memory allows them
-    st->tb2 = p->tb2 && (long long)cells <= kFusedCells;
-    if (st->tb2) {
-        st->tb2 = dev_alloc(p, (void **)&st->slots, (size_t)std::max(2 * T, T + 1) * cells * sizeof(float)) == AWE_OK;
-        if (st->tb2 && dev_alloc(p, (void **)&st->xy2, 2 * cells * sizeof(float)) != AWE_OK) {
-            dev_free(p, st->slots);
-            st->slots = nullptr;
-            st->tb2 = false;
-        }
-        cudaGetLastError();
-    }
-    if (!st->tb2) AWE_TRY(dev_alloc(p, (void **)&st->slots, (size_t)(st->tma ? T : T + 1) * cells * sizeof(float)));
     AWE_TRY(dev_alloc(p, &st->ckpt, (size_t)2 * st->nseg * cells * es));
     st->nblk = fmt == AWE_CKPT_BFP16 ? ((long long)cells + kBfpBlock - 1) / kBfpBlock : 1;
     AWE_TRY(dev_alloc(p, (void **)&st->scales, (size_t)2 * st->nseg * st->nblk * sizeof(float)));
@@ -129,13 +124,41 @@ static awe_status grad_alloc(awe_plan *p, int T, int fmt) {
     AWE_TRY(dev_alloc(p, (void **)&st->Y, cells * sizeof(float)));
     if (d.ndim == 3 && d.dabc && d.scheme == AWE_SCHEME_CPU) AWE_TRY(dev_alloc(p, (void **)&st->kap, cells * sizeof(float)));
     AWE_TRY(dev_alloc(p, (void **)&st->G, cells * sizeof(float2)));
-    st->nd_cap = nd;
     AWE_TRY(dev_alloc(p, (void **)&st->dat, nd * sizeof(float)));
     AWE_TRY(dev_alloc(p, (void **)&st->r, nd * sizeof(float)));
     AWE_TRY(dev_alloc(p, (void **)&st->row_sum, (size_t)p->nsmp * sizeof(double)));
     if (st->tma) {
         AWE_TRY(dev_alloc(p, (void **)&st->vr, 3 * cells * sizeof(float)));
         AWE_TRY(dev_alloc(p, (void **)&st->gbuf, cells * sizeof(float)));
+    }
+    // the point lists of the one-step kernels (build_cell_lists)
+    const bool lists = !st->tma && !st->kap && p->g.cells() <= kFusedCells && d.scheme == AWE_SCHEME_CPU;
+    if (lists) {
+        const int nc = d.ndim == 3 ? 8 : 4;
+        st->sc_cap = std::max<size_t>(p->h_src.size() * nc, 1);
+        st->rc_cap = std::max<size_t>(p->h_rec.size() * nc, 1);
+        for (int **q : {&st->sc_start, &st->rc_start}) AWE_TRY(dev_alloc(p, (void **)q, (cells + 1) * sizeof(int)));
+        AWE_TRY(dev_alloc(p, (void **)&st->sc_ent, st->sc_cap * sizeof(int2)));
+        AWE_TRY(dev_alloc(p, (void **)&st->rc_ent, st->rc_cap * sizeof(int2)));
+    }
+    // the slots last: 2D, two a step and two more levels if memory is left for them
+    if (want_tb2(p)) {
+        st->tb2 = dev_alloc_extra(p, (void **)&st->xy2, 2 * cells * sizeof(float)) == AWE_OK &&
+                  dev_alloc_extra(p, (void **)&st->slots, (size_t)std::max(2 * T, T + 1) * cells * sizeof(float)) == AWE_OK;
+        st->tb2_tried = true;
+        if (!st->tb2) {
+            dev_free(p, st->xy2);
+            st->xy2 = nullptr;
+        } else {  // not needed then (what is free now holds them if that changes)
+            dev_free(p, st->rc_start);
+            dev_free(p, st->rc_ent);
+            st->rc_start = nullptr;
+            st->rc_ent = nullptr;
+            st->rc_cap = 0;
+        }
+    }
+    if (!st->tb2) AWE_TRY(dev_alloc(p, (void **)&st->slots, (size_t)(st->tma ? T : T + 1) * cells * sizeof(float)));
+    if (st->tma) {
         int h1, h2, t1, t2;
         stepB3_tma_boxes(&h1, &h2, &t1, &t2);
         const Grid &g = p->g;
@@ -164,8 +187,32 @@ static awe_status grad_alloc(awe_plan *p, int T, int fmt) {
             return AWE_ERR_CUDA;
         }
     }
+    st->nd_cap = nd;
     return AWE_OK;
 }
+
+static awe_status grad_alloc(awe_plan *p, int T, int fmt) {
+    const size_t nd = (size_t)p->nsmp * (p->nr > 0 ? p->nr : 1);
+    GradState *st = p->grad;
+    if (st && st->T == T && st->fmt == fmt && st->nd_cap >= nd && (st->tb2 || st->tb2_tried || !want_tb2(p))) {
+        st->busy = true;
+        return AWE_OK;
+    }
+    plan_gradient_free(p);
+    st = p->grad = new GradState();
+    st->busy = true;
+    const awe_status r = grad_buffers(p, st, T, fmt, nd);
+    if (r != AWE_OK) plan_gradient_free(p);  // (a later call starts anew)
+    return r;
+}
+
+// the end of a call that uses the gradient's buffers
+struct GradUse {
+    awe_plan *p;
+    ~GradUse() {
+        if (p->grad) p->grad->busy = false;
+    }
+};
 
 static int float_bits(float f) {
     int i;
@@ -196,6 +243,7 @@ static awe_status build_cell_lists(awe_plan *p, const std::vector<GeoPoint> &pts
     if (*cap < e.size()) {
         if (*ent) dev_free(p, *ent);
         *ent = nullptr;
+        *cap = 0;
         AWE_TRY(dev_alloc(p, (void **)ent, e.size() * sizeof(int2)));
         *cap = e.size();
     }
@@ -526,6 +574,7 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
         set_error("awe_gradient: unknown checkpoint format %d", o.ckpt_format);
         return AWE_ERR_INVALID;
     }
+    const GradUse use{p};
     AWE_TRY(grad_alloc(p, T, o.ckpt_format));
     GradState *st = p->grad;
     const long long cells = g.cells();
@@ -570,6 +619,7 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
             AWE_TRY(build_cell_lists(p, p->h_src, nc, &st->sc_start, &st->sc_ent, &st->sc_cap, s));
             st->lists_ok = true;
         }
+        // (the lists above may have taken the memory of the two levels)
         tb2 = st->tb2 && p->tb2_fwd.ok && p->tb2_adj.ok && !p->profile;
         if (!tb2 && !st->rc_ok) {
             AWE_TRY(build_cell_lists(p, p->h_rec, nc, &st->rc_start, &st->rc_ent, &st->rc_cap, s));
@@ -581,6 +631,14 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
         ap.sc_ent = st->sc_ent;
         ap.ncs = ncs;
         ap.one_wavelet = ncs == 1;
+    }
+
+    if (!fuse_pts && p->ns > 0 && !xcorr && p->inj.n == 0) {  // no memory for them when the points were set
+        AWE_TRY(set_inj_cells(p));
+        if (p->inj.n == 0) {
+            set_error("awe_gradient: no device memory for the sources' cells");
+            return AWE_ERR_NOMEM;
+        }
     }
 
     // the whole gradient as stream work on `s`

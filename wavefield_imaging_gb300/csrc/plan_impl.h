@@ -145,6 +145,8 @@ struct awe_plan {
 
 namespace awe {
 awe_status dev_alloc(awe_plan *p, void **ptr, size_t bytes);
+// memory the plan can do without (dev_alloc takes it back when it needs it)
+awe_status dev_alloc_extra(awe_plan *p, void **ptr, size_t bytes);
 // forget the captured time loop (the model, geometry or buffers it baked in changed)
 void plan_graph_drop(awe_plan *p);
 void dev_free(awe_plan *p, void *ptr);
@@ -209,6 +211,8 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
 void plan_gradient_free(awe_plan *p);
 // drops the gradient's captured graph and its per-cell point lists
 void plan_gradient_graph_drop(awe_plan *p);
+// frees a gradient state that holds more than one step a launch needs and is not in use
+bool plan_gradient_release(awe_plan *p);
 
 awe_status planA_init(awe_plan *p);
 // the per-corner injection scales, when the model or the points changed since

@@ -187,7 +187,7 @@ awe_status set_tb2_lists(awe_plan *p, Tb2Lists &t, const std::vector<GeoPoint> &
         dev_free(p, t.buf);
         t.buf = nullptr;
         t.cap = 0;
-        AWE_TRY(dev_alloc(p, (void **)&t.buf, total * sizeof(int)));
+        if (dev_alloc_extra(p, (void **)&t.buf, total * sizeof(int)) != AWE_OK) return AWE_OK;
         t.cap = total;
     }
     CUDA_TRY(cudaMemcpy(t.buf, h.buf.data(), total * sizeof(int), cudaMemcpyHostToDevice));
@@ -234,6 +234,28 @@ void tb2_launch(awe_plan *p, bool adj, const float *prv, const float *cur, float
     launch_tb2(p->nop, adj ? 2 : slots ? 3 : d.precision == AWE_EXACT ? 1 : 0, q, sh, tb2_smem(sh, t.most), s);
 }
 
+// the one-way ABC's coefficient tables: cells of table k
+static size_t abc_cells(const Grid &g, int k) {
+    return k < 2 ? (size_t)g.n2 * g.n3 : k < 4 ? (size_t)g.n1 * g.n3 : (size_t)g.n1 * g.n2;
+}
+
+// the two levels, the model and its tables: all of them or none
+static awe_status alloc_levels(awe_plan *p) {
+    const awe_desc &d = p->d;
+    std::vector<std::pair<float **, size_t>> want;
+    for (float **q : {&p->u[0], &p->u[1], &p->vel}) want.push_back({q, (size_t)p->g.cells()});
+    for (int k = 0; d.dabc && k < (d.ndim == 3 ? 6 : 4); k++) want.push_back({&p->abc[k], abc_cells(p->g, k)});
+    awe_status st = AWE_OK;
+    for (auto &w : want)
+        if (st == AWE_OK) st = dev_alloc(p, (void **)w.first, w.second * sizeof(float));
+    for (auto &w : want)
+        if (st != AWE_OK) {
+            dev_free(p, *w.first);
+            *w.first = nullptr;
+        }
+    return st;
+}
+
 awe_status planB_init(awe_plan *p) {
     awe_desc &d = p->d;
     if (d.fdorder == 0) d.fdorder = 4;  // MAWEFDcart2Dcpu.c:126
@@ -249,19 +271,24 @@ awe_status planB_init(awe_plan *p) {
     // compare both)
     const char *kern = std::getenv("AWE_STEP_KERNEL");
     const bool force_simple = kern && std::strcmp(kern, "simple") == 0;
+    // lines of a 3D level on 16-byte boundaries, so that the TMA step takes any
+    // n1; plain ones where memory does not hold them
+    const Grid plain = p->g;
     {
-        // lines of a 3D level on 16-byte boundaries, so that the TMA step takes any n1
-        const Grid pitched(p->g.n1, p->g.n2, p->g.n3, (p->g.n1 + 3) / 4 * 4);
+        const Grid pitched(plain.n1, plain.n2, plain.n3, (plain.n1 + 3) / 4 * 4);
         if (!force_simple && stepB3_tma_eligible(d.ndim, p->nop, false, pitched)) p->g = pitched;
     }
     for (int a = 0; a < d.ndim; a++) p->opad[a] = d.o[a] - nb * d.d[a];  // fdutil_init
     float dd[3] = {d.d[0], d.d[1], d.ndim == 3 ? d.d[2] : 1.f};
     fd_coefficients(p->nop, d.ndim, dd, d.optfd, p->k);
 
+    awe_status st = alloc_levels(p);
+    if (st != AWE_OK && p->g.p1 != plain.p1) {
+        p->g = plain;
+        st = alloc_levels(p);
+    }
+    if (st != AWE_OK) return st;
     const size_t cells = (size_t)p->g.cells();
-    AWE_TRY(dev_alloc(p, (void **)&p->u[0], cells * sizeof(float)));
-    AWE_TRY(dev_alloc(p, (void **)&p->u[1], cells * sizeof(float)));
-    AWE_TRY(dev_alloc(p, (void **)&p->vel, cells * sizeof(float)));
     AWE_TRY(dev_alloc(p, (void **)&p->corner_off, 8 * sizeof(long long)));
 
     if (d.dabc && !d.hybrid) {
@@ -309,15 +336,18 @@ awe_status planB_init(awe_plan *p) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
         p->tb2_shape = tb2_shape(p->g, p->nop, sms > 0 ? sms : 1);
         // (without room for two more levels: one step a launch)
-        p->tb2 = dev_alloc(p, (void **)&p->tb2_u, 2 * cells * sizeof(float)) == AWE_OK;
-        cudaGetLastError();
+        p->tb2 = dev_alloc_extra(p, (void **)&p->tb2_u, 2 * cells * sizeof(float)) == AWE_OK;
     }
     // line-end copies of the 3D boundary launch (made before any capture of
-    // the time loop; AWE_BND_ENDS=0: the launch reads the level itself)
+    // the time loop; AWE_BND_ENDS=0, or no memory: the launch reads the level itself)
     const char *eenv = std::getenv("AWE_BND_ENDS");
     if (d.ndim == 3 && d.dabc && !d.hybrid && bnd3_eligible(p->nop, p->g) && !(eenv && std::strcmp(eenv, "0") == 0))
         for (int k = 0; k < 2; k++)
-            AWE_TRY(dev_alloc(p, (void **)&p->ends[k], (size_t)p->g.n2 * p->g.n3 * 16 * sizeof(float)));
+            if (dev_alloc_extra(p, (void **)&p->ends[k], (size_t)p->g.n2 * p->g.n3 * 16 * sizeof(float)) != AWE_OK) {
+                dev_free(p, p->ends[0]);
+                p->ends[0] = nullptr;
+                break;
+            }
 
     p->nsmp = (d.nt - 1) / d.jdata + 1;
     p->nsnap = d.jsnap > 0 ? (d.nt - 1) / d.jsnap + 1 : 0;
@@ -368,14 +398,9 @@ awe_status planB_model(awe_plan *p, const float *vel, const float *den) {
     CUDA_TRY(cudaDeviceSynchronize());
     CUDA_TRY(cudaMemcpyAsync(stage, vel, raw * sizeof(float), cudaMemcpyHostToDevice, s));
     if (d.dabc) {
-        const size_t sz[6] = {(size_t)g.n2 * g.n3, (size_t)g.n2 * g.n3, (size_t)g.n1 * g.n3, (size_t)g.n1 * g.n3,
-                              (size_t)g.n1 * g.n2, (size_t)g.n1 * g.n2};
-        for (int k = 0; k < (d.ndim == 3 ? 6 : 4); k++)
-            if (!p->abc[k]) AWE_TRY(dev_alloc(p, (void **)&p->abc[k], sz[k] * sizeof(float)));
         float *const tabs[6] = {p->abc[0], p->abc[1], p->abc[2], p->abc[3], p->abc[4], p->abc[5]};
         launch_model_abc(stage, m, tabs, s);
     }
-    if (!p->vel) AWE_TRY(dev_alloc(p, (void **)&p->vel, cells * sizeof(float)));
     launch_model_pad(stage, p->vel, m, true, s);
     if (den) {
         CUDA_TRY(cudaMemcpyAsync(stage, den, raw * sizeof(float), cudaMemcpyHostToDevice, s));
@@ -424,7 +449,8 @@ awe_status set_inj_cells(awe_plan *p) {
         dev_free(p, p->inj_buf);
         p->inj_buf = nullptr;
         p->inj_cap = 0;
-        AWE_TRY(dev_alloc(p, &p->inj_buf, bytes));
+        // (without memory for them: one thread walks the sources)
+        if (dev_alloc(p, &p->inj_buf, bytes) != AWE_OK) return AWE_OK;
         p->inj_cap = bytes;
     }
     char *b = (char *)p->inj_buf;
@@ -714,6 +740,8 @@ awe_status planB_run_hooked(awe_plan *p, const float *d_wav, int ncs, float *d_d
         CUDA_TRY(cudaMemsetAsync(p->sched_counter, 0, sizeof(unsigned long long), s));
         p->sched_base = 0;
     }
+    if (p->nsnap > 0 && !d_wfl && p->snap_cb && !p->d_snap_tmp)
+        AWE_TRY(dev_alloc(p, (void **)&p->d_snap_tmp, p->snap_elems * sizeof(float)));
     // the boundary launches pass the line ends from step to step; the first
     // step reads those of the zero level
     struct EndsOff {
@@ -726,8 +754,6 @@ awe_status planB_run_hooked(awe_plan *p, const float *d_wav, int ncs, float *d_d
         p->ends_idx = 0;
         p->ends_run = true;
     }
-    if (p->nsnap > 0 && !d_wfl && p->snap_cb && !p->d_snap_tmp)
-        AWE_TRY(dev_alloc(p, (void **)&p->d_snap_tmp, p->snap_elems * sizeof(float)));
     p->snap_pending = -1;  // a frame left queued by a failed run is not delivered
 
     const StepBParams sp = stepB_params(p);
