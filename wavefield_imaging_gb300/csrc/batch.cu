@@ -33,7 +33,8 @@ struct awe_batch {
     int ntile_items = 0;
     long long cells = 0, ndat = 0;
     int nsmp = 0;
-    std::vector<void *> allocs;
+    std::vector<std::pair<void *, size_t>> allocs;
+    size_t held = 0;  // their bytes
     float *u[2] = {nullptr, nullptr}, *vel = nullptr, *wz = nullptr, *wx = nullptr, *wav = nullptr, *dat = nullptr;
     BatchShot *d_shots = nullptr;
     int4 *d_items = nullptr;
@@ -77,6 +78,7 @@ struct awe_batch {
         int most[3] = {};
     } tb2_fwd, tb2_adj;
     bool tb2_grad = false, tb2_tried = false;  // the gradient's slots hold both sweeps of a segment; asked for
+    bool grad_busy = false;                    // a call uses the gradient's buffers
     std::vector<GeoPoint> h_src;
 };
 
@@ -89,21 +91,82 @@ struct awe_batch {
         }                                                                                         \
     } while (0)
 
-static awe_status balloc(awe_batch *b, void **p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
-    if (e != cudaSuccess) {
-        set_error("cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
-        return AWE_ERR_NOMEM;
-    }
-    b->allocs.push_back(*p);
-    return AWE_OK;
-}
-
 static void drop_graph(awe_batch *b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     b->exec = nullptr;
     b->graph = nullptr;
+}
+
+// Optional cap on the device memory one batch may hold (AWE_BATCH_BYTES_LIMIT,
+// bytes, read at every allocation), as AWE_DEVICE_BYTES_LIMIT is for a plan.
+static size_t batch_bytes_limit() {
+    const char *e = std::getenv("AWE_BATCH_BYTES_LIMIT");
+    return e && *e ? (size_t)std::strtoull(e, nullptr, 10) : (size_t)0;
+}
+
+// memory the batch can do without; null and AWE_ERR_NOMEM where there is none left
+static awe_status balloc_extra(awe_batch *b, void **p, size_t bytes) {
+    *p = nullptr;
+    if (bytes == 0) bytes = 16;
+    const size_t lim = batch_bytes_limit();
+    if (lim && b->held + bytes > lim) {
+        set_error("device memory limit: %zu bytes held + %zu requested > AWE_BATCH_BYTES_LIMIT %zu", b->held, bytes,
+                  lim);
+        return AWE_ERR_NOMEM;
+    }
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+        set_error("cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
+        return AWE_ERR_NOMEM;
+    }
+    b->allocs.push_back({*p, bytes});
+    b->held += bytes;
+    return AWE_OK;
+}
+
+template <class T>
+static void bfree(awe_batch *b, T *&p) {
+    for (auto it = b->allocs.begin(); it != b->allocs.end(); ++it)
+        if (it->first == (void *)p) {
+            b->held -= it->second;
+            b->allocs.erase(it);
+            cudaFree(p);
+            break;
+        }
+    p = nullptr;
+}
+
+// Gives back what the batch can do without: the gradient's slots for several
+// steps a launch while no call uses them (the next one allocates what then
+// fits), then the levels, lists and tiles of k_tb2d.cu.
+static bool release_extra(awe_batch *b) {
+    if (b->tb2_grad && !b->grad_busy) {
+        bfree(b, b->slots);
+        bfree(b, b->tb2_xy);
+        b->gT = 0;
+        b->tb2_grad = b->tb2_tried = false;
+        return true;
+    }
+    if (!b->tb2_ok) return false;
+    drop_graph(b);  // reads them
+    bfree(b, b->tb2_u);
+    bfree(b, b->tb2_xy);
+    bfree(b, b->d_tb2_cols);
+    for (awe_batch::Lists *l : {&b->tb2_fwd, &b->tb2_adj}) {
+        bfree(b, l->buf);
+        bfree(b, l->tiles);
+    }
+    b->tb2_ok = b->tb2 = b->tb2_grad = false;
+    return true;
+}
+
+static awe_status balloc(awe_batch *b, void **p, size_t bytes) {
+    awe_status st = balloc_extra(b, p, bytes);
+    while (st != AWE_OK && release_extra(b)) st = balloc_extra(b, p, bytes);
+    return st;
 }
 
 static void build_items(awe_batch *b) {
@@ -118,11 +181,7 @@ static void build_items(awe_batch *b) {
 }
 
 static awe_status upload_items(awe_batch *b) {
-    if (b->d_items) {
-        cudaFree(b->d_items);
-        b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), (void *)b->d_items));
-        b->d_items = nullptr;
-    }
+    bfree(b, b->d_items);
     awe_status st = balloc(b, (void **)&b->d_items, b->items.size() * sizeof(int4));
     if (st != AWE_OK) return st;
     CUDA_TRY(cudaMemcpy(b->d_items, b->items.data(), b->items.size() * sizeof(int4), cudaMemcpyHostToDevice));
@@ -137,11 +196,7 @@ static awe_status build_col_items(awe_batch *b, int L) {
     b->ncol_items = (int)b->col_items.size();
     for (int s = 0; s < (int)b->shots.size(); s++)
         for (int r = 0; r < b->shots[s].nr; r += kBatchRecBlock) b->col_items.push_back(make_int4(s, r, 0, 1));
-    if (b->d_col_items) {
-        cudaFree(b->d_col_items);
-        b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), (void *)b->d_col_items));
-        b->d_col_items = nullptr;
-    }
+    bfree(b, b->d_col_items);
     awe_status st = balloc(b, (void **)&b->d_col_items, b->col_items.size() * sizeof(int4));
     if (st != AWE_OK) return st;
     CUDA_TRY(cudaMemcpy(b->d_col_items, b->col_items.data(), b->col_items.size() * sizeof(int4),
@@ -198,9 +253,12 @@ static awe_status upload_lists(awe_batch *b, awe_batch::Lists &l, const Tb2HostL
             tiles.push_back({q.off, q.dat_off, q.n2, q.wx_off, q.nr, k % sh.ntz * sh.tz, k / sh.ntz * sh.tx, r[0],
                              r[1] - r[0], c[0], c[1] - c[0], e[0], e[1] - e[0], 0});
         }
-    awe_status st = balloc(b, (void **)&l.buf, h.buf.size() * sizeof(int));
-    if (st == AWE_OK) st = balloc(b, (void **)&l.tiles, tiles.size() * sizeof(Tb2Tile));
-    if (st != AWE_OK) return st;
+    awe_status st = balloc_extra(b, (void **)&l.buf, h.buf.size() * sizeof(int));
+    if (st == AWE_OK) st = balloc_extra(b, (void **)&l.tiles, tiles.size() * sizeof(Tb2Tile));
+    if (st != AWE_OK) {
+        bfree(b, l.buf);
+        return st;
+    }
     CUDA_TRY(cudaMemcpy(l.tiles, tiles.data(), tiles.size() * sizeof(Tb2Tile), cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(l.buf, h.buf.data(), h.buf.size() * sizeof(int), cudaMemcpyHostToDevice));
     std::copy(h.off, h.off + 7, l.off);
@@ -238,11 +296,17 @@ static awe_status set_tb2(awe_batch *b) {
     Tb2HostLists h;
     if (!tb2_host_lists(sh, b->tb2_grids, b->tb2_tiles, h)) return AWE_OK;
     awe_status st = upload_lists(b, b->tb2_fwd, h);
-    if (st == AWE_OK) st = balloc(b, (void **)&b->d_tb2_cols, cols.size() * sizeof(int2));
+    if (st == AWE_OK) st = balloc_extra(b, (void **)&b->d_tb2_cols, cols.size() * sizeof(int2));
+    if (st == AWE_OK) st = balloc_extra(b, (void **)&b->tb2_u, (size_t)2 * b->cells * sizeof(float));
+    if (st == AWE_ERR_NOMEM) {
+        bfree(b, b->tb2_fwd.buf);
+        bfree(b, b->tb2_fwd.tiles);
+        bfree(b, b->d_tb2_cols);
+        return AWE_OK;
+    }
     if (st != AWE_OK) return st;
     CUDA_TRY(cudaMemcpy(b->d_tb2_cols, cols.data(), cols.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    b->tb2_ok = balloc(b, (void **)&b->tb2_u, (size_t)2 * b->cells * sizeof(float)) == AWE_OK;
-    cudaGetLastError();
+    b->tb2_ok = true;
     b->tb2 = b->tb2_ok;
     return AWE_OK;
 }
@@ -513,7 +577,7 @@ awe_status awe_batch_destroy(awe_batch *b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     drop_graph(b);
-    for (void *p : b->allocs) cudaFree(p);
+    for (auto &a : b->allocs) cudaFree(a.first);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return AWE_OK;
@@ -598,6 +662,7 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
         return AWE_ERR_STATE;
     }
     CUDA_TRY(cudaSetDevice(b->device));
+    drop_graph(b);  // recaptured with the chosen kernel on the next forward (its items are freed here)
     steps = std::min(steps, b->d.nt);
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
@@ -689,7 +754,7 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
         if (st != AWE_OK) return st;
         b->col_grid = best_col_grid;
     }
-    b->tb2 = tb2_ms < best;
+    b->tb2 = b->tb2_ok && tb2_ms < best;
     b->selected = false;
     int bad = 0;
     CUDA_TRY(cudaMemcpy(&bad, b->d_err, sizeof bad, cudaMemcpyDeviceToHost));
@@ -700,7 +765,6 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
     build_items(b);
     awe_status st = upload_items(b);
     if (st != AWE_OK) return st;
-    drop_graph(b);  // recaptured with the chosen shape on the next forward
     CUDA_TRY(cudaGetLastError());
     if (tile_out) *tile_out = b->tb2 ? kBatchNumTiles + 1 : b->colL > 0 ? kBatchNumTiles : best_tile;
     if (grid_out) *grid_out = b->tb2 ? b->tb2_tiles : b->colL > 0 ? b->col_grid : best_grid;
@@ -730,13 +794,8 @@ static awe_status build_rec_cells(awe_batch *b) {
                                          e0, (int)ws.size(), 0});
         }
     }
-    for (void *q : {(void *)b->rec_cells, (void *)b->rec_ws}) {
-        if (!q) continue;
-        cudaFree(q);
-        b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), q));
-    }
-    b->rec_cells = nullptr;
-    b->rec_ws = nullptr;
+    bfree(b, b->rec_cells);
+    bfree(b, b->rec_ws);
     awe_status st = balloc(b, (void **)&b->rec_cells, std::max<size_t>(cells.size(), 1) * sizeof(BatchRecCell));
     if (st == AWE_OK) st = balloc(b, (void **)&b->rec_ws, std::max<size_t>(ws.size(), 1) * sizeof(BatchRecW));
     if (st != AWE_OK) return st;
@@ -752,66 +811,57 @@ static awe_status grad_alloc(awe_batch *b, int T, int fmt) {
     const bool want = b->tb2_ok && !b->selected;
     if (b->gT == T && b->gfmt == fmt && (b->tb2_grad || b->tb2_tried || !want)) return AWE_OK;
     b->gT = 0;
-    for (void *q : {(void *)b->slots, b->ckpt, (void *)b->scales}) {
-        if (!q) continue;
-        cudaFree(q);
-        b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), q));
-    }
-    b->slots = nullptr;
-    b->ckpt = nullptr;
-    b->scales = nullptr;
+    b->tb2_grad = b->tb2_tried = false;
+    bfree(b, b->slots);
+    bfree(b, b->ckpt);
+    bfree(b, b->scales);
     const int nseg = (b->d.nt + T - 1) / T;
-    const size_t es = fmt == AWE_CKPT_FP32 ? 4 : 2;
-    awe_status st = balloc(b, &b->ckpt, (size_t)2 * nseg * b->cells * es);
+    const size_t es = fmt == AWE_CKPT_FP32 ? 4 : 2, cb = (size_t)b->cells * sizeof(float);
+    const size_t nd = (size_t)std::max(b->ndat, 1LL);
     b->gscale_per = fmt == AWE_CKPT_BFP16 ? (b->cells + kBfpBlock - 1) / kBfpBlock : (long long)b->shots.size();
-    if (st == AWE_OK) st = balloc(b, (void **)&b->scales, (size_t)2 * nseg * b->gscale_per * sizeof(float));
+    const bool first = !b->win;
+    const std::pair<void **, size_t> need[] = {
+        {&b->ckpt, (size_t)2 * nseg * b->cells * es},
+        {(void **)&b->scales, (size_t)2 * nseg * b->gscale_per * sizeof(float)},
+        {(void **)&b->gX, cb},
+        {(void **)&b->gY, cb},
+        {(void **)&b->G, (size_t)b->cells * sizeof(float2)},
+        {(void **)&b->res, nd * sizeof(float)},
+        {(void **)&b->dobs, nd * sizeof(float)},
+        {(void **)&b->part, ((nd + 1023) / 1024) * sizeof(double)},
+        {(void **)&b->grad, (size_t)b->d.n[0] * b->d.n[1] * sizeof(double)},
+        {(void **)&b->win, b->shots.size() * sizeof(int2)}};
+    awe_status st = AWE_OK;
+    for (const auto &q : need)
+        if (st == AWE_OK && !*q.first) st = balloc(b, q.first, q.second);
     if (st != AWE_OK) return st;
-    if (!b->gX) {
-        const size_t cb = (size_t)b->cells * sizeof(float);
-        const size_t nd = (size_t)std::max(b->ndat, 1LL);
-        for (void **q : {(void **)&b->gX, (void **)&b->gY})
-            if (st == AWE_OK) st = balloc(b, q, cb);
-        if (st == AWE_OK) st = balloc(b, (void **)&b->G, (size_t)b->cells * sizeof(float2));
-        if (st == AWE_OK) st = balloc(b, (void **)&b->res, nd * sizeof(float));
-        if (st == AWE_OK) st = balloc(b, (void **)&b->dobs, nd * sizeof(float));
-        if (st == AWE_OK) st = balloc(b, (void **)&b->part, ((nd + 1023) / 1024) * sizeof(double));
-        if (st == AWE_OK) st = balloc(b, (void **)&b->grad, (size_t)b->d.n[0] * b->d.n[1] * sizeof(double));
-        if (st == AWE_OK) st = balloc(b, (void **)&b->win, b->shots.size() * sizeof(int2));
-        if (st != AWE_OK) return st;
+    if (first) {
         std::vector<int2> w(b->shots.size());
         for (size_t s = 0; s < w.size(); s++) w[s] = make_int2(b->shots_in[s].x0, b->shots_in[s].nx);
         CUDA_TRY(cudaMemcpy(b->win, w.data(), w.size() * sizeof(int2), cudaMemcpyHostToDevice));
     }
+    if (b->nrec_cells < 0) {
+        st = build_rec_cells(b);
+        if (st != AWE_OK) return st;
+    }
     // several steps a launch: slots for both sweeps of a segment and two more
     // levels, where memory is left for them when all else is allocated
-    b->tb2_grad = false;
-    b->tb2_tried = want;
-    if (want) {
+    if (b->tb2_ok && want) {
+        b->tb2_tried = true;
         if (!b->tb2_adj.buf) {
             std::vector<Tb2Grid> grids = b->tb2_grids;
             for (Tb2Grid &g : grids) g.inj = g.rec, g.ninj = g.nrec, g.rec = nullptr, g.nrec = 0;
             Tb2HostLists h;
             if (tb2_host_lists(b->tb2_shape, grids, b->tb2_tiles, h)) {
                 st = upload_lists(b, b->tb2_adj, h);
-                if (st != AWE_OK) return st;
+                if (st != AWE_OK && st != AWE_ERR_NOMEM) return st;
             }
         }
-        if (b->tb2_adj.buf && !b->tb2_xy &&
-            balloc(b, (void **)&b->tb2_xy, (size_t)2 * b->cells * sizeof(float)) != AWE_OK)
-            b->tb2_xy = nullptr;
-        b->tb2_grad = b->tb2_adj.buf && b->tb2_xy &&
-                      balloc(b, (void **)&b->slots, (size_t)std::max(2 * T, T + 1) * b->cells * sizeof(float)) == AWE_OK;
-        if (!b->tb2_grad) {
-            b->slots = nullptr;
-            if (b->tb2_xy) {
-                cudaFree(b->tb2_xy);
-                b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), (void *)b->tb2_xy));
-                b->tb2_xy = nullptr;
-            }
-        }
-        cudaGetLastError();
+        b->tb2_grad = b->tb2_adj.buf && balloc_extra(b, (void **)&b->tb2_xy, 2 * cb) == AWE_OK &&
+                      balloc_extra(b, (void **)&b->slots, (size_t)std::max(2 * T, T + 1) * cb) == AWE_OK;
+        if (!b->tb2_grad) bfree(b, b->tb2_xy);
     }
-    if (!b->tb2_grad) st = balloc(b, (void **)&b->slots, (size_t)(T + 1) * b->cells * sizeof(float));
+    if (!b->tb2_grad) st = balloc(b, (void **)&b->slots, (size_t)(T + 1) * cb);
     if (st != AWE_OK) return st;
     b->gT = T;
     b->gfmt = fmt;
@@ -948,8 +998,12 @@ awe_status awe_batch_gradient(awe_batch *b, const float *wav, const float *dobs,
     CUDA_TRY(cudaSetDevice(b->device));
     int T = o.ckpt_every > 0 ? o.ckpt_every : (int)std::ceil(std::sqrt((double)b->d.nt));
     T = std::max(1, std::min(T, b->d.nt));
+    struct Use {
+        awe_batch *b;
+        explicit Use(awe_batch *q) : b(q) { b->grad_busy = true; }
+        ~Use() { b->grad_busy = false; }
+    } use(b);
     awe_status st = grad_alloc(b, T, o.ckpt_format);
-    if (st == AWE_OK && b->nrec_cells < 0) st = build_rec_cells(b);
     if (st == AWE_OK) {
         const int cpsm = b->colL > 0 ? batch2d_col_adj_ctas_per_sm(b->n1) : 0;
         b->col_adj_grid = cpsm > 0 ? cpsm * b->sms : 0;
