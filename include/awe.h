@@ -350,10 +350,12 @@ awe_status awe_batch_forward_device(awe_batch *batch, const float *d_wav, float 
  * launch; grid_out: the forward's grid. */
 awe_status awe_batch_tune(awe_batch *batch, int steps, int *tile_out, int *grid_out);
 awe_status awe_batch_info(const awe_batch *batch, awe_batch_info_t *info);
-/* Picks a one-step kernel without timing: kernel 0-3 = the tile shapes,
- * 4 = the column march with `chunk` columns per item (8th order only);
- * grid <= 0 = the default (4 CTAs per SM for tiles, every resident CTA for
- * the column march). */
+/* Picks a kernel without timing (an answer of awe_batch_tune, for instance):
+ * kernel 0-3 = the tile shapes, 4 = the column march with `chunk` columns per
+ * item (8th order only), both one step a launch, also in the gradient; 5 = the
+ * kernel that takes several steps a launch (chunk and grid are not used;
+ * AWE_ERR_UNSUPPORTED where it does not apply).  grid <= 0 = the default (4
+ * CTAs per SM for tiles, every resident CTA for the column march). */
 awe_status awe_batch_select(awe_batch *batch, int kernel, int chunk, int grid);
 /* Misfit gradient of the whole batch: J = 0.5 sum over shots and samples of
  * (d - dobs)^2, dJ/dm (m = 1/v^2) on the whole model [n2][n1] (each shot's

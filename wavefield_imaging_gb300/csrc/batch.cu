@@ -1034,11 +1034,22 @@ awe_status awe_batch_gradient(awe_batch *b, const float *wav, const float *dobs,
 }
 
 awe_status awe_batch_select(awe_batch *b, int kernel, int chunk, int grid) {
-    if (!b || kernel < 0 || kernel > kBatchNumTiles) {
-        set_error("awe_batch_select: kernel must be 0-%d", kBatchNumTiles);
+    if (!b || kernel < 0 || kernel > kBatchNumTiles + 1) {
+        set_error("awe_batch_select: kernel must be 0-%d", kBatchNumTiles + 1);
         return AWE_ERR_INVALID;
     }
     CUDA_TRY(cudaSetDevice(b->device));
+    if (kernel == kBatchNumTiles + 1) {
+        if (!b->tb2_ok) {
+            set_error("awe_batch_select: several steps a launch need order 8 or less, no source in the sponge, no "
+                      "point on a window's last line, few enough in a tile, and memory for two more levels");
+            return AWE_ERR_UNSUPPORTED;
+        }
+        drop_graph(b);
+        b->tb2 = true;
+        b->selected = false;
+        return AWE_OK;
+    }
     drop_graph(b);
     if (kernel < kBatchNumTiles) {
         b->tb2 = false;

@@ -398,8 +398,9 @@ class Batch:
         return grad, J.value
 
     def select(self, kernel: int, chunk: int = 32, grid: int = 0):
-        """Forward kernel without timing (awe_batch_select): 0-3 tile shapes,
-        4 = the column march with `chunk` columns per item."""
+        """Kernel without timing (awe_batch_select): 0-3 tile shapes, 4 = the
+        column march with `chunk` columns per item, 5 = several steps a launch
+        (the default where it applies)."""
         _check(lib().awe_batch_select(self._h, kernel, chunk, grid))
         self.info = self._info()
 
