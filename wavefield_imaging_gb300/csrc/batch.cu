@@ -38,6 +38,7 @@ struct awe_batch {
     float *u[2] = {nullptr, nullptr}, *vel = nullptr, *wz = nullptr, *wx = nullptr, *wav = nullptr, *dat = nullptr;
     BatchShot *d_shots = nullptr;
     int4 *d_items = nullptr;
+    size_t items_cap = 0;
     GeoPoint *src = nullptr, *rec = nullptr;
     bool model_set = false;
     int tile = 0, grid = 0, sms = 1;
@@ -61,6 +62,7 @@ struct awe_batch {
     int colL = 0, col_grid = 0, ncol_items = 0;
     std::vector<int4> col_items;
     int4 *d_col_items = nullptr;
+    size_t col_cap = 0;
     int *d_err = nullptr;  // set by a bulk-copy wait that timed out
     int col_adj_grid = 0;  // column-march adjoint's grid (0: the tile adjoint)
     // several steps a launch (k_tb2d.cu): possible for these points, the forward's; two more
@@ -180,12 +182,22 @@ static void build_items(awe_batch *b) {
         for (int r = 0; r < b->shots[s].nr; r += kBatchRecBlock) b->items.push_back(make_int4(s, r, 0, 1));
 }
 
-static awe_status upload_items(awe_batch *b) {
-    bfree(b, b->d_items);
-    awe_status st = balloc(b, (void **)&b->d_items, b->items.size() * sizeof(int4));
-    if (st != AWE_OK) return st;
-    CUDA_TRY(cudaMemcpy(b->d_items, b->items.data(), b->items.size() * sizeof(int4), cudaMemcpyHostToDevice));
+// items to a device buffer that is kept while large enough (the tuner tries
+// several lists); no launch that reads it may be in flight
+static awe_status upload(awe_batch *b, const std::vector<int4> &v, int4 *&d, size_t &cap) {
+    if (cap < v.size()) {
+        bfree(b, d);
+        cap = 0;
+        const awe_status st = balloc(b, (void **)&d, v.size() * sizeof(int4));
+        if (st != AWE_OK) return st;
+        cap = v.size();
+    }
+    CUDA_TRY(cudaMemcpy(d, v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice));
     return AWE_OK;
+}
+
+static awe_status upload_items(awe_batch *b) {
+    return upload(b, b->items, b->d_items, b->items_cap);
 }
 
 // column items (shot, x0) for chunks of L columns, then the receiver items
@@ -196,13 +208,9 @@ static awe_status build_col_items(awe_batch *b, int L) {
     b->ncol_items = (int)b->col_items.size();
     for (int s = 0; s < (int)b->shots.size(); s++)
         for (int r = 0; r < b->shots[s].nr; r += kBatchRecBlock) b->col_items.push_back(make_int4(s, r, 0, 1));
-    bfree(b, b->d_col_items);
-    awe_status st = balloc(b, (void **)&b->d_col_items, b->col_items.size() * sizeof(int4));
-    if (st != AWE_OK) return st;
-    CUDA_TRY(cudaMemcpy(b->d_col_items, b->col_items.data(), b->col_items.size() * sizeof(int4),
-                        cudaMemcpyHostToDevice));
-    b->colL = L;
-    return AWE_OK;
+    const awe_status st = upload(b, b->col_items, b->d_col_items, b->col_cap);
+    if (st == AWE_OK) b->colL = L;
+    return st;
 }
 
 // Tile of k_tb2d.cu for all windows: 4 columns a thread, up to 256 threads, two
@@ -213,6 +221,9 @@ static awe_status build_col_items(awe_batch *b, int L) {
 // 8th order, where 48 x 48 cells took 14.3 us a step with 2 steps a launch, 18.1
 // with one (56 x 56), 15.5 with three (40 x 40), and the one-step kernels 17.8.
 static bool tb2_batch_shape(const std::vector<BatchShot> &shots, int n1, int nop, int sms, Tb2Shape &best) {
+    long long ntx[31] = {};  // tile columns of all windows by tx / 4 (one pass: there may be thousands of windows)
+    for (const BatchShot &sh : shots)
+        for (int q = 2; q <= 30; q++) ntx[q] += (sh.n2 + 4 * q - 1) / (4 * q);
     double cost = 1e30;
     for (int tz0 = 8; tz0 <= 120; tz0 += 4)
         for (int tx = 8; tx <= 120; tx += 4)
@@ -229,8 +240,7 @@ static bool tb2_batch_shape(const std::vector<BatchShot> &shots, int n1, int nop
                 s.rz = s.tz + 2 * s.hz;
                 s.rx = (s.tx + 2 * s.hx + 3) / 4 * 4;
                 if ((s.rz / 4) * (s.rx / 4) > kTb2BatchThreads) break;
-                long long tiles = 0;
-                for (const BatchShot &sh : shots) tiles += (long long)s.ntz * ((sh.n2 + tx - 1) / tx);
+                const long long tiles = s.ntz * ntx[tx / 4];
                 const double r = (double)s.rz * s.rx;
                 const double rounds = tiles <= sms ? 1.0 : std::max(1.0, 0.6 * tiles / sms);
                 const double c = rounds * (2.0 / k + 0.25 + 1.5e-4 * r) * (s.rz % 32 ? 1.05 : 1.0);
@@ -662,7 +672,8 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
         return AWE_ERR_STATE;
     }
     CUDA_TRY(cudaSetDevice(b->device));
-    drop_graph(b);  // recaptured with the chosen kernel on the next forward (its items are freed here)
+    CUDA_TRY(cudaDeviceSynchronize());  // no earlier run (on any stream) still reads the items
+    drop_graph(b);  // recaptured with the chosen kernel on the next forward
     steps = std::min(steps, b->d.nt);
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
@@ -670,12 +681,13 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
     float best = 1e30f, tb2_ms = 1e30f;
     int best_tile = b->tile, best_grid = b->grid;
     const size_t bytes = (size_t)b->cells * sizeof(float);
+    // (once: the time of a step does not depend on what the levels hold)
+    CUDA_TRY(cudaMemsetAsync(b->u[0], 0, bytes, b->stream));
+    CUDA_TRY(cudaMemsetAsync(b->u[1], 0, bytes, b->stream));
     b->colL = 0;
     if (b->tb2_ok) {
         const int n = std::min((steps + b->tb2_shape.k - 1) / b->tb2_shape.k * b->tb2_shape.k, b->d.nt);
         b->tb2 = true;
-        cudaMemsetAsync(b->u[0], 0, bytes, b->stream);
-        cudaMemsetAsync(b->u[1], 0, bytes, b->stream);
         launch_range(b, 0, std::min(n, b->tb2_shape.k), b->stream);  // warm
         cudaEventRecord(e0, b->stream);
         launch_range(b, 0, n, b->stream);
@@ -692,8 +704,6 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
         if (st != AWE_OK) return st;
         for (int mult : {2, 4, 8, 16}) {
             b->grid = mult * b->sms;
-            cudaMemsetAsync(b->u[0], 0, bytes, b->stream);
-            cudaMemsetAsync(b->u[1], 0, bytes, b->stream);
             launch_range(b, 0, 1, b->stream);  // warm
             cudaEventRecord(e0, b->stream);
             launch_range(b, 0, steps, b->stream);
@@ -724,14 +734,14 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
         const long long t = (items + (long long)cpsm * b->sms - 1) / ((long long)cpsm * b->sms) * (L + 8);
         if (cols_best < 0 || t < cols_best) cols_best = t, Lw = L;
     }
-    for (int L : {16, 32, 64, Lw}) {
+    std::vector<int> chunks = {16, 32, 64};
+    if (Lw != 16 && Lw != 32 && Lw != 64) chunks.push_back(Lw);
+    for (int L : chunks) {
         if (cpsm <= 0) break;
         awe_status st = build_col_items(b, L);
         if (st != AWE_OK) return st;
         for (int mult : {1, 2}) {
             b->col_grid = mult * cpsm * b->sms;
-            cudaMemsetAsync(b->u[0], 0, bytes, b->stream);
-            cudaMemsetAsync(b->u[1], 0, bytes, b->stream);
             launch_range(b, 0, 1, b->stream);  // warm
             cudaEventRecord(e0, b->stream);
             launch_range(b, 0, steps, b->stream);
@@ -1039,6 +1049,7 @@ awe_status awe_batch_select(awe_batch *b, int kernel, int chunk, int grid) {
         return AWE_ERR_INVALID;
     }
     CUDA_TRY(cudaSetDevice(b->device));
+    CUDA_TRY(cudaDeviceSynchronize());  // no earlier run (on any stream) still reads the items
     if (kernel == kBatchNumTiles + 1) {
         if (!b->tb2_ok) {
             set_error("awe_batch_select: several steps a launch need order 8 or less, no source in the sponge, no "
