@@ -17,7 +17,7 @@ import hashlib
 import numpy as np, wavefield_imaging_gb300 as awe
 from helpers import ricker
 kind = sys.argv[1]
-n = dict(grad2d=(300, 290), frames2d=(300, 290), fwd3d=(70, 60, 52))[kind]
+n = dict(grad2d=(300, 290), frames2d=(300, 290), fwd3d=(70, 60, 52), shell=(101, 40, 40))[kind]
 nt, d = 60, (5.0,) * len(n)
 rng = np.random.default_rng(1)
 vel = (150 + 30 * rng.random(n[::-1])).astype(np.float32)
@@ -35,20 +35,29 @@ def call(f):
     except awe.AweError as e:
         res.append("E%d" % e.status)
 wav, obs = ricker(nt, 0.005), rng.standard_normal((nt, 40)).astype(np.float32)
+if kind == "shell":  # r, theta, phi
+    d = (0.005, 1.5e-6, 1.5e-6)
+    o = (3387.0, np.pi / 2 - 20 * d[1], -20 * d[2])
+    vel, axes = vel / 1000, (0, 2, 1)
+    pt = lambda f: [o[a] + f * (n[a] - 1) * d[a] for a in axes]
+    sou, rec = np.array([pt(0.5)], np.float32), np.array([pt(0.3 + 0.01 * k) for k in range(40)], np.float32)
+    desc = awe.make_desc(3, n, d, o, nt, 0.005, coords=awe.SPHER, scheme=awe.SCHEME_GPU, nb=8, precision=awe.FAST)
 held = launches = 0
 try:
     p = awe.Plan(desc)
     p.set_model(vel); p.set_geometry(sou, rec)
     for _ in range(3):  # launched, captured, replayed
-        if kind != "fwd3d":
+        if kind not in ("fwd3d", "shell"):
             call(lambda: h(p.gradient(wav, obs, ckpt_every=5)[0]))
             launches = p.last_launch_count()
         if kind == "frames2d":
             call(lambda: h(*p.forward(wav, snapshots=True)))
-        if kind == "fwd3d":
+        if kind in ("fwd3d", "shell"):
             call(lambda: h(p.forward(wav)))
             launches = p.last_launch_count()
     held = p.device_bytes()
+    if kind == "shell":
+        res.append(p.step_kernel)
 except awe.AweError as e:
     res.append("C%d" % e.status)
 print(held, launches, " ".join(res))
@@ -76,6 +85,16 @@ def test_what_fits_one_step_a_launch_fits(kind):
     for limit in (need, need + level // 2, need + 2 * level, need + 4 * level, (need + top) // 2, top + 8 * level):
         held, _, res = _run(kind, limit)
         assert res == want and held <= limit
+
+
+def test_padded_lines_of_a_shell_give_way():
+    need, _, want = _run("shell", kernel="simple")
+    level = 117 * 56 * 56 * 4
+    held, _, res = _run("shell", need)  # less than three padded levels
+    assert need < 3 * level * 120 // 117 and held <= need
+    assert res == want and res[-1] == "simple"
+    _, _, res = _run("shell", need + level)
+    assert res[-1] == "tma_sph" and not any(r.startswith(("E", "C")) for r in res)
 
 
 def test_too_little_memory_is_an_error_every_time():

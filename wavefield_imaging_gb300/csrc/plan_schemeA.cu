@@ -42,6 +42,13 @@ static awe_status upload_t(awe_plan *p, T **dst, const T *src, size_t n) {
 
 static int floor_first(float o, float opad, float d, float eps) { return (int)(std::floor)((o - opad) / d + eps); }
 
+// the two levels and the velocity
+static awe_status alloc_levels(awe_plan *p) {
+    for (float **q : {&p->u[0], &p->u[1], &p->vel})
+        AWE_TRY(dev_alloc(p, (void **)q, (size_t)p->g.cells() * sizeof(float)));
+    return AWE_OK;
+}
+
 awe_status planA_init(awe_plan *p) {
     awe_desc &d = p->d;
     p->ndim = d.ndim;
@@ -51,19 +58,6 @@ awe_status planA_init(awe_plan *p) {
     const int nb = d.nb < kNopA ? kNopA : d.nb;  // MAWEFDcart2Dgpu.cu:144
     p->nbd = nb;
     p->g = Grid{d.n[0] + 2 * nb, d.n[1] + 2 * nb, d.ndim == 3 ? d.n[2] + 2 * nb : 1};
-    // TMA-staged spherical step for AWE_FAST; AWE_STEP_KERNEL=simple keeps the
-    // register-march kernel (the tests compare both).  Lines of its levels
-    // start on 16-byte boundaries: n1 % 4 != 0 takes padded ones from 2^17
-    // cells on.  (A step of 185 x 122 x 122 ragged cells: 25 us against 33;
-    // below, launches bound both, 19 us against 25, and the plan stays with
-    // the kernels that step_kernel has always reported for such grids.)
-    const char *kern = std::getenv("AWE_STEP_KERNEL");
-    bool sph_tma = geom == 3 && d.precision == AWE_FAST && !(kern && std::strcmp(kern, "simple") == 0);
-    if (sph_tma) {
-        const Grid pitched(p->g.n1, p->g.n2, p->g.n3, (p->g.n1 + 3) / 4 * 4);
-        sph_tma = sphA_tma_eligible(pitched, nb) && (p->g.n1 % 4 == 0 || pitched.cells() >= 1 << 17);
-        if (sph_tma) p->g = pitched;
-    }
     const Grid &g = p->g;
     if (g.n1 < 12 || g.n2 < 12 || (d.ndim == 3 && g.n3 < 12)) {
         set_error("the GPU-program scheme needs at least 12 padded samples per axis");
@@ -75,6 +69,33 @@ awe_status planA_init(awe_plan *p) {
         set_error("the cartesian 3D GPU program is defined only for nx == nz (got nz=%d nx=%d)", d.n[0], d.n[1]);
         return AWE_ERR_UNSUPPORTED;
     }
+    // TMA-staged spherical step for AWE_FAST; AWE_STEP_KERNEL=simple keeps the
+    // register-march kernel (the tests compare both).  Lines of its levels
+    // start on 16-byte boundaries: n1 % 4 != 0 takes padded ones from 2^17
+    // cells on.  (A step of 185 x 122 x 122 ragged cells: 25 us against 33;
+    // below, launches bound both, 19 us against 25, and the plan stays with
+    // the kernels that step_kernel has always reported for such grids.)
+    const char *kern = std::getenv("AWE_STEP_KERNEL");
+    bool sph_tma = geom == 3 && d.precision == AWE_FAST && !(kern && std::strcmp(kern, "simple") == 0);
+    if (sph_tma) {
+        const Grid pitched(p->g.n1, p->g.n2, p->g.n3, (p->g.n1 + 3) / 4 * 4);
+        sph_tma = sphA_tma_eligible(pitched, nb) && (p->g.n1 % 4 == 0 || pitched.cells() >= 1 << 17);
+        // the register kernels take plain lines only: padded ones once their
+        // levels are allocated and the tensor maps encoded
+        if (sph_tma) {
+            const Grid plain = p->g;
+            p->g = pitched;
+            sph_tma = alloc_levels(p) == AWE_OK && sphA_tma_maps(p->sph_maps, p->u, p->vel, p->g, 1);
+            if (!sph_tma) {
+                for (float **q : {&p->u[0], &p->u[1], &p->vel}) {
+                    dev_free(p, *q);
+                    *q = nullptr;
+                }
+                p->g = plain;
+            }
+        }
+    }
+    if (!sph_tma) AWE_TRY(alloc_levels(p));
     for (int a = 0; a < d.ndim; a++) p->opad[a] = d.o[a] - nb * d.d[a];
 
     StepAParams &pa = p->pa;
@@ -174,18 +195,14 @@ awe_status planA_init(awe_plan *p) {
     }
 
     const size_t cells = (size_t)g.cells();
-    AWE_TRY(dev_alloc(p, (void **)&p->u[0], cells * sizeof(float)));
-    AWE_TRY(dev_alloc(p, (void **)&p->u[1], cells * sizeof(float)));
-    AWE_TRY(dev_alloc(p, (void **)&p->vel, cells * sizeof(float)));
     AWE_TRY(dev_alloc(p, (void **)&p->corner_off, 8 * sizeof(long long)));
     if (geom != 3) AWE_TRY(dev_alloc(p, (void **)&p->u3, cells * sizeof(float)));
 
     pa.nshot = 1;
     pa.shot_cells = g.cells();
-    // (the TMA kernels' sponge index walks the axes in this grid's priority
-    // order (r, phi, theta) = memory axes (1, 3, 2))
-    const bool pri_rpt = pa.pri[0] == 0 && pa.pri[1] == 2 && pa.pri[2] == 1;
-    if (sph_tma && pri_rpt && sphA_tma_maps(p->sph_maps, p->u, p->vel, g, 1)) {
+    // (the TMA kernels' sponge index walks the axes in the spherical grid's
+    // priority order (r, phi, theta) = memory axes (1, 3, 2), pa.pri above)
+    if (sph_tma) {
         AWE_TRY(dev_alloc(p, (void **)&p->sched_counter, sizeof(unsigned long long)));
         AWE_TRY(dev_alloc(p, (void **)&p->d_err, sizeof(int)));
         CUDA_TRY(cudaMemset(p->sched_counter, 0, sizeof(unsigned long long)));
@@ -234,7 +251,6 @@ awe_status planA_model(awe_plan *p, const float *vel, const float *rfl) {
     p->inj_scale_ok = false;
     p->h_vel_raw.assign(cells, 0.f);
     expand_model(d.ndim, vel, p->h_vel_raw.data(), nb, d.n);
-    if (!p->vel) AWE_TRY(dev_alloc(p, (void **)&p->vel, (size_t)g.cells() * sizeof(float)));
     CUDA_TRY(cudaMemcpy2D(p->vel, g.p1 * sizeof(float), p->h_vel_raw.data(), g.n1 * sizeof(float),
                           g.n1 * sizeof(float), lines, cudaMemcpyHostToDevice));
     const std::vector<float> &v = p->h_vel_raw;
