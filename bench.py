@@ -1366,7 +1366,8 @@ def run_fwd2d(args):
            "config": {"workload": "2D %dx%d at 5 m (nb=40), 8th order, nt=%d, dabc=y, 1 source, %d receivers; "
                                   "time loop as one CUDA graph" % (nz, nx, nt, nx), "padded_cells": cells,
                       "l2": "the 1.4 MB fields stay in L2: launch- and latency-bound, no HBM claim"},
-           "step_kernel_us_directly_launched": avg * 1e6, "us_per_time_step": 1e3 * ms / nt,
+           "step_kernel_us_directly_launched": avg * 1e6, "steps_per_launch": nt / max(kern_n, 1),
+           "us_per_time_step": 1e3 * ms / nt,
            "gpu_launches": plan.last_launch_count(), "clocks": clocks}
     print(json.dumps(out))
     plan.close()

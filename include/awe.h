@@ -195,7 +195,10 @@ long long awe_last_launch_count(const awe_plan *plan);
  * stream; awe_profile_read returns the step kernels' summed duration (ms) and
  * launch count after the runs have completed, awe_profile_read_kinds both
  * kinds (arrays of AWE_PROF_KINDS, indexed by AWE_PROF_STEP and
- * AWE_PROF_ADJOINT).  Reading resets the record.  Off by default. */
+ * AWE_PROF_ADJOINT).  A launch that takes several steps (2D) counts as one; the
+ * imaging condition of such a gradient is a launch of its own and not bracketed.
+ * Profiled runs use the kernels that other runs do, launched directly.  Reading
+ * resets the record.  Off by default. */
 #define AWE_PROF_STEP 0
 #define AWE_PROF_ADJOINT 1
 #define AWE_PROF_KINDS 2

@@ -620,7 +620,7 @@ awe_status plan_gradient(awe_plan *p, const float *d_wav, int ncs, const float *
             st->lists_ok = true;
         }
         // (the lists above may have taken the memory of the two levels)
-        tb2 = st->tb2 && p->tb2_fwd.ok && p->tb2_adj.ok && !p->profile;
+        tb2 = st->tb2 && p->tb2_fwd.ok && p->tb2_adj.ok;
         if (!tb2 && !st->rc_ok) {
             AWE_TRY(build_cell_lists(p, p->h_rec, nc, &st->rc_start, &st->rc_ent, &st->rc_cap, s));
             st->rc_ok = true;

@@ -231,7 +231,9 @@ void tb2_launch(awe_plan *p, bool adj, const float *prv, const float *cur, float
     q.jdata = d.jdata;
     q.nr = p->nr;
     q.dat = d_dat;
+    prof_begin(p, s, adj ? AWE_PROF_ADJOINT : AWE_PROF_STEP);
     launch_tb2(p->nop, adj ? 2 : slots ? 3 : d.precision == AWE_EXACT ? 1 : 0, q, sh, tb2_smem(sh, t.most), s);
+    prof_end(p, s);
 }
 
 // the one-way ABC's coefficient tables: cells of table k
@@ -765,7 +767,7 @@ awe_status planB_run_hooked(awe_plan *p, const float *d_wav, int ncs, float *d_d
     // 2D: the traces of step it (the level the step reads, pending sponge
     // applied, as the reference extracts after its swap) are gathered by the
     // step's own launch; 3D: by the step's boundary launch
-    if (p->tb2_fwd.ok && !p->den && !p->profile) {
+    if (p->tb2_fwd.ok && !p->den) {
         // several steps a launch, stopping at steps whose levels the hook or a frame reads
         float *alt_prv = p->tb2_u, *alt_cur = p->tb2_u + g.cells();
         float *prv = nxt;
