@@ -109,7 +109,7 @@ struct Tb2Params {
     int tz, tx, hz, hx, rz, rx;
     float c0, cz[5], cx[5];
     const float *cur, *prv, *vel;  // levels it, it - 1; v^2 dt^2
-    float *ocur, *oprv;            // levels it + k, it + k - 1 (other buffers; null: not stored)
+    float *ocur, *oprv;            // levels it + k, it + k - 1 (other buffers)
     // stored by step j at slots + j * slot_stride (null: nothing): L of the level
     // it reads, or (slot_level) that level; the adjoint step nu_k
     float *slots;
@@ -278,6 +278,7 @@ struct StepAParams {
     const float *tb[6];                  // cart 3D one-way coefficient tables
     int nshot;                           // shots advanced together (spherical 3D, AWE_FAST), fields back to back
     long long shot_cells;                // cells of one shot's field
+    int sms;                             // of the device
 };
 // out of place (the spherical AWE_FAST march kernels): prv the previous level, out the new one
 void launch_stepA_oop(const float *cur, const float *prv, float *out, const float *vel,
@@ -490,9 +491,6 @@ bool stepB3_tma_eligible(int ndim, int nop, bool rho, const Grid &g);
 bool stepB3_tma_maps(CUtensorMap *maps, float *const u[2], const float *vel, const Grid &g, int nop);
 int march_planes(int n3, long long columns, int slots, int halo);
 Step3Launch stepB3_tma_shape(const Grid &g, int num_sms, int L, int nop = 4);
-cudaError_t launch_stepB3_tma(bool exact, const CUtensorMap *maps, int icur, float *nxt, const StepBParams &sp,
-                              const Step3Launch &sh, unsigned long long *counter, unsigned long long base, int *err,
-                              cudaStream_t s);
 // lap_out (AWE_FAST only, may be null): also store L(cur) of interior cells
 cudaError_t launch_stepB3_tma_with(bool exact, const CUtensorMap &cur, const CUtensorMap &prv, const CUtensorMap &vel,
                                    float *nxt, const StepBParams &sp, const Step3Launch &sh,

@@ -251,7 +251,7 @@ void launch_stepA3(bool exact, const float *cur, const float *prv, float *nxt, c
     // cells: 5.4 us a step with one plane, 13.7 with 16; 100^3: 12.4 with two,
     // 16.6 with 16; 290^3: 228 with two, 132 with 16.
     int L = 16;
-    while (L > 1 && (long long)grid.x * grid.y * (2 + (p.g.n3 - 10 + L - 1) / L) < 16 * 152) L /= 2;
+    while (L > 1 && (long long)grid.x * grid.y * (2 + (p.g.n3 - 10 + L - 1) / L) < 16LL * p.sms) L /= 2;
     const int segs = 2 + (p.g.n3 - 10 + L - 1) / L;
     grid.z = (unsigned)segs;
     const unsigned per = grid.x * grid.y * TZ * TX;

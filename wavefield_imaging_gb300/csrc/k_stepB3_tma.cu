@@ -473,12 +473,6 @@ Step3Launch stepB3_tma_shape(const Grid &g, int num_sms, int L, int nop) {
 }
 
 // launch one step: cur = u[icur], nxt = u[1-icur]
-cudaError_t launch_stepB3_tma(bool exact, const CUtensorMap *maps, int icur, float *nxt, const StepBParams &sp,
-                              const Step3Launch &sh, unsigned long long *counter, unsigned long long base, int *err,
-                              cudaStream_t s) {
-    return launch_stepB3_tma_with(exact, maps[icur], maps[2 + (1 - icur)], maps[4], nxt, sp, sh, counter, base, err,
-                                  s, nullptr);
-}
 
 static Step3Params step3_params(const StepBParams &sp, const Step3Launch &sh, unsigned long long *counter,
                                 unsigned long long base, int *err, float *nxt) {

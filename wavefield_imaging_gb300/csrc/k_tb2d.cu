@@ -392,7 +392,6 @@ __global__ void __launch_bounds__(BATCH ? kTb2BatchThreads : kTb2Threads, BATCH 
     };
     if (inner && !damp) steps(std::false_type());
     else steps(std::true_type());
-    if (!p.ocur) return;
 #pragma unroll
     for (int c = 0; c < CX; c++) {  // the last two levels
         store(p.ocur, c, cur[c]);

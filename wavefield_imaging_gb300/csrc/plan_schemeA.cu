@@ -200,6 +200,9 @@ awe_status planA_init(awe_plan *p) {
 
     pa.nshot = 1;
     pa.shot_cells = g.cells();
+    cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device);
+    if (p->num_sms < 1) p->num_sms = 1;
+    pa.sms = p->num_sms;
     // (the TMA kernels' sponge index walks the axes in the spherical grid's
     // priority order (r, phi, theta) = memory axes (1, 3, 2), pa.pri above)
     if (sph_tma) {
@@ -207,8 +210,6 @@ awe_status planA_init(awe_plan *p) {
         AWE_TRY(dev_alloc(p, (void **)&p->d_err, sizeof(int)));
         CUDA_TRY(cudaMemset(p->sched_counter, 0, sizeof(unsigned long long)));
         CUDA_TRY(cudaMemset(p->d_err, 0, sizeof(int)));
-        cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device);
-        if (p->num_sms < 1) p->num_sms = 1;
         const char *spin = std::getenv("AWE_PIPELINE_SPIN_LIMIT");
         if (spin && *spin) p->spin_limit = std::atoll(spin);
         p->sph_tma = true;
