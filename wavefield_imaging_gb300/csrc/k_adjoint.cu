@@ -54,7 +54,9 @@ __global__ void __launch_bounds__(256) k_adjB(const float *__restrict__ X, float
     const int i3 = (NDIM == 3) ? (int)blockIdx.z : 0;
     const Grid g = p.g;
     if (i1 >= g.n1 || i2 >= g.n2) return;
-    const long long s2 = g.p1, s3 = (long long)g.p1 * g.n2;
+    // (lines are padded in 3D up to 8th order only)
+    const int line = NDIM == 3 && NOP <= 4 ? g.p1 : g.n1;
+    const long long s2 = line, s3 = (long long)line * g.n2;
     const long long i = i3 * s3 + i2 * s2 + i1;
     const bool in = interior<NOP, NDIM>(g, i1, i2, i3);
     const float x = X[i];

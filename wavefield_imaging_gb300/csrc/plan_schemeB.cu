@@ -278,7 +278,9 @@ awe_status planB_init(awe_plan *p) {
     const Grid plain = p->g;
     {
         const Grid pitched(plain.n1, plain.n2, plain.n3, (plain.n1 + 3) / 4 * 4);
-        if (!force_simple && stepB3_tma_eligible(d.ndim, p->nop, false, pitched)) p->g = pitched;
+        // (k_stepB steps across padded lines with 32-bit offsets)
+        const bool small = pitched.p1 == plain.p1 || pitched.s3() < 1LL << 29;
+        if (!force_simple && small && stepB3_tma_eligible(d.ndim, p->nop, false, pitched)) p->g = pitched;
     }
     for (int a = 0; a < d.ndim; a++) p->opad[a] = d.o[a] - nb * d.d[a];  // fdutil_init
     float dd[3] = {d.d[0], d.d[1], d.ndim == 3 ? d.d[2] : 1.f};
