@@ -438,13 +438,17 @@ bool stepB3_tma_maps(CUtensorMap *maps, float *const u[2], const float *vel, con
 
 // Planes per work item of the marching kernels.  An item of L planes takes
 // L + halo plane times (the halo planes only fill the queue), and `slots` CTAs
-// run at once.  With many waves of items the work counter evens them out and
-// 64 planes keep the halo re-reads low.  Below that the launch takes
+// run at once.  From 3.5 waves of 64-plane items on the work counter evens them
+// out (the short last chunks come last), and 64 planes keep the halo re-reads
+// low: in 13 of 15 forward runs with 3.6 to 5.6 waves the chunk count of the rule
+// below was slower, by up to 4.5 %.  Below that the launch takes
 // ceil(items / slots) * (L + halo) plane times, and the chunk count that makes
 // this least is taken: 208 x 192 x 198 cells had 192 items of 64 planes on 304
 // slots (72 plane times, 65 us); 288 items of 33 planes take 41 plane times.
+// (2.5 to 3.5 waves, 20 runs: from 5.5 % slower to 5.8 % faster than 64 planes,
+// 0.7 % faster in the mean; fewer waves: up to 1.6 times.)
 int march_planes(int n3, long long columns, int slots, int halo) {
-    if (columns * ((n3 + 63) / 64) >= 6LL * slots) return 64;
+    if (2 * columns * ((n3 + 63) / 64) >= 7LL * slots) return 64;
     int best = n3 < 64 ? n3 : 64;
     long long cost = -1;
     for (int c = (n3 + 95) / 96; c <= (n3 + 7) / 8; c++) {
