@@ -181,7 +181,7 @@ def measured_peak():
 
 # DRAM bytes per cell of one step-kernel launch (k_stepB3 at 8th order, AWE_FAST),
 # from the ncu capture of a 384^3-padded launch: 895.2 MB read + written
-# over 56.62 M padded cells (profiles/k_stepB3_o8_tma_n320.md).  A full
+# over 56.62 M padded cells (profiles/k_stepB3_tma_n320.md).  A full
 # 576^3 launch is too large for a capture; DRAM traffic scales with the cells
 # a launch processes.
 STEP_DRAM_BYTES_PER_CELL = 15.810
@@ -466,7 +466,7 @@ def run_ours(args):
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                         "frac": achieved / peak, "traffic": traffic,
                         "traffic_source": ("ncu DRAM bytes per cell of a 384^3-padded launch of the same kernel "
-                                           "(profiles/k_stepB3_o8_tma_n320.md) x this launch's cells"
+                                           "(profiles/k_stepB3_tma_n320.md) x this launch's cells"
                                            if traffic else None),
                         "kernel": ("k_stepB3 (TMA-staged, 3D 8th order)" if plan.step_kernel == "tma3d"
                                    else "k_stepB (one thread per cell, 3D 8th order)"),
