@@ -131,17 +131,18 @@ static awe_status grad_buffers(awe_plan *p, GradState *st, int T, int fmt, size_
         AWE_TRY(dev_alloc(p, (void **)&st->vr, 3 * cells * sizeof(float)));
         AWE_TRY(dev_alloc(p, (void **)&st->gbuf, cells * sizeof(float)));
     }
-    // the point lists of the one-step kernels (build_cell_lists)
+    // the sources' lists (build_cell_lists); the receivers' with one step a launch only
     const bool lists = !st->tma && !st->kap && p->g.cells() <= kFusedCells && d.scheme == AWE_SCHEME_CPU;
-    if (lists) {
-        const int nc = d.ndim == 3 ? 8 : 4;
-        st->sc_cap = std::max<size_t>(p->h_src.size() * nc, 1);
-        st->rc_cap = std::max<size_t>(p->h_rec.size() * nc, 1);
-        for (int **q : {&st->sc_start, &st->rc_start}) AWE_TRY(dev_alloc(p, (void **)q, (cells + 1) * sizeof(int)));
-        AWE_TRY(dev_alloc(p, (void **)&st->sc_ent, st->sc_cap * sizeof(int2)));
-        AWE_TRY(dev_alloc(p, (void **)&st->rc_ent, st->rc_cap * sizeof(int2)));
-    }
-    // the slots last: 2D, two a step and two more levels if memory is left for them
+    const int nc = d.ndim == 3 ? 8 : 4;
+    auto list = [&](int **start, int2 **ent, size_t &cap, size_t points) -> awe_status {
+        cap = std::max<size_t>(points * nc, 1);
+        AWE_TRY(dev_alloc(p, (void **)start, (cells + 1) * sizeof(int)));
+        return dev_alloc(p, (void **)ent, cap * sizeof(int2));
+    };
+    if (lists) AWE_TRY(list(&st->sc_start, &st->sc_ent, st->sc_cap, p->h_src.size()));
+    // the slots last: 2D, two a step and two more levels if memory is left for
+    // them (the plan's two levels give way to the receivers' lists if a
+    // geometry needs those after all)
     if (want_tb2(p)) {
         st->tb2 = dev_alloc_extra(p, (void **)&st->xy2, 2 * cells * sizeof(float)) == AWE_OK &&
                   dev_alloc_extra(p, (void **)&st->slots, (size_t)std::max(2 * T, T + 1) * cells * sizeof(float)) == AWE_OK;
@@ -149,15 +150,10 @@ static awe_status grad_buffers(awe_plan *p, GradState *st, int T, int fmt, size_
         if (!st->tb2) {
             dev_free(p, st->xy2);
             st->xy2 = nullptr;
-        } else {  // not needed then (what is free now holds them if that changes)
-            dev_free(p, st->rc_start);
-            dev_free(p, st->rc_ent);
-            st->rc_start = nullptr;
-            st->rc_ent = nullptr;
-            st->rc_cap = 0;
         }
     }
     if (!st->tb2) AWE_TRY(dev_alloc(p, (void **)&st->slots, (size_t)(st->tma ? T : T + 1) * cells * sizeof(float)));
+    if (lists && !st->tb2) AWE_TRY(list(&st->rc_start, &st->rc_ent, st->rc_cap, p->h_rec.size()));
     if (st->tma) {
         int h1, h2, t1, t2;
         stepB3_tma_boxes(&h1, &h2, &t1, &t2);
