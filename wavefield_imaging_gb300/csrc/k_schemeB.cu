@@ -31,25 +31,27 @@ __device__ __forceinline__ float damp_cell(float v, int i1, int i2, int i3, cons
     return v;
 }
 
+// Blocks per SM asked of the compiler (0: as it likes): 3D steps without a
+// density run in 32 registers up to 20th order (34 took AWE_EXACT at 16th order
+// from 561 to 628 us a step of 340^3 cells).
+constexpr int stepB_blocks(int ndim, bool rho, bool pad) { return ndim == 3 && !rho && !pad ? 8 : 0; }
+
 // One time step, one thread per cell (grid: x = axis-1 tiles, y = axis 2, z = axis 3).
-// PAD: lines p1 cells apart (3D up to 8th order); else n1, and the pitch as one
-// more variable costs nothing: it took the density loop at 6th order from 40 to
-// 56 registers and 340^3 cells from 597 to 787 us a step, 20th order alike.
-constexpr int stepB_blocks(int nop, int ndim, bool rho, bool pad) {  // per SM, at least
-    if (ndim == 3 && !rho) return 8;
-    return 0;
-}
+// PAD: lines p1 cells apart (3D up to 8th order), else n1.  A case of its own,
+// since the pitch as one more variable everywhere took the density loop at 6th
+// order from 40 to 56 registers and 340^3 cells from 597 to 787 us a step.
 template <int NOP, int NDIM, bool EXACT, bool RHO, bool PAD>
-__global__ void __launch_bounds__(256, stepB_blocks(NOP, NDIM, RHO, PAD)) k_stepB(const float *__restrict__ cur, float *__restrict__ nxt,
-                                               const float *__restrict__ vel, const float *__restrict__ rho,
-                                               const StepBParams p) {
+__global__ void __launch_bounds__(256, stepB_blocks(NDIM, RHO, PAD))
+    k_stepB(const float *__restrict__ cur, float *__restrict__ nxt, const float *__restrict__ vel,
+            const float *__restrict__ rho, const StepBParams p) {
     // programmatic dependent launch (2D): wait for the previous grid before
     // touching memory (a no-op for an ordinary launch), then let the next
     // step's grid be scheduled once every block of this one has started
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
     const Grid g = p.g;
-    using Step = typename std::conditional<PAD, int, long long>::type;  // (padded planes hold less than 2^29 cells)
+    // (padded planes hold less than 2^29 cells; 32-bit offsets gain with a density only)
+    using Step = typename std::conditional<PAD && RHO, int, long long>::type;
     const int line = PAD ? g.p1 : g.n1;
     const Step s2 = line, s3 = (Step)line * g.n2;
     if (NDIM == 2 && p.ext_n > 0) {
