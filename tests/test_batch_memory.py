@@ -79,3 +79,28 @@ def test_what_fits_one_step_a_launch_fits(monkeypatch):
             assert bad and set(bad) == {3}  # AWE_ERR_NOMEM
             for a, b in zip(out[:1], want[:1]):
                 np.testing.assert_array_equal(a, b)
+
+
+def test_a_refused_selection_leaves_the_batch_usable(monkeypatch):
+    """Items of another kernel that do not fit: an error, and the next runs use
+    what the batch had, one step a launch if its extra memory was given back."""
+    import wavefield_imaging_gb300 as awe
+
+    nz, nxm, vel, shots, obs = _survey()
+    desc = awe.make_desc(2, (nz, nxm), (D, D), (0.0, 0.0), NT, 0.005, nb=10, fdorder=8, dabc=1, expl=1,
+                         precision=awe.FAST)
+    wav = ricker(NT, 0.005)
+    with awe.Batch(desc, shots) as b:
+        b.set_model(vel)
+        want, (grad, J) = np.concatenate(b.forward(wav), 1), b.gradient(wav, obs)
+        assert np.abs(want).max() > 0
+        for call in (lambda: b.select(4, chunk=1), lambda: b.select(3), lambda: b.tune(2)):
+            monkeypatch.setenv("AWE_BATCH_BYTES_LIMIT", "1")
+            with pytest.raises(awe.AweError) as e:
+                call()
+            assert e.value.status == 3
+            np.testing.assert_array_equal(np.concatenate(b.forward(wav), 1), want)
+            monkeypatch.delenv("AWE_BATCH_BYTES_LIMIT")
+            g, J1 = b.gradient(wav, obs)
+            np.testing.assert_array_equal(g, grad)
+            assert J1 == J

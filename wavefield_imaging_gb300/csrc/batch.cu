@@ -171,46 +171,58 @@ static awe_status balloc(awe_batch *b, void **p, size_t bytes) {
     return st;
 }
 
-static void build_items(awe_batch *b) {
-    const int TZ = kBatchTiles[b->tile][0], TX = kBatchTiles[b->tile][1];
-    b->items.clear();
-    for (int s = 0; s < (int)b->shots.size(); s++)
-        for (int x0 = 0; x0 < b->shots[s].n2; x0 += TX)
-            for (int z0 = 0; z0 < b->n1; z0 += TZ) b->items.push_back(make_int4(s, z0, x0, 0));
-    b->ntile_items = (int)b->items.size();
-    for (int s = 0; s < (int)b->shots.size(); s++)
-        for (int r = 0; r < b->shots[s].nr; r += kBatchRecBlock) b->items.push_back(make_int4(s, r, 0, 1));
-}
-
 // items to a device buffer that is kept while large enough (the tuner tries
-// several lists); no launch that reads it may be in flight
+// several lists) and stays as it is if a larger one cannot be had; no launch
+// that reads it may be in flight
 static awe_status upload(awe_batch *b, const std::vector<int4> &v, int4 *&d, size_t &cap) {
     if (cap < v.size()) {
-        bfree(b, d);
-        cap = 0;
-        const awe_status st = balloc(b, (void **)&d, v.size() * sizeof(int4));
+        int4 *larger = nullptr;
+        const awe_status st = balloc(b, (void **)&larger, v.size() * sizeof(int4));
         if (st != AWE_OK) return st;
+        bfree(b, d);
+        d = larger;
         cap = v.size();
     }
     CUDA_TRY(cudaMemcpy(d, v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice));
     return AWE_OK;
 }
 
-static awe_status upload_items(awe_batch *b) {
-    return upload(b, b->items, b->d_items, b->items_cap);
+// the receiver blocks of every shot, after its tiles or column chunks
+static void add_rec_items(const awe_batch *b, std::vector<int4> &v) {
+    for (int s = 0; s < (int)b->shots.size(); s++)
+        for (int r = 0; r < b->shots[s].nr; r += kBatchRecBlock) v.push_back(make_int4(s, r, 0, 1));
 }
 
-// column items (shot, x0) for chunks of L columns, then the receiver items
-static awe_status build_col_items(awe_batch *b, int L) {
-    b->col_items.clear();
+// the tile kernels' items (shot, tile) for a tile shape
+static awe_status set_tile(awe_batch *b, int tile) {
+    const int TZ = kBatchTiles[tile][0], TX = kBatchTiles[tile][1];
+    std::vector<int4> v;
     for (int s = 0; s < (int)b->shots.size(); s++)
-        for (int x0 = 0; x0 < b->shots[s].n2; x0 += L) b->col_items.push_back(make_int4(s, 0, x0, 0));
-    b->ncol_items = (int)b->col_items.size();
+        for (int x0 = 0; x0 < b->shots[s].n2; x0 += TX)
+            for (int z0 = 0; z0 < b->n1; z0 += TZ) v.push_back(make_int4(s, z0, x0, 0));
+    const int n = (int)v.size();
+    add_rec_items(b, v);
+    const awe_status st = upload(b, v, b->d_items, b->items_cap);
+    if (st != AWE_OK) return st;
+    b->items.swap(v);
+    b->ntile_items = n;
+    b->tile = tile;
+    return AWE_OK;
+}
+
+// the column march's items (shot, x0) for chunks of L columns
+static awe_status set_columns(awe_batch *b, int L) {
+    std::vector<int4> v;
     for (int s = 0; s < (int)b->shots.size(); s++)
-        for (int r = 0; r < b->shots[s].nr; r += kBatchRecBlock) b->col_items.push_back(make_int4(s, r, 0, 1));
-    const awe_status st = upload(b, b->col_items, b->d_col_items, b->col_cap);
-    if (st == AWE_OK) b->colL = L;
-    return st;
+        for (int x0 = 0; x0 < b->shots[s].n2; x0 += L) v.push_back(make_int4(s, 0, x0, 0));
+    const int n = (int)v.size();
+    add_rec_items(b, v);
+    const awe_status st = upload(b, v, b->d_col_items, b->col_cap);
+    if (st != AWE_OK) return st;
+    b->col_items.swap(v);
+    b->ncol_items = n;
+    b->colL = L;
+    return AWE_OK;
 }
 
 // Tile of k_tb2d.cu for all windows: 4 columns a thread, up to 256 threads, two
@@ -569,10 +581,7 @@ awe_status awe_batch_create(const awe_desc *desc, int nshots, const awe_shot *sh
             st = AWE_ERR_CUDA;
         }
     }
-    if (st == AWE_OK) {
-        build_items(b);
-        st = upload_items(b);
-    }
+    if (st == AWE_OK) st = set_tile(b, 0);
     if (st == AWE_OK) st = set_tb2(b);
     if (st != AWE_OK) {
         awe_batch_destroy(b);
@@ -698,9 +707,7 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
         b->tb2 = false;
     }
     for (int t = 0; t < kBatchNumTiles; t++) {
-        b->tile = t;
-        build_items(b);
-        awe_status st = upload_items(b);
+        awe_status st = set_tile(b, t);
         if (st != AWE_OK) return st;
         for (int mult : {2, 4, 8, 16}) {
             b->grid = mult * b->sms;
@@ -719,7 +726,6 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
         }
     }
     // the column-march kernel: chunk lengths x (1, 2) persistent waves
-    b->tile = best_tile;
     b->grid = best_grid;
     int best_col = 0, best_col_grid = 0;
     const int cpsm = batch2d_col_shape(b->nop, b->n1, nullptr) ? batch2d_col_ctas_per_sm(b->n1) : 0;
@@ -738,7 +744,7 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
     if (Lw != 16 && Lw != 32 && Lw != 64) chunks.push_back(Lw);
     for (int L : chunks) {
         if (cpsm <= 0) break;
-        awe_status st = build_col_items(b, L);
+        awe_status st = set_columns(b, L);
         if (st != AWE_OK) return st;
         for (int mult : {1, 2}) {
             b->col_grid = mult * cpsm * b->sms;
@@ -760,7 +766,7 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
     cudaEventDestroy(e1);
     b->colL = 0;
     if (best_col > 0) {
-        awe_status st = build_col_items(b, best_col);
+        awe_status st = set_columns(b, best_col);
         if (st != AWE_OK) return st;
         b->col_grid = best_col_grid;
     }
@@ -772,8 +778,7 @@ awe_status awe_batch_tune(awe_batch *b, int steps, int *tile_out, int *grid_out)
         set_error("awe_batch_tune: a bulk-copy wait of the column kernel timed out");
         return AWE_ERR_CUDA;
     }
-    build_items(b);
-    awe_status st = upload_items(b);
+    awe_status st = set_tile(b, best_tile);
     if (st != AWE_OK) return st;
     CUDA_TRY(cudaGetLastError());
     if (tile_out) *tile_out = b->tb2 ? kBatchNumTiles + 1 : b->colL > 0 ? kBatchNumTiles : best_tile;
@@ -1067,13 +1072,13 @@ awe_status awe_batch_select(awe_batch *b, int kernel, int chunk, int grid) {
     }
     drop_graph(b);
     if (kernel < kBatchNumTiles) {
-        b->tb2 = false;
-        b->selected = true;
-        b->tile = kernel;
+        const awe_status st = set_tile(b, kernel);
+        if (st != AWE_OK) return st;
         b->grid = grid > 0 ? grid : 4 * std::max(b->sms, 1);
         b->colL = 0;
-        build_items(b);
-        return upload_items(b);
+        b->tb2 = false;
+        b->selected = true;
+        return AWE_OK;
     }
     if (chunk < 1 || !batch2d_col_shape(b->nop, b->n1, nullptr)) {
         set_error("awe_batch_select: the column march needs 8th order, nz + 2 nb <= 2048 and chunk >= 1");
@@ -1084,11 +1089,11 @@ awe_status awe_batch_select(awe_batch *b, int kernel, int chunk, int grid) {
         set_error("awe_batch_select: the column march does not fit on this device");
         return AWE_ERR_UNSUPPORTED;
     }
-    b->tb2 = false;
-    b->selected = true;
-    awe_status st = build_col_items(b, chunk);
+    const awe_status st = set_columns(b, chunk);
     if (st != AWE_OK) return st;
     b->col_grid = grid > 0 ? grid : cpsm * b->sms;
+    b->tb2 = false;
+    b->selected = true;
     return AWE_OK;
 }
 
