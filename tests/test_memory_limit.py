@@ -102,3 +102,47 @@ def test_too_little_memory_is_an_error_every_time():
     _, _, res = _run("grad2d", need - (1 << 19))
     assert set(res) == {"E3"} or res[0].startswith("C3")  # AWE_ERR_NOMEM
     assert len(want) == 3
+
+
+_GEOMETRY = r'''
+import sys; sys.path.insert(0, "."); sys.path.insert(0, "tests")
+import numpy as np, wavefield_imaging_gb300 as awe
+from helpers import ricker
+shell = sys.argv[1] == "shell"
+n = (40, 30, 28) if shell else (60, 50)
+d = (0.005, 1.5e-6, 1.5e-6) if shell else (5.0, 5.0)
+o = (3387.0, np.pi / 2 - 15 * d[1], -14 * d[2]) if shell else (0.0, 0.0)
+desc = awe.make_desc(len(n), n, d, o, 40, 0.005, coords=awe.SPHER if shell else awe.CART,
+                     scheme=awe.SCHEME_GPU if shell else awe.SCHEME_CPU, nb=6, dabc=not shell, expl=not shell)
+axes = (0, 2, 1) if shell else (1, 0)
+sou = np.array([[o[a] + 0.5 * n[a] * d[a] for a in axes]], np.float32)
+rec = sou + np.array([2 * d[a] for a in axes], np.float32)
+p, wav, res = awe.Plan(desc), ricker(40, 0.005), []
+p.set_model(np.full(n[::-1], 0.168 if shell else 168.0, np.float32))
+p.set_geometry(sou, rec)
+ref = p.forward(wav)
+many = np.repeat(sou, 400000, 0)
+def call(f):
+    try:
+        f(); res.append(0)
+    except awe.AweError as e:
+        res.append(e.status)
+for g in (lambda: p.set_geometry(many, rec), lambda: p.set_shots([(many, rec)] * 2) if shell else p.set_geometry(sou, many),
+          lambda: p.set_moving_geometry(many, 400000, rec, 1)):
+    call(g)
+    call(lambda: p.forward(wav))
+    call(lambda: p.gradient(wav, np.zeros((40, p.nr), np.float32)))
+    p.set_geometry(sou, rec)
+    assert np.array_equal(p.forward(wav), ref) and np.abs(ref).max() > 0
+print(*res)
+'''
+
+
+@pytest.mark.parametrize("kind", ["plane", "shell"])
+def test_points_that_do_not_fit_leave_no_half_set_geometry(kind):
+    env = dict(os.environ, AWE_DEVICE_BYTES_LIMIT=str(8 << 20))
+    r = subprocess.run([sys.executable, "-c", _GEOMETRY, kind], cwd=ROOT, env=env, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    # AWE_ERR_NOMEM, then AWE_ERR_STATE until a geometry is set
+    assert r.stdout.split() == ["3", "6", "6"] * 3

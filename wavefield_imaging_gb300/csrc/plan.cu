@@ -431,6 +431,7 @@ awe_status awe_set_geometry(awe_plan *p, int ns, const float *sou, int nr, const
     CUDA_TRY(cudaSetDevice(p->device));
     set_move_mode(p, -1, 1, 1);
     p->inj_scale_ok = false;
+    p->geom_set = false;  // until all of it is: a failed call can leave points without a buffer
     awe_status st = set_geometry_common(p, ns, sou, nr, rec);
     if (st == AWE_OK) st = set_inj_cells(p);
     if (st == AWE_OK) st = set_tb2_lists(p, p->tb2_fwd, p->h_src, &p->h_rec);
@@ -479,6 +480,7 @@ awe_status awe_set_moving_geometry(awe_plan *p, int ns, int nst, const float *so
     plan_graph_drop(p);  // the captured time loop baked in the old state
     CUDA_TRY(cudaSetDevice(p->device));
     p->inj_scale_ok = false;
+    p->geom_set = false;
     awe_status st = set_geometry_common(p, ns * nst, sou, nr * nrt, rec);
     if (st != AWE_OK) return st;
     p->inj = InjCells{};  // the lists hold fixed sources
@@ -520,6 +522,7 @@ awe_status awe_set_shots(awe_plan *p, int nshots, const int *ns, const float *so
     CUDA_TRY(cudaSetDevice(p->device));
     set_move_mode(p, -1, 1, 1);
     p->inj_scale_ok = false;
+    p->geom_set = false;
     awe_status st = set_geometry_common(p, NS, sou, NR, rec);
     if (st != AWE_OK) return st;
     // points of shot s address field s
