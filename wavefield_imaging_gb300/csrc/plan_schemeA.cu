@@ -252,6 +252,7 @@ awe_status planA_model(awe_plan *p, const float *vel, const float *rfl) {
     p->inj_scale_ok = false;
     p->h_vel_raw.assign(cells, 0.f);
     expand_model(d.ndim, vel, p->h_vel_raw.data(), nb, d.n);
+    CUDA_TRY(cudaDeviceSynchronize());  // earlier runs (on any stream) may still read the old model
     CUDA_TRY(cudaMemcpy2D(p->vel, g.p1 * sizeof(float), p->h_vel_raw.data(), g.n1 * sizeof(float),
                           g.n1 * sizeof(float), lines, cudaMemcpyHostToDevice));
     const std::vector<float> &v = p->h_vel_raw;
@@ -296,7 +297,8 @@ awe_status planA_model(awe_plan *p, const float *vel, const float *rfl) {
                 byl[iz * nxpad + ix] = coef(v[kNopA * n2 + iz * nxpad + ix] * (dt / d.d[2]));
                 byh[iz * nxpad + ix] = coef(v[(nypad - kNopA - 1) * n2 + iz * nxpad + ix] * (dt / d.d[2]));
             }
-        float *t[6] = {nullptr};
+        float *t[6];  // (kept from model to model)
+        for (int k = 0; k < 6; k++) t[k] = const_cast<float *>(pa.tb[k]);
         AWE_TRY(upload_t(p, &t[0], bzl.data(), bzl.size()));
         AWE_TRY(upload_t(p, &t[1], bzh.data(), bzh.size()));
         AWE_TRY(upload_t(p, &t[2], bxl.data(), bxl.size()));
