@@ -624,6 +624,7 @@ awe_status awe_batch_set_model(awe_batch *b, const float *vel) {
             for (int x = 0; x < sh.n2; x++)
                 for (int z = 0; z < b->nb + 1 && z < b->n1; z++) v[(size_t)x * b->n1 + z] = 0.f;  // :292-295
     }
+    CUDA_TRY(cudaDeviceSynchronize());  // earlier runs (on any stream) may still read the old model
     CUDA_TRY(cudaMemcpy(b->vel, all.data(), all.size() * sizeof(float), cudaMemcpyHostToDevice));
     b->model_set = true;
     return AWE_OK;
